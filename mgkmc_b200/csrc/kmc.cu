@@ -46,19 +46,39 @@ __device__ __forceinline__ double soft_base(double g_p, double g_t, double t_las
   return g;
 }
 
+// D*D doubles from global memory; VEC: 16-byte loads (the caller checked that
+// the base is 16-byte aligned; D = 2 tensors then all are)
+template <int D, bool VEC>
+__device__ __forceinline__ void load_tensor(const double* __restrict__ p, double* __restrict__ t) {
+  if constexpr (VEC && D == 2) {
+    const double2 a = __ldg(reinterpret_cast<const double2*>(p)), b = __ldg(reinterpret_cast<const double2*>(p) + 1);
+    t[0] = a.x; t[1] = a.y; t[2] = b.x; t[3] = b.y;
+  } else {
+#pragma unroll
+    for (int q = 0; q < D * D; ++q) t[q] = __ldg(p + q);
+  }
+}
+
+// voxel of mode index i: 32-bit division where the index fits
+__device__ __forceinline__ long long voxel_of(long long i, int M) {
+  return i <= 0xffffffffLL ? (long long)((unsigned int)i / (unsigned int)M) : i / M;
+}
+
 // One thread per (voxel, mode).  D = 2 or 3 (tensor dimension); SP = soft_prop
 // stride (2 in 2D, 4 in 3D).
-template <int D, int SP>
+template <int D, int SP, bool VEC>
 __device__ __forceinline__ double barrier_mode(long long i, int M, double* __restrict__ Q,
                                                const double* __restrict__ Q0, const double* __restrict__ sig,
                                                const double* __restrict__ cat, double volume,
                                                const double* __restrict__ soft, const double* __restrict__ t_last,
                                                double t, const double* __restrict__ prev, double cap, int scheme,
                                                double tau) {
-  const long long v = i / M;
+  const long long v = voxel_of(i, M);
+  double c[D * D], s[D * D];
+  load_tensor<D, VEC>(cat + i * D * D, c);
+  load_tensor<D, VEC>(sig + v * D * D, s);
+  const double q0 = __ldg(Q0 + i);
   const double g_base = soft_base(soft[SP * v], soft[SP * v + 1], t_last[v], t, cap, tau);
-  const double* c = cat + i * D * D;
-  const double* s = sig + v * D * D;
   double modifier = 1.0;
   if (scheme == 1) {
     const double* p = prev + v * D * D;
@@ -83,19 +103,23 @@ __device__ __forceinline__ double barrier_mode(long long i, int M, double* __res
 #pragma unroll
   for (int q = 0; q < D * D; ++q) w = add(w, mul(s[q], c[q]));
   const double w_val = mul(mul(mul(0.5, volume), __ddiv_rn(w, 1e9)), GPA_NM3_TO_EV);
-  const double q = sub(mul(Q0[i], exp(-g_eff)), w_val);
+  // exp(-0) is 1 exactly, so an unsoftened voxel needs no exponential
+  const double q = sub(g_eff == 0.0 ? q0 : mul(q0, exp(-g_eff)), w_val);
   Q[i] = q;
   return q;
 }
 
-template <int D, int SP>
-__global__ void barrier_kernel(long long nvox, int M, double* __restrict__ Q, const double* __restrict__ Q0,
+// 55 bytes per mode at M = 8, bound by HBM once the tensors come in 16-byte
+// loads, the voxel index by a 32-bit division and unsoftened voxels skip the
+// exponential: 1024^2 x 8 modes took 120 us before and 84 us now (5.5 TB/s).
+template <int D, int SP, bool VEC>
+__global__ void __launch_bounds__(256) barrier_kernel(long long nvox, int M, double* __restrict__ Q, const double* __restrict__ Q0,
                                const double* __restrict__ sig, const double* __restrict__ cat, double volume,
                                const double* __restrict__ soft, const double* __restrict__ t_last, double t,
                                const double* __restrict__ prev, double cap, int scheme, double tau) {
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= nvox * M) return;
-  barrier_mode<D, SP>(i, M, Q, Q0, sig, cat, volume, soft, t_last, t, prev, cap, scheme, tau);
+  barrier_mode<D, SP, VEC>(i, M, Q, Q0, sig, cat, volume, soft, t_last, t, prev, cap, scheme, tau);
 }
 
 // rate of one mode (kmc_simulator_functions.py:41-48)
@@ -103,13 +127,13 @@ __device__ __forceinline__ double mode_rate(double q, double beta, double vnu) {
   return q <= 0 ? vnu : mul(vnu, exp(-mul(q, beta)));
 }
 
-__device__ __forceinline__ double beta_of(double T) { return T > 0.0 ? __ddiv_rn(1.0, mul(KB_EV, T)) : INFINITY; }
+__host__ __device__ inline double beta_of(double T) { return T > 0.0 ? 1.0 / (KB_EV * T) : INFINITY; }
 
 // Fused barrier, rate and block-sum pass (fast selection mode): the barriers
 // as barrier_kernel, each mode's KMC-mode rate from its new barrier, and the
 // FP64 sum of the rates per CTA (grid-stride, fixed grid: a deterministic
 // order); no rate array is written.
-template <int D, int SP>
+template <int D, int SP, bool VEC>
 __global__ void __launch_bounds__(256) barrier_total_kernel(long long nvox, int M, double* __restrict__ Q,
                                                             const double* __restrict__ Q0,
                                                             const double* __restrict__ sig,
@@ -124,8 +148,8 @@ __global__ void __launch_bounds__(256) barrier_total_kernel(long long nvox, int 
   double acc = 0.0;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nvox * M;
        i += (long long)gridDim.x * blockDim.x) {
-    const double q = barrier_mode<D, SP>(i, M, Q, Q0, sig, cat, volume, soft, t_last, t, prev, cap, scheme, tau);
-    acc += mode_rate(q, T ? beta_of(T[i / M]) : beta_s, vnu);
+    const double q = barrier_mode<D, SP, VEC>(i, M, Q, Q0, sig, cat, volume, soft, t_last, t, prev, cap, scheme, tau);
+    acc += mode_rate(q, T ? beta_of(T[voxel_of(i, M)]) : beta_s, vnu);
   }
   acc = block_sum(acc, red);
   if (threadIdx.x == 0) partials[blockIdx.x] = acc;
@@ -141,16 +165,15 @@ __global__ void __launch_bounds__(256) partials_total_kernel(const double* __res
   if (threadIdx.x == 0) *d_total = acc;
 }
 
-// Non-compacting rates (KMC mode: every mode is an event).
+// Non-compacting rates (KMC mode: every mode is an event); beta_s is the
+// scalar temperature's (used when T is NULL).
 __global__ void rates_full_kernel(long long nvox, int M, const double* __restrict__ Q, double vnu,
-                                  const double* __restrict__ T, double Ts, double* __restrict__ rates,
+                                  const double* __restrict__ T, double beta_s, double* __restrict__ rates,
                                   long long* __restrict__ indices, long long* __restrict__ d_count) {
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i == 0 && d_count) *d_count = nvox * M;
   if (i >= nvox * M) return;
-  const long long v = i / M;
-  const double beta = beta_of(T ? T[v] : Ts);
-  rates[i] = mode_rate(Q[i], beta, vnu);
+  rates[i] = mode_rate(Q[i], T ? beta_of(T[voxel_of(i, M)]) : beta_s, vnu);
   if (indices) indices[i] = i;
 }
 
@@ -238,152 +261,184 @@ __global__ void rates_scatter_kernel(long long nvox, int M, const double* __rest
 //
 // The array is cut into chunks of kExactChunk rates, processed in five
 // launches:
-//   1. chunk sums in FP64, any order (an estimate of the running sum);
+//   1. chunk sums in FP64, any order (an estimate of the running sum; the
+//      KMC-mode rate kernel forms them with the rates);
 //   2. one CTA scans them: the estimated running sum at each chunk start;
 //   3. per chunk, with the binade e of that estimate: the exact int64 sum Q
 //      of q_i, and whether every element is representable and tie-free;
-//   4. one CTA walks the chunks in order with the exact running sum s: a
-//      chunk whose record holds (s in binade e, M + Q < 2^53) ends at
-//      (M + Q) u exactly and costs a few instructions; any other chunk (the
-//      first, the last short one, a binade crossing, a tie, a wrong estimate)
-//      runs the sequential-exact CTA algorithm above on its own rates;
+//   4. one CTA walks the chunks with the exact running sum s: a scan of the
+//      records' Q finds the first chunk whose record does not hold (s leaves
+//      binade e, M + Q >= 2^53, a tie, a wrong estimate, the first or last
+//      short chunk); all chunks before it are accepted at once, and that one
+//      runs the same scan over its own rates, once per binade it crosses;
 //   5. per chunk that the walk accepted: prefix_i = (M + Q_i) u from a block
 //      scan of its q_i.
 // A chunk's records sit in its own first four prefix entries until the walk
 // (rejected chunks) or launch 5 (accepted ones) writes its final values; the
 // walk marks accepted chunks with -0.0 in entry 3, a value no running sum
-// from +0.0 can take.  The walk's cost is about the number of binades the
-// sum crosses, times one chunk.
-constexpr int kExactThreads = 1024;
-constexpr int kExactPer = 8;  // rates per thread per chunk
+// from +0.0 can take.
+//
+// The walk is bound by its serial chain: a scan of the records and one or
+// more of a chunk's rates per rejected chunk, about as many as the binades the
+// sum crosses (20 at 1024^2 x 8 modes).  Each link is one scan by 256 threads
+// of eight values each, with three barriers: with 1024 threads of two values
+// the 64-bit shuffles of 32 warps bound it.  At 1024^2 x 8 modes the walk took
+// 347 us with chunks of 8192 and one thread accepting chunk by chunk, 215 us
+// with warp-wide steps inside a rejected chunk, 106 us with 1024 threads, and
+// 102 us now.
+constexpr int kExactThreads = 256;                        // of launches 1, 3 and 5
+constexpr int kExactPer = 8;                              // rates per thread per chunk
 constexpr int kExactChunk = kExactThreads * kExactPer;
-// q_i < 2^53, so sums of q are saturated at 2^61 (no int64 overflow); any
-// saturated sum is far above 2^53 - M and reads as leaving the binade
-constexpr long long kQCap = 1LL << 61;
-__device__ __forceinline__ long long qsat(long long a, long long b) { return min(a + b, kQCap); }
+constexpr int kExactPad = kExactChunk + kExactChunk / 8;  // shared copy: one slot of slack per 8 rates
+constexpr int kScanThreads = 1024, kScanPer = 4;          // launch 2: chunk sums per thread and round
+constexpr int kWalkThreads = 256, kWalkWarps = kWalkThreads / 32;
+constexpr int kWalkPer = 8;                               // values per thread of a scan of the walk
+static_assert(kWalkThreads * kWalkPer == kExactChunk, "one scan covers one chunk's rates");
+// Any q >= 2^52 leaves the binade (M >= 2^52), so q and Q are clamped there
+// and the scan of 2048 of them fits 64 bits.
+constexpr unsigned long long kQMax = 1ULL << 52;
 constexpr long long kRecOk = 1LL << 62;                      // record tag: chunk tie-free, q representable
 constexpr long long kRecMark = (long long)0x8000000000000000ULL;  // bits of -0.0: accepted by the walk
 
 __device__ __forceinline__ bool normal_finite(double s) { return s >= 2.2250738585072014e-308 && s < 1.0 / 0.0; }
 __device__ __forceinline__ int binade_of(double s) { return (int)((__double_as_longlong(s) >> 52) & 0x7ff) - 1023; }
+__device__ __forceinline__ unsigned long long mantissa_of(double s) {
+  return ((unsigned long long)__double_as_longlong(s) & (kQMax - 1)) | kQMax;
+}
+__device__ __forceinline__ int pad8(int i) { return i + (i >> 3); }
 
-// The sequential-exact algorithm on rates[p0, end) from running sum s0, by
-// all kExactThreads threads of the CTA; writes prefix[p0, end) and returns
-// the running sum after element end - 1 (in every thread).
-__device__ double exact_range(const double* __restrict__ rates, long long p0, long long end, double s0,
-                              double* __restrict__ prefix, long long* w_sum, long long* w_fail, double* s_s,
-                              long long* s_p) {
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  __syncthreads();
-  if (tid == 0) { *s_s = s0; *s_p = p0; }
-  __syncthreads();
-  while (true) {
-    const double s = *s_s;
-    const long long p = *s_p;
-    if (p >= end) break;
-    if (!normal_finite(s)) {
-      // zero, subnormal or non-finite running sum: one ordinary add
-      __syncthreads();
-      if (tid == 0) {
-        const double v = add(s, rates[p]);
-        prefix[p] = v;
-        *s_s = v;
-        *s_p = p + 1;
-      }
-      __syncthreads();
-      continue;
-    }
-    const long long bits = __double_as_longlong(s);
-    const int e = binade_of(s);
-    const long long M = (bits & ((1LL << 52) - 1)) | (1LL << 52);
-    const double scale = ldexp(1.0, 52 - e);  // 1/u, exact power of two
-    const double u = ldexp(1.0, e - 52);
-    const long long base = p + (long long)tid * kExactPer;
-    long long q[kExactPer];
-    long long fail = LLONG_MAX;  // first tie or unrepresentable element of this thread
-    long long tot = 0;
+// 1/u = 2^(52 - e) and u = 2^(e - 52), exact.  Below e = -971 the scale is
+// infinite and every rate reads as not representable.
+__device__ __forceinline__ double binade_scale(int e) {
+  return e >= -971 ? __longlong_as_double((long long)(1075 - e) << 52) : INFINITY;
+}
+__device__ __forceinline__ double binade_ulp(int e) {
+  return e >= -970 ? __longlong_as_double((long long)(971 + e) << 52) : ldexp(1.0, e - 52);
+}
+
+// q = rint(r * scale) of rate r; bad when it is a tie or not below 2^52.
+// Adding 2^52 rounds x to an integer, which the sum's mantissa holds.
+__device__ __forceinline__ unsigned long long exact_q(double r, double scale, bool& bad) {
+  const double x = r * scale, y = add(x, 4503599627370496.0);
+  bad = !(x >= 0.0 && x < 4503599627370496.0) || fabs(sub(x, sub(y, 4503599627370496.0))) == 0.5;
+  return bad ? kQMax : (unsigned long long)(__double_as_longlong(y) - 0x4330000000000000LL);
+}
+
+__device__ __forceinline__ unsigned long long warp_scan_q(unsigned long long v, int lane) {
 #pragma unroll
-    for (int k = 0; k < kExactPer; ++k) {
-      const long long i = base + k;
-      q[k] = 0;
-      if (i < end) {
-        const double x = rates[i] * scale;
-        if (!(x >= 0.0) || !(x < 9007199254740992.0) || x - floor(x) == 0.5) {
-          if (fail == LLONG_MAX) fail = i;
-        } else {
-          q[k] = (long long)rint(x);
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned long long t = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += t;
+  }
+  return v;
+}
+
+// One scan of the walk, by all kWalkThreads threads: values q[] of the items
+// kWalkPer tid + j (0 outside the range, kQMax where the item cannot be
+// taken).  Returns the first item with M + (inclusive sum) >= 2^53, INT_MAX if
+// none; before: the sum of all items ahead of this thread's; all: of every item.
+struct WalkShared {
+  unsigned long long q[kWalkWarps];
+  int fail[kWalkWarps];
+  double s;
+};
+__device__ __forceinline__ int walk_first(int v, WalkShared& W) {
+  v = __reduce_min_sync(0xffffffffu, v);
+  if ((threadIdx.x & 31) == 0) W.fail[threadIdx.x >> 5] = v;
+  __syncthreads();
+  int f = W.fail[0];
+#pragma unroll
+  for (int w = 1; w < kWalkWarps; ++w) f = min(f, W.fail[w]);
+  return f;
+}
+__device__ __forceinline__ int walk_scan(const unsigned long long* q, unsigned long long M, WalkShared& W,
+                                         unsigned long long& before, unsigned long long& all) {
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  unsigned long long tot = 0;
+#pragma unroll
+  for (int j = 0; j < kWalkPer; ++j) tot += q[j];
+  const unsigned long long incl = warp_scan_q(tot, lane);
+  if (lane == 31) W.q[wid] = incl;
+  __syncthreads();
+  before = incl - tot;
+  all = 0;
+#pragma unroll
+  for (int w = 0; w < kWalkWarps; ++w) {
+    const unsigned long long t = W.q[w];
+    if (w < wid) before += t;
+    all += t;
+  }
+  int fail = INT_MAX;
+  unsigned long long after = M + before + tot;
+#pragma unroll
+  for (int j = kWalkPer - 1; j >= 0; --j) {
+    if (after >= 2 * kQMax) fail = kWalkPer * tid + j;
+    after -= q[j];
+  }
+  return walk_first(fail, W);
+}
+
+// The running sums of the m <= kExactChunk rates at `rates` from running sum
+// s, by all kWalkThreads threads; writes them to `prefix` and returns the
+// last one (in every thread).
+__device__ double walk_chunk(const double* __restrict__ rates, int m, double s, double* __restrict__ prefix,
+                             WalkShared& W) {
+  const int i0 = kWalkPer * threadIdx.x;
+  double r[kWalkPer];
+#pragma unroll
+  for (int k = 0; k < kWalkPer; ++k) r[k] = i0 + k < m ? rates[i0 + k] : 0.0;
+  int p = 0;
+  while (p < m) {
+    int stop = p;  // the rate added the ordinary way
+    if (normal_finite(s)) {
+      const int e = binade_of(s);
+      const unsigned long long M = mantissa_of(s);
+      const double scale = binade_scale(e), u = binade_ulp(e);
+      unsigned long long q[kWalkPer], before, all;
+#pragma unroll
+      for (int k = 0; k < kWalkPer; ++k) {
+        bool bad;
+        q[k] = exact_q(r[k], scale, bad);
+        if (i0 + k < p || i0 + k >= m) q[k] = 0;
+      }
+      stop = walk_scan(q, M, W, before, all);
+#pragma unroll
+      for (int k = 0; k < kWalkPer; ++k) {
+        const int i = i0 + k;
+        const unsigned long long after = before + q[k];
+        if (i >= p && i < m) {
+          if (i < stop) prefix[i] = (double)(M + after) * u;
+          if (i == stop) W.s = prefix[i] = add((double)(M + before) * u, r[k]);
+        }
+        before = after;
+      }
+      if (stop == INT_MAX) return (double)(M + all) * u;
+    } else {
+      // zero stays zero up to the first other rate; a subnormal or non-finite
+      // sum takes one ordinary add
+      if (s == 0.0) {
+        int f = INT_MAX;
+#pragma unroll
+        for (int k = kWalkPer - 1; k >= 0; --k)
+          if (i0 + k >= p && i0 + k < m && !(r[k] == 0.0)) f = i0 + k;
+        stop = walk_first(f, W);
+      }
+#pragma unroll
+      for (int k = 0; k < kWalkPer; ++k) {
+        const int i = i0 + k;
+        if (i >= p && i < m) {
+          if (i < stop) prefix[i] = s;
+          if (i == stop) W.s = prefix[i] = add(s, r[k]);
         }
       }
-      tot += q[k];
-    }
-    // exclusive block scan of the per-thread totals (int64, exact)
-    long long incl = tot;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const long long t = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl = qsat(incl, t);
-    }
-    long long wf = fail;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) wf = min(wf, __shfl_xor_sync(0xffffffffu, wf, o));
-    if (lane == 31) w_sum[wid] = incl;
-    if (lane == 0) w_fail[wid] = wf;
-    __syncthreads();
-    if (wid == 0) {
-      long long v = w_sum[lane];
-      long long f = w_fail[lane];
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const long long t = __shfl_up_sync(0xffffffffu, v, o);
-        if (lane >= o) v = qsat(v, t);
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) f = min(f, __shfl_xor_sync(0xffffffffu, f, o));
-      w_sum[lane] = v;  // inclusive warp totals
-      if (lane == 0) w_fail[0] = f;
+      if (stop == INT_MAX) return s;
     }
     __syncthreads();
-    // before this thread's first element (a saturated incl minus tot stays far above 2^53)
-    long long Q = qsat(wid > 0 ? w_sum[wid - 1] : 0, incl - tot);
-    long long first_bad = w_fail[0];
-    // first element whose candidate leaves the binade (Q is nondecreasing)
-    long long cross = LLONG_MAX;
-#pragma unroll
-    for (int k = 0; k < kExactPer; ++k) {
-      const long long i = base + k;
-      if (i < end && i < first_bad) {
-        Q = qsat(Q, q[k]);
-        if (M + Q >= (1LL << 53)) { cross = i; break; }
-        prefix[i] = (double)(M + Q) * u;
-      }
-    }
-    // the step is valid up to min(first tie, first crossing)
-    long long wc = cross;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) wc = min(wc, __shfl_xor_sync(0xffffffffu, wc, o));
-    __syncthreads();  // everyone has read w_fail[0]
-    if (lane == 0) w_sum[wid] = wc;
-    __syncthreads();
-    if (tid == 0) {
-      long long stop = first_bad;
-      for (int w = 0; w < kExactThreads / 32; ++w) stop = min(stop, w_sum[w]);
-      const long long stp_end = min(p + (long long)kExactChunk, end);
-      if (stop >= stp_end) {
-        // whole step valid: the running sum is its last prefix
-        *s_s = prefix[stp_end - 1];
-        *s_p = stp_end;
-      } else {
-        // elements [p, stop) were written; stop is added the ordinary way
-        const double prev = stop > p ? prefix[stop - 1] : s;
-        const double v = add(prev, rates[stop]);
-        prefix[stop] = v;
-        *s_s = v;
-        *s_p = stop + 1;
-      }
-    }
-    __syncthreads();
+    s = W.s;
+    __syncthreads();  // W is free again
+    p = stop + 1;
   }
-  return *s_s;
+  return s;
 }
 
 __device__ __forceinline__ long long exact_count(long long n_fixed, const long long* d_count) {
@@ -392,49 +447,73 @@ __device__ __forceinline__ long long exact_count(long long n_fixed, const long l
 // chunks that carry records: not the first, at least 4 rates long
 __device__ __forceinline__ bool has_record(long long c0, long long n) { return c0 > 0 && n - c0 >= 4; }
 
-__device__ __forceinline__ double block_sum_d(double v, double* red) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  double t = 0;
-  if (threadIdx.x < 32) {
-    t = threadIdx.x < (blockDim.x + 31) / 32 ? red[threadIdx.x] : 0.0;
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+// KMC-mode rates of one chunk per CTA with the chunk's FP64 sum (launch 1 of
+// the exact running sum) in its entry 0: the sums cost no pass of their own.
+__global__ void __launch_bounds__(kExactThreads) rates_sum_kernel(long long n, int M, const double* __restrict__ Q,
+                                                                  double vnu, const double* __restrict__ T,
+                                                                  double beta_s, double* __restrict__ rates,
+                                                                  long long* __restrict__ indices,
+                                                                  long long* __restrict__ d_count,
+                                                                  double* __restrict__ prefix) {
+  __shared__ double red[32];
+  const long long c0 = (long long)blockIdx.x * kExactChunk;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *d_count = n;
+  const int m = (int)min((long long)kExactChunk, n - c0);
+  double v = 0;
+#pragma unroll
+  for (int k = 0; k < kExactPer; ++k) {
+    const int i = threadIdx.x + k * kExactThreads;
+    if (i < m) {
+      const double r = mode_rate(Q[c0 + i], T ? beta_of(T[voxel_of(c0 + i, M)]) : beta_s, vnu);
+      rates[c0 + i] = r;
+      indices[c0 + i] = c0 + i;
+      v += r;
+    }
   }
-  return t;  // valid in thread 0
+  v = block_sum(v, red);
+  if (threadIdx.x == 0 && m >= 4) prefix[c0] = v;
 }
 
 // 1. FP64 sum of each chunk (an estimate) into the chunk's entry 0; grid = chunks
-__global__ void __launch_bounds__(256) exact_chunk_sum_kernel(const double* __restrict__ rates, long long n_fixed,
-                                                              const long long* __restrict__ d_count,
-                                                              double* __restrict__ prefix) {
+__global__ void __launch_bounds__(kExactThreads) exact_chunk_sum_kernel(const double* __restrict__ rates,
+                                                                        long long n_fixed,
+                                                                        const long long* __restrict__ d_count,
+                                                                        double* __restrict__ prefix) {
   __shared__ double red[32];
   const long long n = exact_count(n_fixed, d_count);
   const long long c0 = (long long)blockIdx.x * kExactChunk;
   if (c0 >= n || n - c0 < 4) return;  // the last short chunk needs no estimate
-  const long long c1 = min(c0 + (long long)kExactChunk, n);
+  const int m = (int)min((long long)kExactChunk, n - c0);
   double v = 0;
-  for (long long i = c0 + threadIdx.x; i < c1; i += blockDim.x) v += rates[i];
-  v = block_sum_d(v, red);
+#pragma unroll
+  for (int k = 0; k < kExactPer; ++k) {
+    const int i = threadIdx.x + k * kExactThreads;
+    if (i < m) v += rates[c0 + i];
+  }
+  v = block_sum(v, red);
   if (threadIdx.x == 0) prefix[c0] = v;
 }
 
 // 2. one CTA: estimated running sum at each chunk start into entry 1
-__global__ void __launch_bounds__(1024) exact_chunk_scan_kernel(long long n_fixed, const long long* __restrict__ d_count,
-                                                                double* __restrict__ prefix) {
+__global__ void __launch_bounds__(kScanThreads) exact_chunk_scan_kernel(long long n_fixed,
+                                                                        const long long* __restrict__ d_count,
+                                                                        double* __restrict__ prefix) {
   __shared__ double wtot[32];
-  __shared__ double carry;
   const long long n = exact_count(n_fixed, d_count);
   const long long K = (n + kExactChunk - 1) / kExactChunk;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (threadIdx.x == 0) carry = 0.0;
-  __syncthreads();
-  for (long long kb = 0; kb < K; kb += 1024) {
-    const long long k = kb + threadIdx.x;
-    const long long c0 = k * kExactChunk;
-    const double v = (k < K && n - c0 >= 4) ? prefix[c0] : 0.0;
-    double incl = v;
+  double carry = 0.0;
+  for (long long kb = 0; kb < K; kb += kScanThreads * kScanPer) {
+    const long long k0 = kb + (long long)threadIdx.x * kScanPer;
+    double v[kScanPer], tot = 0.0;
+#pragma unroll
+    for (int j = 0; j < kScanPer; ++j) {
+      const long long c0 = (k0 + j) * kExactChunk;
+      v[j] = (k0 + j < K && n - c0 >= 4) ? prefix[c0] : 0.0;
+    }
+#pragma unroll
+    for (int j = 0; j < kScanPer; ++j) tot += v[j];
+    double incl = tot;
     for (int o = 1; o < 32; o <<= 1) {
       const double t = __shfl_up_sync(0xffffffffu, incl, o);
       if (lane >= o) incl += t;
@@ -450,20 +529,16 @@ __global__ void __launch_bounds__(1024) exact_chunk_scan_kernel(long long n_fixe
       wtot[lane] = w;
     }
     __syncthreads();
-    const double excl = carry + (wid > 0 ? wtot[wid - 1] : 0.0) + (incl - v);
-    if (k < K && has_record(c0, n)) prefix[c0 + 1] = excl;
-    __syncthreads();
-    if (threadIdx.x == 0) carry += wtot[31];
+    double excl = carry + (wid > 0 ? wtot[wid - 1] : 0.0) + (incl - tot);
+#pragma unroll
+    for (int j = 0; j < kScanPer; ++j) {
+      const long long c0 = (k0 + j) * kExactChunk;
+      if (k0 + j < K && has_record(c0, n)) prefix[c0 + 1] = excl;
+      excl += v[j];
+    }
+    carry += wtot[31];
     __syncthreads();
   }
-}
-
-// q_i = rint(r_i * scale) of rate i, or -1 when it is a tie or not
-// representable (then the chunk is left to the sequential algorithm)
-__device__ __forceinline__ long long exact_q(double r, double scale) {
-  const double x = r * scale;
-  if (!(x >= 0.0) || !(x < 9007199254740992.0) || x - floor(x) == 0.5) return -1;
-  return (long long)rint(x);
 }
 
 // 3. per chunk with a record: Q = sum of q_i at the binade of its estimated
@@ -472,107 +547,101 @@ __global__ void __launch_bounds__(kExactThreads) exact_chunk_q_kernel(const doub
                                                                       long long n_fixed,
                                                                       const long long* __restrict__ d_count,
                                                                       double* __restrict__ prefix) {
-  __shared__ long long w_q[32];
-  __shared__ int w_bad[32];
-  __shared__ double s_est;
+  __shared__ unsigned long long w_q[kExactThreads / 32];
+  __shared__ int w_bad[kExactThreads / 32];
   const long long n = exact_count(n_fixed, d_count);
   const long long c0 = (long long)blockIdx.x * kExactChunk;
   if (c0 >= n || !has_record(c0, n)) return;
-  const long long c1 = min(c0 + (long long)kExactChunk, n);
+  const int m = (int)min((long long)kExactChunk, n - c0);
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  if (tid == 0) s_est = prefix[c0 + 1];
-  __syncthreads();
-  const double est = s_est;
-  const bool est_ok = normal_finite(est);
-  const int e = est_ok ? binade_of(est) : 0;
-  const double scale = ldexp(1.0, 52 - e);
-  long long tot = 0;
-  int bad = est_ok ? 0 : 1;
-  const long long base = c0 + (long long)tid * kExactPer;
+  const double est = prefix[c0 + 1];
+  double r[kExactPer];
 #pragma unroll
   for (int k = 0; k < kExactPer; ++k) {
-    const long long i = base + k;
-    if (i < c1 && !bad) {
-      const long long q = exact_q(rates[i], scale);
-      if (q < 0) bad = 1;
-      else tot = qsat(tot, q);
-    }
+    const int i = tid + k * kExactThreads;
+    r[k] = i < m ? rates[c0 + i] : 0.0;
+  }
+  const bool est_ok = normal_finite(est);
+  const int e = est_ok ? binade_of(est) : 0;
+  const double scale = binade_scale(e);
+  unsigned long long tot = 0;
+  bool any_bad = !est_ok;
+#pragma unroll
+  for (int k = 0; k < kExactPer; ++k) {
+    bool bad;
+    tot += exact_q(r[k], scale, bad);
+    any_bad |= bad;
   }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    tot = qsat(tot, __shfl_xor_sync(0xffffffffu, tot, o));
-    bad |= __shfl_xor_sync(0xffffffffu, bad, o);
-  }
-  if (lane == 0) { w_q[wid] = tot; w_bad[wid] = bad; }
-  __syncthreads();  // every thread has read entry 1 (s_est) before entry 2/3 change
+  for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+  const int wb = __any_sync(0xffffffffu, any_bad);
+  if (lane == 0) { w_q[wid] = tot; w_bad[wid] = wb; }
+  __syncthreads();
   if (tid == 0) {
-    long long Q = 0;
+    unsigned long long Q = 0;
     int b = 0;
-    for (int w = 0; w < kExactThreads / 32; ++w) { Q = qsat(Q, w_q[w]); b |= w_bad[w]; }
-    prefix[c0 + 2] = __longlong_as_double(Q);
+    for (int w = 0; w < kExactThreads / 32; ++w) { Q += w_q[w]; b |= w_bad[w]; }
+    prefix[c0 + 2] = __longlong_as_double((long long)min(Q, kQMax));
     prefix[c0 + 3] = __longlong_as_double(b ? 0LL : (kRecOk | (long long)(e + 2048)));
   }
 }
 
-// 4. one CTA walks the chunks in order with the exact running sum; writes the
-// total.  Accepted chunks get (M, e, mark) in entries 0, 1, 3.
-__global__ void __launch_bounds__(kExactThreads) exact_walk_kernel(const double* __restrict__ rates, long long n_fixed,
-                                                                   const long long* __restrict__ d_count,
-                                                                   double* __restrict__ prefix,
-                                                                   double* __restrict__ d_total) {
-  __shared__ long long w_sum[32];
-  __shared__ long long w_fail[32];
-  __shared__ double s_s;
-  __shared__ long long s_p;
-  __shared__ long long rec_q[kExactThreads];
-  __shared__ long long rec_t[kExactThreads];
-  __shared__ double w_s;
-  __shared__ long long w_k;
+// 4. one CTA walks the chunks with the exact running sum; writes the total.
+// Accepted chunks get (M, e, mark) in entries 0, 1, 3.
+__global__ void __launch_bounds__(kWalkThreads) exact_walk_kernel(const double* __restrict__ rates, long long n_fixed,
+                                                                  const long long* __restrict__ d_count,
+                                                                  double* __restrict__ prefix,
+                                                                  double* __restrict__ d_total) {
+  __shared__ WalkShared W;
   const long long n = exact_count(n_fixed, d_count);
   const long long K = (n + kExactChunk - 1) / kExactChunk;
-  double s = 0.0;
-  for (long long kb = 0; kb < K; kb += kExactThreads) {
-    const long long kend = min(kb + (long long)kExactThreads, K);
-    {
-      const long long k = kb + threadIdx.x;
-      const long long c0 = k * kExactChunk;
-      const bool rec = k < kend && has_record(c0, n);
-      rec_q[threadIdx.x] = rec ? __double_as_longlong(prefix[c0 + 2]) : 0;
-      rec_t[threadIdx.x] = rec ? __double_as_longlong(prefix[c0 + 3]) : 0;
+  const int j0 = kWalkPer * threadIdx.x;
+  double s = 0.0;  // the exact running sum, the same in every thread
+  for (long long kb = 0; kb < K; kb += kWalkThreads * kWalkPer) {
+    const int wend = (int)min((long long)(kWalkThreads * kWalkPer), K - kb);
+    // this thread's records of the window
+    unsigned long long rq[kWalkPer];
+    long long rt[kWalkPer];
+#pragma unroll
+    for (int j = 0; j < kWalkPer; ++j) {
+      const long long c0 = (kb + j0 + j) * kExactChunk;
+      const bool rec = j0 + j < wend && has_record(c0, n);
+      rq[j] = rec ? (unsigned long long)__double_as_longlong(prefix[c0 + 2]) : 0;
+      rt[j] = rec ? __double_as_longlong(prefix[c0 + 3]) : 0;
     }
-    __syncthreads();
-    long long k = kb;
-    while (k < kend) {
-      if (threadIdx.x == 0) {
-        // accept chunks while their records hold at the exact running sum
-        while (k < kend) {
-          const long long c0 = k * kExactChunk;
-          const long long t = rec_t[k - kb];
-          if (!has_record(c0, n) || !(t & kRecOk) || !normal_finite(s)) break;
-          const int e = (int)(t & 0xffff) - 2048;
-          if (binade_of(s) != e) break;
-          const long long M = (__double_as_longlong(s) & ((1LL << 52) - 1)) | (1LL << 52);
-          const long long Q = rec_q[k - kb];
-          if (M + Q >= (1LL << 53)) break;
-          prefix[c0] = __longlong_as_double(M);
-          prefix[c0 + 1] = __longlong_as_double((long long)e);
-          prefix[c0 + 3] = __longlong_as_double(kRecMark);
-          s = (double)(M + Q) * ldexp(1.0, e - 52);
-          ++k;
+    int k = 0;  // next chunk of the window
+    while (k < wend) {
+      int stop = k;
+      if (normal_finite(s)) {
+        const int e = binade_of(s);
+        const unsigned long long M = mantissa_of(s);
+        const long long tag = kRecOk | (long long)(e + 2048);
+        unsigned long long q[kWalkPer], before, all;
+#pragma unroll
+        for (int j = 0; j < kWalkPer; ++j)
+          q[j] = j0 + j < k || j0 + j >= wend ? 0 : rt[j] == tag ? rq[j] : kQMax;
+        stop = min(walk_scan(q, M, W, before, all), wend);
+#pragma unroll
+        for (int j = 0; j < kWalkPer; ++j) {
+          const int c = j0 + j;
+          if (c >= k && c < stop) {
+            const long long c0 = (kb + c) * kExactChunk;
+            prefix[c0] = __longlong_as_double((long long)(M + before));
+            prefix[c0 + 1] = __longlong_as_double((long long)e);
+            prefix[c0 + 3] = __longlong_as_double(kRecMark);
+          }
+          if (c == stop) W.s = (double)(M + before) * binade_ulp(e);
+          before += q[j];
         }
-        w_s = s;
-        w_k = k;
+        __syncthreads();
+        s = stop < wend ? W.s : (double)(M + all) * binade_ulp(e);
       }
-      __syncthreads();
-      s = w_s;
-      k = w_k;
-      if (k < kend) {
-        // chunk k by the sequential-exact algorithm
-        const long long c0 = k * kExactChunk;
-        s = exact_range(rates, c0, min(c0 + (long long)kExactChunk, n), s, prefix, w_sum, w_fail, &s_s, &s_p);
-        ++k;
+      if (stop < wend) {
+        const long long c0 = (kb + stop) * kExactChunk;
+        s = walk_chunk(rates + c0, (int)min((long long)kExactChunk, n - c0), s, prefix + c0, W);
       }
-      __syncthreads();
+      k = stop + 1;
+      __syncthreads();  // W is free again
     }
   }
   if (threadIdx.x == 0) *d_total = n > 0 ? s : 0.0;
@@ -583,66 +652,65 @@ __global__ void __launch_bounds__(kExactThreads) exact_walk_kernel(const double*
 __global__ void __launch_bounds__(kExactThreads) exact_write_kernel(const double* __restrict__ rates, long long n_fixed,
                                                                     const long long* __restrict__ d_count,
                                                                     double* __restrict__ prefix) {
-  __shared__ long long w_sum[32];
-  __shared__ long long s_rec[3];
+  __shared__ double buf[kExactPad];
+  __shared__ unsigned long long w_sum[kExactThreads / 32];
   const long long n = exact_count(n_fixed, d_count);
   const long long c0 = (long long)blockIdx.x * kExactChunk;
   if (c0 >= n || !has_record(c0, n)) return;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  if (tid < 3) s_rec[tid] = __double_as_longlong(prefix[c0 + (tid == 2 ? 3 : tid)]);
-  __syncthreads();
-  if (s_rec[2] != kRecMark) return;  // the walk wrote this chunk
-  const long long M = s_rec[0];
-  const int e = (int)s_rec[1];
-  const long long c1 = min(c0 + (long long)kExactChunk, n);
-  const double scale = ldexp(1.0, 52 - e), u = ldexp(1.0, e - 52);
-  const long long base = c0 + (long long)tid * kExactPer;
-  long long q[kExactPer];
-  long long tot = 0;
+  const unsigned long long M = (unsigned long long)__double_as_longlong(prefix[c0]);
+  const int e = (int)__double_as_longlong(prefix[c0 + 1]);
+  if (__double_as_longlong(prefix[c0 + 3]) != kRecMark) return;  // the walk wrote this chunk
+  const int m = (int)min((long long)kExactChunk, n - c0);
+  const double scale = binade_scale(e), u = binade_ulp(e);
 #pragma unroll
   for (int k = 0; k < kExactPer; ++k) {
-    const long long i = base + k;
-    q[k] = i < c1 ? exact_q(rates[i], scale) : 0;  // >= 0: the chunk's record said so
+    const int i = tid + k * kExactThreads;
+    if (i < m) buf[pad8(i)] = rates[c0 + i];
+  }
+  __syncthreads();  // also: every thread has read the record
+  unsigned long long q[kExactPer];
+  unsigned long long tot = 0;
+#pragma unroll
+  for (int k = 0; k < kExactPer; ++k) {
+    const int i = tid * kExactPer + k;
+    bool bad;
+    q[k] = i < m ? exact_q(buf[pad8(i)], scale, bad) : 0;  // not bad: the chunk's record said so
     tot += q[k];
   }
-  long long incl = tot;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const long long t = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += t;
-  }
+  const unsigned long long incl = warp_scan_q(tot, lane);
   if (lane == 31) w_sum[wid] = incl;
   __syncthreads();
-  if (wid == 0) {
-    long long v = w_sum[lane];
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const long long t = __shfl_up_sync(0xffffffffu, v, o);
-      if (lane >= o) v += t;
-    }
-    w_sum[lane] = v;
-  }
-  __syncthreads();
-  long long Q = (wid > 0 ? w_sum[wid - 1] : 0) + (incl - tot);
+  unsigned long long Q = incl - tot;
+  for (int w = 0; w < wid; ++w) Q += w_sum[w];
 #pragma unroll
   for (int k = 0; k < kExactPer; ++k) {
-    const long long i = base + k;
-    if (i < c1) {
-      Q += q[k];
-      prefix[i] = (double)(M + Q) * u;
-    }
+    const int i = tid * kExactPer + k;
+    Q += q[k];
+    if (i < m) buf[pad8(i)] = (double)(M + Q) * u;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kExactPer; ++k) {
+    const int i = tid + k * kExactThreads;
+    if (i < m) prefix[c0 + i] = buf[pad8(i)];
   }
 }
 
-// the five launches for up to n_max rates (the count is *d_count when given)
+static unsigned int exact_chunks(long long n) {
+  return (unsigned int)std::max(1LL, (n + kExactChunk - 1) / kExactChunk);
+}
+
+// the launches for up to n_max rates (the count is *d_count when given);
+// have_sums: the chunk sums are already in the chunks' entries 0
 static int launch_exact_prefix(const double* rates, long long n_max, const long long* d_count, double* prefix,
-                               double* d_total, cudaStream_t s) {
+                               double* d_total, bool have_sums, cudaStream_t s) {
   const long long nfix = d_count ? 0 : n_max;
-  const unsigned int K = (unsigned int)std::max(1LL, (n_max + kExactChunk - 1) / kExactChunk);
-  exact_chunk_sum_kernel<<<K, 256, 0, s>>>(rates, nfix, d_count, prefix);
-  exact_chunk_scan_kernel<<<1, 1024, 0, s>>>(nfix, d_count, prefix);
+  const unsigned int K = exact_chunks(n_max);
+  if (!have_sums) exact_chunk_sum_kernel<<<K, kExactThreads, 0, s>>>(rates, nfix, d_count, prefix);
+  exact_chunk_scan_kernel<<<1, kScanThreads, 0, s>>>(nfix, d_count, prefix);
   exact_chunk_q_kernel<<<K, kExactThreads, 0, s>>>(rates, nfix, d_count, prefix);
-  exact_walk_kernel<<<1, kExactThreads, 0, s>>>(rates, nfix, d_count, prefix, d_total);
+  exact_walk_kernel<<<1, kWalkThreads, 0, s>>>(rates, nfix, d_count, prefix, d_total);
   exact_write_kernel<<<K, kExactThreads, 0, s>>>(rates, nfix, d_count, prefix);
   MGK_CUDA(cudaGetLastError());
   return MGK_OK;
@@ -960,11 +1028,21 @@ __global__ void scan_block_kernel(const double* __restrict__ r, long long n, dou
 }
 
 __global__ void scan_bsum_kernel(double* bsum, int nb, long long n, double* d_total) {
-  // single-thread exclusive scan of the (few hundred) block totals
-  if (threadIdx.x != 0) return;
+  // exclusive scan of the block totals, added in order by one thread from
+  // shared memory (in order from global memory each add waits for its load)
+  __shared__ double buf[1024];
   double run = 0.0;
-  for (int b = 0; b < nb; ++b) { const double t = bsum[b]; bsum[b] = run; run += t; }
-  *d_total = n > 0 ? run : 0.0;
+  for (int b0 = 0; b0 < nb; b0 += 1024) {
+    const int m = min(1024, nb - b0);
+    for (int i = threadIdx.x; i < m; i += blockDim.x) buf[i] = bsum[b0 + i];
+    __syncthreads();
+    if (threadIdx.x == 0)
+      for (int i = 0; i < m; ++i) { const double t = buf[i]; buf[i] = run; run += t; }
+    __syncthreads();
+    for (int i = threadIdx.x; i < m; i += blockDim.x) bsum[b0 + i] = buf[i];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) *d_total = n > 0 ? run : 0.0;
 }
 
 __global__ void scan_add_kernel(double* prefix, long long n, const double* bsum) {
@@ -977,6 +1055,10 @@ __global__ void scan_add_kernel(double* prefix, long long n, const double* bsum)
 using namespace mgk;
 
 static int blocks_for(long long n, int bs) { return (int)((n + bs - 1) / bs); }
+// 16-byte tensor loads need both bases aligned (a caller may pass a view)
+static bool aligned16(const void* a, const void* b) {
+  return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15) == 0;
+}
 
 extern "C" int mgk_kmc2d_barrier(int nx, int ny, int M, double* Q, const double* Q0, const double* sig,
                                  const double* catalog, double volume, const double* soft_prop,
@@ -987,7 +1069,8 @@ extern "C" int mgk_kmc2d_barrier(int nx, int ny, int M, double* Q, const double*
   MGK_REQUIRE(Q && Q0 && sig && catalog && soft_prop && last_event_time, "mgk_kmc2d_barrier: null argument");
   MGK_REQUIRE(scheme == 0 || (scheme == 1 && prev_strain_dir), "mgk_kmc2d_barrier: bad scheme");
   const long long nvox = (long long)nx * ny;
-  barrier_kernel<2, 2><<<blocks_for(nvox * M, 256), 256, 0, (cudaStream_t)stream>>>(
+  auto kern = aligned16(sig, catalog) ? barrier_kernel<2, 2, true> : barrier_kernel<2, 2, false>;
+  kern<<<blocks_for(nvox * M, 256), 256, 0, (cudaStream_t)stream>>>(
       nvox, M, Q, Q0, sig, catalog, volume, soft_prop, last_event_time, current_time, prev_strain_dir,
       softening_cap, scheme, tau);
   MGK_CUDA(cudaGetLastError());
@@ -1010,9 +1093,9 @@ extern "C" int mgk_kmc2d_barrier_total(int nx, int ny, int M, double* Q, const d
   const double vnu = rate_volume * nu0;  // host product, as in mgk_kmc2d_rates
   cudaStream_t s = (cudaStream_t)stream;
   double* partials = reinterpret_cast<double*>(work);
-  barrier_total_kernel<2, 2><<<nb, 256, 0, s>>>(nvox, M, Q, Q0, sig, catalog, volume, soft_prop, last_event_time,
-                                                current_time, prev_strain_dir, softening_cap, scheme, tau,
-                                                temperature, temperature_scalar, vnu, partials);
+  auto kern = aligned16(sig, catalog) ? barrier_total_kernel<2, 2, true> : barrier_total_kernel<2, 2, false>;
+  kern<<<nb, 256, 0, s>>>(nvox, M, Q, Q0, sig, catalog, volume, soft_prop, last_event_time, current_time,
+                          prev_strain_dir, softening_cap, scheme, tau, temperature, temperature_scalar, vnu, partials);
   partials_total_kernel<<<1, 256, 0, s>>>(partials, nb, d_total);
   MGK_CUDA(cudaGetLastError());
   return MGK_OK;
@@ -1028,10 +1111,10 @@ static int kmc_rates_impl(long long nvox, int M, const double* Q, double volume,
   const long long n = nvox * M;
   const double vnu = volume * nu0;  // host product, same rounding as (volume * nu0) in the reference
   if (!cascade_mode) {
-    rates_full_kernel<<<blocks_for(n, 256), 256, 0, s>>>(nvox, M, Q, vnu, T, Ts, rates, (long long*)indices,
-                                                         (long long*)d_count);
+    rates_sum_kernel<<<exact_chunks(n), kExactThreads, 0, s>>>(n, M, Q, vnu, T, beta_of(Ts), rates,
+                                                               (long long*)indices, (long long*)d_count, prefix);
     MGK_CUDA(cudaGetLastError());
-    int rc = launch_exact_prefix(rates, n, nullptr, prefix, d_total, s);
+    int rc = launch_exact_prefix(rates, n, nullptr, prefix, d_total, true, s);
     if (rc) return rc;
   } else {
     MGK_REQUIRE(work != nullptr, "mgk_kmc2d_rates: cascade mode needs the work buffer");
@@ -1043,7 +1126,7 @@ static int kmc_rates_impl(long long nvox, int M, const double* Q, double volume,
     MGK_CUDA(cudaGetLastError());
     rates_scatter_kernel<<<nb, 256, 0, s>>>(nvox, M, Q, vnu, T, Ts, bcount, rates, (long long*)indices);
     MGK_CUDA(cudaGetLastError());
-    int rc = launch_exact_prefix(rates, n, (const long long*)d_count, prefix, d_total, s);
+    int rc = launch_exact_prefix(rates, n, (const long long*)d_count, prefix, d_total, false, s);
     if (rc) return rc;
   }
   return MGK_OK;
@@ -1067,7 +1150,7 @@ extern "C" int mgk_kmc_prefix(const double* rates, int64_t n, double* prefix, in
   cudaStream_t s = (cudaStream_t)stream;
   set_count_kernel<<<1, 1, 0, s>>>((long long*)d_count, (long long)n);
   MGK_CUDA(cudaGetLastError());
-  return launch_exact_prefix(rates, n, nullptr, prefix, d_total, s);
+  return launch_exact_prefix(rates, n, nullptr, prefix, d_total, false, s);
 }
 
 extern "C" int mgk_kmc_select(const double* prefix, const int64_t* d_count, const double* d_total, double u,
@@ -1100,7 +1183,7 @@ extern "C" int mgk_kmc3d_barrier(int nx, int ny, int nz, int M, double* Q, const
   MGK_REQUIRE(Q && Q0 && sig && catalog && soft_prop && last_event_time, "mgk_kmc3d_barrier: null argument");
   MGK_REQUIRE(scheme == 0 || (scheme == 1 && prev_strain_dir), "mgk_kmc3d_barrier: bad scheme");
   const long long nvox = (long long)nx * ny * nz;
-  barrier_kernel<3, 4><<<blocks_for(nvox * M, 256), 256, 0, (cudaStream_t)stream>>>(
+  barrier_kernel<3, 4, false><<<blocks_for(nvox * M, 256), 256, 0, (cudaStream_t)stream>>>(
       nvox, M, Q, Q0, sig, catalog, volume, soft_prop, last_event_time, current_time, prev_strain_dir,
       softening_cap, scheme, tau);
   MGK_CUDA(cudaGetLastError());
@@ -1198,10 +1281,10 @@ extern "C" int mgk_kmc_prefix_fast(const double* rates, int64_t n, double* prefi
   set_count_kernel<<<1, 1, 0, s>>>((long long*)d_count, (long long)n);
   if (nb > 0) {
     scan_block_kernel<<<nb, 256, 0, s>>>(rates, n, prefix, bsum);
-    scan_bsum_kernel<<<1, 32, 0, s>>>(bsum, nb, n, d_total);
+    scan_bsum_kernel<<<1, 256, 0, s>>>(bsum, nb, n, d_total);
     scan_add_kernel<<<(int)((n + 255) / 256), 256, 0, s>>>(prefix, n, bsum);
   } else {
-    scan_bsum_kernel<<<1, 32, 0, s>>>(bsum, 0, 0, d_total);
+    scan_bsum_kernel<<<1, 256, 0, s>>>(bsum, 0, 0, d_total);
   }
   MGK_CUDA(cudaGetLastError());
   return MGK_OK;
@@ -1212,7 +1295,7 @@ extern "C" int mgk_kmc2d_rates_only(int nx, int ny, int M, const double* Q, doub
   MGK_REQUIRE(nx > 0 && ny > 0 && M > 0 && Q && rates, "mgk_kmc2d_rates_only: bad argument");
   const long long nvox = (long long)nx * ny, n = nvox * M;
   rates_full_kernel<<<blocks_for(n, 256), 256, 0, (cudaStream_t)stream>>>(nvox, M, Q, volume * nu0, temperature,
-                                                                          temperature_scalar, rates, nullptr, nullptr);
+                                                                          beta_of(temperature_scalar), rates, nullptr, nullptr);
   MGK_CUDA(cudaGetLastError());
   return MGK_OK;
 }
