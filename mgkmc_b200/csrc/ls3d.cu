@@ -33,185 +33,25 @@
 
 #include "common.cuh"
 #include "fft.cuh"
-#include "tma.cuh"
+#include "ls3d_dev.cuh"
+#include "ls3d_line.cuh"
 
 namespace mgk {
 
 const void* twiddles(int n, int prec);
 
-struct Ls3dRep {
-  int nx, ny, nz, nzh, ld, tc;
-  int zl_items;      // z-line pairs = nx*ny/2
-  int y_items;       // nx * ceil(nzh/tc)
-  int x_items;       // ny * ceil(nzh/tc)
-  long long N;
-  FftLen fx, fy, fz;
-  double* mu;
-  double* lam;
-  double* eps;   // 6 planes
-  double* ep;    // 6 planes
-  double* epf;   // 9 planes or null
-  double2* spec;
-  // mixed-precision plans (warp-line kernels only): FP32 copies and tables;
-  // the FP32 spectrum reuses `spec`
-  float* mu32;
-  float* lam32;
-  float* eps32;  // 6 planes
-  float* ep32;   // 6 planes
-  FftLen fx32, fy32, fz32;
-  // per call
-  const double* init;
-  double* out_eps;
-  double* out_sig;
-  double eb[9];
-  double tol;
-  int max_iter;
-  int zl_first;
-  // constitutive law: 0 linear (elasticity.py:62-67); 1 the secant
-  // degradation law with magnitude law_a and rate law_b (FP64 plans)
-  int law;
-  double law_a, law_b;
-  // law 3, Landau: v1, v2, v3, g1, g2, g3, g4, capping (0 none, 1 piecewise,
-  // 2 smooth), E_cap, tangent ratio, smooth power
-  double lp[11];
-};
-
-struct Ls3dState {
-  double mu0, lam0, Bc, inv2mu0;
-  double ebar[6];
-  double abar[3];  // (xy - yx)/2, (xz - zx)/2, (yz - zy)/2 of eps_bar
-  double extra_d0, extra_n0;
-  int iter, done, status, phase_iter;  // done: 0 active, 1 phase 1 finished, 2 finished
-  double diff;
-  double means[9];
-  double out_eps_mean[9];
-  double out_sig_mean[9];
-};
-
-struct Ls3dCtl {
-  unsigned int n_active, decided, still, bodies;
-  int any;
-  int error;  // a bounded wait gave up (MGK_TIMEOUT)
-};
-
-constexpr double kL3Phase1Tol = 2e-6;  // mixed plans: FP32 iterations down to max(tol, this)
-constexpr int kL3Phase1Cap = 64;
-
-// symmetric component c -> (i, j): xx yy zz yz xz xy
-__device__ __constant__ int kSymI[6] = {0, 1, 2, 1, 0, 0};
-__device__ __constant__ int kSymJ[6] = {0, 1, 2, 2, 2, 1};
-
-__device__ __forceinline__ int fftfreq3(int k, int n) { return (k < (n + 1) / 2) ? k : k - n; }
-
-// eps~^ = -Gamma0(n) : tau^ for symmetric tau (3D), n a unit vector.
-// t[6] / e[6] in the symmetric order above.
-// R = double for the FP64 iterations, float for the FP32 phase of a mixed plan.
-template <typename R>
-__device__ __forceinline__ void gamma3d_apply_t(const C_t<R>* t, R n0, R n1, R n2, R inv2mu0, R Bc, C_t<R>* e) {
-  constexpr int kI[6] = {0, 1, 2, 1, 0, 0}, kJ[6] = {0, 1, 2, 2, 2, 1};
-  const R n[3] = {n0, n1, n2};
-  // full symmetric tau as 3x3 of complex
-  C_t<R> T[3][3];
-  T[0][0] = t[0]; T[1][1] = t[1]; T[2][2] = t[2];
-  T[1][2] = T[2][1] = t[3];
-  T[0][2] = T[2][0] = t[4];
-  T[0][1] = T[1][0] = t[5];
-  C_t<R> tn[3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    tn[i].x = T[i][0].x * n[0] + T[i][1].x * n[1] + T[i][2].x * n[2];
-    tn[i].y = T[i][0].y * n[0] + T[i][1].y * n[1] + T[i][2].y * n[2];
-  }
-  C_t<R> ntn;
-  ntn.x = tn[0].x * n[0] + tn[1].x * n[1] + tn[2].x * n[2];
-  ntn.y = tn[0].y * n[0] + tn[1].y * n[1] + tn[2].y * n[2];
-#pragma unroll
-  for (int c = 0; c < 6; ++c) {
-    const int k = kI[c], h = kJ[c];
-    e[c].x = -(inv2mu0 * (n[h] * tn[k].x + n[k] * tn[h].x) - Bc * n[k] * n[h] * ntn.x);
-    e[c].y = -(inv2mu0 * (n[h] * tn[k].y + n[k] * tn[h].y) - Bc * n[k] * n[h] * ntn.y);
-  }
-}
-__device__ __forceinline__ void gamma3d_apply(const double2* t, double n0, double n1, double n2, double inv2mu0,
-                                              double Bc, double2* e) {
-  gamma3d_apply_t<double>(t, n0, n1, n2, inv2mu0, Bc, e);
+const Ls3Line* ls3_line_a(int n, int prec);
+const Ls3Line* ls3_line_b(int n, int prec);
+const Ls3Line* ls3_line_c(int n, int prec);
+const Ls3Line* ls3_line_d(int n, int prec);
+const Ls3Line* ls3_line(int n, int prec) {
+  for (auto f : {ls3_line_a, ls3_line_b, ls3_line_c, ls3_line_d})
+    if (const Ls3Line* k = f(n, prec)) return k;
+  return nullptr;
 }
 
 // -------------------------------------------------------------- kernels ---
 
-// Secant shear modulus mu (1 - d (1 - exp(-k eq))) (elasticity.py:703-728) at
-// the von Mises equivalent strain sqrt(2/3 e':e') of the elastic strain
-// (elasticity.py:665-700) given by its symmetric components; each pair of
-// shear entries sums to twice the symmetric one.
-// 3D Landau small-strain stress (elasticity.py:811-857) of the symmetric
-// elastic strain a = (xx, yy, zz, yz, xz, xy), with the strain capping of
-// elasticity.py:297-334: deviator scaled by f above the cap E_cap (piecewise)
-// or by the tanh profile (smooth), plus 2 (ratio mu) (a - capped) w.
-// sigma = (lam I1 + v1/2 I1^2 + v2 I2 + g1/6 I1^3 + g2 I1 I2 + 4/3 g3 I3) I
-//       + 2 (mu + v2 I1 + g2/2 I1^2 + g4 I2) e + 4 (v3 + g3 I1) e^2.
-__device__ __forceinline__ void landau_sigma3(double mu, double lam, const double* a, const double* __restrict__ lp,
-                                              double* sg) {
-  const double v1 = lp[0], v2 = lp[1], v3 = lp[2], g1 = lp[3], g2 = lp[4], g3 = lp[5], g4 = lp[6];
-  const int cap = (int)lp[7];
-  double c[6];
-  for (int q = 0; q < 6; ++q) c[q] = a[q];
-  double w = 0.0;
-  if (cap) {
-    const double I1a = a[0] + a[1] + a[2];
-    const double m3 = (1.0 / 3.0) * I1a;
-    const double d0 = a[0] - m3, d1 = a[1] - m3, d2 = a[2] - m3;
-    const double dd = d0 * d0 + d1 * d1 + d2 * d2 + 2.0 * (a[3] * a[3] + a[4] * a[4] + a[5] * a[5]);
-    const double Eeq = sqrt(fmax(0.0, (2.0 / 3.0) * dd));
-    const double Ecap = lp[8];
-    double f = 1.0;
-    if (cap == 2) {
-      const double pw = lp[10];
-      if (Eeq > 1e-12) f = (Ecap / Eeq) * pow(tanh(fmin(100.0, pow(Eeq / Ecap, pw))), 1.0 / pw);
-      const double t = tanh(fmin(100.0, pow(Eeq / Ecap, pw)));
-      w = t * t;
-    } else if (Eeq > Ecap) {
-      f = Ecap / Eeq;
-      w = 1.0;
-    }
-    c[0] = d0 * f + m3;
-    c[1] = d1 * f + m3;
-    c[2] = d2 * f + m3;
-    c[3] = a[3] * f;
-    c[4] = a[4] * f;
-    c[5] = a[5] * f;
-  }
-  // e^2 of the symmetric tensor [[xx, xy, xz], [xy, yy, yz], [xz, yz, zz]]
-  const double xx = c[0], yy = c[1], zz = c[2], yz = c[3], xz = c[4], xy = c[5];
-  double e2[6];
-  e2[0] = xx * xx + xy * xy + xz * xz;
-  e2[1] = xy * xy + yy * yy + yz * yz;
-  e2[2] = xz * xz + yz * yz + zz * zz;
-  e2[3] = xy * xz + yy * yz + yz * zz;
-  e2[4] = xx * xz + xy * yz + xz * zz;
-  e2[5] = xx * xy + xy * yy + xz * yz;
-  const double I1 = xx + yy + zz;
-  const double I2 = e2[0] + e2[1] + e2[2];
-  const double I3 = (e2[0] * xx + e2[5] * xy + e2[4] * xz) + (e2[5] * xy + e2[1] * yy + e2[3] * yz) +
-                    (e2[4] * xz + e2[3] * yz + e2[2] * zz);
-  const double cI = lam * I1 + 0.5 * v1 * (I1 * I1) + v2 * I2 + (1.0 / 6.0) * g1 * (I1 * I1 * I1) + g2 * I1 * I2 +
-                    (4.0 / 3.0) * g3 * I3;
-  const double ce = 2.0 * (mu + v2 * I1 + 0.5 * g2 * (I1 * I1) + g4 * I2);
-  const double ce2 = 4.0 * (v3 + g3 * I1);
-  for (int q = 0; q < 6; ++q) sg[q] = (q < 3 ? cI : 0.0) + ce * c[q] + ce2 * e2[q];
-  if (cap) {
-    const double r = 2.0 * (lp[9] * mu) * w;
-    for (int q = 0; q < 6; ++q) sg[q] += r * (a[q] - c[q]);
-  }
-}
-
-__device__ __forceinline__ double secant_mu3(double m, double xx, double yy, double zz, double yz, double xz,
-                                             double xy, double d, double k) {
-  const double tr3 = (xx + yy + zz) / 3.0;
-  const double a = xx - tr3, b = yy - tr3, c = zz - tr3;
-  const double s1 = 2.0 * xy, s2 = 2.0 * xz, s3 = 2.0 * yz;
-  const double eq = sqrt((2.0 / 3.0) * (a * a + b * b + c * c + 0.5 * (s1 * s1 + s2 * s2 + s3 * s3)));
-  return m * (1.0 - d * (1.0 - exp(-k * eq)));
-}
 
 __global__ void ls3d_material_kernel(const Ls3dRep* reps, int rep, const double* __restrict__ E,
                                      const double* __restrict__ nu, const double* __restrict__ epsp,
@@ -360,68 +200,6 @@ __global__ void ls3d_begin_kernel(const Ls3dRep* reps, Ls3dState* st, const int*
       S.extra_d0 = 0;
       S.extra_n0 = 2.0 * (double)N * (ab[0] * ab[0] + ab[1] * ab[1] + ab[2] * ab[2]);
     }
-  }
-}
-
-// Partial sums of this z-line item, and (last item of the replica) the
-// fixed-order reduction, the convergence decision and the loop condition.
-template <bool FINAL>
-__device__ void ls3d_decide(const Ls3dRep& R, Ls3dState& S, int r, int item, double d2, double n2,
-                            double* partials, unsigned int* rep_counter, Ls3dCtl* ctl,
-                            cudaGraphConditionalHandle cond, int use_cond, int guard_cap, double* red,
-                            int* s_last_p) {
-  int& s_last = *s_last_p;
-  const long long N = R.N;
-  d2 = block_sum(d2, red);
-  n2 = block_sum(n2, red);
-  if (threadIdx.x == 0) {
-    partials[2 * item] = d2;
-    partials[2 * item + 1] = n2;
-    __threadfence();
-    const unsigned int t = atomicInc(&rep_counter[r], (unsigned int)R.zl_items - 1);
-    s_last = (t == (unsigned int)R.zl_items - 1);
-  }
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  double a = 0, b = 0;
-  for (int i = threadIdx.x; i < R.zl_items; i += blockDim.x) {
-    a += __ldcg(&partials[2 * (R.zl_first + i)]);
-    b += __ldcg(&partials[2 * (R.zl_first + i) + 1]);
-  }
-  a = block_sum(a, red);
-  b = block_sum(b, red);
-  if (threadIdx.x != 0) return;
-  if (S.iter == 0) { a += S.extra_d0; b += S.extra_n0; }
-  else b += 2.0 * (double)N * (S.abar[0] * S.abar[0] + S.abar[1] * S.abar[1] + S.abar[2] * S.abar[2]);
-  const double diff = sqrt(a) / (sqrt(b) + 1e-20);
-  S.diff = diff;
-  S.iter += 1;
-  S.phase_iter += 1;
-  int keep = 0;
-  if (!isfinite(diff)) { S.done = 2; S.status = MGK_NONFINITE; }
-  else if (FINAL) {
-    if (diff < R.tol) { S.done = 2; S.status = MGK_OK; }
-    else if (S.iter >= R.max_iter) { S.done = 2; S.status = MGK_NOT_CONVERGED; }
-    else keep = 1;
-  } else {
-    const double tol1 = R.tol > kL3Phase1Tol ? R.tol : kL3Phase1Tol;
-    if (S.iter >= R.max_iter) { S.done = 2; S.status = diff < R.tol ? MGK_OK : MGK_NOT_CONVERGED; }
-    else if (diff < tol1 || S.phase_iter >= kL3Phase1Cap) S.done = 1;
-    else keep = 1;
-  }
-  const unsigned int n_act = ctl->n_active;
-  if (keep) atomicAdd(&ctl->still, 1u);
-  __threadfence();
-  const unsigned int dcount = atomicAdd(&ctl->decided, 1u);
-  if (dcount == n_act - 1) {
-    __threadfence();
-    const unsigned int still = atomicExch(&ctl->still, 0u);
-    ctl->decided = 0;
-    ctl->n_active = still;
-    const bool go = still > 0 && atomicAdd(&ctl->bodies, 0u) <= (unsigned int)guard_cap;
-    ctl->any = go ? 1 : 0;
-    if (use_cond) cudaGraphSetConditional(cond, go ? 1u : 0u);
   }
 }
 
@@ -627,347 +405,6 @@ __global__ void __launch_bounds__(256) ls3d_axis_kernel(const Ls3dRep* __restric
   }
 }
 
-// --------------------------------------------- warp-line iteration kernels ---
-// The same iteration for replicas whose sides are all 64, 96 or 128:
-//   z-line kernel: CTA of 3 warps per pair of z-lines; one elected thread
-//     stages the pair's eps (6), mu, lambda and eps_p (6) lines in shared
-//     memory with bulk copies while warp w inverts components 2w, 2w+1 of the
-//     spectrum; after one CTA barrier every thread updates its voxels and
-//     builds tau; warp w transforms and stores its two components.
-//   axis kernels: per tile of kL3Tile kz columns at one x (y passes) or one y
-//     (x pass with Gamma0_sym between the transforms), warp c owns component
-//     c's lines; the x pass CTA holds all 6 components, an FP64 y pass CTA 3.
-constexpr int kL3Tile = 4;
-
-template <typename T> struct L3F;
-template <> struct L3F<double> {
-  static __device__ __forceinline__ double* eps(const Ls3dRep& R) { return R.eps; }
-  static __device__ __forceinline__ const double* ep(const Ls3dRep& R) { return R.ep; }
-  static __device__ __forceinline__ const double* mu(const Ls3dRep& R) { return R.mu; }
-  static __device__ __forceinline__ const double* lam(const Ls3dRep& R) { return R.lam; }
-  static __device__ __forceinline__ double2* spec(const Ls3dRep& R) { return R.spec; }
-  static __device__ __forceinline__ const FftLen& fx(const Ls3dRep& R) { return R.fx; }
-  static __device__ __forceinline__ const FftLen& fy(const Ls3dRep& R) { return R.fy; }
-  static __device__ __forceinline__ const FftLen& fz(const Ls3dRep& R) { return R.fz; }
-};
-template <> struct L3F<float> {
-  static __device__ __forceinline__ float* eps(const Ls3dRep& R) { return R.eps32; }
-  static __device__ __forceinline__ const float* ep(const Ls3dRep& R) { return R.ep32; }
-  static __device__ __forceinline__ const float* mu(const Ls3dRep& R) { return R.mu32; }
-  static __device__ __forceinline__ const float* lam(const Ls3dRep& R) { return R.lam32; }
-  static __device__ __forceinline__ float2* spec(const Ls3dRep& R) { return reinterpret_cast<float2*>(R.spec); }
-  static __device__ __forceinline__ const FftLen& fx(const Ls3dRep& R) { return R.fx32; }
-  static __device__ __forceinline__ const FftLen& fy(const Ls3dRep& R) { return R.fy32; }
-  static __device__ __forceinline__ const FftLen& fz(const Ls3dRep& R) { return R.fz32; }
-};
-__host__ __device__ constexpr bool ls3_fast_len(int n) { return n == 64 || n == 96 || n == 128; }
-__host__ __device__ constexpr int ls3_pl(int n, int csz) { return csz == 16 ? n + n / 8 + 1 : ((n + n / 16 + 2) & ~1); }
-__host__ __device__ constexpr int ls3_zl_smem(int nz, int csz) {
-  return ((6 * ls3_pl(nz, csz) * csz + 127) / 128) * 128 + 14 * 2 * nz * (csz / 2);
-}
-__host__ __device__ constexpr int ls3_ax_smem(int n, int csz) { return 6 * kL3Tile * ls3_pl(n, csz) * csz; }
-
-template <typename T, bool IN_SPEC, bool FINAL, int NZ, int LAW>
-__device__ __forceinline__ void ls3_zline_body(const Ls3dRep& R, Ls3dState& S, int item, int r, long long l0,
-                                               double* partials, unsigned int* rep_counter, Ls3dCtl* ctl,
-                                               cudaGraphConditionalHandle cond, int use_cond, int guard_cap,
-                                               unsigned char* smem, uint64_t* bar, double* red, int* s_last) {
-  using C = C_t<T>;
-  constexpr int PL = padded_len<C>(NZ);
-  constexpr int NZH = NZ / 2 + 1;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int ld = R.ld;
-  const long long N = R.N;
-  const long long plane = (long long)R.nx * R.ny * ld;
-  C* lines = reinterpret_cast<C*>(smem);
-  T* stg = reinterpret_cast<T*>(smem + ((6 * PL * (int)sizeof(C) + 127) / 128) * 128);
-  T* eps = L3F<T>::eps(R);
-  const T* ep = L3F<T>::ep(R);
-  C* spec = L3F<T>::spec(R);
-  constexpr uint32_t rb = 2u * NZ * sizeof(T);
-  if (threadIdx.x == 0) {
-    fence_proxy_async_smem();
-    mbar_arrive_expect_tx(bar, 14u * rb);
-#pragma unroll
-    for (int c = 0; c < 6; ++c) bulk_g2s(stg + c * 2 * NZ, eps + c * N + l0 * NZ, rb, bar);
-    bulk_g2s(stg + 12 * NZ, L3F<T>::mu(R) + l0 * NZ, rb, bar);
-    bulk_g2s(stg + 14 * NZ, L3F<T>::lam(R) + l0 * NZ, rb, bar);
-#pragma unroll
-    for (int c = 0; c < 6; ++c) bulk_g2s(stg + (16 + 2 * c) * NZ, ep + c * N + l0 * NZ, rb, bar);
-  }
-  const C* tw = reinterpret_cast<const C*>(L3F<T>::fz(R).tw);
-  C* lw = lines + 2 * warp * PL;
-  if (IN_SPEC) {
-    constexpr int U = (NZH + 31) / 32;
-    for (int cc = 0; cc < 2; ++cc) {
-      const int c = 2 * warp + cc;
-      C* ln = lines + c * PL;
-      const C* ra = spec + c * plane + l0 * ld;
-      // the component's half-spectrum rows into registers first: one memory
-      // round trip, not one per strided step behind the shared-memory stores
-      C av[U], bv[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int k = lane + 32 * u;
-        if (k < NZH) { av[u] = ra[k]; bv[u] = ra[ld + k]; }
-      }
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int k = lane + 32 * u;
-        if (k < NZH) {
-          C a = av[u], b = bv[u];
-          if (k == 0 || 2 * k == NZ) { a.y = 0; b.y = 0; }
-          ln[pidx<C>(k)] = mk<C>(a.x - b.y, a.y + b.x);
-          if (k > 0 && 2 * k < NZ) ln[pidx<C>(NZ - k)] = mk<C>(a.x + b.y, b.x - a.y);
-        }
-      }
-    }
-    __syncwarp();
-    warp_fft<NZ, +1, 2>(lw, PL, tw, lane);
-  }
-  const bool ok = mbar_wait(bar, 0);
-  if (!__syncthreads_and(ok ? 1 : 0)) {
-    if (threadIdx.x == 0) { ctl->error = 1; ctl->any = 0; }
-    return;
-  }
-  const double mu0 = S.mu0, lam0 = S.lam0;
-  double d2 = 0, n2 = 0;
-  for (int z = threadIdx.x; z < NZ; z += 96) {
-    const int pz = pidx<C>(z);
-    C zz[6];
-    if (IN_SPEC) {
-#pragma unroll
-      for (int c = 0; c < 6; ++c) zz[c] = lines[c * PL + pz];
-    }
-    T tr[2][6];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int j = h * NZ + z;
-      const long long i = (l0 + h) * NZ + z;
-      double e[6];
-#pragma unroll
-      for (int c = 0; c < 6; ++c) {
-        const double o = (double)stg[c * 2 * NZ + j];
-        if (IN_SPEC) {
-          const double nw = S.ebar[c] + (double)(h == 0 ? zz[c].x : zz[c].y);
-          const double dd = nw - o;
-          const double w = c < 3 ? 1.0 : 2.0;
-          d2 += w * dd * dd;
-          n2 += w * o * o;
-          eps[c * N + i] = (T)nw;
-          e[c] = nw;
-        } else {
-          e[c] = o;
-        }
-      }
-      double m = (double)stg[12 * NZ + j];
-      const double l = (double)stg[14 * NZ + j];
-      double d[6];
-#pragma unroll
-      for (int c = 0; c < 6; ++c) d[c] = e[c] - (double)stg[(16 + 2 * c) * NZ + j];
-      if constexpr (LAW == 1) m = secant_mu3(m, d[0], d[1], d[2], d[3], d[4], d[5], R.law_a, R.law_b);
-      const double trd = d[0] + d[1] + d[2], tre = e[0] + e[1] + e[2];
-      if constexpr (LAW == 3) {
-        double sg[6];
-        landau_sigma3(m, l, d, R.lp, sg);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) tr[h][c] = (T)(sg[c] - (2 * mu0 * e[c] + lam0 * tre));
-#pragma unroll
-        for (int c = 3; c < 6; ++c) tr[h][c] = (T)(sg[c] - 2 * mu0 * e[c]);
-      } else {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) tr[h][c] = (T)((2 * m * d[c] + l * trd) - (2 * mu0 * e[c] + lam0 * tre));
-#pragma unroll
-        for (int c = 3; c < 6; ++c) tr[h][c] = (T)(2 * m * d[c] - 2 * mu0 * e[c]);
-      }
-    }
-#pragma unroll
-    for (int c = 0; c < 6; ++c) lines[c * PL + pz] = mk<C>(tr[0][c], tr[1][c]);
-  }
-  __syncthreads();
-  warp_fft<NZ, -1, 2>(lw, PL, tw, lane);
-  for (int cc = 0; cc < 2; ++cc) {
-    const int c = 2 * warp + cc;
-    const C* ln = lines + c * PL;
-    C* ra = spec + c * plane + l0 * ld;
-    for (int k = lane; k < NZH; k += 32) {
-      const C z = ln[pidx<C>(k)];
-      const C w = ln[pidx<C>(k == 0 ? 0 : NZ - k)];
-      ra[k] = mk<C>(T(0.5) * (z.x + w.x), T(0.5) * (z.y - w.y));
-      ra[ld + k] = mk<C>(T(0.5) * (z.y + w.y), T(-0.5) * (z.x - w.x));
-    }
-  }
-  if (!IN_SPEC) return;
-  ls3d_decide<FINAL>(R, S, r, item, d2, n2, partials, rep_counter, ctl, cond, use_cond, guard_cap, red, s_last);
-}
-
-template <typename T, bool IN_SPEC, bool FINAL, int LAW = 0>
-__device__ __forceinline__ void ls3d_zline_fast_entry(const Ls3dRep* __restrict__ reps, Ls3dState* st,
-                                                      const int* __restrict__ map, const int* __restrict__ loc,
-                                                      double* partials, unsigned int* rep_counter, Ls3dCtl* ctl,
-                                                      cudaGraphConditionalHandle cond, int use_cond, int guard_cap) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ double red[32];
-  __shared__ int s_last;
-  __shared__ __align__(8) uint64_t bar;
-  const int item = blockIdx.x;
-  const int r = map[item];
-  const Ls3dRep& R = reps[r];
-  Ls3dState& S = st[r];
-  if (IN_SPEC && use_cond && item == 0 && threadIdx.x == 0) {
-    const unsigned int b = atomicAdd(&ctl->bodies, 1u) + 1u;
-    if (ctl->n_active == 0 || b > (unsigned int)guard_cap || *(volatile int*)&ctl->error != 0) {
-      ctl->any = 0;
-      cudaGraphSetConditional(cond, 0u);
-    }
-  }
-  if (S.done != 0) return;
-  if (threadIdx.x == 0) {
-    mbar_init(&bar, 1);
-    fence_mbar_init();
-  }
-  __syncthreads();
-  const long long l0 = 2LL * loc[item];
-#define MGK_Z3_CASE(n) case n: ls3_zline_body<T, IN_SPEC, FINAL, n, LAW>(R, S, item, r, l0, partials, rep_counter, ctl, cond, use_cond, guard_cap, smem_raw, &bar, red, &s_last); break;
-  switch (R.nz) {
-    MGK_Z3_CASE(64) MGK_Z3_CASE(96) MGK_Z3_CASE(128)
-    default: break;
-  }
-#undef MGK_Z3_CASE
-}
-
-// FP32 phase kernel with a register target of 8 resident CTAs per SM, and
-// the FP64 kernel with one of 5 (both measured faster at 128^3 than the
-// compiler's own choice, despite some spilled registers)
-template <typename T, bool IN_SPEC, bool FINAL>
-__global__ void __launch_bounds__(96, 8) ls3d_zline_fast_kernel(const Ls3dRep* __restrict__ reps, Ls3dState* st,
-                                                            const int* __restrict__ map, const int* __restrict__ loc,
-                                                            double* partials, unsigned int* rep_counter, Ls3dCtl* ctl,
-                                                            cudaGraphConditionalHandle cond, int use_cond,
-                                                            int guard_cap) {
-  ls3d_zline_fast_entry<T, IN_SPEC, FINAL>(reps, st, map, loc, partials, rep_counter, ctl, cond, use_cond, guard_cap);
-}
-template <bool IN_SPEC, bool FINAL, int LAW = 0>  // LAW 1: the secant law, 3: the Landau law
-__global__ void __launch_bounds__(96, 5) ls3d_zline_fast64_kernel(const Ls3dRep* __restrict__ reps, Ls3dState* st,
-                                                                const int* __restrict__ map, const int* __restrict__ loc,
-                                                                double* partials, unsigned int* rep_counter,
-                                                                Ls3dCtl* ctl, cudaGraphConditionalHandle cond,
-                                                                int use_cond, int guard_cap) {
-  ls3d_zline_fast_entry<double, IN_SPEC, FINAL, LAW>(reps, st, map, loc, partials, rep_counter, ctl, cond,
-                                                     use_cond, guard_cap);
-}
-
-template <typename T, int AXIS, int SIGN, int NL, int NC>
-__device__ __forceinline__ void ls3_axis_body(const Ls3dRep& R, const Ls3dState& S, int o, int k0, int c0,
-                                              unsigned char* smem) {
-  using C = C_t<T>;
-  constexpr int PL = padded_len<C>(NL);
-  constexpr int TC = kL3Tile;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nx = R.nx, ny = R.ny, nz = R.nz, nzh = R.nzh, ld = R.ld;
-  const int tcw = min(TC, nzh - k0);
-  const long long plane = (long long)nx * ny * ld;
-  const long long jstride = AXIS == 1 ? ld : (long long)ny * ld;
-  const long long obase = AXIS == 1 ? (long long)o * ny * ld : (long long)o * ld;
-  C* lines = reinterpret_cast<C*>(smem);  // line (c * TC + t), c relative to c0
-  C* spec = L3F<T>::spec(R) + c0 * plane;
-  constexpr int TOT = NC * NL * TC;
-  for (int e = threadIdx.x; e < TOT; e += NC * 32) {
-    const int c = e / (NL * TC);
-    const int rem = e - c * NL * TC;
-    const int j = rem / TC, t = rem - j * TC;
-    if (t < tcw) cp_async_elem(&lines[(c * TC + t) * PL + pidx<C>(j)], &spec[c * plane + obase + j * jstride + k0 + t]);
-  }
-  cp_async_wait_all();
-  __syncthreads();
-  const C* tw = reinterpret_cast<const C*>((AXIS == 1 ? L3F<T>::fy(R) : L3F<T>::fx(R)).tw);
-  C* l0 = lines + warp * TC * PL;
-  warp_fft<NL, AXIS == 1 ? SIGN : -1, 2>(l0, PL, tw, lane);
-  warp_fft<NL, AXIS == 1 ? SIGN : -1, 2>(l0 + 2 * PL, PL, tw, lane);
-  if constexpr (AXIS == 0) {
-    // Gamma0 in the precision of the pass: FP64 iterations in double, the
-    // FP32 phase of a mixed plan in float (its errors are those of its FP32
-    // fields; the FP64 phase that follows removes both)
-    __syncthreads();
-    const T scale = T(1.0 / (double)R.N);
-    const T inv2mu0 = (T)S.inv2mu0, Bc = (T)S.Bc;
-    const int ky = o;
-    const T uy = (T)fftfreq3(ky, ny) / (T)ny;
-    const bool nqy = (ny & 1) == 0 && 2 * ky == ny;
-    for (int e = threadIdx.x; e < tcw * NL; e += NC * 32) {
-      const int t = e / NL, kx = e - t * NL;
-      const int kz = k0 + t;
-      const int pk = pidx<C>(kx);
-      C tv[6], ev[6];
-#pragma unroll
-      for (int c = 0; c < 6; ++c) tv[c] = lines[(c * TC + t) * PL + pk];
-      if (kx == 0 && ky == 0 && kz == 0) {
-        for (int c = 0; c < 6; ++c) lines[(c * TC + t) * PL + pk] = mk<C>(T(0), T(0));
-        continue;
-      }
-      const T ux = (T)fftfreq3(kx, nx) / (T)nx, uz = (T)fftfreq3(kz, nz) / (T)nz;
-      const T inv = T(1) / sqrt(ux * ux + uy * uy + uz * uz);
-      const T n0 = ux * inv, n1 = uy * inv, n2 = uz * inv;
-      gamma3d_apply_t<T>(tv, n0, n1, n2, inv2mu0, Bc, ev);
-      const bool nqx = (nx & 1) == 0 && 2 * kx == nx, nqz = (nz & 1) == 0 && 2 * kz == nz;
-      if (nqx || nqy || nqz) {
-        C fv[6];
-        gamma3d_apply_t<T>(tv, nqx ? -n0 : n0, nqy ? -n1 : n1, nqz ? -n2 : n2, inv2mu0, Bc, fv);
-#pragma unroll
-        for (int c = 0; c < 6; ++c) ev[c] = mk<C>(T(0.5) * (ev[c].x + fv[c].x), T(0.5) * (ev[c].y + fv[c].y));
-      }
-#pragma unroll
-      for (int c = 0; c < 6; ++c) lines[(c * TC + t) * PL + pk] = mk<C>(ev[c].x * scale, ev[c].y * scale);
-    }
-    __syncthreads();
-    warp_fft<NL, +1, 2>(l0, PL, tw, lane);
-    warp_fft<NL, +1, 2>(l0 + 2 * PL, PL, tw, lane);
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < TOT; e += NC * 32) {
-    const int c = e / (NL * TC);
-    const int rem = e - c * NL * TC;
-    const int j = rem / TC, t = rem - j * TC;
-    if (t < tcw) spec[c * plane + obase + j * jstride + k0 + t] = lines[(c * TC + t) * PL + pidx<C>(j)];
-  }
-}
-
-// components per CTA of the axis kernels: the x pass applies Gamma0 across
-// all 6 components; the FP64 y passes transform 3 components per CTA (two
-// CTAs per tile: 5 resident CTAs of 3 warps per SM instead of 2 of 6 at the
-// registers an FP64 line pair needs).  FP32 y passes keep 6 per CTA (measured
-// faster at 128^3).  Second value: resident-CTA target for the allocator
-// (the FP32 x pass: 3, at most 96 registers).
-__host__ __device__ constexpr int ls3_axis_nc(int axis, int tsz) { return axis == 0 || tsz == 4 ? 6 : 3; }
-__host__ __device__ constexpr int ls3_axis_minb(int axis, int tsz) {
-  return ls3_axis_nc(axis, tsz) == 3 ? 5 : (axis == 0 && tsz == 4 ? 3 : 2);
-}
-
-// grid = items * (6 / NC), the component group fastest
-template <typename T, int AXIS, int SIGN>
-__global__ void __launch_bounds__(ls3_axis_nc(AXIS, sizeof(T)) * 32, ls3_axis_minb(AXIS, sizeof(T)))
-    ls3d_axis_fast_kernel(const Ls3dRep* __restrict__ reps, const Ls3dState* __restrict__ st,
-                          const int* __restrict__ map, const int* __restrict__ loc) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  constexpr int NC = ls3_axis_nc(AXIS, sizeof(T));
-  const int item = blockIdx.x / (6 / NC);
-  const int c0 = (blockIdx.x % (6 / NC)) * NC;
-  const int r = map[item];
-  const Ls3dRep& R = reps[r];
-  const Ls3dState& S = st[r];
-  if (S.done != 0) return;
-  const int ntile = (R.nzh + kL3Tile - 1) / kL3Tile;
-  const int o = loc[item] / ntile;
-  const int k0 = (loc[item] - o * ntile) * kL3Tile;
-  const int nl = AXIS == 1 ? R.ny : R.nx;
-#define MGK_A3_CASE(n) case n: ls3_axis_body<T, AXIS, SIGN, n, NC>(R, S, o, k0, c0, smem_raw); break;
-  switch (nl) {
-    MGK_A3_CASE(64) MGK_A3_CASE(96) MGK_A3_CASE(128)
-    default: break;
-  }
-#undef MGK_A3_CASE
-}
-
 // Mixed plans, between the phases: FP64 field from the FP32 one; grid (G, nsel)
 __global__ void ls3d_promote_kernel(const Ls3dRep* reps, const int* sel) {
   const int r = sel[blockIdx.y];
@@ -1078,10 +515,10 @@ int tc3(int n) {
 struct mgk_ls3d_plan {
   int nrep = 0;
   long long maxN = 0;
-  size_t zl_smem = 0, ax_smem = 0;
-  int fast = 0;  // warp-line kernels (every side 64, 96 or 128)
+  size_t zl_smem = 0, ax_smem = 0;  // CTA-wide passes
+  std::vector<char> line;           // replicas on the register-FFT kernels (every side has one)
+  bool mixed_ok = false;            // every side of every replica 64, 96 or 128
   int prec = MGK_FP64;
-  size_t zl_smem32 = 0, ax_smem32 = 0;
   std::vector<Ls3dRep> reps;
   std::vector<char> has_material;
   std::vector<void*> allocations;
@@ -1099,10 +536,15 @@ struct mgk_ls3d_plan {
   double* d_part = nullptr;
   double* d_mat_part = nullptr;
   int tot_zl = 0, tot_y = 0, tot_x = 0;
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
-  int graph_mode = -1, graph_cap = 0;
-  int nsel = 0, s_zl = 0, s_y = 0, s_x = 0;
+  // instantiated loop graphs by the selection's shapes (its signature)
+  struct GraphEntry {
+    std::vector<int> sig;
+    int cap;
+    cudaGraph_t g;
+    cudaGraphExec_t x;
+  };
+  std::vector<GraphEntry> gcache;
+  int graph_mode = 1;  // 0: host-driven loop
   int law = 0;  // 1: secant degradation law (mgk_ls3d_set_secant)
 };
 
@@ -1116,13 +558,32 @@ static int a3(mgk_ls3d_t p, void** ptr, size_t bytes) {
   return MGK_OK;
 }
 
-// Precision form (warp-line plans only): MGK_MIXED runs FP32 iterations
+// raises the shared-memory limits of a replica's register-FFT kernels
+static int ls3_attrs(const Ls3dRep& R, int prec) {
+  const Ls3Line *kx = ls3_line(R.nx, prec), *ky = ls3_line(R.ny, prec), *kz = ls3_line(R.nz, prec);
+  for (int law : {0, 1, 3})
+    if (kz->zline[law]) MGK_CUDA(raise_smem(kz->zline[law], kz->z_bytes));
+  MGK_CUDA(raise_smem(ky->y[0], ky->y_bytes));
+  MGK_CUDA(raise_smem(ky->y[1], ky->y_bytes));
+  MGK_CUDA(raise_smem(kx->x, kx->x_bytes));
+  return MGK_OK;
+}
+
+static void drop_graphs3(mgk_ls3d_t p) {
+  for (auto& e : p->gcache) {
+    cudaGraphExecDestroy(e.x);
+    cudaGraphDestroy(e.g);
+  }
+  p->gcache.clear();
+}
+
+// Precision form (sides 64, 96 and 128): MGK_MIXED runs FP32 iterations
 // (FP32 fields, spectra and Gamma0) until the update norm is below
 // max(tol, 2e-6), then FP64 iterations from that field to tol.
 extern "C" int mgk_ls3d_set_precision(mgk_ls3d_t p, int precision) {
   MGK_REQUIRE(p, "mgk_ls3d_set_precision: null plan");
   MGK_REQUIRE(precision == MGK_FP64 || precision == MGK_MIXED, "mgk_ls3d_set_precision: bad precision");
-  MGK_REQUIRE(precision == MGK_FP64 || p->fast,
+  MGK_REQUIRE(precision == MGK_FP64 || p->mixed_ok,
               "mgk_ls3d_set_precision: the mixed form needs every side in {64, 96, 128}");
   if (precision == MGK_MIXED && !p->reps[0].mu32) {
     for (int r = 0; r < p->nrep; ++r) {
@@ -1132,22 +593,23 @@ extern "C" int mgk_ls3d_set_precision(mgk_ls3d_t p, int precision) {
       if (st) return st;
       float* fl = reinterpret_cast<float*>(f);
       R.mu32 = fl; R.lam32 = fl + R.N; R.eps32 = fl + 2 * R.N; R.ep32 = fl + 8 * R.N;
-      R.fx32 = R.fx; R.fy32 = R.fy; R.fz32 = R.fz;
-      R.fx32.tw = twiddles(R.nx, 1); R.fy32.tw = twiddles(R.ny, 1); R.fz32.tw = twiddles(R.nz, 1);
-      if (!R.fx32.tw || !R.fy32.tw || !R.fz32.tw) return MGK_OOM;
+      const int n[3] = {R.nx, R.ny, R.nz};
+      for (int q = 0; q < 3; ++q) {
+        R.rtw32[q] = reinterpret_cast<const float2*>(twiddles_reg(n[q], 1));
+        if (!R.rtw32[q]) return MGK_OOM;
+      }
+      if (ls3_attrs(R, MGK_MIXED)) return MGK_CUDA_ERROR;
       p->has_material[r] = 0;  // the FP32 copies come with the next set_material
     }
     MGK_CUDA(cudaMemcpy(p->d_reps, p->reps.data(), sizeof(Ls3dRep) * p->nrep, cudaMemcpyHostToDevice));
   }
-  if (precision != p->prec) p->graph_mode = -1;
   p->prec = precision;
   return MGK_OK;
 }
 
 extern "C" int mgk_ls3d_destroy(mgk_ls3d_t p) {
   if (!p) return MGK_OK;
-  if (p->exec) cudaGraphExecDestroy(p->exec);
-  if (p->graph) cudaGraphDestroy(p->graph);
+  drop_graphs3(p);
   if (p->staged) cudaEventDestroy(p->staged);
   for (void* a : p->allocations) cudaFree(a);
   if (p->h_reps) cudaFreeHost(p->h_reps);
@@ -1177,32 +639,39 @@ extern "C" int mgk_ls3d_create_batch(int nrep, const int* nxs, const int* nys, c
   p->nrep = nrep;
   p->reps.resize(nrep);
   p->has_material.assign(nrep, 0);
-  {
-    bool fast = true;
-    for (int r = 0; r < nrep; ++r) fast = fast && ls3_fast_len(nxs[r]) && ls3_fast_len(nys[r]) && ls3_fast_len(nzs[r]);
-    const char* env = getenv("MGK_FAST");
-    p->fast = fast && !(env && env[0] == '0');
-  }
+  const char* env = getenv("MGK_FAST");
+  const bool use_line = !(env && env[0] == '0');
+  p->mixed_ok = use_line;
+  p->line.assign(nrep, 0);
   for (int r = 0; r < nrep; ++r) {
     Ls3dRep& R = p->reps[r];
     memset(&R, 0, sizeof(R));
     R.nx = nxs[r]; R.ny = nys[r]; R.nz = nzs[r];
     R.nzh = R.nz / 2 + 1;
-    R.ld = R.nzh;
+    const int side[3] = {R.nx, R.ny, R.nz};
+    bool line = use_line;
+    for (int n : side) {
+      line = line && ls3_line(n, MGK_FP64);
+      p->mixed_ok = p->mixed_ok && (n == 64 || n == 96 || n == 128);
+    }
+    p->line[r] = line;
+    R.ld = line ? (R.nzh + 3) / 4 * 4 : R.nzh;  // register-FFT tiles read rows of 64 aligned bytes
     R.N = (long long)R.nx * R.ny * R.nz;
-    R.tc = p->fast ? kL3Tile : tc3(std::max(R.nx, R.ny));
+    R.tc = tc3(std::max(R.nx, R.ny));
     const int ntile = (R.nzh + R.tc - 1) / R.tc;
-    R.zl_items = R.nx * R.ny / 2;
+    R.zl_items = line ? (R.nx * R.ny / 2 + ls3_line(R.nz, MGK_FP64)->zp - 1) / ls3_line(R.nz, MGK_FP64)->zp
+                      : R.nx * R.ny / 2;
     R.y_items = R.nx * ntile;
     R.x_items = R.ny * ntile;
     fft_schedule(R.nx, &R.fx); fft_schedule(R.ny, &R.fy); fft_schedule(R.nz, &R.fz);
     R.fx.tw = twiddles(R.nx, MGK_FP64); R.fy.tw = twiddles(R.ny, MGK_FP64); R.fz.tw = twiddles(R.nz, MGK_FP64);
     if (!R.fx.tw || !R.fy.tw || !R.fz.tw) return fail(MGK_OOM);
-    if (p->fast) {
-      p->zl_smem = std::max(p->zl_smem, (size_t)ls3_zl_smem(R.nz, 16));
-      p->ax_smem = std::max(p->ax_smem, (size_t)ls3_ax_smem(std::max(R.nx, R.ny), 16));
-      p->zl_smem32 = std::max(p->zl_smem32, (size_t)ls3_zl_smem(R.nz, 8));
-      p->ax_smem32 = std::max(p->ax_smem32, (size_t)ls3_ax_smem(std::max(R.nx, R.ny), 8));
+    if (line) {
+      for (int q = 0; q < 3; ++q) {
+        R.rtw[q] = reinterpret_cast<const double2*>(twiddles_reg(side[q], MGK_FP64));
+        if (!R.rtw[q]) return fail(MGK_OOM);
+      }
+      if (int rc = ls3_attrs(R, MGK_FP64)) return fail(rc);
     } else {
       p->zl_smem = std::max(p->zl_smem, 2 * 6 * (size_t)R.nz * sizeof(double2));
       p->ax_smem = std::max(p->ax_smem, 2 * 6 * (size_t)R.tc * std::max(R.nx, R.ny) * sizeof(double2));
@@ -1220,25 +689,7 @@ extern "C" int mgk_ls3d_create_batch(int nrep, const int* nxs, const int* nys, c
     R.spec = reinterpret_cast<double2*>(sp);
   }
   int st;
-  if (p->fast &&
-      (raise_smem((const void*)ls3d_zline_fast64_kernel<true, true>, (int)p->zl_smem) ||
-       raise_smem((const void*)ls3d_zline_fast64_kernel<false, true>, (int)p->zl_smem) ||
-       raise_smem((const void*)ls3d_zline_fast64_kernel<true, true, 1>, (int)p->zl_smem) ||
-       raise_smem((const void*)ls3d_zline_fast64_kernel<false, true, 1>, (int)p->zl_smem) ||
-       raise_smem((const void*)ls3d_zline_fast64_kernel<true, true, 3>, (int)p->zl_smem) ||
-       raise_smem((const void*)ls3d_zline_fast64_kernel<false, true, 3>, (int)p->zl_smem) ||
-       raise_smem((const void*)ls3d_axis_fast_kernel<double, 1, -1>, (int)p->ax_smem) ||
-       raise_smem((const void*)ls3d_axis_fast_kernel<double, 1, 1>, (int)p->ax_smem) ||
-       raise_smem((const void*)ls3d_axis_fast_kernel<double, 0, 0>, (int)p->ax_smem) ||
-       raise_smem((const void*)ls3d_zline_fast_kernel<float, true, false>, (int)p->zl_smem32) ||
-       raise_smem((const void*)ls3d_zline_fast_kernel<float, false, false>, (int)p->zl_smem32) ||
-       raise_smem((const void*)ls3d_axis_fast_kernel<float, 1, -1>, (int)p->ax_smem32) ||
-       raise_smem((const void*)ls3d_axis_fast_kernel<float, 1, 1>, (int)p->ax_smem32) ||
-       raise_smem((const void*)ls3d_axis_fast_kernel<float, 0, 0>, (int)p->ax_smem32))) {
-    set_error("mgk_ls3d_create: cudaFuncSetAttribute failed");
-    return fail(MGK_CUDA_ERROR);
-  }
-  if (!p->fast && (raise_smem((const void*)ls3d_zline_kernel<true>, (int)p->zl_smem) ||
+  if (p->zl_smem && (raise_smem((const void*)ls3d_zline_kernel<true>, (int)p->zl_smem) ||
       raise_smem((const void*)ls3d_zline_kernel<false>, (int)p->zl_smem) ||
       raise_smem((const void*)ls3d_axis_kernel<1, -1>, (int)p->ax_smem) ||
       raise_smem((const void*)ls3d_axis_kernel<1, 1>, (int)p->ax_smem) ||
@@ -1337,7 +788,7 @@ extern "C" int mgk_ls3d_set_secant(mgk_ls3d_t p, double d, double k) {
   const int law = d != 0.0 ? 1 : 0;
   for (auto& R : p->reps) { R.law = law; R.law_a = d; R.law_b = k; }
   if (law != p->law) {
-    if (p->graph_mode == 1) p->graph_mode = -1;
+    drop_graphs3(p);
     p->law = law;
   }
   return MGK_OK;
@@ -1362,7 +813,7 @@ extern "C" int mgk_ls3d_set_landau(mgk_ls3d_t p, const double* v, int capping, d
     R.lp[10] = smooth_power;
   }
   if (p->law != 3) {
-    if (p->graph_mode == 1) p->graph_mode = -1;
+    drop_graphs3(p);
     p->law = 3;
   }
   return MGK_OK;
@@ -1373,63 +824,104 @@ extern "C" int mgk_ls3d_set_eigenstrain_rep(mgk_ls3d_t p, int rep, const double*
   return set3(p, rep, nullptr, nullptr, epsp, 0, (cudaStream_t)stream);
 }
 
+// One launch group of a solve: the selected replicas of one shape on the
+// register-FFT kernels (kx, ky, kz), or every other replica on the CTA-wide
+// passes (kz null), which find their replica in work maps.
+struct Grp3 {
+  const Ls3Line *kx = nullptr, *ky = nullptr, *kz = nullptr;
+  const Ls3Line *kx32 = nullptr, *ky32 = nullptr, *kz32 = nullptr;
+  const int* sel = nullptr;  // the group's slice of the selection (device)
+  int n = 0;                 // replicas
+  int nx = 0, ny = 0, nzh = 0, zl_items = 0;  // of one replica
+  // CTA-wide group: maps and item counts over its replicas
+  const int *zm = nullptr, *zl = nullptr, *ym = nullptr, *yl = nullptr, *xm = nullptr, *xl = nullptr;
+  int czl = 0, cy = 0, cx = 0;
+  int lead = 0;  // counts the loop bodies
+};
+
 struct Loop3 {
   const Ls3dRep* reps;
   Ls3dState* st;
-  const int *zm, *zl, *ym, *yl, *xm, *xl;
   double* part;
   unsigned int* ctr;
   Ls3dCtl* ctl;
-  int nzl, ny, nx;
-  size_t zs, as;
-  int fast;
-  // mixed plans: FP32 phase shared memory, the selection and the
-  // per-voxel grid of the promote kernel
-  size_t zs32, as32;
+  size_t zs, as;  // shared memory of the CTA-wide passes
   const int* sel;
-  int nsel, G;
-  int law;
+  int nsel, G, law;
+  std::vector<Grp3> grp;
 };
 
-// kernels of one iteration: `f32` selects the FP32 phase of a mixed plan
-// (warp-line kernels only; its decisions end phase 1, not the solve)
-static void* zline_fn(int fast, bool in_spec, bool f32 = false, int law = 0) {
-  if (fast && !f32 && law == 1)
-    return in_spec ? (void*)ls3d_zline_fast64_kernel<true, true, 1> : (void*)ls3d_zline_fast64_kernel<false, true, 1>;
-  if (fast && !f32 && law == 3)
-    return in_spec ? (void*)ls3d_zline_fast64_kernel<true, true, 3> : (void*)ls3d_zline_fast64_kernel<false, true, 3>;
-  if (fast && f32)
-    return in_spec ? (void*)ls3d_zline_fast_kernel<float, true, false> : (void*)ls3d_zline_fast_kernel<float, false, false>;
-  if (fast)
-    return in_spec ? (void*)ls3d_zline_fast64_kernel<true, true> : (void*)ls3d_zline_fast64_kernel<false, true>;
-  return in_spec ? (void*)ls3d_zline_kernel<true> : (void*)ls3d_zline_kernel<false>;
-}
-template <int AXIS, int SIGN> static void* axis_fn(int fast, bool f32 = false) {
-  if (fast && f32) return (void*)ls3d_axis_fast_kernel<float, AXIS, SIGN>;
-  return fast ? (void*)ls3d_axis_fast_kernel<double, AXIS, SIGN> : (void*)ls3d_axis_kernel<AXIS, SIGN>;
+// The stages of one iteration of a group: 0 y forward, 1 x with Gamma0, 2 y
+// inverse, 3 z-lines; 4: the first z-line pass of a phase.
+struct Launch3 {
+  const void* fn;
+  dim3 grid, block;
+  size_t smem;
+};
+static Launch3 stage3(const Loop3& a, const Grp3& g, int stage, bool f32) {
+  if (!g.kz) {
+    switch (stage) {
+      case 0: return {(const void*)ls3d_axis_kernel<1, -1>, dim3(g.cy), dim3(kT3), a.as};
+      case 1: return {(const void*)ls3d_axis_kernel<0, 0>, dim3(g.cx), dim3(kT3), a.as};
+      case 2: return {(const void*)ls3d_axis_kernel<1, 1>, dim3(g.cy), dim3(kT3), a.as};
+      case 3: return {(const void*)ls3d_zline_kernel<true>, dim3(g.czl), dim3(kT3), a.zs};
+      default: return {(const void*)ls3d_zline_kernel<false>, dim3(g.czl), dim3(kT3), a.zs};
+    }
+  }
+  const Ls3Line *kx = f32 ? g.kx32 : g.kx, *ky = f32 ? g.ky32 : g.ky, *kz = f32 ? g.kz32 : g.kz;
+  if (stage >= 3)
+    return {kz->zline[f32 ? 0 : a.law], dim3(g.n * g.zl_items), dim3(kz->z_threads), (size_t)kz->z_bytes};
+  if (stage == 1)
+    return {kx->x, dim3(g.n * g.ny * ceil_div(g.nzh, kx->tile)), dim3(kx->x_threads), (size_t)kx->x_bytes};
+  return {ky->y[stage == 0 ? 0 : 1], dim3(2 * g.n * g.nx * ceil_div(g.nzh, ky->tile)), dim3(ky->y_threads),
+          (size_t)ky->y_bytes};
 }
 
-static int body3(const Loop3& a, cudaStream_t s, bool f32 = false) {
-  const dim3 ab(a.fast ? 192 : kT3), zb(a.fast ? 96 : kT3);
-  const size_t as = f32 ? a.as32 : a.as, zs = f32 ? a.zs32 : a.zs;
-  const bool ysplit = a.fast && ls3_axis_nc(1, f32 ? 4 : 8) == 3;  // FP64 y passes: 3 components per CTA
-  const size_t asy = ysplit ? as / 2 : as;
-  const dim3 gy(ysplit ? 2 * a.ny : a.ny), aby(ysplit ? 96 : ab.x);
-  void* ay[] = {(void*)&a.reps, (void*)&a.st, (void*)&a.ym, (void*)&a.yl};
-  void* ax[] = {(void*)&a.reps, (void*)&a.st, (void*)&a.xm, (void*)&a.xl};
-  cudaGraphConditionalHandle h = 0;
-  int zero = 0;
-  void* az[] = {(void*)&a.reps, (void*)&a.st, (void*)&a.zm, (void*)&a.zl, (void*)&a.part, (void*)&a.ctr,
-                (void*)&a.ctl, &h, &zero, &zero};
-  MGK_CUDA(cudaLaunchKernel(axis_fn<1, -1>(a.fast, f32), gy, aby, ay, asy, s));
-  MGK_CUDA(cudaLaunchKernel(axis_fn<0, 0>(a.fast, f32), dim3(a.nx), ab, ax, as, s));
-  MGK_CUDA(cudaLaunchKernel(axis_fn<1, 1>(a.fast, f32), gy, aby, ay, asy, s));
-  MGK_CUDA(cudaLaunchKernel(zline_fn(a.fast, true, f32, a.law), dim3(a.nzl), zb, az, zs, s));
+// Calls f(fn, grid, block, smem, args) with a stage's launch and arguments.
+template <typename F>
+static cudaError_t with_stage3(Loop3& a, Grp3& g, int stage, bool f32, cudaGraphConditionalHandle h, int use, int cap,
+                               F f) {
+  const Launch3 L = stage3(a, g, stage, f32);
+  if (g.kz) {
+    int first = stage == 4;
+    if (stage >= 3) {
+      void* z[] = {&a.reps, &a.st, &g.sel, &a.part, &a.ctr, &a.ctl, &h, &use, &cap, &g.lead, &first};
+      return f(L, z);
+    }
+    void* x[] = {&a.reps, &a.st, &g.sel};
+    return f(L, x);
+  }
+  if (stage >= 3) {
+    void* z[] = {&a.reps, &a.st, &g.zm, &g.zl, &a.part, &a.ctr, &a.ctl, &h, &use, &cap};
+    return f(L, z);
+  }
+  void* x[] = {&a.reps, &a.st, stage == 1 ? &g.xm : &g.ym, stage == 1 ? &g.xl : &g.yl};
+  return f(L, x);
+}
+
+static int launch3(Loop3& a, int stage, bool f32, cudaStream_t s) {
+  for (Grp3& g : a.grp)
+    MGK_CUDA(with_stage3(a, g, stage, f32, 0, 0, 0, [&](const Launch3& L, void** args) {
+      return cudaLaunchKernel(L.fn, L.grid, L.block, args, L.smem, s);
+    }));
   return MGK_OK;
 }
 
-// one while node running iterations of the FP32 (phase 1) or FP64 kernels
-static int add_while3(cudaGraph_t g, const cudaGraphNode_t* dep, Loop3& a, bool f32, int* cap,
+static cudaError_t add_node3(cudaGraph_t g, cudaGraphNode_t* node, const cudaGraphNode_t* dep, int ndep,
+                             const Launch3& L, void** args) {
+  cudaKernelNodeParams k;
+  memset(&k, 0, sizeof(k));
+  k.func = const_cast<void*>(L.fn);
+  k.gridDim = L.grid;
+  k.blockDim = L.block;
+  k.sharedMemBytes = (unsigned)L.smem;
+  k.kernelParams = args;
+  return cudaGraphAddKernelNode(node, g, dep, ndep, &k);
+}
+
+// One while node running iterations of the FP32 (phase 1) or FP64 kernels;
+// the groups' stages are independent chains of the body.
+static int add_while3(cudaGraph_t g, const cudaGraphNode_t* dep, int ndep, Loop3& a, bool f32, int cap,
                       cudaGraphNode_t* out) {
   cudaGraphConditionalHandle h;
   if (cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault)) return MGK_CUDA_ERROR;
@@ -1440,80 +932,56 @@ static int add_while3(cudaGraph_t g, const cudaGraphNode_t* dep, Loop3& a, bool 
   cp.conditional.handle = h;
   cp.conditional.type = cudaGraphCondTypeWhile;
   cp.conditional.size = 1;
-  if (cudaGraphAddNode(out, g, dep, dep ? 1 : 0, &cp)) return MGK_CUDA_ERROR;
+  if (cudaGraphAddNode(out, g, dep, ndep, &cp)) return MGK_CUDA_ERROR;
   cudaGraph_t body = cp.conditional.phGraph_out[0];
-  cudaGraphNode_t prev = nullptr, node;
-  auto add = [&](void* fn, dim3 grid, size_t smem, void** args, int block) {
-    cudaKernelNodeParams k;
-    memset(&k, 0, sizeof(k));
-    k.func = fn; k.gridDim = grid; k.blockDim = dim3(block); k.sharedMemBytes = (unsigned)smem; k.kernelParams = args;
-    cudaError_t e = cudaGraphAddKernelNode(&node, body, prev ? &prev : nullptr, prev ? 1 : 0, &k);
-    prev = node;
-    return e;
-  };
-  void* ay[] = {&a.reps, &a.st, &a.ym, &a.yl};
-  void* ax[] = {&a.reps, &a.st, &a.xm, &a.xl};
-  int use = 1;
-  void* az[] = {&a.reps, &a.st, &a.zm, &a.zl, &a.part, &a.ctr, &a.ctl, &h, &use, cap};
-  const int ab = a.fast ? 192 : kT3, zb = a.fast ? 96 : kT3;
-  const size_t as = f32 ? a.as32 : a.as, zs = f32 ? a.zs32 : a.zs;
-  const bool ysplit = a.fast && ls3_axis_nc(1, f32 ? 4 : 8) == 3;  // FP64 y passes: 3 components per CTA
-  const size_t asy = ysplit ? as / 2 : as;
-  const dim3 gy(ysplit ? 2 * a.ny : a.ny);
-  const int aby = ysplit ? 96 : ab;
-  cudaError_t e = add(axis_fn<1, -1>(a.fast, f32), gy, asy, ay, aby);
-  if (!e) e = add(axis_fn<0, 0>(a.fast, f32), dim3(a.nx), as, ax, ab);
-  if (!e) e = add(axis_fn<1, 1>(a.fast, f32), gy, asy, ay, aby);
-  if (!e) e = add(zline_fn(a.fast, true, f32, a.law), dim3(a.nzl), zs, az, zb);
-  return e ? MGK_CUDA_ERROR : MGK_OK;
+  for (Grp3& gr : a.grp) {
+    cudaGraphNode_t prev = nullptr;
+    for (int stage = 0; stage < 4; ++stage) {
+      cudaGraphNode_t node;
+      if (with_stage3(a, gr, stage, f32, h, 1, cap, [&](const Launch3& L, void** args) {
+            return add_node3(body, &node, prev ? &prev : nullptr, prev ? 1 : 0, L, args);
+          }))
+        return MGK_CUDA_ERROR;
+      prev = node;
+    }
+  }
+  return MGK_OK;
 }
 
 // Loop graph: FP64 plans one while node; mixed plans [FP32 while, promote,
 // phase-2 set-up, first FP64 z-line pass, FP64 while].
-static int graph3(mgk_ls3d_t p, Loop3& a, int cap) {
-  if (p->exec) { cudaGraphExecDestroy(p->exec); p->exec = nullptr; }
-  if (p->graph) { cudaGraphDestroy(p->graph); p->graph = nullptr; }
+static int graph3(mgk_ls3d_t p, Loop3& a, int cap, cudaGraph_t* gout, cudaGraphExec_t* xout) {
   cudaGraph_t g;
   MGK_CUDA(cudaGraphCreate(&g, 0));
-  int capv = cap;
   int rc = MGK_OK;
   cudaGraphNode_t last;
   if (p->prec == MGK_MIXED) {
-    cudaGraphNode_t w1, np, n2, nz0;
-    rc = add_while3(g, nullptr, a, true, &capv, &w1);
+    cudaGraphNode_t w1, np, n2;
+    std::vector<cudaGraphNode_t> nz0(a.grp.size());
+    rc = add_while3(g, nullptr, 0, a, true, cap, &w1);
     if (rc == MGK_OK) {
-      cudaKernelNodeParams k;
-      memset(&k, 0, sizeof(k));
-      void* ap[] = {&a.reps, (void*)&a.sel};
-      k.func = (void*)ls3d_promote_kernel; k.gridDim = dim3(a.G, a.nsel); k.blockDim = dim3(kT3); k.kernelParams = ap;
-      if (cudaGraphAddKernelNode(&np, g, &w1, 1, &k)) rc = MGK_CUDA_ERROR;
+      void* ap[] = {&a.reps, &a.sel};
+      if (add_node3(g, &np, &w1, 1, {(const void*)ls3d_promote_kernel, dim3(a.G, a.nsel), dim3(kT3), 0}, ap))
+        rc = MGK_CUDA_ERROR;
     }
     if (rc == MGK_OK) {
-      cudaKernelNodeParams k;
-      memset(&k, 0, sizeof(k));
-      void* ap[] = {&a.st, (void*)&a.sel, &a.nsel, &a.ctl};
-      k.func = (void*)ls3d_phase2_kernel; k.gridDim = dim3(1); k.blockDim = dim3(32); k.kernelParams = ap;
-      if (cudaGraphAddKernelNode(&n2, g, &np, 1, &k)) rc = MGK_CUDA_ERROR;
+      void* ap[] = {&a.st, &a.sel, &a.nsel, &a.ctl};
+      if (add_node3(g, &n2, &np, 1, {(const void*)ls3d_phase2_kernel, dim3(1), dim3(32), 0}, ap)) rc = MGK_CUDA_ERROR;
     }
-    if (rc == MGK_OK) {
-      cudaKernelNodeParams k;
-      memset(&k, 0, sizeof(k));
-      cudaGraphConditionalHandle h0 = 0;
-      int zero = 0;
-      void* ap[] = {&a.reps, &a.st, &a.zm, &a.zl, &a.part, &a.ctr, &a.ctl, &h0, &zero, &zero};
-      k.func = zline_fn(a.fast, false, false); k.gridDim = dim3(a.nzl); k.blockDim = dim3(a.fast ? 96 : kT3);
-      k.sharedMemBytes = (unsigned)a.zs; k.kernelParams = ap;
-      if (cudaGraphAddKernelNode(&nz0, g, &n2, 1, &k)) rc = MGK_CUDA_ERROR;
-    }
-    if (rc == MGK_OK) rc = add_while3(g, &nz0, a, false, &capv, &last);
+    for (size_t i = 0; i < a.grp.size() && rc == MGK_OK; ++i)
+      if (with_stage3(a, a.grp[i], 4, false, 0, 0, 0, [&](const Launch3& L, void** args) {
+            return add_node3(g, &nz0[i], &n2, 1, L, args);
+          }))
+        rc = MGK_CUDA_ERROR;
+    if (rc == MGK_OK) rc = add_while3(g, nz0.data(), (int)nz0.size(), a, false, cap, &last);
   } else {
-    rc = add_while3(g, nullptr, a, false, &capv, &last);
+    rc = add_while3(g, nullptr, 0, a, false, cap, &last);
   }
   cudaGraphExec_t x = nullptr;
   if (rc == MGK_OK && cudaGraphInstantiate(&x, g, 0)) rc = MGK_CUDA_ERROR;
   if (rc) { cudaGraphDestroy(g); cudaGetLastError(); return MGK_CUDA_ERROR; }
-  p->graph = g;
-  p->exec = x;
+  *gout = g;
+  *xout = x;
   return MGK_OK;
 }
 
@@ -1534,41 +1002,82 @@ extern "C" int mgk_ls3d_solve_batch(mgk_ls3d_t p, int nsel, const int* sel, cons
   }
   int rc = wait3(p);
   if (rc) return rc;
-  int nzl = 0, ny_ = 0, nx_ = 0;
-  for (int r : selv) { nzl += p->reps[r].zl_items; ny_ += p->reps[r].y_items; nx_ += p->reps[r].x_items; }
-  const bool changed = nzl != p->s_zl || ny_ != p->s_y || nx_ != p->s_x || nsel != p->nsel;
-  int* zm = p->h_maps; int* zl = zm + nzl; int* ym = zl + nzl; int* yl = ym + ny_;
-  int* xm = yl + ny_; int* xl = xm + nx_; int* sp = xl + nx_;
-  int zi = 0, yi = 0, xi = 0;
+  Loop3 a{p->d_reps, p->d_st, p->d_part, p->d_repctr, p->d_ctl, p->zl_smem, p->ax_smem, p->d_maps, nsel,
+          g3(p->maxN), p->law, {}};
+  // the selection by groups: the CTA-wide replicas first, then each shape
+  std::vector<int> order, sig{p->law, p->prec};
+  order.reserve(nsel);
+  {
+    Grp3 g;
+    for (int r : selv)
+      if (!p->line[r]) {
+        order.push_back(r);
+        ++g.n;
+        g.czl += p->reps[r].zl_items; g.cy += p->reps[r].y_items; g.cx += p->reps[r].x_items;
+      }
+    const int* m = p->d_maps + nsel;
+    g.zm = m; g.zl = g.zm + g.czl; g.ym = g.zl + g.czl; g.yl = g.ym + g.cy; g.xm = g.yl + g.cy; g.xl = g.xm + g.cx;
+    sig.insert(sig.end(), {nsel, g.n, g.czl, g.cy, g.cx});
+    if (g.n) a.grp.push_back(g);
+  }
+  std::vector<char> placed(p->nrep, 0);
   for (int q = 0; q < nsel; ++q) {
-    const int r = selv[q];
+    const Ls3dRep& R = p->reps[selv[q]];
+    if (!p->line[selv[q]] || placed[selv[q]]) continue;
+    Grp3 g;
+    g.kx = ls3_line(R.nx, MGK_FP64); g.ky = ls3_line(R.ny, MGK_FP64); g.kz = ls3_line(R.nz, MGK_FP64);
+    if (p->prec == MGK_MIXED) {
+      g.kx32 = ls3_line(R.nx, MGK_MIXED); g.ky32 = ls3_line(R.ny, MGK_MIXED); g.kz32 = ls3_line(R.nz, MGK_MIXED);
+    }
+    g.nx = R.nx; g.ny = R.ny; g.nzh = R.nzh; g.zl_items = R.zl_items;
+    g.sel = p->d_maps + order.size();
+    for (int w = q; w < nsel; ++w) {
+      const int r = selv[w];
+      const Ls3dRep& O = p->reps[r];
+      if (!p->line[r] || placed[r] || O.nx != R.nx || O.ny != R.ny || O.nz != R.nz) continue;
+      placed[r] = 1;
+      order.push_back(r);
+      ++g.n;
+    }
+    sig.insert(sig.end(), {R.nx, R.ny, R.nz, g.n});
+    a.grp.push_back(g);
+  }
+  a.grp[0].lead = 1;
+  // per-call records, the selection and the CTA-wide group's maps
+  const Grp3& cg = a.grp[0];
+  int* zm = p->h_maps + nsel; int* zl = zm + cg.czl; int* ym = zl + cg.czl; int* yl = ym + cg.cy;
+  int* xm = yl + cg.cy; int* xl = xm + cg.cx;
+  std::vector<int> at(p->nrep, 0);
+  for (int q = 0; q < nsel; ++q) at[selv[q]] = q;
+  int zfirst = 0, zi = 0, yi = 0, xi = 0;
+  for (int k = 0; k < nsel; ++k) {
+    const int r = order[k], q = at[r];
     Ls3dRep& H = p->h_reps[r];
     H = p->reps[r];
     H.init = eps_init ? eps_init[q] : nullptr;
     H.out_eps = eps_out ? eps_out[q] : nullptr;
     H.out_sig = sig_out ? sig_out[q] : nullptr;
-    for (int k = 0; k < 9; ++k) H.eb[k] = eps_bar[9 * q + k];
+    for (int c = 0; c < 9; ++c) H.eb[c] = eps_bar[9 * q + c];
     H.tol = tol;
     H.max_iter = max_iter;
-    H.zl_first = zi;
+    H.zl_first = zfirst;
+    zfirst += H.zl_items;
+    p->h_maps[k] = r;
+    if (p->line[r]) continue;
     for (int i = 0; i < H.zl_items; ++i) { zm[zi] = r; zl[zi] = i; ++zi; }
     for (int i = 0; i < H.y_items; ++i) { ym[yi] = r; yl[yi] = i; ++yi; }
     for (int i = 0; i < H.x_items; ++i) { xm[xi] = r; xl[xi] = i; ++xi; }
-    sp[q] = r;
   }
   const int n_active = max_iter > 0 ? nsel : 0;
   *p->h_ctl = Ls3dCtl{(unsigned int)n_active, 0u, 0u, 0u, n_active > 0, 0};
-  const size_t nm = 2 * (size_t)(nzl + ny_ + nx_) + nsel;
+  const size_t nm = nsel + 2 * (size_t)(zi + yi + xi);
   MGK_CUDA(cudaMemcpyAsync(p->d_maps, p->h_maps, sizeof(int) * nm, cudaMemcpyHostToDevice, s));
   MGK_CUDA(cudaMemcpyAsync(p->d_reps, p->h_reps, sizeof(Ls3dRep) * p->nrep, cudaMemcpyHostToDevice, s));
   MGK_CUDA(cudaMemcpyAsync(p->d_ctl, p->h_ctl, sizeof(Ls3dCtl), cudaMemcpyHostToDevice, s));
   MGK_CUDA(cudaEventRecord(p->staged, s));
   p->staged_pending = true;
-  p->s_zl = nzl; p->s_y = ny_; p->s_x = nx_; p->nsel = nsel;
-  const int* d_zm = p->d_maps; const int* d_zl = d_zm + nzl; const int* d_ym = d_zl + nzl;
-  const int* d_yl = d_ym + ny_; const int* d_xm = d_yl + ny_; const int* d_xl = d_xm + nx_;
-  const int* d_sel = d_xl + nx_;
-  const int G = g3(p->maxN);
+  const int* d_sel = a.sel;
+  const int G = a.G;
   bool any_init = false;
   for (int q = 0; q < nsel && eps_init; ++q) any_init |= eps_init[q] != nullptr;
   if (any_init) {
@@ -1585,43 +1094,43 @@ extern "C" int mgk_ls3d_solve_batch(mgk_ls3d_t p, int nsel, const int* sel, cons
     MGK_CUDA(cudaGetLastError());
   }
   if (n_active > 0) {
-    Loop3 a{p->d_reps, p->d_st, d_zm, d_zl, d_ym, d_yl, d_xm, d_xl, p->d_part, p->d_repctr, p->d_ctl,
-            nzl, ny_, nx_, p->zl_smem, p->ax_smem, p->fast, p->zl_smem32, p->ax_smem32, d_sel, nsel, G, p->law};
     const bool mixed = p->prec == MGK_MIXED;
-    {
-      cudaGraphConditionalHandle h0 = 0;
-      int zero = 0;
-      void* az0[] = {(void*)&p->d_reps, (void*)&p->d_st, (void*)&d_zm, (void*)&d_zl, (void*)&p->d_part,
-                     (void*)&p->d_repctr, (void*)&p->d_ctl, &h0, &zero, &zero};
-      MGK_CUDA(cudaLaunchKernel(zline_fn(p->fast, false, mixed, p->law), dim3(nzl), dim3(p->fast ? 96 : kT3), az0,
-                                mixed ? p->zl_smem32 : p->zl_smem, s));
-    }
+    rc = launch3(a, 4, mixed, s);
+    if (rc) return rc;
     const int cap = max_iter + 2 > 1000 ? max_iter + 2 : 1000;
-    if (p->graph_mode == 1 && (changed || cap > p->graph_cap)) p->graph_mode = -1;
-    if (p->graph_mode < 0) {
-      const char* env = getenv("MGK_NO_GRAPH_WHILE");
-      if (env && env[0] == '1') p->graph_mode = 0;
-      else {
-        p->graph_mode = graph3(p, a, cap) == MGK_OK ? 1 : 0;
-        p->graph_cap = cap;
+    const char* env = getenv("MGK_NO_GRAPH_WHILE");
+    if (env && env[0] == '1') p->graph_mode = 0;
+    cudaGraphExec_t exec = nullptr;
+    if (p->graph_mode == 1) {
+      for (auto& e : p->gcache)
+        if (e.cap >= cap && e.sig == sig) exec = e.x;
+      if (!exec) {
+        cudaGraph_t g;
+        if (graph3(p, a, cap, &g, &exec) == MGK_OK) {
+          constexpr size_t kMaxGraphs3 = 16;
+          if (p->gcache.size() >= kMaxGraphs3) {
+            cudaGraphExecDestroy(p->gcache.front().x);
+            cudaGraphDestroy(p->gcache.front().g);
+            p->gcache.erase(p->gcache.begin());
+          }
+          p->gcache.push_back({sig, cap, g, exec});
+        } else {
+          p->graph_mode = 0;
+        }
       }
     }
     if (p->graph_mode == 1) {
-      MGK_CUDA(cudaGraphLaunch(p->exec, s));
+      MGK_CUDA(cudaGraphLaunch(exec, s));
     } else {
       for (int phase = mixed ? 1 : 2; phase <= 2; ++phase) {
         if (phase == 2 && mixed) {
           ls3d_promote_kernel<<<dim3(G, nsel), kT3, 0, s>>>(p->d_reps, d_sel);
           ls3d_phase2_kernel<<<1, 32, 0, s>>>(p->d_st, d_sel, nsel, p->d_ctl);
-          cudaGraphConditionalHandle h0 = 0;
-          int zero = 0;
-          void* az1[] = {(void*)&p->d_reps, (void*)&p->d_st, (void*)&d_zm, (void*)&d_zl, (void*)&p->d_part,
-                         (void*)&p->d_repctr, (void*)&p->d_ctl, &h0, &zero, &zero};
-          MGK_CUDA(cudaLaunchKernel(zline_fn(p->fast, false, false, p->law), dim3(nzl), dim3(96), az1, p->zl_smem, s));
+          if ((rc = launch3(a, 4, false, s))) return rc;
         }
         for (int it = 0; it < max_iter; ++it) {
-          rc = body3(a, s, phase == 1);
-          if (rc) return rc;
+          for (int stage = 0; stage < 4; ++stage)
+            if ((rc = launch3(a, stage, phase == 1, s))) return rc;
           Ls3dCtl hc;
           MGK_CUDA(cudaMemcpyAsync(&hc, p->d_ctl, sizeof(Ls3dCtl), cudaMemcpyDeviceToHost, s));
           MGK_CUDA(cudaStreamSynchronize(s));
@@ -1646,7 +1155,7 @@ extern "C" int mgk_ls3d_solve_batch(mgk_ls3d_t p, int nsel, const int* sel, cons
     MGK_CUDA(cudaMemcpyAsync(&hc3, p->d_ctl, sizeof(Ls3dCtl), cudaMemcpyDeviceToHost, s));
     MGK_CUDA(cudaStreamSynchronize(s));
     if (hc3.error) {
-      set_error("mgk_ls3d_solve: a bulk copy wait gave up (device timeout)");
+      set_error("mgk_ls3d_solve: a device wait gave up");
       return MGK_TIMEOUT;
     }
     int worst = MGK_OK;

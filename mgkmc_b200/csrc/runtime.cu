@@ -10,6 +10,7 @@
 
 #include "common.cuh"
 #include "fft.cuh"
+#include "fft_reg.cuh"
 
 namespace mgk {
 
@@ -89,6 +90,57 @@ const void* twiddles(int n, int prec) {
     if (cudaMemcpy(d, h.data(), bytes, cudaMemcpyHostToDevice) != cudaSuccess) return nullptr;
   }
   cache[key] = d;
+  return d;
+}
+
+// Step twiddles of the register FFT of length n: for each step s >= 1 the
+// entries W_{NS R}^{r k} at [r - 1][k], k < NS; one table per (device, n,
+// precision), kept until process exit.
+template <typename C> static void fill_reg(int n, std::vector<C>& h) {
+  const RegSched q = reg_sched(n);
+  int ns = q.r[0];
+  for (int s = 1; s < q.ns; ++s) {
+    for (int r = 1; r < q.r[s]; ++r)
+      for (int k = 0; k < ns; ++k) {
+        const long double ang =
+            -2.0L * 3.14159265358979323846264338327950288L * (long double)(r * k) / (long double)(ns * q.r[s]);
+        C c;
+        c.x = (decltype(C::x))cosl(ang);
+        c.y = (decltype(C::x))sinl(ang);
+        h.push_back(c);
+      }
+    ns *= q.r[s];
+  }
+}
+
+template <typename C> static void* upload(const std::vector<C>& h) {
+  void* d = nullptr;
+  if (cudaMalloc(&d, h.size() * sizeof(C)) != cudaSuccess) return nullptr;
+  if (cudaMemcpy(d, h.data(), h.size() * sizeof(C), cudaMemcpyHostToDevice) != cudaSuccess) {
+    cudaFree(d);
+    return nullptr;
+  }
+  return d;
+}
+
+const void* twiddles_reg(int n, int prec) {
+  static std::mutex mu;
+  static std::map<std::tuple<int, int, int>, void*> cache;
+  int dev = 0;
+  if (!reg_len(n) || cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+  std::lock_guard<std::mutex> lock(mu);
+  void*& d = cache[std::make_tuple(dev, n, prec)];
+  if (!d) {
+    if (prec == MGK_FP64) {
+      std::vector<double2> h;
+      fill_reg(n, h);
+      d = upload(h);
+    } else {
+      std::vector<float2> h;
+      fill_reg(n, h);
+      d = upload(h);
+    }
+  }
   return d;
 }
 
