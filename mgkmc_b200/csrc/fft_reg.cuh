@@ -232,11 +232,12 @@ __device__ __forceinline__ void reg_bfly(C* v, int j, const C* __restrict__ tw) 
 //   store(i, v)  the result point i; it may write at(reg_slot<N>(i)) in place
 //   sync()       synchronises the threads that share the line
 // Threads with act == false take part in the synchronisations only.
-// presync: the inputs are read from the exchange buffer itself, so the first
-// exchange has to wait for every thread's reads.
-template <int N, int SIGN, bool PRESYNC, typename C, typename Load, typename At, typename Store, typename Sync>
+//   pre()        called once by every thread between its loads and the first
+//                exchange: inputs that lie in exchange buffers have been read
+//                by the threads it synchronises
+template <int N, int SIGN, typename C, typename Load, typename At, typename Store, typename Sync, typename Pre>
 __device__ __forceinline__ void reg_line(int t, bool act, const C* __restrict__ tw, Load load, At at, Store store,
-                                         Sync sync) {
+                                         Sync sync, Pre pre) {
   constexpr RegSched Q = reg_sched(N);
   constexpr int R0 = Q.r[0], T = Q.t, P0 = reg_p0(N);
   {
@@ -250,7 +251,7 @@ __device__ __forceinline__ void reg_line(int t, bool act, const C* __restrict__ 
         for (int r = 0; r < R0; ++r) v[u][r] = load(j + r * NB);
       }
     }
-    if (PRESYNC) sync();
+    pre();
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int j = t + T * u;

@@ -9,7 +9,7 @@
 //   mu, lam           2 planes
 //   eps[6]            symmetric components xx, yy, zz, yz, xz, xy
 //   ep[6]             eigenstrain, symmetric components
-//   epf[9]            eigenstrain as given (only when given; output stress)
+//   epa[6]            its off-diagonal entries as given (only when given; output)
 //   spec[6]           half spectrum [c][x][y][kz], kz < nz/2+1
 // The antisymmetric part of eps is uniform after the first iteration and is
 // carried as three scalars.
@@ -52,41 +52,97 @@ const Ls3Line* ls3_line(int n, int prec) {
 
 // -------------------------------------------------------------- kernels ---
 
+constexpr int kT3 = 256;
+// per-voxel kernels: at most 4 CTAs per SM (they loop over tiles of kT3)
+constexpr int kG3 = 592;
 
-__global__ void ls3d_material_kernel(const Ls3dRep* reps, int rep, const double* __restrict__ E,
-                                     const double* __restrict__ nu, const double* __restrict__ epsp,
-                                     int set_moduli, double* partials) {
-  __shared__ double red[32];
+
+// Block sums of K values per thread in a fixed order: warp trees, then one
+// warp per value; value q of the block to out[q].
+template <int K> __device__ __forceinline__ void block_sums(const double* v, double* out) {
+  __shared__ double w[kT3 / 32][K];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+  for (int q = 0; q < K; ++q) {
+    const double t = warp_sum(v[q]);
+    if (lane == 0) w[wid][q] = t;
+  }
+  __syncthreads();
+  if (threadIdx.x < K) {
+    double t = 0;
+#pragma unroll
+    for (int k = 0; k < kT3 / 32; ++k) t += w[k][threadIdx.x];
+    out[threadIdx.x] = t;
+  }
+}
+
+// kT3 voxels' 3x3 tensors between the caller's interleaved layout and one
+// thread per voxel, through shared memory: the warp's accesses are contiguous
+// (a thread's own nine doubles would be 72 bytes apart from its neighbour's).
+// m: voxels in this tile.
+__device__ __forceinline__ void tile_load9(const double* __restrict__ src, int m, double* buf, double* v) {
+  __syncthreads();
+  for (int i = threadIdx.x; i < 9 * m; i += kT3) buf[i] = __ldcs(src + i);
+  __syncthreads();
+  if ((int)threadIdx.x < m)
+#pragma unroll
+    for (int q = 0; q < 9; ++q) v[q] = buf[9 * threadIdx.x + q];
+}
+__device__ __forceinline__ void tile_store9(double* __restrict__ dst, int m, double* buf, const double* v) {
+  __syncthreads();
+  if ((int)threadIdx.x < m)
+#pragma unroll
+    for (int q = 0; q < 9; ++q) buf[9 * threadIdx.x + q] = v[q];
+  __syncthreads();
+  for (int i = threadIdx.x; i < 9 * m; i += kT3) __stcs(dst + i, buf[i]);
+}
+
+// Moduli and eigenstrain planes of one replica, per-CTA partial sums of the
+// two moduli inputs.  HBM-bound: 25 planes per voxel with an eigenstrain.
+__global__ void __launch_bounds__(kT3, 3) ls3d_material_kernel(const Ls3dRep* reps, int rep,
+                                                               const double* __restrict__ E,
+                                                               const double* __restrict__ nu,
+                                                               const double* __restrict__ epsp, int set_moduli,
+                                                               double* partials) {
+  __shared__ double buf[9 * kT3];
   const Ls3dRep& R = reps[rep];
   const long long N = R.N;
-  double sE = 0, sn = 0;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N;
-       i += (long long)gridDim.x * blockDim.x) {
+  double sm[2] = {0, 0};
+  for (long long i0 = blockIdx.x * (long long)kT3; i0 < N; i0 += (long long)gridDim.x * kT3) {
+    const int m = (int)min((long long)kT3, N - i0);
+    const long long i = i0 + threadIdx.x;
+    const bool in = (int)threadIdx.x < m;
+    double p[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    double e = 0, v = 0;
+    if (set_moduli && in) { e = E[i]; v = nu[i]; }
+    if (epsp) tile_load9(epsp + 9 * i0, m, buf, p);
+    if (!in) continue;
     if (set_moduli) {
       // elasticity.py:55-59 (set_moduli 1); set_moduli 2: E holds lambda and
       // nu holds mu, as the secant solver takes them
-      const double e = E[i], v = nu[i];
-      R.mu[i] = set_moduli == 2 ? v : e / (2 * (1 + v));
-      R.lam[i] = set_moduli == 2 ? e : e * v / ((1 + v) * (1 - 2 * v));
-      if (R.mu32) { R.mu32[i] = (float)R.mu[i]; R.lam32[i] = (float)R.lam[i]; }
-      sE += e;
-      sn += v;
+      const double mu = set_moduli == 2 ? v : e / (2 * (1 + v));
+      const double lam = set_moduli == 2 ? e : e * v / ((1 + v) * (1 - 2 * v));
+      R.mu[i] = mu;
+      R.lam[i] = lam;
+      if (R.mu32) { R.mu32[i] = (float)mu; R.lam32[i] = (float)lam; }
+      sm[0] += e;
+      sm[1] += v;
     }
-    double p[9];
-    for (int q = 0; q < 9; ++q) p[q] = epsp ? epsp[9 * i + q] : 0.0;
+#pragma unroll
     for (int c = 0; c < 6; ++c) {
-      const int a = 3 * kSymI[c] + kSymJ[c], b = 3 * kSymJ[c] + kSymI[c];
-      R.ep[c * N + i] = (p[a] == p[b]) ? p[a] : 0.5 * (p[a] + p[b]);
-      if (R.ep32) R.ep32[c * N + i] = (float)R.ep[c * N + i];
+      constexpr int kI[6] = {0, 1, 2, 1, 0, 0}, kJ[6] = {0, 1, 2, 2, 2, 1};
+      const int a = 3 * kI[c] + kJ[c], b = 3 * kJ[c] + kI[c];
+      const double sy = (p[a] == p[b]) ? p[a] : 0.5 * (p[a] + p[b]);
+      R.ep[c * N + i] = sy;
+      if (R.ep32) R.ep32[c * N + i] = (float)sy;
+      // the off-diagonal entries as given (the output stress uses them)
+      if (c >= 3 && R.epa) {
+        R.epa[(c - 3) * N + i] = p[a];
+        R.epa[c * N + i] = p[b];
+      }
     }
-    if (R.epf)
-      for (int q = 0; q < 9; ++q) R.epf[q * N + i] = p[q];
   }
-  if (set_moduli) {
-    double a = block_sum(sE, red);
-    double b = block_sum(sn, red);
-    if (threadIdx.x == 0) { partials[2 * blockIdx.x] = a; partials[2 * blockIdx.x + 1] = b; }
-  }
+  if (set_moduli) block_sums<2>(sm, partials + 2 * blockIdx.x);
 }
 
 // reference medium from the means of E and nu (linear_elastic_simulator.py:
@@ -112,40 +168,39 @@ __global__ void ls3d_medium_kernel(const Ls3dRep* reps, Ls3dState* st, int rep, 
 }
 
 // per-CTA partials of the 9 components of the warm-start field; grid (G, nsel)
-__global__ void ls3d_means_kernel(const Ls3dRep* reps, const int* sel, double* partials) {
-  __shared__ double red[32];
+__global__ void __launch_bounds__(kT3, 4) ls3d_means_kernel(const Ls3dRep* reps, const int* sel, double* partials) {
+  __shared__ double buf[9 * kT3];
   const Ls3dRep& R = reps[sel[blockIdx.y]];
   if (!R.init) return;
   double s[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < R.N;
-       i += (long long)gridDim.x * blockDim.x)
-    for (int q = 0; q < 9; ++q) s[q] += R.init[9 * i + q];
-  for (int q = 0; q < 9; ++q) {
-    double t = block_sum(s[q], red);
-    if (threadIdx.x == 0) partials[((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 18 + q] = t;
+  for (long long i0 = blockIdx.x * (long long)kT3; i0 < R.N; i0 += (long long)gridDim.x * kT3) {
+    double v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    tile_load9(R.init + 9 * i0, (int)min((long long)kT3, R.N - i0), buf, v);
+#pragma unroll
+    for (int q = 0; q < 9; ++q) s[q] += v[q];
   }
+  block_sums<9>(s, partials + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 18);
 }
 
-// fixed-order sums (stride 18 per CTA slot); mode 0: means of every replica,
-// 1: means for warm-started replicas, 2: plain sums for warm-started replicas
+// fixed-order sums (stride 18 per CTA slot), one warp per value; mode 0:
+// means of every replica, 1: means for warm-started replicas, 2: plain sums
+// for warm-started replicas
 __global__ void ls3d_finalize_kernel(const Ls3dRep* reps, Ls3dState* st, const int* sel, const double* partials,
-                                     int G, int K, int off, int mode) {
-  __shared__ double red[32];
-  const int r = sel[blockIdx.x];
+                                     int G, int off, int mode) {
+  const int r = sel[blockIdx.x], q = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (mode && !reps[r].init) return;
-  const double scale = mode == 2 ? 1.0 : 1.0 / (double)reps[r].N;
   double* out = reinterpret_cast<double*>(reinterpret_cast<char*>(&st[r]) + off);
-  for (int q = 0; q < K; ++q) {
-    double a = 0;
-    for (int i = threadIdx.x; i < G; i += blockDim.x) a += partials[((size_t)blockIdx.x * G + i) * 18 + q];
-    a = block_sum(a, red);
-    if (threadIdx.x == 0) out[q] = a * scale;
-  }
+  double a = 0;
+#pragma unroll 4
+  for (int i = lane; i < G; i += 32) a += partials[((size_t)blockIdx.x * G + i) * 18 + q];
+  a = warp_sum(a);
+  if (lane == 0) out[q] = a * (mode == 2 ? 1.0 : 1.0 / (double)reps[r].N);
 }
 
 // initial field (linear_elastic_simulator.py:302-313); grid (G, nsel)
-__global__ void ls3d_begin_kernel(const Ls3dRep* reps, Ls3dState* st, const int* sel, double* partials) {
-  __shared__ double red[32];
+__global__ void __launch_bounds__(kT3, 3) ls3d_begin_kernel(const Ls3dRep* reps, Ls3dState* st, const int* sel,
+                                                            double* partials) {
+  __shared__ double buf[9 * kT3];
   const int r = sel[blockIdx.y];
   const Ls3dRep& R = reps[r];
   Ls3dState& S = st[r];
@@ -157,37 +212,39 @@ __global__ void ls3d_begin_kernel(const Ls3dRep* reps, Ls3dState* st, const int*
     const int a = 3 * kSymI[c] + kSymJ[c], b = 3 * kSymJ[c] + kSymI[c];
     sb[c] = (eb[a] == eb[b]) ? eb[a] : 0.5 * (eb[a] + eb[b]);
   }
-  double d2 = 0, n2 = 0;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N;
-       i += (long long)gridDim.x * blockDim.x) {
+  double dn[2] = {0, 0};
+  for (long long i0 = blockIdx.x * (long long)kT3; i0 < N; i0 += (long long)gridDim.x * kT3) {
+    const int m = (int)min((long long)kT3, N - i0);
+    const long long i = i0 + threadIdx.x;
     if (R.init) {
       double v[9];
-      for (int q = 0; q < 9; ++q) v[q] = R.init[9 * i + q] + (eb[q] - S.means[q]);
+      tile_load9(R.init + 9 * i0, m, buf, v);
+      if ((int)threadIdx.x >= m) continue;
+#pragma unroll
+      for (int q = 0; q < 9; ++q) v[q] += eb[q] - S.means[q];
+#pragma unroll
       for (int c = 0; c < 6; ++c) {
-        const int a = 3 * kSymI[c] + kSymJ[c], b = 3 * kSymJ[c] + kSymI[c];
-        R.eps[c * N + i] = (v[a] == v[b]) ? v[a] : 0.5 * (v[a] + v[b]);
-        if (R.eps32) R.eps32[c * N + i] = (float)R.eps[c * N + i];
+        constexpr int kI[6] = {0, 1, 2, 1, 0, 0}, kJ[6] = {0, 1, 2, 2, 2, 1};
+        const int a = 3 * kI[c] + kJ[c], b = 3 * kJ[c] + kI[c];
+        const double sy = (v[a] == v[b]) ? v[a] : 0.5 * (v[a] + v[b]);
+        R.eps[c * N + i] = sy;
+        if (R.eps32) R.eps32[c * N + i] = (float)sy;
       }
       const double a0[3] = {0.5 * (v[1] - v[3]), 0.5 * (v[2] - v[6]), 0.5 * (v[5] - v[7])};
+#pragma unroll
       for (int q = 0; q < 3; ++q) {
-        d2 += 2 * (ab[q] - a0[q]) * (ab[q] - a0[q]);
-        n2 += 2 * a0[q] * a0[q];
+        dn[0] += 2 * (ab[q] - a0[q]) * (ab[q] - a0[q]);
+        dn[1] += 2 * a0[q] * a0[q];
       }
-    } else {
+    } else if ((int)threadIdx.x < m) {
+#pragma unroll
       for (int c = 0; c < 6; ++c) {
         R.eps[c * N + i] = sb[c];
         if (R.eps32) R.eps32[c * N + i] = (float)sb[c];
       }
     }
   }
-  if (R.init) {
-    d2 = block_sum(d2, red);
-    n2 = block_sum(n2, red);
-    if (threadIdx.x == 0) {
-      partials[((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 18 + 0] = d2;
-      partials[((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 18 + 1] = n2;
-    }
-  }
+  if (R.init) block_sums<2>(dn, partials + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 18);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     for (int c = 0; c < 6; ++c) S.ebar[c] = sb[c];
     for (int q = 0; q < 3; ++q) S.abar[q] = ab[q];
@@ -430,38 +487,47 @@ __global__ void ls3d_phase2_kernel(Ls3dState* st, const int* sel, int nsel, Ls3d
 }
 
 // outputs (nx,ny,nz,3,3) and partial sums for the means; grid (G, nsel)
+// Stores through shared memory (tile_store9): written one double per
+// thread at a time the 18 output planes' sectors are touched four times each,
+// and the pass took 239 us at 128^3 with 256 CTAs; 96 us so (705 MB).
 template <int LAW = 0>  // 1: the secant law, 3: the Landau law
-__global__ void ls3d_output_kernel(const Ls3dRep* reps, const Ls3dState* st, const int* sel, double* partials) {
-  __shared__ double red[32];
+__global__ void __launch_bounds__(kT3, 2) ls3d_output_kernel(const Ls3dRep* reps, const Ls3dState* st, const int* sel,
+                                                             double* partials) {
+  __shared__ double buf[9 * kT3];
   const int r = sel[blockIdx.y];
   const Ls3dRep& R = reps[r];
   const Ls3dState& S = st[r];
   const long long N = R.N;
+  const double ab[3] = {S.abar[0], S.abar[1], S.abar[2]};
   double s[18];
+#pragma unroll
   for (int q = 0; q < 18; ++q) s[q] = 0;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N;
-       i += (long long)gridDim.x * blockDim.x) {
+  for (long long i0 = blockIdx.x * (long long)kT3; i0 < N; i0 += (long long)gridDim.x * kT3) {
+    const int m = (int)min((long long)kT3, N - i0);
+    const long long i = i0 + min((int)threadIdx.x, m - 1);  // idle threads of the last tile repeat its last voxel
     double e[9], p[9];
     const double sxx = R.eps[i], syy = R.eps[N + i], szz = R.eps[2 * N + i];
     const double syz = R.eps[3 * N + i], sxz = R.eps[4 * N + i], sxy = R.eps[5 * N + i];
-    e[0] = sxx; e[4] = syy; e[8] = szz;
-    e[1] = S.abar[0] == 0 ? sxy : sxy + S.abar[0];
-    e[3] = S.abar[0] == 0 ? sxy : sxy - S.abar[0];
-    e[2] = S.abar[1] == 0 ? sxz : sxz + S.abar[1];
-    e[6] = S.abar[1] == 0 ? sxz : sxz - S.abar[1];
-    e[5] = S.abar[2] == 0 ? syz : syz + S.abar[2];
-    e[7] = S.abar[2] == 0 ? syz : syz - S.abar[2];
-    if (R.epf) {
-      for (int q = 0; q < 9; ++q) p[q] = R.epf[q * N + i];
+    p[0] = R.ep[i]; p[4] = R.ep[N + i]; p[8] = R.ep[2 * N + i];
+    if (R.epa) {
+      p[5] = R.epa[i]; p[2] = R.epa[N + i]; p[1] = R.epa[2 * N + i];
+      p[7] = R.epa[3 * N + i]; p[6] = R.epa[4 * N + i]; p[3] = R.epa[5 * N + i];
     } else {
-      p[0] = R.ep[i]; p[4] = R.ep[N + i]; p[8] = R.ep[2 * N + i];
       p[5] = p[7] = R.ep[3 * N + i];
       p[2] = p[6] = R.ep[4 * N + i];
       p[1] = p[3] = R.ep[5 * N + i];
     }
     double mu = R.mu[i];
     const double lam = R.lam[i];
+    e[0] = sxx; e[4] = syy; e[8] = szz;
+    e[1] = ab[0] == 0 ? sxy : sxy + ab[0];
+    e[3] = ab[0] == 0 ? sxy : sxy - ab[0];
+    e[2] = ab[1] == 0 ? sxz : sxz + ab[1];
+    e[6] = ab[1] == 0 ? sxz : sxz - ab[1];
+    e[5] = ab[2] == 0 ? syz : syz + ab[2];
+    e[7] = ab[2] == 0 ? syz : syz - ab[2];
     double d[9];
+#pragma unroll
     for (int q = 0; q < 9; ++q) d[q] = e[q] - p[q];
     if constexpr (LAW == 1)
       mu = secant_mu3(mu, d[0], d[4], d[8], 0.5 * (d[5] + d[7]), 0.5 * (d[2] + d[6]), 0.5 * (d[1] + d[3]),
@@ -478,19 +544,20 @@ __global__ void ls3d_output_kernel(const Ls3dRep* reps, const Ls3dState* st, con
       sg[2] = sg[6] = s6[4];
       sg[1] = sg[3] = s6[5];
     } else {
+#pragma unroll
       for (int q = 0; q < 9; ++q) sg[q] = 2 * mu * d[q] + ((q % 4) == 0 ? lam * tr : 0.0);
     }
-    for (int q = 0; q < 9; ++q) {
-      if (R.out_eps) R.out_eps[9 * i + q] = e[q];
-      if (R.out_sig) R.out_sig[9 * i + q] = sg[q];
-      s[q] += e[q];
-      s[9 + q] += sg[q];
+    if (R.out_eps) tile_store9(R.out_eps + 9 * i0, m, buf, e);
+    if (R.out_sig) tile_store9(R.out_sig + 9 * i0, m, buf, sg);
+    if ((int)threadIdx.x < m) {
+#pragma unroll
+      for (int q = 0; q < 9; ++q) {
+        s[q] += e[q];
+        s[9 + q] += sg[q];
+      }
     }
   }
-  for (int q = 0; q < 18; ++q) {
-    double t = block_sum(s[q], red);
-    if (threadIdx.x == 0) partials[((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 18 + q] = t;
-  }
+  block_sums<18>(s, partials + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 18);
 }
 
 }  // namespace mgk
@@ -499,8 +566,6 @@ __global__ void ls3d_output_kernel(const Ls3dRep* reps, const Ls3dState* st, con
 using namespace mgk;
 
 namespace {
-constexpr int kT3 = 256;
-constexpr int kG3 = 256;
 int g3(long long N) {
   long long b = (N + kT3 - 1) / kT3;
   return (int)std::max(1LL, std::min((long long)kG3, b));
@@ -655,7 +720,7 @@ extern "C" int mgk_ls3d_create_batch(int nrep, const int* nxs, const int* nys, c
       p->mixed_ok = p->mixed_ok && (n == 64 || n == 96 || n == 128);
     }
     p->line[r] = line;
-    R.ld = line ? (R.nzh + 3) / 4 * 4 : R.nzh;  // register-FFT tiles read rows of 64 aligned bytes
+    R.ld = line ? ls3_ld(R.nz) : R.nzh;  // register-FFT tiles read rows of 64 aligned bytes
     R.N = (long long)R.nx * R.ny * R.nz;
     R.tc = tc3(std::max(R.nx, R.ny));
     const int ntile = (R.nzh + R.tc - 1) / R.tc;
@@ -679,10 +744,10 @@ extern "C" int mgk_ls3d_create_batch(int nrep, const int* nxs, const int* nys, c
     p->maxN = std::max(p->maxN, R.N);
     p->tot_zl += R.zl_items; p->tot_y += R.y_items; p->tot_x += R.x_items;
     void* f = nullptr;
-    int st = a3(p, &f, sizeof(double) * R.N * 23);
+    int st = a3(p, &f, sizeof(double) * R.N * 20);
     if (st) return fail(st);
     double* d = reinterpret_cast<double*>(f);
-    R.mu = d; R.lam = d + R.N; R.eps = d + 2 * R.N; R.ep = d + 8 * R.N; R.epf = nullptr;
+    R.mu = d; R.lam = d + R.N; R.eps = d + 2 * R.N; R.ep = d + 8 * R.N; R.epa = nullptr;
     void* sp = nullptr;
     st = a3(p, &sp, 6 * (size_t)R.nx * R.ny * R.ld * sizeof(double2));
     if (st) return fail(st);
@@ -744,8 +809,8 @@ static int set3(mgk_ls3d_t p, int rep, const double* E, const double* nu, const 
                 cudaStream_t s) {
   Ls3dRep& R = p->reps[rep];
   const bool want = epsp != nullptr;
-  if (want != (R.epf != nullptr)) {
-    R.epf = want ? R.mu + 14 * R.N : nullptr;
+  if (want != (R.epa != nullptr)) {
+    R.epa = want ? R.mu + 14 * R.N : nullptr;
     int st = wait3(p);
     if (st) return st;
     p->h_reps[rep] = R;
@@ -1082,14 +1147,14 @@ extern "C" int mgk_ls3d_solve_batch(mgk_ls3d_t p, int nsel, const int* sel, cons
   for (int q = 0; q < nsel && eps_init; ++q) any_init |= eps_init[q] != nullptr;
   if (any_init) {
     ls3d_means_kernel<<<dim3(G, nsel), kT3, 0, s>>>(p->d_reps, d_sel, p->d_part);
-    ls3d_finalize_kernel<<<nsel, kT3, 0, s>>>(p->d_reps, p->d_st, d_sel, p->d_part, G, 9,
+    ls3d_finalize_kernel<<<nsel, 32 * 9, 0, s>>>(p->d_reps, p->d_st, d_sel, p->d_part, G,
                                               (int)offsetof(Ls3dState, means), 1);
     MGK_CUDA(cudaGetLastError());
   }
   ls3d_begin_kernel<<<dim3(G, nsel), kT3, 0, s>>>(p->d_reps, p->d_st, d_sel, p->d_part);
   MGK_CUDA(cudaGetLastError());
   if (any_init) {
-    ls3d_finalize_kernel<<<nsel, kT3, 0, s>>>(p->d_reps, p->d_st, d_sel, p->d_part, G, 2,
+    ls3d_finalize_kernel<<<nsel, 32 * 2, 0, s>>>(p->d_reps, p->d_st, d_sel, p->d_part, G,
                                               (int)offsetof(Ls3dState, extra_d0), 2);
     MGK_CUDA(cudaGetLastError());
   }
@@ -1146,7 +1211,7 @@ extern "C" int mgk_ls3d_solve_batch(mgk_ls3d_t p, int nsel, const int* sel, cons
   else
     ls3d_output_kernel<0><<<dim3(G, nsel), kT3, 0, s>>>(p->d_reps, p->d_st, d_sel, p->d_part);
   MGK_CUDA(cudaGetLastError());
-  ls3d_finalize_kernel<<<nsel, kT3, 0, s>>>(p->d_reps, p->d_st, d_sel, p->d_part, G, 18,
+  ls3d_finalize_kernel<<<nsel, 32 * 18, 0, s>>>(p->d_reps, p->d_st, d_sel, p->d_part, G,
                                             (int)offsetof(Ls3dState, out_eps_mean), 0);
   MGK_CUDA(cudaGetLastError());
   if (infos) {

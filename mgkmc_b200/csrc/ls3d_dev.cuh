@@ -20,7 +20,7 @@ struct Ls3dRep {
   double* lam;
   double* eps;   // 6 planes
   double* ep;    // 6 planes
-  double* epf;   // 9 planes or null
+  double* epa;   // eps_p yz, xz, xy, zy, zx, yx as given (6 planes) or null
   double2* spec;
   // mixed-precision plans (warp-line kernels only): FP32 copies and tables;
   // the FP32 spectrum reuses `spec`

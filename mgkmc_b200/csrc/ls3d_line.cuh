@@ -14,9 +14,11 @@
 // steps, two shared-memory accesses per point and step, strided twiddles) ran
 // at 60 % of the L1 rate and 0.25 .. 0.4 of HBM with 12 .. 15 warps per SM.  Here
 // a point crosses shared memory once per transform (twice more around Gamma0),
-// a thread has 8 .. 16 independent global loads in flight, and the fields of a
-// line pair are asked into L2 while the spectrum is inverted.
-// @@FIG@@
+// a thread has 8 .. 16 independent loads in flight, the spectrum rows of the
+// z-lines come by bulk copies, and their fields are asked into L2 while the
+// spectrum is inverted.  FP64 at 128^3, before and now: z-lines 197 and 130 us
+// (540 MB: 0.63 of the measured copy rate), x pass 113 and 70 us, y pass 71 and
+// 42 us (204 MB each: 0.45 and 0.74).
 #pragma once
 #include "fft_reg.cuh"
 #include "ls3d_dev.cuh"
@@ -26,16 +28,31 @@ namespace mgk {
 
 // ------------------------------------------------------------ geometry ---
 constexpr int round32(int n) { return (n + 31) / 32 * 32; }
-// line pairs per z-line CTA: about 96 .. 160 threads
-constexpr int ls3_zp(int n) { return reg_sched(n).t <= 12 ? 2 : 1; }
-constexpr int ls3_z_threads(int n) { return round32(6 * reg_sched(n).t * ls3_zp(n)); }
+// Line pairs per z-line CTA, and its threads: those of the transforms, and
+// enough for the voxel stage to run in one round of at most 192 voxel pairs or
+// two equal ones (at 128 points 96 threads would take three rounds).
+constexpr int ls3_zp(int n) { return reg_sched(n).t <= 9 ? 2 : 1; }
+constexpr int ls3_z_threads(int n) {
+  const int fft = 6 * reg_sched(n).t * ls3_zp(n), vox = ls3_zp(n) * n, rounds = (vox + 191) / 192;
+  const int per = (vox + rounds - 1) / rounds;
+  return round32(fft > per ? fft : per);
+}
+// row pitch of the half spectra (see mgk_ls3d_create_batch)
+constexpr int ls3_ld(int n) { return (n / 2 + 1 + 3) / 4 * 4; }
 // kz columns per tile: rows of 64 bytes (whole 32-byte sectors, spectra rows
-// start on 64-byte boundaries), fewer where a CTA would pass 432 threads
+// start on 64-byte boundaries), fewer where a CTA would pass 432 threads.  The
+// x pass spends its time in the load-store pipe (58 % of its rate at 128^3,
+// half of it the exchanges and Gamma0): tiles of 2 columns (79 us) and a third
+// resident CTA at 96 registers (77 us) were slower than this (70 us).
 constexpr int ls3_tile(int n, int csz) {
   return csz == 8 ? 8 : 6 * 4 * reg_sched(n).t <= 432 ? 4 : 2;
 }
 constexpr int ls3_ax_threads(int n, int csz, int nc) { return round32(nc * ls3_tile(n, csz) * reg_sched(n).t); }
-constexpr int ls3_z_bytes(int n, int csz) { return ls3_zp(n) * 6 * reg_slots(n) * csz; }
+// exchange buffers; they first hold the pairs' spectrum rows as copied
+constexpr int ls3_z_bytes(int n, int csz) {
+  const int a = ls3_zp(n) * 6 * reg_slots(n), b = ls3_zp(n) * 12 * ls3_ld(n);
+  return (a > b ? a : b) * csz;
+}
 constexpr int ls3_ax_bytes(int n, int csz, int nc) { return nc * ls3_tile(n, csz) * reg_slots(n) * csz; }
 // resident CTAs asked of the register allocator: 128 registers per thread in
 // FP64, 80 in FP32
@@ -83,6 +100,7 @@ __global__ void __launch_bounds__(ls3_z_threads(NZ), ls3_minb(ls3_z_threads(NZ),
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double red[32];
   __shared__ int s_last;
+  __shared__ __align__(8) uint64_t bar;
   const int per = reps[sel[0]].zl_items;
   const int r = sel[blockIdx.x / per], loc = blockIdx.x % per;
   const Ls3dRep& R = reps[r];
@@ -91,7 +109,7 @@ __global__ void __launch_bounds__(ls3_z_threads(NZ), ls3_minb(ls3_z_threads(NZ),
     // a body with no active replica has no decider: stop here; the body
     // count bounds the loop whatever happens to the deciders
     const unsigned int b = atomicAdd(&ctl->bodies, 1u) + 1u;
-    if (ctl->n_active == 0 || b > (unsigned int)guard_cap) {
+    if (ctl->n_active == 0 || b > (unsigned int)guard_cap || *(volatile int*)&ctl->error != 0) {
       ctl->any = 0;
       cudaGraphSetConditional(cond, 0u);
     }
@@ -104,12 +122,22 @@ __global__ void __launch_bounds__(ls3_z_threads(NZ), ls3_minb(ls3_z_threads(NZ),
   const int np = (int)min((long long)P, (long long)R.nx * R.ny / 2 - p0);
   T* eps = L3F<T>::eps(R);
   const T *mu = L3F<T>::mu(R), *lam = L3F<T>::lam(R), *ep = L3F<T>::ep(R);
-  if (threadIdx.x < 14) {
-    const int q = threadIdx.x;
+  C* lines = reinterpret_cast<C*>(smem_raw);
+  if (!first && threadIdx.x == 0) {
+    // the pairs' half-spectrum rows, contiguous per component
+    const uint32_t bytes = 2u * np * ld * sizeof(C);
+    mbar_init(&bar, 1);
+    fence_mbar_init();
+    mbar_arrive_expect_tx(&bar, 6u * bytes);
+#pragma unroll
+    for (int q = 0; q < 6; ++q)
+      bulk_g2s(lines + q * 2 * P * ld, L3F<T>::spec(R) + q * plane + 2 * p0 * ld, bytes, &bar);
+  }
+  if (threadIdx.x >= 32 && threadIdx.x < 46) {
+    const int q = threadIdx.x - 32;
     const T* f = q < 6 ? eps + q * N : q == 6 ? mu : q == 7 ? lam : ep + (q - 8) * N;
     l2_prefetch(f + 2 * p0 * NZ, (uint32_t)(2 * np * NZ * sizeof(T)));
   }
-  C* lines = reinterpret_cast<C*>(smem_raw);
   const C* tw = L3F<T>::tw(R, 2);
   const int line = threadIdx.x / TL, t = threadIdx.x % TL;  // line = 6 pair + component
   const int pr = line / 6, c = line - 6 * pr;
@@ -123,13 +151,19 @@ __global__ void __launch_bounds__(ls3_z_threads(NZ), ls3_minb(ls3_z_threads(NZ),
     else __syncthreads();
   };
   if (!first) {
+    __syncthreads();  // the barrier is initialised
+    if (!__syncthreads_and(mbar_wait(&bar, 0) ? 1 : 0)) {
+      if (threadIdx.x == 0) { ctl->error = 1; ctl->any = 0; }
+      return;
+    }
+    const C* sa = lines + (c * P + pr) * 2 * ld;
     auto load = [&](int k) -> C {
       const int ks = 2 * k <= NZ ? k : NZ - k;
-      C a = ra[ks], b = ra[ld + ks];
+      C a = sa[ks], b = sa[ld + ks];
       if (k == 0 || 2 * k == NZ) { a.y = 0; b.y = 0; }
       return 2 * k <= NZ ? mk<C>(a.x - b.y, a.y + b.x) : mk<C>(a.x + b.y, b.x - a.y);
     };
-    reg_line<NZ, +1, false, C>(t, act, tw, load, at, put, sync);
+    reg_line<NZ, +1, C>(t, act, tw, load, at, put, sync, [] { __syncthreads(); });
   }
   __syncthreads();
   const double mu0 = S.mu0, lam0 = S.lam0;
@@ -193,7 +227,7 @@ __global__ void __launch_bounds__(ls3_z_threads(NZ), ls3_minb(ls3_z_threads(NZ),
     for (int k = 0; k < 6; ++k) vx[k * SL] = mk<C>(tr[0][k], tr[1][k]);
   }
   __syncthreads();
-  reg_line<NZ, -1, true, C>(t, act, tw, [&](int i) -> C { return buf[reg_slot<NZ>(i)]; }, at, put, sync);
+  reg_line<NZ, -1, C>(t, act, tw, [&](int i) -> C { return buf[reg_slot<NZ>(i)]; }, at, put, sync, sync);
   sync();
   if (act) {
     for (int k = t; k < NZH; k += TL) {
@@ -249,10 +283,10 @@ __global__ void __launch_bounds__(ls3_ax_threads(NL, 2 * (int)sizeof(T), AXIS ? 
   };
   auto load = [&](int i) -> C { return g[i * js]; };
   if constexpr (AXIS) {
-    reg_line<NL, SIGN, false, C>(t, act, tw, load, at, [&](int i, C v) { g[i * js] = v; }, sync);
+    reg_line<NL, SIGN, C>(t, act, tw, load, at, [&](int i, C v) { g[i * js] = v; }, sync, [] {});
   } else {
     auto put = [&](int i, C v) { buf[reg_slot<NL>(i) * W] = v; };
-    reg_line<NL, -1, false, C>(t, act, tw, load, at, put, sync);
+    reg_line<NL, -1, C>(t, act, tw, load, at, put, sync, [] {});
     __syncthreads();
     // Gamma0 in the precision of the pass: FP64 iterations in double, the
     // FP32 phase of a mixed plan in float.  With u the wave vector, n = u/|u|
@@ -287,8 +321,8 @@ __global__ void __launch_bounds__(ls3_ax_threads(NL, 2 * (int)sizeof(T), AXIS ? 
       for (int k = 0; k < 6; ++k) p[k * (SL * W)] = ev[k];
     }
     __syncthreads();
-    reg_line<NL, +1, true, C>(t, act, tw, [&](int i) -> C { return buf[reg_slot<NL>(i) * W]; }, at,
-                              [&](int i, C v) { g[i * js] = v; }, sync);
+    reg_line<NL, +1, C>(t, act, tw, [&](int i) -> C { return buf[reg_slot<NL>(i) * W]; }, at,
+                        [&](int i, C v) { g[i * js] = v; }, sync, sync);
   }
 }
 
