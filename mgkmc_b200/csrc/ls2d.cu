@@ -56,338 +56,86 @@
 
 #include "common.cuh"
 #include "fft.cuh"
-#include "tma.cuh"
+#include "ls2d_dev.cuh"
+#include "ls2d_line.cuh"
 
 namespace mgk {
 
 const void* twiddles(int n, int prec);
 
-constexpr int kAaMax = 8;  // deepest Anderson history
-struct Ls2dAA;
-
-struct Ls2dRep {
-  int nx, ny, nyh, ld, tc;
-  int row_items, col_items;
-  long long N;
-  // constitutive law: 0 linear (elasticity.py:12-18); 1 secant degradation
-  // (law_a = d, law_b = k); 2 Rose (law_a = eta, law_b = floor fraction,
-  // law_ps = 1 for plane stress); 3 Landau, law_ps = 1 for plane stress (lp: v1, v2, v3,
-  // g1, g2, g3, g4, capping 0 none / 1 piecewise / 2 smooth, E_cap, tangent
-  // ratio, smooth power)
-  int law, law_ps;
-  double law_a, law_b;
-  double lp[11];
-  FftLen fx64, fy64, fx32, fy32;
-  double* mu;
-  double* lam;
-  double* eps;   // 3 planes
-  double* ep;    // 3 planes
-  double* epa;   // 2 planes or null
-  float* mu32;   // mixed plans only
-  float* lam32;
-  float* eps32;
-  float* ep32;
-  void* spec;    // 3 planes of nx*ld complex (double2, or float2 in FP32 phases)
-  // per call
-  const double* init;
-  double* out_eps;
-  double* out_sig;
-  double* out_e33;  // Landau plane stress: the out-of-plane strain per voxel (set_e33_out; may be null)
-  double eb[4];
-  double tol;
-  int max_iter;
-  int row_first, col_first;  // first work item of this replica in the call's maps
-  // Anderson mixing of this call (null: none): state, the ring's dG slots
-  // and its x (the mix is applied by the first row pass of each iterate and,
-  // when the iteration cap ends the loop, by the output kernel)
-  const Ls2dAA* aa;
-  const double* aa_dG;
-  double* aa_x;
-};
-
-struct Ls2dState {
-  double mu0, lam0, Bc, inv2mu0;
-  double ebar[3];
-  double abar;
-  double extra_d0, extra_n0;
-  int iter;
-  int phase_iter;
-  int done;    // 0 active, 1 finished the current phase, 2 finished
-  int status;
-  double diff;
-  double means[4];  // warm-start means (xx, xy, yx, yy)
-  double out_eps_mean[4];
-  double out_sig_mean[4];
-};
-
-struct Ls2dCtl {
-  unsigned int n_active;  // replicas iterating at the start of the current body
-  unsigned int decided;
-  unsigned int still;
-  unsigned int bodies;    // loop bodies run in the current phase (guard)
-  int any;
-  int error;              // a bounded wait gave up (MGK_TIMEOUT)
-};
-
-struct Ls2dAA {
-  int k;          // valid difference columns, in slots 0 .. k-1
-  int slot_next;  // ring slot of the next column
-  int have_prev;  // a previous (f, g) pair exists
-  int nmix;       // columns of the current mix (0: the plain step)
-  unsigned int ctr;  // blocks of the update kernel done (self-resetting)
-  int pad;
-  double A[kAaMax][kAaMax];  // Gram matrix <dF_i, dF_j>
-  double gamma[kAaMax];
-};
-
-// The Anderson mix x = g - dG gamma of voxel i's three strain planes (g in
-// e), written to the plan's strain planes and the ring's x.
-__device__ __forceinline__ void aa_mix_voxel(const Ls2dRep& R, long long i, int nmix, const double* gam, double* e) {
-  const long long N = R.N, n3 = 3 * N;
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    double sm = 0.0;
-#pragma unroll
-    for (int j = 0; j < kAaMax; ++j)
-      if (j < nmix) sm += gam[j] * R.aa_dG[(size_t)j * n3 + c * N + i];
-    e[c] -= sm;
-    R.eps[c * N + i] = e[c];
-    R.aa_x[c * N + i] = e[c];
-  }
+const Ls2Line* ls2_line_a(int n, int kind);
+const Ls2Line* ls2_line_b(int n, int kind);
+const Ls2Line* ls2_line_c(int n, int kind);
+const Ls2Line* ls2_line_d(int n, int kind);
+const Ls2Line* ls2_line_e(int n, int kind);
+const Ls2Line* ls2_line_f(int n, int kind);
+const Ls2Line* ls2_line_g(int n, int kind);
+const Ls2Line* ls2_line_h(int n, int kind);
+const Ls2Line* ls2_line(int n, int kind) {
+  for (auto f : {ls2_line_a, ls2_line_b, ls2_line_c, ls2_line_d, ls2_line_e, ls2_line_f, ls2_line_g, ls2_line_h})
+    if (const Ls2Line* k = f(n, kind)) return k;
+  return nullptr;
 }
-
-__device__ __forceinline__ int aa_load(const Ls2dRep& R, double* gam) {
-  const int nmix = R.aa->nmix;
-#pragma unroll
-  for (int j = 0; j < kAaMax; ++j) gam[j] = j < nmix ? R.aa->gamma[j] : 0.0;
-  return nmix;
-}
-
-constexpr double kMixedPhase1Tol = 2e-6;
-constexpr int kMixedPhase1Cap = 64;
-
-// --------------------------------------------------------------- helpers ---
-
-// eps~^ = -Gamma0(n) : tau^ for symmetric tau (2D), n a unit vector.
-template <typename C, typename T>
-__device__ __forceinline__ void gamma2d_apply(const C& txx, const C& tyy, const C& txy, T nx, T ny,
-                                              T inv2mu0, T Bc, C& exx, C& eyy, C& exy) {
-  C tnx = mk<C>(txx.x * nx + txy.x * ny, txx.y * nx + txy.y * ny);
-  C tny = mk<C>(txy.x * nx + tyy.x * ny, txy.y * nx + tyy.y * ny);
-  C ntn = mk<C>(tnx.x * nx + tny.x * ny, tnx.y * nx + tny.y * ny);
-  const T a = T(2) * inv2mu0;
-  exx = mk<C>(-(a * nx * tnx.x - Bc * nx * nx * ntn.x), -(a * nx * tnx.y - Bc * nx * nx * ntn.y));
-  eyy = mk<C>(-(a * ny * tny.x - Bc * ny * ny * ntn.x), -(a * ny * tny.y - Bc * ny * ny * ntn.y));
-  exy = mk<C>(-(inv2mu0 * (ny * tnx.x + nx * tny.x) - Bc * nx * ny * ntn.x),
-              -(inv2mu0 * (ny * tnx.y + nx * tny.y) - Bc * nx * ny * ntn.y));
-}
-
-__device__ __forceinline__ int fftfreq(int k, int n) { return (k < (n + 1) / 2) ? k : k - n; }
-
-template <typename TS> struct Fields;
-template <> struct Fields<double> {
-  static __device__ __forceinline__ const double* mu(const Ls2dRep& R) { return R.mu; }
-  static __device__ __forceinline__ const double* lam(const Ls2dRep& R) { return R.lam; }
-  static __device__ __forceinline__ double* eps(const Ls2dRep& R) { return R.eps; }
-  static __device__ __forceinline__ const double* ep(const Ls2dRep& R) { return R.ep; }
-  static __device__ __forceinline__ const FftLen& fx(const Ls2dRep& R) { return R.fx64; }
-  static __device__ __forceinline__ const FftLen& fy(const Ls2dRep& R) { return R.fy64; }
-};
-template <> struct Fields<float> {
-  static __device__ __forceinline__ const float* mu(const Ls2dRep& R) { return R.mu32; }
-  static __device__ __forceinline__ const float* lam(const Ls2dRep& R) { return R.lam32; }
-  static __device__ __forceinline__ float* eps(const Ls2dRep& R) { return R.eps32; }
-  static __device__ __forceinline__ const float* ep(const Ls2dRep& R) { return R.ep32; }
-  static __device__ __forceinline__ const FftLen& fx(const Ls2dRep& R) { return R.fx32; }
-  static __device__ __forceinline__ const FftLen& fy(const Ls2dRep& R) { return R.fy32; }
-};
 
 // -------------------------------------------------------------- kernels ---
 
-// Secant shear modulus mu (1 - d (1 - exp(-k eps_eq))) (elasticity.py:189-214)
-// at the von Mises equivalent strain of the elastic strain (dxx, dyy, sym
-// dxy): sqrt(2/3 eps':eps') with the plane-strain eps'_33 = -(dxx + dyy)/3
-// (elasticity.py:112-150; the two shear entries sum to 2 dxy).
-__device__ __forceinline__ double secant_mu(double m, double dxx, double dyy, double dxy, double d, double k) {
-  const double tr3 = (dxx + dyy) / 3.0;
-  const double a = dxx - tr3, b = dyy - tr3, c = -(dxx + dyy) / 3.0, sh = 2.0 * dxy;
-  const double eq = sqrt((2.0 / 3.0) * (a * a + b * b + c * c + 0.5 * sh * sh));
-  return m * (1.0 - d * (1.0 - exp(-k * eq)));
-}
+constexpr int kThreads = 256;
 
-// Rose secant model (elasticity.py:868-944) at the elastic strain (dxx, dyy,
-// dxy = its [0,1] entry): G = max(mu exp(-eta eq), floor mu), bulk modulus
-// K = lam + 2 mu / 3 kept, lam_eff = K - 2 G / 3; plane stress solves
-// eps_zz by the reference's five fixed-point steps.  Returns the trace
-// (eps_zz included) and sets G and lam_eff.
-__device__ __forceinline__ double rose_moduli(double l, double m, double dxx, double dyy, double dxy, double eta,
-                                              double floor_f, int pstress, double& G, double& lam_eff) {
-  const double K = l + (2.0 / 3.0) * m;
-  double ezz = 0.0;
-  auto eq_of = [&](double zz) {
-    const double tr3 = (dxx + dyy + zz) / 3.0;
-    const double a = dxx - tr3, b = dyy - tr3, c = zz - tr3;
-    return sqrt((2.0 / 3.0) * (a * a + b * b + c * c + 2.0 * dxy * dxy));
-  };
-  auto g_of = [&](double eq) { return fmax(m * exp(-eta * eq), floor_f * m); };
-  if (pstress) {
-    ezz = -l / (l + 2.0 * m) * (dxx + dyy);
-    for (int it = 0; it < 5; ++it) {
-      const double g = g_of(eq_of(ezz));
-      ezz = -((3.0 * K - 2.0 * g) / (3.0 * K + 4.0 * g)) * (dxx + dyy);
-    }
+// Sums over a replica's CTAs of K <= 8 values per thread, in a fixed order:
+// warp trees, the warps, then (in the CTA that arrives last) one warp per
+// value over the CTAs' partials.  part: the replica's gridDim.x slots of 8;
+// ctr: its arrival counter (left at zero).  True in the last CTA only, with
+// the sums in res.  A launch for the last step alone took 4 .. 7 us.
+template <int K>
+__device__ __forceinline__ bool grid_sums(const double* v, double* part, unsigned int* ctr, double* res) {
+  __shared__ double w[kThreads / 32][K];
+  __shared__ int s_last;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+  for (int q = 0; q < K; ++q) {
+    const double t = warp_sum(v[q]);
+    if (lane == 0) w[wid][q] = t;
   }
-  G = g_of(eq_of(ezz));
-  lam_eff = K - (2.0 / 3.0) * G;
-  return dxx + dyy + ezz;
-}
-
-// Landau small-strain stress, plane strain (elasticity.py:487-639 with
-// e33 = 0), parameters lp as in Ls2dRep; a12, a21 the two shear entries of
-// the elastic strain.  With capping on, every voxel's strain goes through the
-// capped form f (a - m) + m, as in the reference.
-// Capped components, invariants and coefficients of the Landau law at the
-// block-diagonal strain (in-plane a, out-of-plane e33)
-// (elasticity.py:527-569).
-struct LandauScal {
-  double c11, c22, c12, c21, c33, w, I1, I2, cI, ce, ce2;
-};
-
-__device__ __forceinline__ LandauScal landau_scal(double mu, double lam, double a11, double a22, double a12,
-                                                  double a21, double e33, const double* __restrict__ lp) {
-  const double v1 = lp[0], v2 = lp[1], v3 = lp[2], g1 = lp[3], g2 = lp[4], g3 = lp[5], g4 = lp[6];
-  const int cap = (int)lp[7];
-  LandauScal s;
-  s.c11 = a11; s.c22 = a22; s.c12 = a12; s.c21 = a21; s.c33 = e33; s.w = 0.0;
-  if (cap) {
-    const double m3 = (a11 + a22 + e33) / 3.0;
-    const double d11 = a11 - m3, d22 = a22 - m3, d33 = e33 - m3;
-    const double Ecap = lp[8];
-    const double Eeq = sqrt(fmax(0.0, (2.0 / 3.0) * (d11 * d11 + d22 * d22 + d33 * d33 + 2.0 * a12 * a21)));
-    double f = 1.0;
-    if (cap == 2) {
-      const double pw = lp[10];
-      if (Eeq > 1e-12) f = (Ecap / Eeq) * pow(tanh(fmin(100.0, pow(Eeq / Ecap, pw))), 1.0 / pw);
-      const double t = tanh(fmin(100.0, pow(Eeq / Ecap, pw)));
-      s.w = t * t;
-    } else if (Eeq > Ecap) {
-      f = Ecap / Eeq;
-      s.w = 1.0;
-    }
-    s.c11 = f * d11 + m3;
-    s.c22 = f * d22 + m3;
-    s.c12 = f * a12;
-    s.c21 = f * a21;
-    s.c33 = f * d33 + m3;
+  __syncthreads();
+  if (threadIdx.x < K) {
+    double t = 0;
+#pragma unroll
+    for (int k = 0; k < kThreads / 32; ++k) t += w[k][threadIdx.x];
+    part[blockIdx.x * 8 + threadIdx.x] = t;
+    __threadfence();
   }
-  const double c11 = s.c11, c22 = s.c22, c33 = s.c33;
-  const double I1 = c11 + c22 + c33;
-  const double cross = s.c12 * s.c21;
-  const double tr2 = c11 * c11 + c22 * c22 + 2.0 * cross;
-  const double I2 = tr2 + c33 * c33;
-  const double t_ip = c11 + c22;
-  const double I3 = t_ip * (tr2 - (c11 * c22 - cross)) + c33 * c33 * c33;
-  s.I1 = I1;
-  s.I2 = I2;
-  s.cI = lam * I1 + 0.5 * v1 * (I1 * I1) + v2 * I2 + (1.0 / 6.0) * g1 * (I1 * I1 * I1) + g2 * I1 * I2 +
-         (4.0 / 3.0) * g3 * I3;
-  s.ce = 2.0 * (mu + v2 * I1 + 0.5 * g2 * (I1 * I1) + g4 * I2);
-  s.ce2 = 4.0 * (v3 + g3 * I1);
-  return s;
-}
-
-// The Landau small-strain stress of a 2D voxel (elasticity.py:487-639).
-// Plane strain: e33 = 0.  Plane stress (ps): e33 from the reference's Newton
-// steps on sigma33 = 0 (:571-616) from the linear guess
-// -lam/(lam + 2 mu) tr a, here until the voxel's step is below 1e-14 (at
-// most 64 steps); the stress is evaluated at the stepped e33.  The
-// reference runs the steps of all voxels together until every step is below
-// 1e-9, evaluates each voxel before its last step and warm-starts the next
-// call from the stepped field, so across its solver's iterations e33
-// converges to the root of sigma33 = 0, which the kernel solves for at
-// every evaluation.  With capping the step's derivative leaves out the
-// capping factor's dependence on e33 and the steps converge linearly, so a
-// single cold solve stopped at 1e-9 would leave ~1e-10 in e33.  e33_out
-// (may be null) receives e33.
-__device__ __forceinline__ void landau_sigma(double mu, double lam, double a11, double a22, double a12, double a21,
-                                             const double* __restrict__ lp, int ps, double& s11, double& s22,
-                                             double& s12, double& s21, double* e33_out = nullptr) {
-  double e33 = 0.0;
-  if (ps) {
-    const double v1 = lp[0], v2 = lp[1], g1 = lp[3], g2 = lp[4], g3 = lp[5], g4 = lp[6];
-    const double Gt = lp[9] * mu;
-    e33 = -lam / (lam + 2.0 * mu) * (a11 + a22);
-#pragma unroll 1
-    for (int it = 0; it < 64; ++it) {
-      const LandauScal t = landau_scal(mu, lam, a11, a22, a12, a21, e33, lp);
-      const double c33 = t.c33, I1 = t.I1, I2 = t.I2;
-      double s33 = t.cI + t.ce * c33 + t.ce2 * (c33 * c33);
-      const double dcI = lam + v1 * I1 + 0.5 * g1 * (I1 * I1) + g2 * I2 + 2.0 * (v2 + g2 * I1) * c33 +
-                         4.0 * g3 * (c33 * c33);
-      const double dce = 2.0 * (v2 + g2 * I1) + 4.0 * g4 * c33;
-      double ds33 = dcI + dce * c33 + t.ce + 4.0 * g3 * (c33 * c33) + 2.0 * t.ce2 * c33;
-      if ((int)lp[7]) {
-        s33 = s33 + 2.0 * Gt * (e33 - c33) * t.w;
-        ds33 = ds33 + 2.0 * Gt * t.w;
-      }
-      const double delta = -s33 / (ds33 + 1e-12);
-      e33 = e33 + delta;
-      if (!(fabs(delta) >= 1e-14)) break;  // also leaves on NaN, which the stress then carries
-    }
-    if (e33_out) *e33_out = e33;
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicInc(ctr, gridDim.x - 1) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return false;
+  __threadfence();
+  if (wid < K) {
+    double a = 0;
+    for (int i = lane; i < (int)gridDim.x; i += 32) a += __ldcg(&part[i * 8 + wid]);
+    a = warp_sum(a);
+    if (lane == 0) res[wid] = a;
   }
-  const LandauScal t = landau_scal(mu, lam, a11, a22, a12, a21, e33, lp);
-  const double cross = t.c12 * t.c21;
-  const double t_ip = t.c11 + t.c22;
-  s11 = t.cI + t.ce * t.c11 + t.ce2 * (t.c11 * t.c11 + cross);
-  s22 = t.cI + t.ce * t.c22 + t.ce2 * (t.c22 * t.c22 + cross);
-  s12 = t.ce * t.c12 + t.ce2 * (t.c12 * t_ip);
-  s21 = t.ce * t.c21 + t.ce2 * (t.c21 * t_ip);
-  if ((int)lp[7]) {
-    const double r = 2.0 * (lp[9] * mu) * t.w;
-    s11 += r * (a11 - t.c11);
-    s22 += r * (a22 - t.c22);
-    s12 += r * (a12 - t.c12);
-    s21 += r * (a21 - t.c21);
-  }
-}
-
-// stress of the elastic strain (dxx, dyy, dxy) under law LAW; m, l the voxel's
-// mu, lambda; LAW 0 is Hooke's law with the reference's operation order
-template <int LAW>
-__device__ __forceinline__ void law_sigma(double m, double l, double dxx, double dyy, double dxy, double a, double b,
-                                          int ps, double& sxx, double& syy, double& sxy,
-                                          const double* __restrict__ lp = nullptr) {
-  if constexpr (LAW == 3) {
-    double syx;
-    landau_sigma(m, l, dxx, dyy, dxy, dxy, lp, ps, sxx, syy, sxy, syx);
-  } else if constexpr (LAW == 2) {
-    double G, le;
-    const double tr = rose_moduli(l, m, dxx, dyy, dxy, a, b, ps, G, le);
-    sxx = le * tr + 2.0 * G * dxx;
-    syy = le * tr + 2.0 * G * dyy;
-    sxy = 2.0 * G * dxy;
-  } else {
-    const double ms = LAW == 1 ? secant_mu(m, dxx, dyy, dxy, a, b) : m;
-    const double trd = dxx + dyy;
-    sxx = 2 * ms * dxx + l * trd;
-    syy = 2 * ms * dyy + l * trd;
-    sxy = 2 * ms * dxy;
-  }
+  __syncthreads();
+  return true;
 }
 
 // Per-voxel material prep for one replica: mu, lambda from (E, nu) as in
 // elasticity.py:3-10 (set_moduli 1), or given directly (set_moduli 2: E holds
 // lambda, nu holds mu, as the secant solver takes them), eigenstrain planes
-// (and FP32 copies for mixed plans), per-CTA partial sums of the two inputs
-// for the reference medium.
-__global__ void ls2d_material_kernel(const Ls2dRep* reps, int rep, const double* __restrict__ E,
-                                     const double* __restrict__ nu, const double* __restrict__ epsp,
-                                     int plane_mode, int set_moduli, double* partials) {
-  __shared__ double red[32];
+// (and FP32 copies for mixed plans), and the reference medium from the means:
+// of E and nu (linear_elastic_simulator.py:22-26), or of lambda and mu (lame_in
+// 1: the secant solver, :679-681; lame_in 2: the Rose solver's (mean lambda,
+// (mean mu + floor mean mu) / 2), :866-869).
+__global__ void __launch_bounds__(kThreads) ls2d_material_kernel(const Ls2dRep* reps, Ls2dState* st, int rep,
+                                                                 const double* __restrict__ E,
+                                                                 const double* __restrict__ nu,
+                                                                 const double* __restrict__ epsp, int plane_mode,
+                                                                 int set_moduli, int lame_in, double floor_f,
+                                                                 double* partials, unsigned int* ctr) {
+  __shared__ double res[2];
   const Ls2dRep& R = reps[rep];
   const long long N = R.N;
-  double sE = 0, sn = 0;
+  double sm[2] = {0, 0};
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N;
        i += (long long)gridDim.x * blockDim.x) {
     if (set_moduli) {
@@ -399,8 +147,8 @@ __global__ void ls2d_material_kernel(const Ls2dRep* reps, int rep, const double*
       R.mu[i] = mu;
       R.lam[i] = lam;
       if (R.mu32) { R.mu32[i] = (float)mu; R.lam32[i] = (float)lam; }
-      sE += e;
-      sn += v;
+      sm[0] += e;
+      sm[1] += v;
     }
     double pxx = 0, pxy = 0, pyx = 0, pyy = 0;
     if (epsp) {
@@ -417,45 +165,23 @@ __global__ void ls2d_material_kernel(const Ls2dRep* reps, int rep, const double*
       R.epa[N + i] = pyx;
     }
   }
-  if (set_moduli) {
-    double a = block_sum(sE, red);
-    double b = block_sum(sn, red);
-    if (threadIdx.x == 0) {
-      partials[2 * blockIdx.x] = a;
-      partials[2 * blockIdx.x + 1] = b;
-    }
-  }
+  if (!set_moduli || !grid_sums<2>(sm, partials, ctr, res) || threadIdx.x != 0) return;
+  const double a = res[0] / (double)N, v = res[1] / (double)N;
+  const double mu0 = lame_in == 2 ? 0.5 * (v + floor_f * v) : lame_in ? v : a / (2 * (1 + v));
+  const double lam0 = lame_in ? a
+                      : plane_mode == MGK_PLANE_STRESS ? a * v / (1 - v * v) : a * v / ((1 + v) * (1 - 2 * v));
+  Ls2dState& S = st[rep];
+  S.mu0 = mu0;
+  S.lam0 = lam0;
+  S.Bc = (lam0 + mu0) / (mu0 * (lam0 + 2 * mu0));
+  S.inv2mu0 = 1.0 / (2 * mu0);
 }
 
-// Reference medium from the means: of E and nu (linear_elastic_simulator.py:
-// 22-26), or of lambda and mu (lame_in 1: the secant solver, :679-681;
-// lame_in 2: the Rose solver's (mean lambda, (mean mu + floor mean mu) / 2),
-// :866-869).
-__global__ void ls2d_medium_kernel(const Ls2dRep* reps, Ls2dState* st, int rep, const double* partials,
-                                   int nblocks, int plane_mode, int lame_in, double floor_f) {
-  __shared__ double red[32];
-  double a = 0, b = 0;
-  for (int i = threadIdx.x; i < nblocks; i += blockDim.x) { a += partials[2 * i]; b += partials[2 * i + 1]; }
-  a = block_sum(a, red);
-  b = block_sum(b, red);
-  if (threadIdx.x == 0) {
-    const double N = (double)reps[rep].N;
-    const double E = a / N, v = b / N;
-    const double mu0 = lame_in == 2 ? 0.5 * (v + floor_f * v) : lame_in ? v : E / (2 * (1 + v));
-    const double lam0 = lame_in ? E
-                        : plane_mode == MGK_PLANE_STRESS ? E * v / (1 - v * v) : E * v / ((1 + v) * (1 - 2 * v));
-    Ls2dState& S = st[rep];
-    S.mu0 = mu0;
-    S.lam0 = lam0;
-    S.Bc = (lam0 + mu0) / (mu0 * (lam0 + 2 * mu0));
-    S.inv2mu0 = 1.0 / (2 * mu0);
-  }
-}
-
-// Warm-start means: per-CTA partials of the 4 components of each selected
-// replica's init field.  grid = (G, nsel).
-__global__ void ls2d_means_kernel(const Ls2dRep* reps, const int* sel, double* partials) {
-  __shared__ double red[32];
+// Warm-start means of the 4 components of each selected replica's init
+// field.  grid = (G, nsel).
+__global__ void __launch_bounds__(kThreads) ls2d_means_kernel(const Ls2dRep* reps, Ls2dState* st, const int* sel,
+                                                              double* partials, unsigned int* ctr) {
+  __shared__ double res[4];
   const int r = sel[blockIdx.y];
   const Ls2dRep& R = reps[r];
   if (!R.init) return;
@@ -466,36 +192,17 @@ __global__ void ls2d_means_kernel(const Ls2dRep* reps, const int* sel, double* p
     const double4 v = reinterpret_cast<const double4*>(R.init)[i];
     s[0] += v.x; s[1] += v.y; s[2] += v.z; s[3] += v.w;
   }
-  for (int q = 0; q < 4; ++q) {
-    double t = block_sum(s[q], red);
-    if (threadIdx.x == 0) partials[((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 8 + q] = t;
-  }
-}
-
-// Fixed-order sums of the per-CTA partials of replica sel[blockIdx.x]: K
-// values at byte offset `off` of its state.  need_init: 0 -> means (scaled
-// by 1/N) for every replica, 1 -> means only for replicas with a warm start,
-// 2 -> plain sums only for replicas with a warm start.
-__global__ void ls2d_finalize_kernel(const Ls2dRep* reps, Ls2dState* st, const int* sel, const double* partials,
-                                     int G, int K, int off, int need_init) {
-  __shared__ double red[32];
-  const int r = sel[blockIdx.x];
-  if (need_init && !reps[r].init) return;
-  const double scale = need_init == 2 ? 1.0 : 1.0 / (double)reps[r].N;
-  double* out = reinterpret_cast<double*>(reinterpret_cast<char*>(&st[r]) + off);
-  for (int q = 0; q < K; ++q) {
-    double a = 0;
-    for (int i = threadIdx.x; i < G; i += blockDim.x) a += partials[((size_t)blockIdx.x * G + i) * 8 + q];
-    a = block_sum(a, red);
-    if (threadIdx.x == 0) out[q] = a * scale;
-  }
+  if (grid_sums<4>(s, partials + (size_t)blockIdx.y * gridDim.x * 8, ctr + r, res) && threadIdx.x < 4)
+    st[r].means[threadIdx.x] = res[threadIdx.x] * (1.0 / (double)N);
 }
 
 // Solve start for each selected replica: eps_bar, caps and the initial field
-// (linear_elastic_simulator.py:32-41), and partial sums of the antisymmetric
-// part's contribution to the first diff and norm.  grid = (G, nsel).
-__global__ void ls2d_begin_kernel(const Ls2dRep* reps, Ls2dState* st, const int* sel, double* partials) {
-  __shared__ double red[32];
+// (linear_elastic_simulator.py:32-41), and the antisymmetric part's
+// contribution to the first diff and norm.  fp32: the loop starts with a mixed
+// plan's FP32 phase, which needs the FP32 field only.  grid = (G, nsel).
+__global__ void __launch_bounds__(kThreads) ls2d_begin_kernel(const Ls2dRep* reps, Ls2dState* st, const int* sel,
+                                                              double* partials, unsigned int* ctr, int fp32) {
+  __shared__ double res[2];
   const int r = sel[blockIdx.y];
   const Ls2dRep& R = reps[r];
   Ls2dState& S = st[r];
@@ -504,7 +211,7 @@ __global__ void ls2d_begin_kernel(const Ls2dRep* reps, Ls2dState* st, const int*
   const double abar = 0.5 * (e01 - e10);
   const double sbar = (e01 == e10) ? e01 : 0.5 * (e01 + e10);
   const double* init = R.init;
-  double d2 = 0, n2 = 0;
+  double dn[2] = {0, 0};
   double m00 = 0, m01 = 0, m10 = 0, m11 = 0;
   if (init) { m00 = S.means[0]; m01 = S.means[1]; m10 = S.means[2]; m11 = S.means[3]; }
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N;
@@ -517,23 +224,21 @@ __global__ void ls2d_begin_kernel(const Ls2dRep* reps, Ls2dState* st, const int*
       yy = v.w + (e11 - m11);
       sy = (xy == yx) ? xy : 0.5 * (xy + yx);
       const double a0 = 0.5 * (xy - yx);
-      d2 += 2 * (abar - a0) * (abar - a0);
-      n2 += 2 * a0 * a0;
+      dn[0] += 2 * (abar - a0) * (abar - a0);
+      dn[1] += 2 * a0 * a0;
     } else {
       xx = e00; yy = e11; sy = sbar;
     }
-    R.eps[i] = xx;
-    R.eps[N + i] = yy;
-    R.eps[2 * N + i] = sy;
+    if (!fp32) {
+      R.eps[i] = xx;
+      R.eps[N + i] = yy;
+      R.eps[2 * N + i] = sy;
+    }
     if (R.eps32) { R.eps32[i] = (float)xx; R.eps32[N + i] = (float)yy; R.eps32[2 * N + i] = (float)sy; }
   }
-  if (init) {
-    d2 = block_sum(d2, red);
-    n2 = block_sum(n2, red);
-    if (threadIdx.x == 0) {
-      partials[((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 8 + 0] = d2;
-      partials[((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 8 + 1] = n2;
-    }
+  if (init && grid_sums<2>(dn, partials + (size_t)blockIdx.y * gridDim.x * 8, ctr + r, res) && threadIdx.x == 0) {
+    S.extra_d0 = res[0];
+    S.extra_n0 = res[1];
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     S.ebar[0] = e00;
@@ -546,53 +251,6 @@ __global__ void ls2d_begin_kernel(const Ls2dRep* reps, Ls2dState* st, const int*
     S.status = MGK_OK;
     S.diff = 0;
     if (!init) { S.extra_d0 = 0; S.extra_n0 = 2.0 * (double)N * abar * abar; }
-  }
-}
-
-// Convergence decision of replica r once the last of its row items has
-// written its partial sums (all threads of the CTA call; thread 0 decides).
-// The last replica to decide sets the graph while-node's condition.
-template <bool FINAL>
-__device__ void ls2d_decide(const Ls2dRep& R, Ls2dState& S, const double* partials, Ls2dCtl* ctl,
-                            cudaGraphConditionalHandle cond, int use_cond, int guard_cap, double* red) {
-  double a = 0, b = 0;
-  for (int i = threadIdx.x; i < R.row_items; i += blockDim.x) {
-    a += __ldcg(&partials[2 * (R.row_first + i)]);
-    b += __ldcg(&partials[2 * (R.row_first + i) + 1]);
-  }
-  a = block_sum(a, red);
-  b = block_sum(b, red);
-  if (threadIdx.x != 0) return;
-  if (S.iter == 0) { a += S.extra_d0; b += S.extra_n0; }
-  else { b += 2.0 * (double)R.N * S.abar * S.abar; }
-  const double diff = sqrt(a) / (sqrt(b) + 1e-20);
-  S.diff = diff;
-  S.iter += 1;
-  S.phase_iter += 1;
-  int keep = 0;
-  if (!isfinite(diff)) { S.done = 2; S.status = MGK_NONFINITE; }
-  else if (FINAL) {
-    if (diff < R.tol) { S.done = 2; S.status = MGK_OK; }
-    else if (S.iter >= R.max_iter) { S.done = 2; S.status = MGK_NOT_CONVERGED; }
-    else keep = 1;
-  } else {
-    const double tol1 = R.tol > kMixedPhase1Tol ? R.tol : kMixedPhase1Tol;
-    if (S.iter >= R.max_iter) { S.done = 2; S.status = diff < R.tol ? MGK_OK : MGK_NOT_CONVERGED; }
-    else if (diff < tol1 || S.phase_iter >= kMixedPhase1Cap) S.done = 1;
-    else keep = 1;
-  }
-  const unsigned int n_act = ctl->n_active;  // stable until every active replica has decided
-  if (keep) atomicAdd(&ctl->still, 1u);
-  __threadfence();
-  const unsigned int d = atomicAdd(&ctl->decided, 1u);
-  if (d == n_act - 1) {
-    __threadfence();
-    const unsigned int still = atomicExch(&ctl->still, 0u);
-    ctl->decided = 0;
-    ctl->n_active = still;
-    const bool go = still > 0 && atomicAdd(&ctl->bodies, 0u) <= (unsigned int)guard_cap && *(volatile int*)&ctl->error == 0;
-    ctl->any = go ? 1 : 0;
-    if (use_cond) cudaGraphSetConditional(cond, go ? 1u : 0u);
   }
 }
 
@@ -681,7 +339,8 @@ __global__ void __launch_bounds__(256) ls2d_row_kernel(const Ls2dRep* __restrict
   C* out = (IN_SPEC && cur == bufA) ? bufB : bufA;
   double gam[kAaMax];
   const int nmix = (!IN_SPEC && sizeof(TS) == 8 && R.aa) ? aa_load(R, gam) : 0;
-  // with Anderson mixing the image's tau is never used (see row_fast_body)
+  // with Anderson mixing the image's tau is never used (the next tau is the
+  // mixed iterate's): the pass stops at the image and its update norm
   const bool img_only = IN_SPEC && sizeof(TS) == 8 && law != 0 && R.aa != nullptr;
   for (int y = threadIdx.x; y < ny; y += blockDim.x) {
     TC tr[2][3];
@@ -750,191 +409,7 @@ __global__ void __launch_bounds__(256) ls2d_row_kernel(const Ls2dRep* __restrict
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  ls2d_decide<FINAL>(R, S, partials, ctl, cond, use_cond, guard_cap, red);
-}
-
-// Persistent row kernel (IN_SPEC iterations) with double-buffered bulk
-// prefetch: each CTA walks the items blockIdx.x, +gridDim.x, ...; while it
-// transforms one row pair, the inputs of its next row pair (two spectrum rows
-// and two rows of eps, mu, lambda, eps_p, all contiguous) stream into the
-// other shared-memory stage through cp.async.bulk.  Requires ny even (16-byte
-// aligned rows).  Stage layout (bytes): spec [3][2][ld] C | eps [3][2][ny] |
-// mu [2][ny] | lam [2][ny] | ep [3][2][ny] (TS).
-template <typename TS, typename TC, bool FINAL>
-__global__ void __launch_bounds__(256, 1) ls2d_row_tma_kernel(const Ls2dRep* __restrict__ reps, Ls2dState* st,
-                                                             const int* __restrict__ row_map,
-                                                             const int* __restrict__ row_local, double* partials,
-                                                             unsigned int* rep_counter, Ls2dCtl* ctl,
-                                                             cudaGraphConditionalHandle cond, int use_cond,
-                                                             int guard_cap, int nitems, int stage_bytes) {
-  using C = C_t<TC>;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ double red[32];
-  __shared__ int s_last;
-  __shared__ __align__(8) uint64_t bars[2];
-  C* bufA = reinterpret_cast<C*>(smem_raw + 2 * (size_t)stage_bytes);
-  if (threadIdx.x == 0) {
-    mbar_init(&bars[0], 1);
-    mbar_init(&bars[1], 1);
-    fence_mbar_init();
-  }
-  if (use_cond && blockIdx.x == 0 && threadIdx.x == 0) {
-    const unsigned int b = atomicAdd(&ctl->bodies, 1u) + 1u;
-    if (ctl->n_active == 0 || b > (unsigned int)guard_cap || *(volatile int*)&ctl->error != 0) {
-      ctl->any = 0;
-      cudaGraphSetConditional(cond, 0u);
-    }
-  }
-  __syncthreads();
-  uint32_t parity[2] = {0u, 0u};
-  // issue the bulk loads of `item` into stage s; returns whether it is active
-  auto issue = [&](int item, int s) -> bool {
-    const int r = row_map[item];
-    if (st[r].done != 0) return false;
-    if (threadIdx.x == 0) {
-      const Ls2dRep& R = reps[r];
-      const int ny = R.ny, ld = R.ld;
-      const long long N = R.N;
-      const long long x0 = 2LL * row_local[item];
-      unsigned char* sb = smem_raw + (size_t)s * stage_bytes;
-      const uint32_t spec_b = 2u * ld * sizeof(C), row_b = 2u * ny * sizeof(TS);
-      // the copy list in stage order; the barrier expects exactly its bytes
-      const void* src[11];
-      uint32_t len[11];
-      int n = 0;
-      const C* spec = reinterpret_cast<const C*>(R.spec);
-      for (int c = 0; c < 3; ++c) { src[n] = spec + ((long long)c * R.nx + x0) * ld; len[n++] = spec_b; }
-      const TS* eps = Fields<TS>::eps(R);
-      const TS* ep = Fields<TS>::ep(R);
-      for (int c = 0; c < 3; ++c) { src[n] = eps + c * N + x0 * ny; len[n++] = row_b; }
-      src[n] = Fields<TS>::mu(R) + x0 * ny; len[n++] = row_b;
-      src[n] = Fields<TS>::lam(R) + x0 * ny; len[n++] = row_b;
-      for (int c = 0; c < 3; ++c) { src[n] = ep + c * N + x0 * ny; len[n++] = row_b; }
-      uint32_t total = 0;
-      for (int q = 0; q < n; ++q) total += len[q];
-      fence_proxy_async_smem();
-      mbar_arrive_expect_tx(&bars[s], total);
-      unsigned char* dst = sb;
-      for (int q = 0; q < n; ++q) { bulk_g2s(dst, src[q], len[q], &bars[s]); dst += len[q]; }
-    }
-    return true;
-  };
-  int item = blockIdx.x;
-  bool act = item < nitems ? issue(item, 0) : false;
-  for (int k = 0; item < nitems; item += gridDim.x, ++k) {
-    const int s = k & 1;
-    const int next = item + gridDim.x;
-    const bool act_next = next < nitems ? issue(next, s ^ 1) : false;
-    if (act) {
-      const bool ok = __syncthreads_and(mbar_wait(&bars[s], parity[s]) ? 1 : 0);
-      parity[s] ^= 1u;
-      if (!ok) {
-        // the copy never completed: record it, wait (bounded) for the other
-        // stage's copy if one is in flight, and leave
-        if (threadIdx.x == 0) { ctl->error = 1; ctl->any = 0; }
-        if (act_next) mbar_wait(&bars[s ^ 1], parity[s ^ 1]);
-        return;
-      }
-      const int r = row_map[item];
-      const Ls2dRep& R = reps[r];
-      Ls2dState& S = st[r];
-      const int ny = R.ny, nyh = R.nyh, ld = R.ld, nx = R.nx;
-      const long long N = R.N;
-      const int x0 = 2 * row_local[item];
-      unsigned char* sb = smem_raw + (size_t)s * stage_bytes;
-      const uint32_t spec_b = 2u * ld * sizeof(C), row_b = 2u * ny * sizeof(TS);
-      const C* sspec = reinterpret_cast<const C*>(sb);
-      const TS* seps = reinterpret_cast<const TS*>(sb + 3 * spec_b);
-      const TS* smu = reinterpret_cast<const TS*>(sb + 3 * spec_b + 3 * row_b);
-      const TS* slam = smu + 2 * ny;
-      const TS* sep = slam + 2 * ny;
-      const FftLen& fy = Fields<TS>::fy(R);
-      for (int e = threadIdx.x; e < 3 * ny; e += blockDim.x) {
-        const int c = e / ny, k2 = e - c * ny;
-        const int ks = (2 * k2 <= ny) ? k2 : ny - k2;
-        C a = sspec[c * 2 * ld + ks], b = sspec[c * 2 * ld + ld + ks];
-        C z;
-        if (2 * k2 <= ny) {
-          if (k2 == 0 || 2 * k2 == ny) { a.y = 0; b.y = 0; }
-          z = mk<C>(a.x - b.y, a.y + b.x);
-        } else {
-          z = mk<C>(a.x + b.y, b.x - a.y);
-        }
-        bufA[e] = z;
-      }
-      __syncthreads();
-      C* bufB = reinterpret_cast<C*>(sb);  // the spectrum rows are consumed
-      C* cur = fft_any<+1>(bufA, bufB, 3, ny, fy);
-      C* out = (cur == bufA) ? bufB : bufA;
-      const double mu0 = S.mu0, lam0 = S.lam0;
-      const int law = R.law, law_ps = R.law_ps;
-  const double law_a = R.law_a, law_b = R.law_b;
-      const double eb0 = S.ebar[0], eb1 = S.ebar[1], eb2 = S.ebar[2];
-      TS* eps = Fields<TS>::eps(R);
-      double d2 = 0, n2 = 0;
-      for (int y = threadIdx.x; y < ny; y += blockDim.x) {
-        TC tr[2][3];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int j = h * ny + y;
-          const long long i = (long long)(x0 + h) * ny + y;
-          const double o0 = (double)seps[j], o1 = (double)seps[2 * ny + j], o2 = (double)seps[4 * ny + j];
-          const double m = (double)smu[j], l = (double)slam[j];
-          const double p0 = (double)sep[j], p1 = (double)sep[2 * ny + j], p2 = (double)sep[4 * ny + j];
-          const C z0 = cur[y], z1 = cur[ny + y], z2 = cur[2 * ny + y];
-          const double e0 = eb0 + (double)(h == 0 ? z0.x : z0.y);
-          const double e1 = eb1 + (double)(h == 0 ? z1.x : z1.y);
-          const double e2 = eb2 + (double)(h == 0 ? z2.x : z2.y);
-          const double q0 = e0 - o0, q1 = e1 - o1, q2 = e2 - o2;
-          d2 += q0 * q0 + q1 * q1 + 2.0 * q2 * q2;
-          n2 += o0 * o0 + o1 * o1 + 2.0 * o2 * o2;
-          eps[i] = (TS)e0;
-          eps[N + i] = (TS)e1;
-          eps[2 * N + i] = (TS)e2;
-          const double dxx = e0 - p0, dyy = e1 - p1, dxy = e2 - p2;
-          const double tre = e0 + e1;
-          double s0, s1, s2;  // nonlinear laws only in FP64 kernels (their plans are FP64)
-          if (sizeof(TS) == 8 && law == 1) law_sigma<1>(m, l, dxx, dyy, dxy, law_a, law_b, law_ps, s0, s1, s2);
-          else if (sizeof(TS) == 8 && law == 2) law_sigma<2>(m, l, dxx, dyy, dxy, law_a, law_b, law_ps, s0, s1, s2);
-          else if (sizeof(TS) == 8 && law == 3) law_sigma<3>(m, l, dxx, dyy, dxy, 0.0, 0.0, law_ps, s0, s1, s2, R.lp);
-          else law_sigma<0>(m, l, dxx, dyy, dxy, 0.0, 0.0, 0, s0, s1, s2);
-          tr[h][0] = (TC)(s0 - (2 * mu0 * e0 + lam0 * tre));
-          tr[h][1] = (TC)(s1 - (2 * mu0 * e1 + lam0 * tre));
-          tr[h][2] = (TC)(s2 - 2 * mu0 * e2);
-        }
-#pragma unroll
-        for (int c = 0; c < 3; ++c) out[c * ny + y] = mk<C>(tr[0][c], tr[1][c]);
-      }
-      __syncthreads();
-      C* scratch = (out == bufA) ? bufB : bufA;
-      C* Z = fft_any<-1>(out, scratch, 3, ny, fy);
-      C* spec = reinterpret_cast<C*>(R.spec);
-      for (int e = threadIdx.x; e < 3 * nyh; e += blockDim.x) {
-        const int c = e / nyh, k2 = e - c * nyh;
-        const C z = Z[c * ny + k2];
-        const C w = Z[c * ny + (k2 == 0 ? 0 : ny - k2)];
-        C* ra = spec + ((size_t)c * nx + x0) * ld;
-        ra[k2] = mk<C>(TC(0.5) * (z.x + w.x), TC(0.5) * (z.y - w.y));
-        ra[ld + k2] = mk<C>(TC(0.5) * (z.y + w.y), TC(-0.5) * (z.x - w.x));
-      }
-      d2 = block_sum(d2, red);
-      n2 = block_sum(n2, red);
-      if (threadIdx.x == 0) {
-        partials[2 * item] = d2;
-        partials[2 * item + 1] = n2;
-        __threadfence();
-        const unsigned int t = atomicInc(&rep_counter[r], (unsigned int)R.row_items - 1);
-        s_last = (t == (unsigned int)R.row_items - 1);
-      }
-      __syncthreads();
-      if (s_last) {
-        __threadfence();
-        ls2d_decide<FINAL>(R, S, partials, ctl, cond, use_cond, guard_cap, red);
-      }
-    }
-    __syncthreads();  // this stage is free for the prefetch two items ahead
-    act = act_next;
-  }
+  ls2d_decide(R, S, partials, ctl, cond, use_cond, guard_cap, red, FINAL);
 }
 
 // Column kernel: FFT along x, Gamma0_sym, inverse FFT along x, for a tile of
@@ -1027,320 +502,9 @@ __global__ void __launch_bounds__(256) ls2d_col_kernel(const Ls2dRep* __restrict
   }
 }
 
-// --------------------------------------------- warp-line iteration kernels ---
-// The same two stages for replicas whose sides have a compiled warp-line FFT
-// (64 .. 512).  Row kernel: one CTA of three warps per pair of x-rows; one
-// elected thread stages the pair's eps, mu, lambda and eps_p rows in shared
-// memory with bulk asynchronous copies at entry, while warp c inverts
-// component c of the spectrum; after one CTA barrier every thread updates its
-// voxels and builds tau, then warp c forward-transforms and stores component
-// c.  Column kernel: one CTA of kColTiles warps per tile of kColTiles ky
-// columns; the tile lands in shared memory through cp.async, then warp t runs
-// FFT, Gamma0_sym and inverse FFT on column t alone.
-// resident-CTA targets for the register allocator (FP32 kernels need fewer
-// registers; more resident warps hide their latency)
-#ifndef MGK_ROW_MINB32
-#define MGK_ROW_MINB32 9
-#endif
-#ifndef MGK_COL_MINB32
-#define MGK_COL_MINB32 4
-#endif
-constexpr int kColTiles = 4;  // ky columns per column-kernel CTA (one warp each)
-// lanes per line and column tiles of a kernel variant (sides up to MAXN):
-// lines longer than 512 points take two warps
-__host__ __device__ constexpr int fast_group(int maxn) { return maxn > 512 ? 64 : 32; }
-__host__ __device__ constexpr int fast_col_tiles(int maxn) { return maxn > 512 ? 2 : kColTiles; }
-__host__ __device__ constexpr int row_threads(int maxn) { return 3 * fast_group(maxn); }
-__host__ __device__ constexpr int col_threads(int maxn) { return fast_col_tiles(maxn) * fast_group(maxn); }
-
-// Shared memory of the row kernel: 3 padded lines, then the row pair's eps
-// (3), mu, lambda and eps_p (3) planes staged by bulk copies (reading eps
-// from global memory instead serialises the loads behind the in-place stores).
-__host__ __device__ constexpr int row_fast_smem(int ny, int csz, int tsz) {
-  return ((3 * (csz == 16 ? ny + ny / 8 + 1 : ((ny + ny / 16 + 2) & ~1)) * csz + 127) / 128) * 128 + 16 * ny * tsz;
-}
-__host__ __device__ constexpr int col_fast_smem(int nx, int csz, int tc) {
-  return 3 * tc * (csz == 16 ? nx + nx / 8 + 1 : ((nx + nx / 16 + 2) & ~1)) * csz;
-}
-
-template <typename T, int NY, int G, bool IN_SPEC, bool FINAL, int LAW>
-__device__ __forceinline__ void row_fast_body(const Ls2dRep& R, Ls2dState& S, int item, int r, int x0,
-                                              double* partials,
-                                              unsigned int* rep_counter, Ls2dCtl* ctl,
-                                              cudaGraphConditionalHandle cond, int use_cond, int guard_cap,
-                                              unsigned char* smem, uint64_t* bar, double* red, int* s_last) {
-  using C = C_t<T>;
-  constexpr int PL = padded_len<C>(NY);
-  constexpr int NYH = NY / 2 + 1;
-  constexpr int NT = 3 * G;
-  const int warp = threadIdx.x / G, lane = threadIdx.x % G;  // line (component) and lane in it
-  const int bid = 1 + warp;
-  const int nx = R.nx, ld = R.ld;
-  const long long N = R.N;
-  C* lines = reinterpret_cast<C*>(smem);
-  T* stg = reinterpret_cast<T*>(smem + ((3 * PL * (int)sizeof(C) + 127) / 128) * 128);
-  T* eps = Fields<T>::eps(R);
-  const T* ep = Fields<T>::ep(R);
-  constexpr uint32_t rb = 2u * NY * sizeof(T);
-  if (threadIdx.x == 0) {
-    const T* src[8] = {eps, eps + N, eps + 2 * N, Fields<T>::mu(R), Fields<T>::lam(R), ep, ep + N, ep + 2 * N};
-    fence_proxy_async_smem();
-    mbar_arrive_expect_tx(bar, 8u * rb);
-#pragma unroll
-    for (int q = 0; q < 8; ++q) bulk_g2s(stg + q * 2 * NY, src[q] + (long long)x0 * NY, rb, bar);
-  }
-  const C* tw = reinterpret_cast<const C*>(Fields<T>::fy(R).tw);
-  C* spec = reinterpret_cast<C*>(R.spec);
-  C* line = lines + warp * PL;
-  C* ra = spec + ((size_t)warp * nx + x0) * ld;
-  C* rbp = ra + ld;
-  if (IN_SPEC) {
-    constexpr int U = (NYH + G - 1) / G;
-    C a[U], b[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int k = lane + G * u;
-      if (k < NYH) { a[u] = ra[k]; b[u] = rbp[k]; }
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int k = lane + G * u;
-      if (k < NYH) {
-        C av = a[u], bv = b[u];
-        if (k == 0 || 2 * k == NY) { av.y = 0; bv.y = 0; }
-        line[pidx<C>(k)] = mk<C>(av.x - bv.y, av.y + bv.x);
-        if (k > 0 && 2 * k < NY) line[pidx<C>(NY - k)] = mk<C>(av.x + bv.y, bv.x - av.y);
-      }
-    }
-    grp_sync<G>(bid);
-    warp_fft<NY, +1, 1, G>(line, PL, tw, lane, bid);
-  }
-  const bool ok = mbar_wait(bar, 0);
-  if (!__syncthreads_and(ok ? 1 : 0)) {
-    if (threadIdx.x == 0) { ctl->error = 1; ctl->any = 0; }
-    return;
-  }
-  const double mu0 = S.mu0, lam0 = S.lam0;
-  const int law = R.law, law_ps = R.law_ps;
-  const double law_a = R.law_a, law_b = R.law_b;
-  const double eb0 = S.ebar[0], eb1 = S.ebar[1], eb2 = S.ebar[2];
-  double gam[kAaMax];
-  const int nmix = (!IN_SPEC && sizeof(T) == 8 && R.aa) ? aa_load(R, gam) : 0;
-  // with Anderson mixing the image's tau is never used (the next tau is the
-  // mixed iterate's): the pass stops at the image and its update norm
-  const bool img_only = IN_SPEC && LAW != 0 && sizeof(T) == 8 && R.aa != nullptr;
-  double d2 = 0, n2 = 0;
-  for (int y = threadIdx.x; y < NY; y += NT) {
-    T tr[2][3];
-    const int py = pidx<C>(y);
-    C z[3];
-    if (IN_SPEC) {
-#pragma unroll
-      for (int c = 0; c < 3; ++c) z[c] = lines[c * PL + py];
-    }
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int j = h * NY + y;
-      const long long i = (long long)(x0 + h) * NY + y;
-      const double o0 = (double)stg[j], o1 = (double)stg[2 * NY + j], o2 = (double)stg[4 * NY + j];
-      const double m = (double)stg[6 * NY + j], l = (double)stg[8 * NY + j];
-      const double p0 = (double)stg[10 * NY + j], p1 = (double)stg[12 * NY + j], p2 = (double)stg[14 * NY + j];
-      double e0, e1, e2;
-      if (IN_SPEC) {
-        e0 = eb0 + (double)(h == 0 ? z[0].x : z[0].y);
-        e1 = eb1 + (double)(h == 0 ? z[1].x : z[1].y);
-        e2 = eb2 + (double)(h == 0 ? z[2].x : z[2].y);
-        const double q0 = e0 - o0, q1 = e1 - o1, q2 = e2 - o2;
-        d2 += q0 * q0 + q1 * q1 + 2.0 * q2 * q2;
-        n2 += o0 * o0 + o1 * o1 + 2.0 * o2 * o2;
-        eps[i] = (T)e0;
-        eps[N + i] = (T)e1;
-        eps[2 * N + i] = (T)e2;
-      } else {
-        e0 = o0; e1 = o1; e2 = o2;
-        if (!IN_SPEC && sizeof(T) == 8 && R.aa) {  // the mixed iterate
-          double e[3] = {o0, o1, o2};
-          aa_mix_voxel(R, i, nmix, gam, e);
-          e0 = e[0]; e1 = e[1]; e2 = e[2];
-        }
-      }
-      if (img_only) continue;
-      const double dxx = e0 - p0, dyy = e1 - p1, dxy = e2 - p2;
-      const double tre = e0 + e1;
-      double s0, s1, s2;  // LAW 0 linear; 1 secant, 2 Rose, 3 Landau (FP64 plans)
-      law_sigma<LAW>(m, l, dxx, dyy, dxy, law_a, law_b, law_ps, s0, s1, s2, R.lp);
-      tr[h][0] = (T)(s0 - (2 * mu0 * e0 + lam0 * tre));
-      tr[h][1] = (T)(s1 - (2 * mu0 * e1 + lam0 * tre));
-      tr[h][2] = (T)(s2 - 2 * mu0 * e2);
-    }
-    if (img_only) continue;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) lines[c * PL + py] = mk<C>(tr[0][c], tr[1][c]);
-  }
-  if (!img_only) {
-    __syncthreads();
-    warp_fft<NY, -1, 1, G>(line, PL, tw, lane, bid);
-    for (int k = lane; k < NYH; k += G) {
-      const C zz = line[pidx<C>(k)];
-      const C w = line[pidx<C>(k == 0 ? 0 : NY - k)];
-      ra[k] = mk<C>(T(0.5) * (zz.x + w.x), T(0.5) * (zz.y - w.y));
-      rbp[k] = mk<C>(T(0.5) * (zz.y + w.y), T(-0.5) * (zz.x - w.x));
-    }
-  }
-  if (!IN_SPEC) return;
-  d2 = block_sum(d2, red);
-  n2 = block_sum(n2, red);
-  if (threadIdx.x == 0) {
-    partials[2 * item] = d2;
-    partials[2 * item + 1] = n2;
-    __threadfence();
-    const unsigned int t = atomicInc(&rep_counter[r], (unsigned int)R.row_items - 1);  // self-resetting
-    *s_last = (t == (unsigned int)R.row_items - 1);
-  }
-  __syncthreads();
-  if (!*s_last) return;
-  __threadfence();
-  ls2d_decide<FINAL>(R, S, partials, ctl, cond, use_cond, guard_cap, red);
-}
-
-template <typename T, int MAXN, bool IN_SPEC, bool FINAL, int LAW = 0>
-__global__ void __launch_bounds__(row_threads(MAXN), sizeof(T) == 4 && MAXN <= 256 ? MGK_ROW_MINB32 : 1) ls2d_row_fast_kernel(
-    const Ls2dRep* __restrict__ reps, Ls2dState* st, const int* __restrict__ row_map,
-    const int* __restrict__ row_local, double* partials, unsigned int* rep_counter, Ls2dCtl* ctl,
-    cudaGraphConditionalHandle cond, int use_cond, int guard_cap) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ double red[32];
-  __shared__ int s_last;
-  __shared__ __align__(8) uint64_t bar;
-  const int item = blockIdx.x;
-  const int r = row_map[item];
-  const Ls2dRep& R = reps[r];
-  Ls2dState& S = st[r];
-  if (IN_SPEC && use_cond && item == 0 && threadIdx.x == 0) {
-    const unsigned int b = atomicAdd(&ctl->bodies, 1u) + 1u;
-    if (ctl->n_active == 0 || b > (unsigned int)guard_cap || *(volatile int*)&ctl->error != 0) {
-      ctl->any = 0;
-      cudaGraphSetConditional(cond, 0u);
-    }
-  }
-  if (S.done != 0) return;
-  if (threadIdx.x == 0) {
-    mbar_init(&bar, 1);
-    fence_mbar_init();
-  }
-  __syncthreads();
-  const int x0 = 2 * row_local[item];
-#define MGK_ROW_CASE(n) \
-  case n: if constexpr (n <= MAXN) row_fast_body<T, n, fast_group(MAXN), IN_SPEC, FINAL, LAW>(R, S, item, r, x0, partials, rep_counter, ctl, cond, use_cond, guard_cap, \
-                                              smem_raw, &bar, red, &s_last); break;
-  switch (R.ny) {
-    MGK_ROW_CASE(64) MGK_ROW_CASE(96) MGK_ROW_CASE(128) MGK_ROW_CASE(192) MGK_ROW_CASE(256) MGK_ROW_CASE(384)
-    MGK_ROW_CASE(512) MGK_ROW_CASE(768) MGK_ROW_CASE(1024)
-    default: break;
-  }
-#undef MGK_ROW_CASE
-}
-
-template <typename T, int NX, int TC, int G>
-__device__ __forceinline__ void col_fast_body(const Ls2dRep& R, const Ls2dState& S, int ky0,
-                                              unsigned char* smem) {
-  using C = C_t<T>;
-  constexpr int kColTiles = TC;
-  constexpr int PL = padded_len<C>(NX);
-  const int warp = threadIdx.x / G, lane = threadIdx.x % G;  // column of the tile and lane in it
-  const int bid = 1 + warp;
-  const int ny = R.ny, nyh = R.nyh, ld = R.ld;
-  const int tcw = min(kColTiles, nyh - ky0);
-  C* lines = reinterpret_cast<C*>(smem);  // line (c * kColTiles + t)
-  C* spec = reinterpret_cast<C*>(R.spec);
-  constexpr int TOT = 3 * NX * kColTiles;
-  for (int e = threadIdx.x; e < TOT; e += G * kColTiles) {
-    const int c = e / (NX * kColTiles);
-    const int rem = e - c * NX * kColTiles;
-    const int x = rem / kColTiles, t = rem - x * kColTiles;
-    if (t < tcw) cp_async_elem(&lines[(c * kColTiles + t) * PL + pidx<C>(x)], &spec[((size_t)c * NX + x) * ld + ky0 + t]);
-  }
-  cp_async_wait_all();
-  __syncthreads();
-  const int t = warp;
-  if (t < tcw) {
-    const C* tw = reinterpret_cast<const C*>(Fields<T>::fx(R).tw);
-    C* l0 = lines + t * PL;
-    constexpr int LS = kColTiles * PL;  // stride between the components of a column
-    warp_fft<NX, -1, 1, G>(l0, LS, tw, lane, bid);
-    warp_fft<NX, -1, 1, G>(l0 + LS, LS, tw, lane, bid);
-    warp_fft<NX, -1, 1, G>(l0 + 2 * LS, LS, tw, lane, bid);
-    const T inv2mu0 = (T)S.inv2mu0, Bc = (T)S.Bc;
-    const T sc = (T)(1.0 / ((double)NX * (double)ny));
-    const int ky = ky0 + t;
-    // the wave direction in the pass precision (FP32 phase: float)
-    const T uy = (T)fftfreq(ky, ny) / (T)ny;
-    const bool nqy = (ny & 1) == 0 && 2 * ky == ny;
-    for (int kx = lane; kx < NX; kx += G) {
-      const int pk = pidx<C>(kx);
-      C* pxx = &l0[pk];
-      C* pyy = &l0[LS + pk];
-      C* pxy = &l0[2 * LS + pk];
-      if (kx == 0 && ky == 0) {
-        *pxx = mk<C>(T(0), T(0)); *pyy = *pxx; *pxy = *pxx;
-        continue;
-      }
-      const T ux = (T)fftfreq(kx, NX) / (T)NX;
-      const T inv = T(1) / sqrt(ux * ux + uy * uy);
-      const T nxv = ux * inv, nyv = uy * inv;
-      const C txx = *pxx, tyy = *pyy, txy = *pxy;
-      C exx, eyy, exy;
-      gamma2d_apply(txx, tyy, txy, nxv, nyv, inv2mu0, Bc, exx, eyy, exy);
-      const bool nqx = 2 * kx == NX;
-      if (nqx || nqy) {
-        C fxx, fyy, fxy;
-        gamma2d_apply(txx, tyy, txy, nqx ? -nxv : nxv, nqy ? -nyv : nyv, inv2mu0, Bc, fxx, fyy, fxy);
-        exx = mk<C>(T(0.5) * (exx.x + fxx.x), T(0.5) * (exx.y + fxx.y));
-        eyy = mk<C>(T(0.5) * (eyy.x + fyy.x), T(0.5) * (eyy.y + fyy.y));
-        exy = mk<C>(T(0.5) * (exy.x + fxy.x), T(0.5) * (exy.y + fxy.y));
-      }
-      *pxx = mk<C>(exx.x * sc, exx.y * sc);
-      *pyy = mk<C>(eyy.x * sc, eyy.y * sc);
-      *pxy = mk<C>(exy.x * sc, exy.y * sc);
-    }
-    grp_sync<G>(bid);
-    warp_fft<NX, +1, 1, G>(l0, LS, tw, lane, bid);
-    warp_fft<NX, +1, 1, G>(l0 + LS, LS, tw, lane, bid);
-    warp_fft<NX, +1, 1, G>(l0 + 2 * LS, LS, tw, lane, bid);
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < TOT; e += G * kColTiles) {
-    const int c = e / (NX * kColTiles);
-    const int rem = e - c * NX * kColTiles;
-    const int x = rem / kColTiles, tt = rem - x * kColTiles;
-    if (tt < tcw) spec[((size_t)c * NX + x) * ld + ky0 + tt] = lines[(c * kColTiles + tt) * PL + pidx<C>(x)];
-  }
-}
-
-template <typename T, int MAXN>
-__global__ void __launch_bounds__(col_threads(MAXN), MAXN <= 256 ? (sizeof(T) == 4 ? MGK_COL_MINB32 : 4) : 1) ls2d_col_fast_kernel(const Ls2dRep* __restrict__ reps,
-                                                                       const Ls2dState* __restrict__ st,
-                                                                       const int* __restrict__ col_map,
-                                                                       const int* __restrict__ col_local) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int item = blockIdx.x;
-  const int r = col_map[item];
-  const Ls2dRep& R = reps[r];
-  const Ls2dState& S = st[r];
-  if (S.done != 0) return;
-  const int ky0 = col_local[item] * fast_col_tiles(MAXN);
-#define MGK_COL_CASE(n) \
-  case n: if constexpr (n <= MAXN) col_fast_body<T, n, fast_col_tiles(MAXN), fast_group(MAXN)>(R, S, ky0, smem_raw); break;
-  switch (R.nx) {
-    MGK_COL_CASE(64) MGK_COL_CASE(96) MGK_COL_CASE(128) MGK_COL_CASE(192) MGK_COL_CASE(256) MGK_COL_CASE(384)
-    MGK_COL_CASE(512) MGK_COL_CASE(768) MGK_COL_CASE(1024)
-    default: break;
-  }
-#undef MGK_COL_CASE
-}
-
-// Mixed plans, between the phases: FP64 field from the FP32 one.
-// grid = (G, nsel).
+// Mixed plans with CTA-wide replicas, between the phases: their FP64 field
+// from the FP32 one (the register-FFT row pass promotes its own).  grid = (G,
+// replicas).
 __global__ void ls2d_promote_kernel(const Ls2dRep* reps, const int* sel) {
   const int r = sel[blockIdx.y];
   const Ls2dRep& R = reps[r];
@@ -1351,13 +515,15 @@ __global__ void ls2d_promote_kernel(const Ls2dRep* reps, const int* sel) {
 }
 
 // Replicas that finished phase 1 re-enter for phase 2; resets the control block.
+// One warp.
 __global__ void ls2d_phase2_kernel(Ls2dState* st, const int* sel, int nsel, Ls2dCtl* ctl) {
-  if (threadIdx.x != 0) return;
   unsigned int n = 0;
-  for (int q = 0; q < nsel; ++q) {
+  for (int q = threadIdx.x; q < nsel; q += 32) {
     Ls2dState& S = st[sel[q]];
     if (S.done == 1) { S.done = 0; S.phase_iter = 0; ++n; }
   }
+  n = __reduce_add_sync(0xffffffffu, n);
+  if (threadIdx.x != 0) return;
   ctl->n_active = n;
   ctl->decided = 0;
   ctl->still = 0;
@@ -1365,15 +531,16 @@ __global__ void ls2d_phase2_kernel(Ls2dState* st, const int* sel, int nsel, Ls2d
   ctl->any = n > 0;
 }
 
-// Outputs in the reference layout: eps, sig (nx,ny,2,2) and partial sums of
-// their components for the means (linear_elastic_simulator.py:83-88).
+// Outputs in the reference layout: eps, sig (nx,ny,2,2) and the means of
+// their components (linear_elastic_simulator.py:83-88).
 // grid = (G, nsel).
 template <int LAW = 0>  // 1: the secant law, 2: the Rose law, 3: the Landau law
-__global__ void ls2d_output_kernel(const Ls2dRep* reps, const Ls2dState* st, const int* sel, double* partials) {
-  __shared__ double red[32];
+__global__ void __launch_bounds__(kThreads) ls2d_output_kernel(const Ls2dRep* reps, Ls2dState* st, const int* sel,
+                                                               double* partials, unsigned int* ctr) {
+  __shared__ double res[8];
   const int r = sel[blockIdx.y];
   const Ls2dRep& R = reps[r];
-  const Ls2dState& S = st[r];
+  Ls2dState& S = st[r];
   const long long N = R.N;
   const double abar = S.abar;
   double* eps_out = R.out_eps;
@@ -1418,10 +585,8 @@ __global__ void ls2d_output_kernel(const Ls2dRep* reps, const Ls2dState* st, con
     s[0] += exx; s[1] += exy; s[2] += eyx; s[3] += eyy;
     s[4] += sxx; s[5] += sxy2; s[6] += syx2; s[7] += syy;
   }
-  for (int q = 0; q < 8; ++q) {
-    double t = block_sum(s[q], red);
-    if (threadIdx.x == 0) partials[((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 8 + q] = t;
-  }
+  if (grid_sums<8>(s, partials + (size_t)blockIdx.y * gridDim.x * 8, ctr + r, res) && threadIdx.x < 8)
+    (threadIdx.x < 4 ? S.out_eps_mean : S.out_sig_mean)[threadIdx.x & 3] = res[threadIdx.x] * (1.0 / (double)N);
 }
 
 // Anderson mixing over fields of n doubles (linear_elastic_simulator.py:
@@ -1807,7 +972,6 @@ using namespace mgk;
 
 namespace {
 
-constexpr int kThreads = 256;
 constexpr int kPerVoxelBlocks = 256;  // G: CTAs per replica for per-voxel kernels
 
 int grid_blocks(long long maxN) {
@@ -1827,18 +991,53 @@ int pick_tc(int nx, size_t csz, size_t cap) {
 
 }  // namespace
 
+// One launch group of a solve: the selected replicas of one shape on the
+// register-FFT kernels, or every other replica on the CTA-wide passes (ky
+// null), which find their replica in work maps.
+struct Grp2 {
+  const Ls2Line *kx = nullptr, *ky = nullptr, *kx32 = nullptr, *ky32 = nullptr;
+  const int* sel = nullptr;  // the group's slice of the selection (device)
+  int n = 0;                 // replicas
+  int nx = 0, nyh = 0;
+  int wr = 0, wc = 0, wc32 = 0;  // narrow or wide forms
+  const int *row_map = nullptr, *row_local = nullptr, *col_map = nullptr, *col_local = nullptr;
+  int rows = 0, cols = 0;    // CTA-wide: items over its replicas
+  int lead = 0;              // counts the loop bodies
+};
+
+struct Loop2 {
+  const Ls2dRep* reps = nullptr;
+  Ls2dState* st = nullptr;
+  double* part = nullptr;
+  unsigned int* ctr = nullptr;
+  Ls2dCtl* ctl = nullptr;
+  size_t rs = 0, cs = 0, rs32 = 0, cs32 = 0;  // shared memory of the CTA-wide passes
+  const int* sel = nullptr;
+  int nsel = 0, G = 0, law = 0;
+  // Anderson mixing (FP64 loop of a one-replica selection; aa_m = 0: none)
+  int aa_m = 0, aa_nb = 0;
+  double* aa_buf = nullptr;
+  Ls2dAA* aa = nullptr;
+  double* aa_part = nullptr;
+  std::vector<Grp2> grp;
+};
+
 struct mgk_ls2d_plan {
   int nrep = 0;
   int plane_mode = 0, prec = 0;
   long long maxN = 0;
-  size_t row_smem = 0, col_smem = 0;      // FP64 iteration kernels
-  size_t row_smem32 = 0, col_smem32 = 0;  // FP32 iteration kernels
-  int fast = 0;                           // kernel family in use: 0 CTA-wide passes, 256/512/1024 warp-line
-  int fast_nat = 0;                       // smallest warp-line family that covers every side (0: none)
+  size_t row_smem = 0, col_smem = 0;      // CTA-wide FP64 iteration kernels
+  size_t row_smem32 = 0, col_smem32 = 0;  // and FP32
+  // Kernel family: 256/512/1024 asks for the register-FFT kernels, 0 for the
+  // CTA-wide passes where every side is one of the lengths 64 .. 1024 of
+  // warp_fft_len (fast_nat: its smallest family); a plan with other sides has
+  // family 0 only, which then means each replica's natural kernels.
+  int fast = 0, fast_nat = 0;
+  std::vector<int> order;                 // the last selection in launch order
+  std::vector<char> line_ok;              // replicas whose sides both have a register-FFT kernel
   int law = 0;                            // 1: secant degradation law, 2: Rose law
   double law_a = 0, law_b = 0;            // the law's parameters (set_secant, set_rose)
   int law_ps = 0;
-  std::vector<int> tc_gen;                // column tiles of the CTA-wide family, per replica
   std::vector<Ls2dRep> reps;      // host copy (static part)
   std::vector<char> has_material;
   Ls2dRep* h_reps = nullptr;      // pinned staging of the table
@@ -1856,32 +1055,22 @@ struct mgk_ls2d_plan {
   double* d_mat_part = nullptr;   // partials of the material kernel
   size_t part_doubles = 0;
   int total_row_items = 0, total_col_items = 0;
+  unsigned int* d_voxctr = nullptr;  // arrival counters of the per-voxel kernels, per replica
   std::vector<void*> allocations;
   // spectra of all replicas, one slab
   void* spec_slab = nullptr;
   size_t spec_bytes = 0;
-  // loop graph for the current selection
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
-  int graph_mode = -1;  // -1 untried, 1 while-node graph, 0 host loop
-  int graph_cap = 0;
-  int graph_aa = 0;     // Anderson depth of the current graph
-  // instantiated loop graphs by selection shape (a serving loop selects
-  // varying numbers of replicas; each shape is built once)
+  // instantiated loop graphs by the selection's shapes and widths (its
+  // signature): a serving loop selects varying numbers of replicas
   struct GraphEntry {
-    int rows, cols, nsel, cap, aa;
+    std::vector<int> sig;
+    int cap;
     cudaGraph_t g;
     cudaGraphExec_t x;
   };
   std::vector<GraphEntry> gcache;
-  // selection of the last call
-  int nsel = 0, sel_rows = 0, sel_cols = 0;
-  // persistent bulk-prefetch row kernels (0 when a replica has odd ny or the
-  // stages do not fit): stage bytes, dynamic smem and resident CTAs per SM
-  int tma = 0;
-  int stage64 = 0, stage32 = 0;
-  size_t tma_smem64 = 0, tma_smem32 = 0;
-  int occ64 = 0, occ32 = 0, num_sms = 0;
+  int graph_mode = 1;  // 0: host-driven loop
+  Loop2 last;          // the last call's launches (the timing hook repeats its stages)
   // Anderson mixing inside the loop (one replica per solve): depth, ring
   // buffer of (3 + 2 m) strain fields, state and per-block partial sums
   int aa_m = 0;
@@ -1902,48 +1091,27 @@ static int plan_alloc(mgk_ls2d_t p, void** ptr, size_t bytes) {
   return MGK_OK;
 }
 
-// warp-line kernel variants: sides up to 256, or up to 512 (more registers)
-template <typename TS, bool IN_SPEC, bool FINAL>
-static void* row_fast_fn(int fast, int law = 0) {
-  if constexpr (sizeof(TS) == 8) {
-    if (law == 1)  // the secant law (FP64 plans only)
-      return fast > 512   ? (void*)ls2d_row_fast_kernel<TS, 1024, IN_SPEC, FINAL, 1>
-             : fast > 256 ? (void*)ls2d_row_fast_kernel<TS, 512, IN_SPEC, FINAL, 1>
-                          : (void*)ls2d_row_fast_kernel<TS, 256, IN_SPEC, FINAL, 1>;
-    if (law == 2)  // the Rose law (FP64 plans only)
-      return fast > 512   ? (void*)ls2d_row_fast_kernel<TS, 1024, IN_SPEC, FINAL, 2>
-             : fast > 256 ? (void*)ls2d_row_fast_kernel<TS, 512, IN_SPEC, FINAL, 2>
-                          : (void*)ls2d_row_fast_kernel<TS, 256, IN_SPEC, FINAL, 2>;
-    if (law == 3)  // the Landau law (FP64 plans only)
-      return fast > 512   ? (void*)ls2d_row_fast_kernel<TS, 1024, IN_SPEC, FINAL, 3>
-             : fast > 256 ? (void*)ls2d_row_fast_kernel<TS, 512, IN_SPEC, FINAL, 3>
-                          : (void*)ls2d_row_fast_kernel<TS, 256, IN_SPEC, FINAL, 3>;
+// raises the shared-memory limits of a replica's register-FFT kernels
+static int ls2d_line_attrs(int nx, int ny, int kind) {
+  const Ls2Line *kx = ls2_line(nx, kind), *ky = ls2_line(ny, kind);
+  for (int w = 0; w < 2; ++w) {
+    for (int law = 0; law < 4; ++law)
+      if (ky->row[law][w]) MGK_CUDA(raise_smem(ky->row[law][w], ky->r_bytes[w]));
+    MGK_CUDA(raise_smem(kx->col[w], kx->c_bytes[w]));
   }
-  return fast > 512   ? (void*)ls2d_row_fast_kernel<TS, 1024, IN_SPEC, FINAL>
-         : fast > 256 ? (void*)ls2d_row_fast_kernel<TS, 512, IN_SPEC, FINAL>
-                      : (void*)ls2d_row_fast_kernel<TS, 256, IN_SPEC, FINAL>;
-}
-template <typename TS>
-static void* col_fast_fn(int fast) {
-  return fast > 512   ? (void*)ls2d_col_fast_kernel<TS, 1024>
-         : fast > 256 ? (void*)ls2d_col_fast_kernel<TS, 512>
-                      : (void*)ls2d_col_fast_kernel<TS, 256>;
-}
-
-template <typename T>
-static int ls2d_set_fast_attrs(int fast, size_t row_smem, size_t col_smem) {
-  void* fns[16] = {row_fast_fn<T, true, true>(fast), row_fast_fn<T, false, true>(fast),
-                   row_fast_fn<T, true, false>(fast), row_fast_fn<T, false, false>(fast),
-                   row_fast_fn<T, true, true>(fast, 1), row_fast_fn<T, false, true>(fast, 1),
-                   row_fast_fn<T, true, false>(fast, 1), row_fast_fn<T, false, false>(fast, 1),
-                   row_fast_fn<T, true, true>(fast, 2), row_fast_fn<T, false, true>(fast, 2),
-                   row_fast_fn<T, true, false>(fast, 2), row_fast_fn<T, false, false>(fast, 2),
-                   row_fast_fn<T, true, true>(fast, 3), row_fast_fn<T, false, true>(fast, 3),
-                   row_fast_fn<T, true, false>(fast, 3), row_fast_fn<T, false, false>(fast, 3)};
-  for (void* f : fns) MGK_CUDA(raise_smem((const void*)f, (int)row_smem));
-  MGK_CUDA(raise_smem((const void*)col_fast_fn<T>(fast), (int)col_smem));
   return MGK_OK;
 }
+
+static void ls2d_drop_graphs(mgk_ls2d_t p) {
+  for (auto& e : p->gcache) {
+    cudaGraphExecDestroy(e.x);
+    cudaGraphDestroy(e.g);
+  }
+  p->gcache.clear();
+}
+
+// whether a replica runs on the register-FFT kernels under the plan's family
+static bool ls2d_on_line(mgk_ls2d_t p, int r) { return p->line_ok[r] && (p->fast != 0 || p->fast_nat == 0); }
 
 template <typename TS, typename TC>
 static int ls2d_set_attrs(size_t row_smem, size_t col_smem) {
@@ -1957,10 +1125,7 @@ static int ls2d_set_attrs(size_t row_smem, size_t col_smem) {
 
 extern "C" int mgk_ls2d_destroy(mgk_ls2d_t p) {
   if (!p) return MGK_OK;
-  for (auto& e : p->gcache) {
-    cudaGraphExecDestroy(e.x);
-    cudaGraphDestroy(e.g);
-  }
+  ls2d_drop_graphs(p);
   if (p->staged) cudaEventDestroy(p->staged);
   for (void* a : p->allocations) cudaFree(a);
   if (p->aa_buf) cudaFree(p->aa_buf);
@@ -2001,6 +1166,8 @@ extern "C" int mgk_ls2d_create_batch(int nrep, const int* nxs, const int* nys, i
   auto fail = [&](int s) { mgk_ls2d_destroy(p); return s; };
   p->reps.resize(nrep);
   p->has_material.assign(nrep, 0);
+  const char* env = getenv("MGK_FAST");
+  const bool no_line = env && env[0] == '0';
   {
     bool fast = true;
     int side = 0;
@@ -2009,29 +1176,22 @@ extern "C" int mgk_ls2d_create_batch(int nrep, const int* nxs, const int* nys, i
       side = std::max(side, std::max(nxs[r], nys[r]));
     }
     p->fast_nat = fast ? (side > 512 ? 1024 : side > 256 ? 512 : 256) : 0;
-    const char* env = getenv("MGK_FAST");
-    p->fast = (env && env[0] == '0') ? 0 : p->fast_nat;
+    p->fast = no_line ? 0 : p->fast_nat;
   }
-  p->tc_gen.resize(nrep);
+  p->line_ok.assign(nrep, 0);
   std::vector<size_t> spec_off(nrep, 0);
-  int total_col_max = 0;
   size_t row_smem = 0, col_smem = 0, row_smem32 = 0, col_smem32 = 0;
   for (int r = 0; r < nrep; ++r) {
     const int nx = nxs[r], ny = nys[r];
     Ls2dRep& R = p->reps[r];
     memset(&R, 0, sizeof(R));
-    R.nx = nx; R.ny = ny; R.nyh = ny / 2 + 1; R.ld = R.nyh;
+    p->line_ok[r] = !no_line && ls2_line(nx, kLs2Fp64) && ls2_line(ny, kLs2Fp64);
+    R.nx = nx; R.ny = ny; R.nyh = ny / 2 + 1;
+    R.ld = p->line_ok[r] ? ls2_ld(ny) : R.nyh;  // register-FFT tiles read rows of 64 aligned bytes
     R.N = (long long)nx * ny;
-    p->tc_gen[r] = pick_tc(nx, c64, 64 * 1024);
-    R.tc = p->fast ? fast_col_tiles(p->fast) : p->tc_gen[r];
+    R.tc = pick_tc(nx, c64, 64 * 1024);
     R.row_items = nx / 2;
     R.col_items = (R.nyh + R.tc - 1) / R.tc;
-    {
-      int cmax = (R.nyh + p->tc_gen[r] - 1) / p->tc_gen[r];
-      for (int v : {256, 512, 1024})
-        if (p->fast_nat && v >= p->fast_nat) cmax = std::max(cmax, (R.nyh + fast_col_tiles(v) - 1) / fast_col_tiles(v));
-      total_col_max += cmax;
-    }
     fft_schedule(nx, &R.fx64);
     fft_schedule(ny, &R.fy64);
     R.fx32 = R.fx64;
@@ -2044,17 +1204,21 @@ extern "C" int mgk_ls2d_create_batch(int nrep, const int* nxs, const int* nys, i
       R.fy32.tw = twiddles(ny, 1 /* float table */);
       if (!R.fx32.tw || !R.fy32.tw) return fail(MGK_OOM);
     }
-    if (p->fast) {
-      row_smem = std::max(row_smem, (size_t)row_fast_smem(ny, 16, 8));
-      col_smem = std::max(col_smem, (size_t)col_fast_smem(nx, 16, R.tc));
-      row_smem32 = std::max(row_smem32, (size_t)row_fast_smem(ny, 8, 4));
-      col_smem32 = std::max(col_smem32, (size_t)col_fast_smem(nx, 8, R.tc));
-    } else {
-      row_smem = std::max(row_smem, 2 * 3 * (size_t)ny * c64);
-      col_smem = std::max(col_smem, 2 * 3 * (size_t)R.tc * nx * c64);
-      row_smem32 = row_smem / 2;
-      col_smem32 = col_smem / 2;
+    if (p->line_ok[r]) {
+      const int n[2] = {nx, ny};
+      for (int q = 0; q < 2; ++q) {
+        R.rtw[q] = reinterpret_cast<const double2*>(twiddles_reg(n[q], MGK_FP64));
+        if (mixed) R.rtw32[q] = reinterpret_cast<const float2*>(twiddles_reg(n[q], MGK_MIXED));
+        if (!R.rtw[q] || (mixed && !R.rtw32[q])) return fail(MGK_OOM);
+      }
+      int rc = ls2d_line_attrs(nx, ny, kLs2Fp64);
+      if (rc == MGK_OK && mixed) rc = ls2d_line_attrs(nx, ny, p->fast ? kLs2Fp32 : kLs2Fp32Wide);
+      if (rc) return fail(rc);
     }
+    row_smem = std::max(row_smem, 2 * 3 * (size_t)ny * c64);
+    col_smem = std::max(col_smem, 2 * 3 * (size_t)R.tc * nx * c64);
+    row_smem32 = row_smem / 2;
+    col_smem32 = col_smem / 2;
     p->maxN = std::max(p->maxN, R.N);
     p->total_row_items += R.row_items;
     p->total_col_items += R.col_items;
@@ -2085,50 +1249,15 @@ extern "C" int mgk_ls2d_create_batch(int nrep, const int* nxs, const int* nys, i
   p->col_smem = col_smem;
   p->row_smem32 = row_smem32;
   p->col_smem32 = col_smem32;
-  int st = p->fast ? ls2d_set_fast_attrs<double>(p->fast, row_smem, col_smem) : ls2d_set_attrs<double, double>(row_smem, col_smem);
-  if (st == MGK_OK && mixed)
-    st = p->fast ? ls2d_set_fast_attrs<float>(p->fast, row_smem32, col_smem32) : ls2d_set_attrs<float, float>(row_smem32, col_smem32);
+  int st = ls2d_set_attrs<double, double>(row_smem, col_smem);
+  if (st == MGK_OK && mixed) st = ls2d_set_attrs<float, float>(row_smem32, col_smem32);
   if (st) return fail(st);
-  {
-    // persistent bulk-prefetch row kernels: every replica needs ny even
-    bool ok = true;
-    int st64 = 0, st32 = 0, maxny = 0;
-    for (const Ls2dRep& R : p->reps) {
-      ok = ok && (R.ny % 2 == 0);
-      st64 = std::max(st64, (int)(6 * R.ld * sizeof(double2) + 16 * R.ny * sizeof(double)));
-      st32 = std::max(st32, (int)(6 * R.ld * sizeof(float2) + 16 * R.ny * sizeof(float)));
-      maxny = std::max(maxny, R.ny);
-    }
-    st64 = (st64 + 127) / 128 * 128;
-    st32 = (st32 + 127) / 128 * 128;
-    const size_t sm64 = 2 * (size_t)st64 + 3 * (size_t)maxny * sizeof(double2);
-    const size_t sm32 = 2 * (size_t)st32 + 3 * (size_t)maxny * sizeof(float2);
-    // opt-in: at 256-point lines the per-CTA FFT work, not load latency,
-    // bounds the row kernel, and the prefetching variant needs one CTA per SM
-    const char* env = getenv("MGK_TMA");
-    ok = ok && !p->fast && (env && env[0] == '1') && sm64 <= 220 * 1024;
-    int dev = 0;
-    if (ok && cudaGetDevice(&dev) == cudaSuccess &&
-        cudaDeviceGetAttribute(&p->num_sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess) {
-      p->stage64 = st64; p->stage32 = st32; p->tma_smem64 = sm64; p->tma_smem32 = sm32;
-      bool good = raise_smem((const void*)ls2d_row_tma_kernel<double, double, true>, (int)sm64) == cudaSuccess &&
-                  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p->occ64, ls2d_row_tma_kernel<double, double, true>,
-                                                                kThreads, sm64) == cudaSuccess;
-      if (good && mixed)
-        good = raise_smem((const void*)ls2d_row_tma_kernel<float, float, false>, (int)sm32) == cudaSuccess &&
-               raise_smem((const void*)ls2d_row_tma_kernel<float, float, true>, (int)sm32) == cudaSuccess &&
-               cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p->occ32, ls2d_row_tma_kernel<float, float, false>,
-                                                             kThreads, sm32) == cudaSuccess;
-      p->tma = good && p->occ64 > 0 && (!mixed || p->occ32 > 0);
-    }
-    cudaGetLastError();
-  }
   const int G = grid_blocks(p->maxN);
   p->part_doubles = std::max((size_t)2 * p->total_row_items, (size_t)nrep * G * 8);
   void* v = nullptr;
   if ((st = plan_alloc(p, &v, sizeof(double) * p->part_doubles))) return fail(st);
   p->d_part = reinterpret_cast<double*>(v);
-  if ((st = plan_alloc(p, &v, sizeof(double) * 2 * kPerVoxelBlocks))) return fail(st);
+  if ((st = plan_alloc(p, &v, sizeof(double) * 8 * kPerVoxelBlocks * nrep))) return fail(st);
   p->d_mat_part = reinterpret_cast<double*>(v);
   if ((st = plan_alloc(p, &v, sizeof(Ls2dRep) * nrep))) return fail(st);
   p->d_reps = reinterpret_cast<Ls2dRep*>(v);
@@ -2136,12 +1265,13 @@ extern "C" int mgk_ls2d_create_batch(int nrep, const int* nxs, const int* nys, i
   p->d_st = reinterpret_cast<Ls2dState*>(v);
   if ((st = plan_alloc(p, &v, sizeof(Ls2dCtl)))) return fail(st);
   p->d_ctl = reinterpret_cast<Ls2dCtl*>(v);
-  const size_t nmaps = 2 * (size_t)p->total_row_items + 2 * (size_t)std::max(p->total_col_items, total_col_max) + nrep;
+  const size_t nmaps = 2 * (size_t)p->total_row_items + 2 * (size_t)p->total_col_items + nrep;
   if ((st = plan_alloc(p, &v, sizeof(int) * nmaps))) return fail(st);
   p->d_maps = reinterpret_cast<int*>(v);
-  if ((st = plan_alloc(p, &v, sizeof(unsigned int) * nrep))) return fail(st);
+  if ((st = plan_alloc(p, &v, sizeof(unsigned int) * 2 * nrep))) return fail(st);
   p->d_repctr = reinterpret_cast<unsigned int*>(v);
-  if (cudaMemset(p->d_repctr, 0, sizeof(unsigned int) * nrep) != cudaSuccess ||
+  p->d_voxctr = p->d_repctr + nrep;
+  if (cudaMemset(p->d_repctr, 0, sizeof(unsigned int) * 2 * nrep) != cudaSuccess ||
       cudaMemset(p->d_st, 0, sizeof(Ls2dState) * nrep) != cudaSuccess ||
       cudaMemset(p->d_ctl, 0, sizeof(Ls2dCtl)) != cudaSuccess)
     return fail(MGK_CUDA_ERROR);
@@ -2185,14 +1315,10 @@ static int ls2d_set_fields(mgk_ls2d_t p, int rep, const double* E, const double*
     p->staged_pending = true;
   }
   const int grid = grid_blocks(R.N);
-  ls2d_material_kernel<<<grid, kThreads, 0, s>>>(p->d_reps, rep, E, nu, epsp, p->plane_mode, set_moduli,
-                                                 p->d_mat_part);
+  ls2d_material_kernel<<<grid, kThreads, 0, s>>>(p->d_reps, p->d_st, rep, E, nu, epsp, p->plane_mode, set_moduli,
+                                                 set_moduli == 2 ? (p->law == 2 ? 2 : 1) : 0, p->law_b,
+                                                 p->d_mat_part + (size_t)rep * 8 * kPerVoxelBlocks, p->d_voxctr + rep);
   MGK_CUDA(cudaGetLastError());
-  if (set_moduli) {
-    ls2d_medium_kernel<<<1, kThreads, 0, s>>>(p->d_reps, p->d_st, rep, p->d_mat_part, grid, p->plane_mode,
-                                              set_moduli == 2 ? (p->law == 2 ? 2 : 1) : 0, p->law_b);
-    MGK_CUDA(cudaGetLastError());
-  }
   return MGK_OK;
 }
 
@@ -2228,15 +1354,7 @@ static int ls2d_set_law(mgk_ls2d_t p, int law, double a, double b, int ps, const
   }
   p->law_a = a; p->law_b = b; p->law_ps = ps;
   if (law != p->law) {
-    for (auto& e : p->gcache) {
-      cudaGraphExecDestroy(e.x);
-      cudaGraphDestroy(e.g);
-    }
-    p->gcache.clear();
-    p->graph = nullptr;
-    p->exec = nullptr;
-    p->sel_rows = p->sel_cols = p->nsel = 0;  // the next solve builds its graph again
-    if (p->graph_mode == 1) p->graph_mode = -1;
+    ls2d_drop_graphs(p);
     p->law = law;
   }
   return MGK_OK;
@@ -2287,16 +1405,7 @@ extern "C" int mgk_ls2d_set_anderson(mgk_ls2d_t p, int m) {
   if (m == p->aa_m) return MGK_OK;
   int rc = staging_wait(p);
   if (rc) return rc;
-  // loop graphs hold the ring's address: rebuild them
-  for (auto& e : p->gcache) {
-    cudaGraphExecDestroy(e.x);
-    cudaGraphDestroy(e.g);
-  }
-  p->gcache.clear();
-  p->graph = nullptr;
-  p->exec = nullptr;
-  p->sel_rows = p->sel_cols = p->nsel = 0;
-  if (p->graph_mode == 1) p->graph_mode = -1;
+  ls2d_drop_graphs(p);  // loop graphs hold the ring's address: rebuild them
   if (m > 0) {
     const size_t need = (size_t)(3 + 2 * m) * 3 * (size_t)p->maxN;
     if (need > p->aa_doubles) {
@@ -2342,57 +1451,54 @@ extern "C" int mgk_ls2d_set_eigenstrain(mgk_ls2d_t p, const double* epsp, mgk_st
 
 // ------------------------------------------------------------- the loop ---
 
-struct LoopArgs {
-  const Ls2dRep* reps;
-  Ls2dState* st;
-  const int* row_map;
-  const int* row_local;
-  const int* col_map;
-  const int* col_local;
-  double* part;
-  unsigned int* repctr;
-  Ls2dCtl* ctl;
-  int rows, cols;
-  size_t row_smem, col_smem;
-  int tma;            // use the persistent bulk-prefetch row kernel
-  int row_grid;       // its grid (resident CTAs), <= rows
-  int stage_bytes;
-  size_t tma_smem;
-  int fast;           // warp-line iteration kernels
-  int law = 0;        // constitutive law of the warp-line row kernel (1: secant, 2: Rose, 3: Landau)
-  // Anderson mixing (FP64 loop of a one-replica selection; aa_m = 0: none)
-  int aa_m = 0;
-  int aa_nb = 0;
-  double* aa_buf = nullptr;
-  Ls2dAA* aa = nullptr;
-  double* aa_part = nullptr;
-  const int* sel = nullptr;
+struct Launch2 {
+  const void* fn;
+  dim3 grid, block;
+  size_t smem;
 };
 
-template <typename TS, bool IN_SPEC, bool FINAL>
-static void launch_row(const LoopArgs& a, cudaStream_t s) {
-  if (a.fast) {
-    void* fn = row_fast_fn<TS, IN_SPEC, FINAL>(a.fast, a.law);
-    cudaGraphConditionalHandle h = 0;
-    int zero = 0;
-    void* args[] = {(void*)&a.reps, (void*)&a.st, (void*)&a.row_map, (void*)&a.row_local, (void*)&a.part,
-                    (void*)&a.repctr, (void*)&a.ctl, &h, &zero, &zero};
-    cudaLaunchKernel(fn, dim3(a.rows), dim3(row_threads(a.fast)), args, a.row_smem, s);
-  } else {
-    ls2d_row_kernel<TS, TS, IN_SPEC, FINAL><<<a.rows, kThreads, a.row_smem, s>>>(
-        a.reps, a.st, a.row_map, a.row_local, a.part, a.repctr, a.ctl, 0, 0, 0);
+// Row stages of a group: 0 an iteration's, 1 the first of a phase (or of a
+// mixed iterate), 2 the first after the FP32 phase; -1 the column stage.
+enum { kCol = -1, kRow = 0, kFirst = 1, kPromote = 2 };
+
+// Calls f(launch, args) with a stage's launch and arguments; final: as
+// ls2d_decide's.
+template <typename F>
+static cudaError_t with_stage2(Loop2& a, Grp2& g, int stage, bool f32, int final, cudaGraphConditionalHandle h, int use,
+                               int cap, F f) {
+  if (g.ky) {
+    const Ls2Line *kx = f32 ? g.kx32 : g.kx, *ky = f32 ? g.ky32 : g.ky;
+    if (stage == kCol) {
+      const int w = f32 ? g.wc32 : g.wc;
+      void* x[] = {&a.reps, &a.st, &g.sel};
+      return f(Launch2{kx->col[w], dim3(g.n * ceil_div(g.nyh, kx->cols[w])), dim3(kx->c_threads[w]),
+                       (size_t)kx->c_bytes[w]}, x);
+    }
+    const int w = g.wr;
+    void* x[] = {&a.reps, &a.st, &g.sel, &a.part, &a.ctr, &a.ctl, &h, &use, &cap, &g.lead, &stage, &final};
+    return f(Launch2{ky->row[f32 ? 0 : a.law][w], dim3(g.n * ceil_div(g.nx / 2, ky->pairs[w])),
+                     dim3(ky->r_threads[w]), (size_t)ky->r_bytes[w]}, x);
   }
+  if (stage == kCol) {
+    void* x[] = {&a.reps, &a.st, &g.col_map, &g.col_local};
+    return f(Launch2{f32 ? (const void*)ls2d_col_kernel<float, float> : (const void*)ls2d_col_kernel<double, double>,
+                     dim3(g.cols), dim3(kThreads), f32 ? a.cs32 : a.cs}, x);
+  }
+  const void* fn = f32 ? (stage == kRow ? (final ? (const void*)ls2d_row_kernel<float, float, true, true>
+                                                 : (const void*)ls2d_row_kernel<float, float, true, false>)
+                                        : (const void*)ls2d_row_kernel<float, float, false, false>)
+                       : (stage == kRow ? (const void*)ls2d_row_kernel<double, double, true, true>
+                                        : (const void*)ls2d_row_kernel<double, double, false, true>);
+  void* x[] = {&a.reps, &a.st, &g.row_map, &g.row_local, &a.part, &a.ctr, &a.ctl, &h, &use, &cap};
+  return f(Launch2{fn, dim3(g.rows), dim3(kThreads), f32 ? a.rs32 : a.rs}, x);
 }
 
-template <typename TS>
-static void launch_col(const LoopArgs& a, cudaStream_t s) {
-  if (a.fast) {
-    void* fn = col_fast_fn<TS>(a.fast);
-    void* args[] = {(void*)&a.reps, (void*)&a.st, (void*)&a.col_map, (void*)&a.col_local};
-    cudaLaunchKernel(fn, dim3(a.cols), dim3(col_threads(a.fast)), args, a.col_smem, s);
-  } else {
-    ls2d_col_kernel<TS, TS><<<a.cols, kThreads, a.col_smem, s>>>(a.reps, a.st, a.col_map, a.col_local);
-  }
+static int launch2(Loop2& a, int stage, bool f32, int final, cudaStream_t s) {
+  for (Grp2& g : a.grp)
+    MGK_CUDA(with_stage2(a, g, stage, f32, final, 0, 0, 0, [&](const Launch2& L, void** args) {
+      return cudaLaunchKernel(L.fn, L.grid, L.block, args, L.smem, s);
+    }));
+  return MGK_OK;
 }
 
 // the history kernel of depth m (1..kAaMax)
@@ -2409,29 +1515,33 @@ static void* aa_update_fn(int m) {
   }
 }
 
-template <typename TS, bool FINAL>
-static int launch_body(const LoopArgs& a, cudaStream_t s) {
-  launch_col<TS>(a, s);
-  MGK_CUDA(cudaGetLastError());
-  if (a.tma)
-    ls2d_row_tma_kernel<TS, TS, FINAL><<<a.row_grid, kThreads, a.tma_smem, s>>>(
-        a.reps, a.st, a.row_map, a.row_local, a.part, a.repctr, a.ctl, 0, 0, 0, a.rows, a.stage_bytes);
-  else
-    launch_row<TS, true, FINAL>(a, s);
-  MGK_CUDA(cudaGetLastError());
-  if (sizeof(TS) == 8 && a.aa_m > 0) {
-    void* args[] = {(void*)&a.reps, (void*)&a.st, (void*)&a.sel, (void*)&a.aa_buf, (void*)&a.aa, (void*)&a.aa_m,
-                    (void*)&a.aa_part};
-    cudaLaunchKernel(aa_update_fn(a.aa_m), dim3(a.aa_nb), dim3(kAaThreads), args, 0, s);
-    launch_row<TS, false, FINAL>(a, s);  // the mix and tau of the mixed iterate
-    MGK_CUDA(cudaGetLastError());
+static int launch_body(Loop2& a, bool f32, cudaStream_t s) {
+  int rc = launch2(a, kCol, f32, !f32, s);
+  if (rc == MGK_OK) rc = launch2(a, kRow, f32, !f32, s);
+  if (rc == MGK_OK && !f32 && a.aa_m > 0) {
+    void* args[] = {&a.reps, &a.st, &a.sel, &a.aa_buf, &a.aa, &a.aa_m, &a.aa_part};
+    MGK_CUDA(cudaLaunchKernel(aa_update_fn(a.aa_m), dim3(a.aa_nb), dim3(kAaThreads), args, 0, s));
+    rc = launch2(a, kFirst, false, 1, s);  // the mix and tau of the mixed iterate
   }
-  return MGK_OK;
+  return rc;
 }
 
-template <typename TS, bool FINAL>
-static int add_while(cudaGraph_t g, cudaGraphNode_t* node, const cudaGraphNode_t* dep, int ndep, LoopArgs& a,
-                     int* guard_cap) {
+static cudaError_t add_node2(cudaGraph_t g, cudaGraphNode_t* node, const cudaGraphNode_t* dep, size_t ndep,
+                             const Launch2& L, void** args) {
+  cudaKernelNodeParams k;
+  memset(&k, 0, sizeof(k));
+  k.func = const_cast<void*>(L.fn);
+  k.gridDim = L.grid;
+  k.blockDim = L.block;
+  k.sharedMemBytes = (unsigned)L.smem;
+  k.kernelParams = args;
+  return cudaGraphAddKernelNode(node, g, dep, ndep, &k);
+}
+
+// One while node running iterations of the FP32 (phase 1) or FP64 kernels;
+// the groups' stages are independent chains of the body.
+static int add_while(cudaGraph_t g, cudaGraphNode_t* node, const cudaGraphNode_t* dep, size_t ndep, Loop2& a, bool f32,
+                     int cap) {
   cudaGraphConditionalHandle h;
   MGK_CUDA(cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault));
   // cudaGraphNodeParams has no default constructor in C++: zeroed storage
@@ -2444,114 +1554,55 @@ static int add_while(cudaGraph_t g, cudaGraphNode_t* node, const cudaGraphNode_t
   cp.conditional.size = 1;
   MGK_CUDA(cudaGraphAddNode(node, g, dep, ndep, &cp));
   cudaGraph_t body = cp.conditional.phGraph_out[0];
-  cudaKernelNodeParams k1;
-  memset(&k1, 0, sizeof(k1));
-  void* a1[] = {&a.reps, &a.st, &a.col_map, &a.col_local};
-  k1.func = a.fast ? col_fast_fn<TS>(a.fast) : (void*)ls2d_col_kernel<TS, TS>;
-  k1.gridDim = dim3(a.cols);
-  k1.blockDim = dim3(a.fast ? col_threads(a.fast) : kThreads);
-  k1.sharedMemBytes = (unsigned)a.col_smem;
-  k1.kernelParams = a1;
-  cudaGraphNode_t n1, n2;
-  MGK_CUDA(cudaGraphAddKernelNode(&n1, body, nullptr, 0, &k1));
-  int use_cond = 1;
-  cudaKernelNodeParams k2;
-  memset(&k2, 0, sizeof(k2));
-  void* a2[] = {&a.reps, &a.st, &a.row_map, &a.row_local, &a.part, &a.repctr, &a.ctl, &h, &use_cond, guard_cap};
-  void* a2t[] = {&a.reps, &a.st, &a.row_map, &a.row_local, &a.part, &a.repctr, &a.ctl, &h, &use_cond, guard_cap,
-                 &a.rows, &a.stage_bytes};
-  if (a.tma) {
-    k2.func = (void*)ls2d_row_tma_kernel<TS, TS, FINAL>;
-    k2.gridDim = dim3(a.row_grid);
-    k2.sharedMemBytes = (unsigned)a.tma_smem;
-    k2.kernelParams = a2t;
-    k2.blockDim = dim3(kThreads);
-  } else {
-    k2.func = a.fast ? row_fast_fn<TS, true, FINAL>(a.fast, a.law) : (void*)ls2d_row_kernel<TS, TS, true, FINAL>;
-    k2.gridDim = dim3(a.rows);
-    k2.sharedMemBytes = (unsigned)a.row_smem;
-    k2.kernelParams = a2;
-    k2.blockDim = dim3(a.fast ? row_threads(a.fast) : kThreads);
-  }
-  MGK_CUDA(cudaGraphAddKernelNode(&n2, body, &n1, 1, &k2));
-  if (sizeof(TS) == 8 && a.aa_m > 0) {
+  for (Grp2& gr : a.grp) {
+    cudaGraphNode_t prev, next;
+    MGK_CUDA(with_stage2(a, gr, kCol, f32, !f32, h, 1, cap, [&](const Launch2& L, void** args) {
+      return add_node2(body, &prev, nullptr, 0, L, args);
+    }));
+    MGK_CUDA(with_stage2(a, gr, kRow, f32, !f32, h, 1, cap, [&](const Launch2& L, void** args) {
+      return add_node2(body, &next, &prev, 1, L, args);
+    }));
+    if (f32 || a.aa_m == 0) continue;
     // Anderson history and least squares, then the mix and tau of the mixed
-    // iterate in the first row pass
-    cudaGraphNode_t n3, n6;
-    cudaKernelNodeParams k3, k6;
-    memset(&k3, 0, sizeof(k3));
-    memset(&k6, 0, sizeof(k6));
-    void* a3[] = {&a.reps, &a.st, &a.sel, &a.aa_buf, &a.aa, &a.aa_m, &a.aa_part};
-    k3.func = aa_update_fn(a.aa_m);
-    k3.gridDim = dim3(a.aa_nb);
-    k3.blockDim = dim3(kAaThreads);
-    k3.kernelParams = a3;
-    MGK_CUDA(cudaGraphAddKernelNode(&n3, body, &n2, 1, &k3));
-    cudaGraphConditionalHandle h0 = 0;
-    int zero = 0;
-    void* a6[] = {&a.reps, &a.st, &a.row_map, &a.row_local, &a.part, &a.repctr, &a.ctl, &h0, &zero, &zero};
-    k6.func = a.fast ? row_fast_fn<TS, false, FINAL>(a.fast, a.law) : (void*)ls2d_row_kernel<TS, TS, false, FINAL>;
-    k6.gridDim = dim3(a.rows);
-    k6.blockDim = dim3(a.fast ? row_threads(a.fast) : kThreads);
-    k6.sharedMemBytes = (unsigned)a.row_smem;
-    k6.kernelParams = a6;
-    MGK_CUDA(cudaGraphAddKernelNode(&n6, body, &n3, 1, &k6));
+    // iterate in the first row pass (one replica, one group)
+    cudaGraphNode_t hist, first;
+    void* ah[] = {&a.reps, &a.st, &a.sel, &a.aa_buf, &a.aa, &a.aa_m, &a.aa_part};
+    MGK_CUDA(add_node2(body, &hist, &next, 1, {aa_update_fn(a.aa_m), dim3(a.aa_nb), dim3(kAaThreads), 0}, ah));
+    MGK_CUDA(with_stage2(a, gr, kFirst, false, 1, 0, 0, 0, [&](const Launch2& L, void** args) {
+      return add_node2(body, &first, &hist, 1, L, args);
+    }));
   }
   return MGK_OK;
 }
 
-// Graph for the current selection: mixed plans run [phase-1 while, promote,
-// phase-2 setup, first FP64 row kernel] before the final while node.  It is
-// rebuilt when the selection's shape or the iteration cap changes.
-static int build_graph(mgk_ls2d_t p, LoopArgs& a64, LoopArgs& a32, const int* d_sel, int nsel, int G,
-                       int guard_cap) {
+// Graph of a selection: mixed plans run [phase-1 while, phase-2 set-up, first
+// FP64 row pass] before the final while node.
+static int build_graph(mgk_ls2d_t p, Loop2& a, int cap, cudaGraph_t* gout, cudaGraphExec_t* xout) {
   cudaGraph_t g = nullptr;
   MGK_CUDA(cudaGraphCreate(&g, 0));
-  int cap = guard_cap;
-  int rc = MGK_OK;
-  cudaGraphNode_t last;
-  if (p->prec == MGK_MIXED) {
-    cudaGraphNode_t w1, n_prom, n_ph2, n_row0;
-    rc = add_while<float, false>(g, &w1, nullptr, 0, a32, &cap);
-    if (rc == MGK_OK) {
-      cudaKernelNodeParams k;
-      memset(&k, 0, sizeof(k));
-      void* ap[] = {&a64.reps, (void*)&d_sel};
-      k.func = (void*)ls2d_promote_kernel;
-      k.gridDim = dim3(G, nsel);
-      k.blockDim = dim3(kThreads);
-      k.kernelParams = ap;
-      rc = cudaGraphAddKernelNode(&n_prom, g, &w1, 1, &k) == cudaSuccess ? MGK_OK : MGK_CUDA_ERROR;
+  auto build = [&]() -> int {
+    cudaGraphNode_t last;
+    if (p->prec != MGK_MIXED) return add_while(g, &last, nullptr, 0, a, false, cap);
+    cudaGraphNode_t w1, ph2;
+    int rc = add_while(g, &w1, nullptr, 0, a, true, cap);
+    if (rc) return rc;
+    if (!a.grp[0].ky) {  // the CTA-wide replicas' FP64 field
+      cudaGraphNode_t prom;
+      void* ap[] = {&a.reps, &a.sel};
+      MGK_CUDA(add_node2(g, &prom, &w1, 1, {(const void*)ls2d_promote_kernel, dim3(a.G, a.grp[0].n), dim3(kThreads), 0},
+                         ap));
+      w1 = prom;
     }
-    if (rc == MGK_OK) {
-      cudaKernelNodeParams k2;
-      memset(&k2, 0, sizeof(k2));
-      void* ap2[] = {&a64.st, (void*)&d_sel, &nsel, &a64.ctl};
-      k2.func = (void*)ls2d_phase2_kernel;
-      k2.gridDim = dim3(1);
-      k2.blockDim = dim3(32);
-      k2.kernelParams = ap2;
-      rc = cudaGraphAddKernelNode(&n_ph2, g, &n_prom, 1, &k2) == cudaSuccess ? MGK_OK : MGK_CUDA_ERROR;
-    }
-    if (rc == MGK_OK) {
-      cudaKernelNodeParams k3;
-      memset(&k3, 0, sizeof(k3));
-      cudaGraphConditionalHandle h0 = 0;
-      int zero = 0;
-      void* ap3[] = {&a64.reps, &a64.st, &a64.row_map, &a64.row_local, &a64.part, &a64.repctr, &a64.ctl,
-                     &h0, &zero, &zero};
-      k3.func = a64.fast ? row_fast_fn<double, false, true>(a64.fast, a64.law)
-                         : (void*)ls2d_row_kernel<double, double, false, true>;
-      k3.gridDim = dim3(a64.rows);
-      k3.blockDim = dim3(a64.fast ? row_threads(a64.fast) : kThreads);
-      k3.sharedMemBytes = (unsigned)a64.row_smem;
-      k3.kernelParams = ap3;
-      rc = cudaGraphAddKernelNode(&n_row0, g, &n_ph2, 1, &k3) == cudaSuccess ? MGK_OK : MGK_CUDA_ERROR;
-    }
-    if (rc == MGK_OK) rc = add_while<double, true>(g, &last, &n_row0, 1, a64, &cap);
-  } else {
-    rc = add_while<double, true>(g, &last, nullptr, 0, a64, &cap);
-  }
+    void* ap2[] = {&a.st, &a.sel, &a.nsel, &a.ctl};
+    MGK_CUDA(add_node2(g, &ph2, &w1, 1, {(const void*)ls2d_phase2_kernel, dim3(1), dim3(32), 0}, ap2));
+    std::vector<cudaGraphNode_t> row0(a.grp.size());
+    for (size_t i = 0; i < a.grp.size(); ++i)
+      MGK_CUDA(with_stage2(a, a.grp[i], kPromote, false, 1, 0, 0, 0, [&](const Launch2& L, void** args) {
+        return add_node2(g, &row0[i], &ph2, 1, L, args);
+      }));
+    return add_while(g, &last, row0.data(), row0.size(), a, false, cap);
+  };
+  int rc = build();
   cudaGraphExec_t x = nullptr;
   if (rc == MGK_OK && cudaGraphInstantiate(&x, g, 0) != cudaSuccess) rc = MGK_CUDA_ERROR;
   if (rc != MGK_OK) {
@@ -2559,61 +1610,17 @@ static int build_graph(mgk_ls2d_t p, LoopArgs& a64, LoopArgs& a32, const int* d_
     cudaGetLastError();
     return rc;
   }
-  constexpr size_t kMaxGraphs = 48;
-  if (p->gcache.size() >= kMaxGraphs) {
-    cudaGraphExecDestroy(p->gcache.front().x);
-    cudaGraphDestroy(p->gcache.front().g);
-    p->gcache.erase(p->gcache.begin());
-  }
-  p->gcache.push_back({a64.rows, a64.cols, nsel, guard_cap, a64.aa_m, g, x});
-  p->graph = g;
-  p->exec = x;
+  *gout = g;
+  *xout = x;
   return MGK_OK;
 }
 
-// Switches the plan's kernel family: 0 = CTA-wide passes, 256/512/1024 =
-// warp-line kernels for sides up to that length (at least the plan's
-// largest side).  Column tiles, shared-memory sizes and the cached loop
-// graphs follow the family.
+// Switches the plan's kernel family (see mgk_ls2d_plan::fast).
 static int ls2d_set_variant(mgk_ls2d_t p, int v) {
   MGK_REQUIRE(v == 0 || (p->fast_nat && v >= p->fast_nat && (v == 256 || v == 512 || v == 1024)),
               "mgk_ls2d: kernel family %d cannot serve this plan", v);
-  const size_t c64 = sizeof(double2);
-  size_t rs = 0, cs = 0, rs32 = 0, cs32 = 0;
-  int tot_cols = 0;
-  for (int r = 0; r < p->nrep; ++r) {
-    Ls2dRep& R = p->reps[r];
-    R.tc = v ? fast_col_tiles(v) : p->tc_gen[r];
-    R.col_items = (R.nyh + R.tc - 1) / R.tc;
-    tot_cols += R.col_items;
-    if (v) {
-      rs = std::max(rs, (size_t)row_fast_smem(R.ny, 16, 8));
-      cs = std::max(cs, (size_t)col_fast_smem(R.nx, 16, R.tc));
-      rs32 = std::max(rs32, (size_t)row_fast_smem(R.ny, 8, 4));
-      cs32 = std::max(cs32, (size_t)col_fast_smem(R.nx, 8, R.tc));
-    } else {
-      rs = std::max(rs, 2 * 3 * (size_t)R.ny * c64);
-      cs = std::max(cs, 2 * 3 * (size_t)R.tc * R.nx * c64);
-      rs32 = rs / 2;
-      cs32 = cs / 2;
-    }
-  }
-  int st = v ? ls2d_set_fast_attrs<double>(v, rs, cs) : ls2d_set_attrs<double, double>(rs, cs);
-  if (st == MGK_OK && p->prec == MGK_MIXED)
-    st = v ? ls2d_set_fast_attrs<float>(v, rs32, cs32) : ls2d_set_attrs<float, float>(rs32, cs32);
-  if (st) return st;
   p->fast = v;
-  p->total_col_items = tot_cols;
-  p->row_smem = rs; p->col_smem = cs; p->row_smem32 = rs32; p->col_smem32 = cs32;
-  for (auto& e : p->gcache) {
-    cudaGraphExecDestroy(e.x);
-    cudaGraphDestroy(e.g);
-  }
-  p->gcache.clear();
-  p->graph = nullptr;
-  p->exec = nullptr;
-  p->graph_mode = -1;
-  p->sel_rows = p->sel_cols = p->nsel = 0;
+  ls2d_drop_graphs(p);
   return MGK_OK;
 }
 
@@ -2629,11 +1636,10 @@ extern "C" int mgk_ls2d_set_family(mgk_ls2d_t p, int family) {
 extern "C" int mgk_ls2d_autotune(mgk_ls2d_t p, int nsel, const int* sel, const double* eps_bar, int reps,
                                  int* chosen, float* best_ms, mgk_stream_t stream) {
   MGK_REQUIRE(p && eps_bar && nsel >= 1 && reps >= 1, "mgk_ls2d_autotune: bad argument");
-  int cands[4];
+  // families 256/512/1024 share their kernels: the natural one stands for them
+  int cands[2];
   int nc = 0;
-  if (p->fast_nat)
-    for (int v : {256, 512, 1024})
-      if (v >= p->fast_nat) cands[nc++] = v;
+  if (p->fast_nat) cands[nc++] = p->fast_nat;
   cands[nc++] = 0;
   int best = p->fast;
   float best_t = 0.0f;
@@ -2688,6 +1694,63 @@ extern "C" int mgk_ls2d_collect(mgk_ls2d_t p, int nsel, const int* sel, mgk_ls_i
   return ls2d_collect(p, nsel, sel, infos, (cudaStream_t)stream);
 }
 
+// The selection by launch groups (the CTA-wide replicas first, then each
+// shape), its order and the loop's signature.  A group takes the wide forms
+// when these give at least two CTAs per SM.
+static void ls2d_group(mgk_ls2d_t p, const std::vector<int>& selv, Loop2& a, std::vector<int>& sig) {
+  const int nsel = (int)selv.size();
+  constexpr int kFill = 296;
+  a = Loop2();
+  a.reps = p->d_reps; a.st = p->d_st; a.part = p->d_part; a.ctr = p->d_repctr; a.ctl = p->d_ctl;
+  a.rs = p->row_smem; a.cs = p->col_smem; a.rs32 = p->row_smem32; a.cs32 = p->col_smem32;
+  a.sel = p->d_maps; a.nsel = nsel; a.G = grid_blocks(p->maxN); a.law = p->law;
+  p->order.clear();
+  Grp2 c;
+  for (int r : selv)
+    if (!ls2d_on_line(p, r)) {
+      p->order.push_back(r);
+      ++c.n;
+      c.rows += p->reps[r].row_items;
+      c.cols += p->reps[r].col_items;
+    }
+  c.row_map = p->d_maps + nsel;
+  c.row_local = c.row_map + c.rows;
+  c.col_map = c.row_local + c.rows;
+  c.col_local = c.col_map + c.cols;
+  sig = {p->law, p->aa_m, nsel, c.n, c.rows, c.cols};
+  if (c.n) a.grp.push_back(c);
+  std::vector<char> placed(p->nrep, 0);
+  for (int q = 0; q < nsel; ++q) {
+    const Ls2dRep& R = p->reps[selv[q]];
+    if (placed[selv[q]] || !ls2d_on_line(p, selv[q])) continue;
+    Grp2 g;
+    g.kx = ls2_line(R.nx, kLs2Fp64);
+    g.ky = ls2_line(R.ny, kLs2Fp64);
+    if (p->prec == MGK_MIXED) {
+      // the FP32 roundings of the kernels that the plan's family stands for
+      const int kind = p->fast ? kLs2Fp32 : kLs2Fp32Wide;
+      g.kx32 = ls2_line(R.nx, kind);
+      g.ky32 = ls2_line(R.ny, kind);
+    }
+    g.nx = R.nx;
+    g.nyh = R.nyh;
+    g.sel = p->d_maps + p->order.size();
+    for (int w = q; w < nsel; ++w) {
+      const int r = selv[w];
+      if (placed[r] || !ls2d_on_line(p, r) || p->reps[r].nx != R.nx || p->reps[r].ny != R.ny) continue;
+      placed[r] = 1;
+      p->order.push_back(r);
+      ++g.n;
+    }
+    g.wr = (long long)g.n * ceil_div(g.nx / 2, g.ky->pairs[1]) >= kFill;
+    g.wc = (long long)g.n * ceil_div(g.nyh, g.kx->cols[1]) >= kFill;
+    if (g.kx32) g.wc32 = (long long)g.n * ceil_div(g.nyh, g.kx32->cols[1]) >= kFill;
+    sig.insert(sig.end(), {R.nx, R.ny, g.n});
+    a.grp.push_back(g);
+  }
+  a.grp[0].lead = 1;
+}
+
 extern "C" int mgk_ls2d_solve_batch(mgk_ls2d_t p, int nsel, const int* sel, const double* eps_bar,
                                     const double* const* eps_init, double* const* eps_out, double* const* sig_out,
                                     int max_iter, double tol, mgk_ls_info* infos, mgk_stream_t stream) {
@@ -2712,35 +1775,40 @@ extern "C" int mgk_ls2d_solve_batch(mgk_ls2d_t p, int nsel, const int* sel, cons
   }
   int rc = staging_wait(p);
   if (rc) return rc;
-  // per-call fields and compact work maps
-  int rows = 0, cols = 0;
-  for (int q = 0; q < nsel; ++q) { rows += p->reps[selv[q]].row_items; cols += p->reps[selv[q]].col_items; }
-  const bool changed = rows != p->sel_rows || cols != p->sel_cols || nsel != p->nsel || p->aa_m != p->graph_aa;
-  int* row_map = p->h_maps;
-  int* row_local = row_map + rows;
-  int* col_map = row_local + rows;
-  int* col_local = col_map + cols;
-  int* selp = col_local + cols;
-  int ri = 0, ci = 0;
-  for (int q = 0; q < nsel; ++q) {
-    const int r = selv[q];
-    Ls2dRep& H = p->h_reps[r];
-    H = p->reps[r];
-    H.init = eps_init ? eps_init[q] : nullptr;
-    H.out_eps = eps_out ? eps_out[q] : nullptr;
-    H.out_sig = sig_out ? sig_out[q] : nullptr;
-    for (int k = 0; k < 4; ++k) H.eb[k] = eps_bar[4 * q + k];
-    H.tol = tol;
-    H.max_iter = max_iter;
-    H.aa = p->aa_m > 0 ? p->d_aa : nullptr;
-    H.aa_x = p->aa_m > 0 ? p->aa_buf : nullptr;
-    H.aa_dG = p->aa_m > 0 ? p->aa_buf + (size_t)(3 + p->aa_m) * 3 * (size_t)H.N : nullptr;
-    H.row_first = ri;
-    H.col_first = ci;
-    for (int i = 0; i < H.row_items; ++i) { row_map[ri] = r; row_local[ri] = i; ++ri; }
-    for (int i = 0; i < H.col_items; ++i) { col_map[ci] = r; col_local[ci] = i; ++ci; }
-    selp[q] = r;
-  }
+  Loop2& a = p->last;
+  std::vector<int> sig;
+  ls2d_group(p, selv, a, sig);
+  // per-call records, the selection and the CTA-wide group's maps
+  const Grp2& cg = a.grp[0];
+  int* row_map = p->h_maps + nsel;
+  int* row_local = row_map + cg.rows;
+  int* col_map = row_local + cg.rows;
+  int* col_local = col_map + cg.cols;
+  std::vector<int> at(p->nrep, 0);
+  for (int q = 0; q < nsel; ++q) at[selv[q]] = q;
+  int first = 0, k = 0, ri = 0, ci = 0;
+  for (const Grp2& g : a.grp)
+    for (int e = 0; e < g.n; ++e, ++k) {
+      const int r = p->order[k], q = at[r];
+      Ls2dRep& H = p->h_reps[r];
+      H = p->reps[r];
+      H.init = eps_init ? eps_init[q] : nullptr;
+      H.out_eps = eps_out ? eps_out[q] : nullptr;
+      H.out_sig = sig_out ? sig_out[q] : nullptr;
+      for (int c = 0; c < 4; ++c) H.eb[c] = eps_bar[4 * q + c];
+      H.tol = tol;
+      H.max_iter = max_iter;
+      H.aa = p->aa_m > 0 ? p->d_aa : nullptr;
+      H.aa_x = p->aa_m > 0 ? p->aa_buf : nullptr;
+      H.aa_dG = p->aa_m > 0 ? p->aa_buf + (size_t)(3 + p->aa_m) * 3 * (size_t)H.N : nullptr;
+      if (g.ky) H.row_items = ceil_div(H.nx / 2, g.ky->pairs[g.wr]);
+      H.row_first = first;
+      first += H.row_items;
+      p->h_maps[k] = r;
+      if (g.ky) continue;
+      for (int i = 0; i < H.row_items; ++i) { row_map[ri] = r; row_local[ri] = i; ++ri; }
+      for (int i = 0; i < H.col_items; ++i) { col_map[ci] = r; col_local[ci] = i; ++ci; }
+    }
   const int n_active = max_iter > 0 ? nsel : 0;
   p->h_ctl->n_active = (unsigned int)n_active;
   p->h_ctl->decided = 0;
@@ -2748,101 +1816,69 @@ extern "C" int mgk_ls2d_solve_batch(mgk_ls2d_t p, int nsel, const int* sel, cons
   p->h_ctl->bodies = 0;
   p->h_ctl->any = n_active > 0;
   p->h_ctl->error = 0;
-  const size_t nm = 2 * (size_t)rows + 2 * (size_t)cols + nsel;
+  const size_t nm = nsel + 2 * (size_t)(ri + ci);
   MGK_CUDA(cudaMemcpyAsync(p->d_maps, p->h_maps, sizeof(int) * nm, cudaMemcpyHostToDevice, s));
   MGK_CUDA(cudaMemcpyAsync(p->d_reps, p->h_reps, sizeof(Ls2dRep) * p->nrep, cudaMemcpyHostToDevice, s));
   MGK_CUDA(cudaMemcpyAsync(p->d_ctl, p->h_ctl, sizeof(Ls2dCtl), cudaMemcpyHostToDevice, s));
   MGK_CUDA(cudaEventRecord(p->staged, s));
   p->staged_pending = true;
-  p->sel_rows = rows;
-  p->sel_cols = cols;
-  p->nsel = nsel;
 
-  const int* d_row_map = p->d_maps;
-  const int* d_row_local = d_row_map + rows;
-  const int* d_col_map = d_row_local + rows;
-  const int* d_col_local = d_col_map + cols;
-  const int* d_sel = d_col_local + cols;
-  const int G = grid_blocks(p->maxN);
+  const int* d_sel = a.sel;
+  const int G = a.G;
+  const bool mixed = p->prec == MGK_MIXED;
   bool any_init = false;
   for (int q = 0; q < nsel && eps_init; ++q) any_init |= eps_init[q] != nullptr;
-  if (any_init) {
-    ls2d_means_kernel<<<dim3(G, nsel), kThreads, 0, s>>>(p->d_reps, d_sel, p->d_part);
-    MGK_CUDA(cudaGetLastError());
-    ls2d_finalize_kernel<<<nsel, kThreads, 0, s>>>(p->d_reps, p->d_st, d_sel, p->d_part, G, 4,
-                                                   (int)offsetof(Ls2dState, means), 1);
-    MGK_CUDA(cudaGetLastError());
-  }
-  ls2d_begin_kernel<<<dim3(G, nsel), kThreads, 0, s>>>(p->d_reps, p->d_st, d_sel, p->d_part);
+  if (any_init)
+    ls2d_means_kernel<<<dim3(G, nsel), kThreads, 0, s>>>(p->d_reps, p->d_st, d_sel, p->d_part, p->d_voxctr);
+  ls2d_begin_kernel<<<dim3(G, nsel), kThreads, 0, s>>>(p->d_reps, p->d_st, d_sel, p->d_part, p->d_voxctr,
+                                                       mixed && n_active > 0);
   MGK_CUDA(cudaGetLastError());
-  if (any_init) {
-    ls2d_finalize_kernel<<<nsel, kThreads, 0, s>>>(p->d_reps, p->d_st, d_sel, p->d_part, G, 2,
-                                                   (int)offsetof(Ls2dState, extra_d0), 2);
-    MGK_CUDA(cudaGetLastError());
-  }
   if (n_active > 0) {
-    const bool mixed = p->prec == MGK_MIXED;
-    LoopArgs a64{p->d_reps, p->d_st, d_row_map, d_row_local, d_col_map, d_col_local, p->d_part, p->d_repctr,
-                 p->d_ctl, rows, cols, p->row_smem, p->col_smem, p->tma, 0, p->stage64, p->tma_smem64, p->fast};
-    a64.row_grid = std::max(1, std::min(rows, p->occ64 * p->num_sms));
-    a64.law = p->law;
-    LoopArgs a32 = a64;
-    a32.law = 0;
     if (p->aa_m > 0) {
-      a64.aa_m = p->aa_m;
-      a64.aa_nb = p->aa_nb;
-      a64.aa_buf = p->aa_buf;
-      a64.aa = p->d_aa;
-      a64.aa_part = p->aa_part;
-      a64.sel = d_sel;
+      a.aa_m = p->aa_m;
+      a.aa_nb = p->aa_nb;
+      a.aa_buf = p->aa_buf;
+      a.aa = p->d_aa;
+      a.aa_part = p->aa_part;
       ls2d_aa_init_kernel<<<p->aa_nb, kThreads, 0, s>>>(p->d_reps, d_sel, p->aa_buf, p->d_aa);
       MGK_CUDA(cudaGetLastError());
     }
-    a32.row_smem = p->row_smem32;
-    a32.col_smem = p->col_smem32;
-    a32.stage_bytes = p->stage32;
-    a32.tma_smem = p->tma_smem32;
-    a32.row_grid = std::max(1, std::min(rows, p->occ32 * p->num_sms));
-    if (mixed) launch_row<float, false, false>(a32, s);
-    else launch_row<double, false, true>(a64, s);
-    MGK_CUDA(cudaGetLastError());
-    const int guard_cap = (max_iter + 2 > 1000 ? max_iter + 2 : 1000);
-    if (p->graph_mode == 1 && (changed || guard_cap > p->graph_cap)) {
-      bool hit = false;
+    if ((rc = launch2(a, kFirst, mixed, !mixed, s))) return rc;
+    const int cap = (max_iter + 2 > 1000 ? max_iter + 2 : 1000);
+    const char* env = getenv("MGK_NO_GRAPH_WHILE");
+    if (env && env[0] == '1') p->graph_mode = 0;
+    cudaGraphExec_t exec = nullptr;
+    if (p->graph_mode == 1) {
       for (auto& e : p->gcache)
-        if (e.rows == rows && e.cols == cols && e.nsel == nsel && e.cap >= guard_cap && e.aa == p->aa_m) {
-          p->graph = e.g;
-          p->exec = e.x;
-          p->graph_cap = e.cap;
-          p->graph_aa = e.aa;
-          hit = true;
-          break;
+        if (e.cap >= cap && e.sig == sig) exec = e.x;
+      if (!exec) {
+        cudaGraph_t g;
+        if (build_graph(p, a, cap, &g, &exec) == MGK_OK) {
+          constexpr size_t kMaxGraphs = 48;
+          if (p->gcache.size() >= kMaxGraphs) {
+            cudaGraphExecDestroy(p->gcache.front().x);
+            cudaGraphDestroy(p->gcache.front().g);
+            p->gcache.erase(p->gcache.begin());
+          }
+          p->gcache.push_back({sig, cap, g, exec});
+        } else {
+          p->graph_mode = 0;
         }
-      if (!hit) p->graph_mode = -1;
-    }
-    if (p->graph_mode < 0) {
-      const char* env = getenv("MGK_NO_GRAPH_WHILE");
-      if (env && env[0] == '1') p->graph_mode = 0;
-      else {
-        p->graph_mode = build_graph(p, a64, a32, d_sel, nsel, G, guard_cap) == MGK_OK ? 1 : 0;
-        p->graph_cap = guard_cap;
-        p->graph_aa = p->aa_m;
       }
     }
     if (p->graph_mode == 1) {
-      MGK_CUDA(cudaGraphLaunch(p->exec, s));
+      MGK_CUDA(cudaGraphLaunch(exec, s));
     } else {
       // host-driven loop: poll the device flag after each iteration
       for (int phase = mixed ? 1 : 2; phase <= 2; ++phase) {
         if (phase == 2 && mixed) {
-          ls2d_promote_kernel<<<dim3(G, nsel), kThreads, 0, s>>>(p->d_reps, d_sel);
+          if (!a.grp[0].ky) ls2d_promote_kernel<<<dim3(G, a.grp[0].n), kThreads, 0, s>>>(p->d_reps, d_sel);
           ls2d_phase2_kernel<<<1, 32, 0, s>>>(p->d_st, d_sel, nsel, p->d_ctl);
-          launch_row<double, false, true>(a64, s);
           MGK_CUDA(cudaGetLastError());
+          if ((rc = launch2(a, kPromote, false, 1, s))) return rc;
         }
         for (int it = 0; it < max_iter; ++it) {
-          rc = (phase == 1) ? launch_body<float, false>(a32, s) : launch_body<double, true>(a64, s);
-          if (rc) return rc;
+          if ((rc = launch_body(a, phase == 1, s))) return rc;
           Ls2dCtl hc;
           MGK_CUDA(cudaMemcpyAsync(&hc, p->d_ctl, sizeof(Ls2dCtl), cudaMemcpyDeviceToHost, s));
           MGK_CUDA(cudaStreamSynchronize(s));
@@ -2851,13 +1887,11 @@ extern "C" int mgk_ls2d_solve_batch(mgk_ls2d_t p, int nsel, const int* sel, cons
       }
     }
   }
-  if (p->law == 1) ls2d_output_kernel<1><<<dim3(G, nsel), kThreads, 0, s>>>(p->d_reps, p->d_st, d_sel, p->d_part);
-  else if (p->law == 2) ls2d_output_kernel<2><<<dim3(G, nsel), kThreads, 0, s>>>(p->d_reps, p->d_st, d_sel, p->d_part);
-  else if (p->law == 3) ls2d_output_kernel<3><<<dim3(G, nsel), kThreads, 0, s>>>(p->d_reps, p->d_st, d_sel, p->d_part);
-  else ls2d_output_kernel<<<dim3(G, nsel), kThreads, 0, s>>>(p->d_reps, p->d_st, d_sel, p->d_part);
-  MGK_CUDA(cudaGetLastError());
-  ls2d_finalize_kernel<<<nsel, kThreads, 0, s>>>(p->d_reps, p->d_st, d_sel, p->d_part, G, 8,
-                                                 (int)offsetof(Ls2dState, out_eps_mean), 0);
+  auto out = p->law == 1   ? ls2d_output_kernel<1>
+             : p->law == 2 ? ls2d_output_kernel<2>
+             : p->law == 3 ? ls2d_output_kernel<3>
+                           : ls2d_output_kernel<0>;
+  out<<<dim3(G, nsel), kThreads, 0, s>>>(p->d_reps, p->d_st, d_sel, p->d_part, p->d_voxctr);
   MGK_CUDA(cudaGetLastError());
   if (infos) return ls2d_collect(p, nsel, selv.data(), infos, s);
   return MGK_OK;
@@ -2872,44 +1906,26 @@ extern "C" int mgk_ls2d_solve(mgk_ls2d_t p, const double* eps_bar, const double*
 
 // ----------------------------------------------------------- profiling ---
 
-template <typename TS>
-static int profile_t(mgk_ls2d_t p, float* row_ms, float* col_ms, int reps, cudaStream_t s) {
-  const int rows = p->sel_rows, cols = p->sel_cols;
-  const int* d_row_map = p->d_maps;
-  const int* d_row_local = d_row_map + rows;
-  const int* d_col_map = d_row_local + rows;
-  const int* d_col_local = d_col_map + cols;
-  const size_t rs = sizeof(TS) == 8 ? p->row_smem : p->row_smem32;
-  const size_t cs = sizeof(TS) == 8 ? p->col_smem : p->col_smem32;
-  LoopArgs a{p->d_reps, p->d_st, d_row_map, d_row_local, d_col_map, d_col_local, p->d_part, p->d_repctr,
-             p->d_ctl, rows, cols, rs, cs, 0, 0, 0, 0, p->fast};
-  a.law = sizeof(TS) == 8 ? p->law : 0;
-  launch_row<TS, false, true>(a, s);
-  MGK_CUDA(cudaGetLastError());
+// times the stages of the plan's last selection
+static int profile_stages(mgk_ls2d_t p, bool f32, float* row_ms, float* col_ms, int reps, cudaStream_t s) {
+  Loop2& a = p->last;
+  int rc = launch2(a, kFirst, f32, 1, s);
+  if (rc) return rc;
   cudaEvent_t ev[3];
   for (int i = 0; i < 3; ++i) MGK_CUDA(cudaEventCreate(&ev[i]));
   float tr = 0, tc = 0;
-  int rc = MGK_OK;
-  for (int r = 0; r < reps; ++r) {
+  for (int r = 0; r < reps && rc == MGK_OK; ++r) {
     cudaEventRecord(ev[0], s);
-    launch_col<TS>(a, s);
+    rc = launch2(a, kCol, f32, 1, s);
     cudaEventRecord(ev[1], s);
-    if (p->tma) {
-      const bool f64 = sizeof(TS) == 8;
-      const int grid = std::max(1, std::min(rows, (f64 ? p->occ64 : p->occ32) * p->num_sms));
-      ls2d_row_tma_kernel<TS, TS, true><<<grid, kThreads, f64 ? p->tma_smem64 : p->tma_smem32, s>>>(
-          p->d_reps, p->d_st, d_row_map, d_row_local, p->d_part, p->d_repctr, p->d_ctl, 0, 0, 0, rows,
-          f64 ? p->stage64 : p->stage32);
-    } else {
-      launch_row<TS, true, true>(a, s);
-    }
+    if (rc == MGK_OK) rc = launch2(a, kRow, f32, 1, s);
     cudaEventRecord(ev[2], s);
     if (cudaEventSynchronize(ev[2]) != cudaSuccess) { rc = MGK_CUDA_ERROR; break; }
-    float a = 0, b = 0;
-    cudaEventElapsedTime(&a, ev[0], ev[1]);
-    cudaEventElapsedTime(&b, ev[1], ev[2]);
-    tc += a;
-    tr += b;
+    float x = 0, y = 0;
+    cudaEventElapsedTime(&x, ev[0], ev[1]);
+    cudaEventElapsedTime(&y, ev[1], ev[2]);
+    tc += x;
+    tr += y;
   }
   for (int i = 0; i < 3; ++i) cudaEventDestroy(ev[i]);
   MGK_CUDA(cudaGetLastError());
@@ -2949,7 +1965,7 @@ extern "C" int mgk_ls2d_profile_batch(mgk_ls2d_t p, int nsel, const int* sel, co
   p->h_ctl->bodies = 0;
   MGK_CUDA(cudaMemcpyAsync(p->d_ctl, p->h_ctl, sizeof(Ls2dCtl), cudaMemcpyHostToDevice, s));
   MGK_CUDA(cudaStreamSynchronize(s));
-  return fp32 ? profile_t<float>(p, row_ms, col_ms, reps, s) : profile_t<double>(p, row_ms, col_ms, reps, s);
+  return profile_stages(p, fp32 != 0, row_ms, col_ms, reps, s);
 }
 
 extern "C" int mgk_ls2d_profile(mgk_ls2d_t p, const double* eps_bar, int reps, float* row_ms, float* col_ms,
@@ -3046,7 +2062,8 @@ __global__ void ls2d_noalloc_setup_kernel(Ls2dRep rep, Ls2dRep* dst, Ls2dState* 
   if (t == 0) {
     *dst = rep;
     sel[0] = 0;
-    *repctr = 0;
+    repctr[0] = 0;
+    repctr[1] = 0;
     Ls2dState z;
     memset(&z, 0, sizeof(z));
     *st = z;
@@ -3122,6 +2139,7 @@ extern "C" int mgk_ls2d_solve_noalloc(int nx, int ny, int plane_mode, const doub
   Ls2dState* d_st = reinterpret_cast<Ls2dState*>(misc + kNaState);
   Ls2dCtl* d_ctl = reinterpret_cast<Ls2dCtl*>(misc + kNaCtl);
   unsigned int* d_ctr = reinterpret_cast<unsigned int*>(misc + kNaCtr);
+  unsigned int* d_vox = d_ctr + 1;  // arrival counter of the per-voxel kernels
   int* d_maps = reinterpret_cast<int*>(misc + kNaMaps);
   static_assert(sizeof(Ls2dRep) <= 1024 && sizeof(Ls2dState) <= 1024 && sizeof(Ls2dCtl) <= 64,
                 "no-alloc record sizes");
@@ -3149,36 +2167,25 @@ extern "C" int mgk_ls2d_solve_noalloc(int nx, int ny, int plane_mode, const doub
                                               max_iter > 0 ? 1 : 0, twx, nx, twy, ny);
   MGK_CUDA(cudaGetLastError());
   const int G = grid_blocks(N);
-  ls2d_material_kernel<<<G, kThreads, 0, s>>>(d_rep, 0, E, nu, eps_plastic, plane_mode, 1, part);
+  ls2d_material_kernel<<<G, kThreads, 0, s>>>(d_rep, d_st, 0, E, nu, eps_plastic, plane_mode, 1, 0, 0.0, part, d_vox);
   MGK_CUDA(cudaGetLastError());
-  ls2d_medium_kernel<<<1, kThreads, 0, s>>>(d_rep, d_st, 0, part, G, plane_mode, 0, 0.0);
+  if (eps_init) ls2d_means_kernel<<<dim3(G, 1), kThreads, 0, s>>>(d_rep, d_st, d_sel, part, d_vox);
+  ls2d_begin_kernel<<<dim3(G, 1), kThreads, 0, s>>>(d_rep, d_st, d_sel, part, d_vox, 0);
   MGK_CUDA(cudaGetLastError());
-  if (eps_init) {
-    ls2d_means_kernel<<<dim3(G, 1), kThreads, 0, s>>>(d_rep, d_sel, part);
-    ls2d_finalize_kernel<<<1, kThreads, 0, s>>>(d_rep, d_st, d_sel, part, G, 4, (int)offsetof(Ls2dState, means), 1);
-    MGK_CUDA(cudaGetLastError());
-  }
-  ls2d_begin_kernel<<<dim3(G, 1), kThreads, 0, s>>>(d_rep, d_st, d_sel, part);
-  MGK_CUDA(cudaGetLastError());
-  if (eps_init) {
-    ls2d_finalize_kernel<<<1, kThreads, 0, s>>>(d_rep, d_st, d_sel, part, G, 2, (int)offsetof(Ls2dState, extra_d0),
-                                                1);
-    MGK_CUDA(cudaGetLastError());
-  }
   if (max_iter > 0) {
     ls2d_row_kernel<double, double, false, true><<<rows, kThreads, row_smem, s>>>(
         d_rep, d_st, d_row_map, d_row_local, part, d_ctr, d_ctl, 0, 0, 0);
     MGK_CUDA(cudaGetLastError());
     // host-driven loop in chunks of 4 iterations; finished replicas skip
     // their work on the device, and the host polls the activity flag
-    LoopArgs a{d_rep, d_st, d_row_map, d_row_local, d_col_map, d_col_local, part, d_ctr, d_ctl, rows, cols,
-               row_smem, col_smem};
     int it = 0;
     while (it < max_iter) {
       const int chunk = max_iter - it < 4 ? max_iter - it : 4;
       for (int c = 0; c < chunk; ++c) {
-        st = launch_body<double, true>(a, s);
-        if (st != MGK_OK) return st;
+        ls2d_col_kernel<double, double><<<cols, kThreads, col_smem, s>>>(d_rep, d_st, d_col_map, d_col_local);
+        ls2d_row_kernel<double, double, true, true><<<rows, kThreads, row_smem, s>>>(
+            d_rep, d_st, d_row_map, d_row_local, part, d_ctr, d_ctl, 0, 0, 0);
+        MGK_CUDA(cudaGetLastError());
       }
       it += chunk;
       Ls2dCtl hc;
@@ -3187,10 +2194,7 @@ extern "C" int mgk_ls2d_solve_noalloc(int nx, int ny, int plane_mode, const doub
       if (!hc.any) break;
     }
   }
-  ls2d_output_kernel<<<dim3(G, 1), kThreads, 0, s>>>(d_rep, d_st, d_sel, part);
-  MGK_CUDA(cudaGetLastError());
-  ls2d_finalize_kernel<<<1, kThreads, 0, s>>>(d_rep, d_st, d_sel, part, G, 8, (int)offsetof(Ls2dState, out_eps_mean),
-                                              0);
+  ls2d_output_kernel<0><<<dim3(G, 1), kThreads, 0, s>>>(d_rep, d_st, d_sel, part, d_vox);
   MGK_CUDA(cudaGetLastError());
   Ls2dState h;
   MGK_CUDA(cudaMemcpyAsync(&h, d_st, sizeof(Ls2dState), cudaMemcpyDeviceToHost, s));

@@ -31,9 +31,9 @@ constexpr int round32(int n) { return (n + 31) / 32 * 32; }
 // Line pairs per z-line CTA, and its threads: those of the transforms, and
 // enough for the voxel stage to run in one round of at most 192 voxel pairs or
 // two equal ones (at 128 points 96 threads would take three rounds).
-constexpr int ls3_zp(int n) { return reg_sched(n).t <= 9 ? 2 : 1; }
-constexpr int ls3_z_threads(int n) {
-  const int fft = 6 * reg_sched(n).t * ls3_zp(n), vox = ls3_zp(n) * n, rounds = (vox + 191) / 192;
+constexpr int ls3_zp(int n) { return reg_sched64(n).t <= 9 ? 2 : 1; }
+constexpr int ls3_z_threads(int n, int csz) {
+  const int fft = 6 * reg_sched(n, csz).t * ls3_zp(n), vox = ls3_zp(n) * n, rounds = (vox + 191) / 192;
   const int per = (vox + rounds - 1) / rounds;
   return round32(fft > per ? fft : per);
 }
@@ -45,15 +45,15 @@ constexpr int ls3_ld(int n) { return (n / 2 + 1 + 3) / 4 * 4; }
 // half of it the exchanges and Gamma0): tiles of 2 columns (79 us) and a third
 // resident CTA at 96 registers (77 us) were slower than this (70 us).
 constexpr int ls3_tile(int n, int csz) {
-  return csz == 8 ? 8 : 6 * 4 * reg_sched(n).t <= 432 ? 4 : 2;
+  return csz == 8 ? 8 : 6 * 4 * reg_sched64(n).t <= 432 ? 4 : 2;
 }
-constexpr int ls3_ax_threads(int n, int csz, int nc) { return round32(nc * ls3_tile(n, csz) * reg_sched(n).t); }
+constexpr int ls3_ax_threads(int n, int csz, int nc) { return round32(nc * ls3_tile(n, csz) * reg_sched(n, csz).t); }
 // exchange buffers; they first hold the pairs' spectrum rows as copied
 constexpr int ls3_z_bytes(int n, int csz) {
-  const int a = ls3_zp(n) * 6 * reg_slots(n), b = ls3_zp(n) * 12 * ls3_ld(n);
+  const int a = ls3_zp(n) * 6 * reg_slots(n, csz), b = ls3_zp(n) * 12 * ls3_ld(n);
   return (a > b ? a : b) * csz;
 }
-constexpr int ls3_ax_bytes(int n, int csz, int nc) { return nc * ls3_tile(n, csz) * reg_slots(n) * csz; }
+constexpr int ls3_ax_bytes(int n, int csz, int nc) { return nc * ls3_tile(n, csz) * reg_slots(n, csz) * csz; }
 // resident CTAs asked of the register allocator: 128 registers per thread in
 // FP64, 80 in FP32
 constexpr int ls3_minb(int threads, int csz) {
@@ -90,12 +90,13 @@ __device__ __forceinline__ void l2_prefetch(const void* p, uint32_t bytes) {
 // previous spectrum is inverted and the field updated.  lead: this launch
 // counts the loop bodies.
 template <typename T, int NZ, bool FINAL, int LAW>
-__global__ void __launch_bounds__(ls3_z_threads(NZ), ls3_minb(ls3_z_threads(NZ), 2 * (int)sizeof(T)))
+__global__ void __launch_bounds__(ls3_z_threads(NZ, 2 * (int)sizeof(T)),
+                                  ls3_minb(ls3_z_threads(NZ, 2 * (int)sizeof(T)), 2 * (int)sizeof(T)))
     ls3_zline_reg(const Ls3dRep* __restrict__ reps, Ls3dState* st, const int* __restrict__ sel, double* partials,
                   unsigned int* rep_counter, Ls3dCtl* ctl, cudaGraphConditionalHandle cond, int use_cond,
                   int guard_cap, int lead, int first) {
   using C = C_t<T>;
-  constexpr int TL = reg_sched(NZ).t, P = ls3_zp(NZ), TH = ls3_z_threads(NZ), SL = reg_slots(NZ);
+  constexpr int TL = reg_sched(NZ, sizeof(C)).t, P = ls3_zp(NZ), TH = ls3_z_threads(NZ, sizeof(C)), SL = reg_slots(NZ, sizeof(C));
   constexpr int NZH = NZ / 2 + 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double red[32];
@@ -145,7 +146,7 @@ __global__ void __launch_bounds__(ls3_z_threads(NZ), ls3_minb(ls3_z_threads(NZ),
   C* buf = lines + (line < 6 * P ? line : 0) * SL;
   C* ra = L3F<T>::spec(R) + c * plane + 2 * (p0 + pr) * ld;  // the pair's two rows: ra, ra + ld
   auto at = [&](int s) -> C& { return buf[s]; };
-  auto put = [&](int i, C v) { buf[reg_slot<NZ>(i)] = v; };
+  auto put = [&](int i, C v) { buf[reg_slot<NZ, C>(i)] = v; };
   auto sync = [] {
     if constexpr (32 % TL == 0) __syncwarp();
     else __syncthreads();
@@ -163,7 +164,7 @@ __global__ void __launch_bounds__(ls3_z_threads(NZ), ls3_minb(ls3_z_threads(NZ),
       if (k == 0 || 2 * k == NZ) { a.y = 0; b.y = 0; }
       return 2 * k <= NZ ? mk<C>(a.x - b.y, a.y + b.x) : mk<C>(a.x + b.y, b.x - a.y);
     };
-    reg_line<NZ, +1, C>(t, act, tw, load, at, put, sync, [] { __syncthreads(); });
+    reg_line<NZ, +1, 0, C>(t, act, tw, load, at, put, sync, [] { __syncthreads(); });
   }
   __syncthreads();
   const double mu0 = S.mu0, lam0 = S.lam0;
@@ -171,7 +172,7 @@ __global__ void __launch_bounds__(ls3_z_threads(NZ), ls3_minb(ls3_z_threads(NZ),
 #pragma unroll 1
   for (int e = threadIdx.x; e < np * NZ; e += TH) {
     const int q = e / NZ, z = e - q * NZ;
-    C* vx = lines + q * 6 * SL + reg_slot<NZ>(z);
+    C* vx = lines + q * 6 * SL + reg_slot<NZ, C>(z);
     // every input of the two voxels before the first store
     T o[2][6], m[2], l[2], pl[2][6];
 #pragma unroll
@@ -227,12 +228,12 @@ __global__ void __launch_bounds__(ls3_z_threads(NZ), ls3_minb(ls3_z_threads(NZ),
     for (int k = 0; k < 6; ++k) vx[k * SL] = mk<C>(tr[0][k], tr[1][k]);
   }
   __syncthreads();
-  reg_line<NZ, -1, C>(t, act, tw, [&](int i) -> C { return buf[reg_slot<NZ>(i)]; }, at, put, sync, sync);
+  reg_line<NZ, -1, 0, C>(t, act, tw, [&](int i) -> C { return buf[reg_slot<NZ, C>(i)]; }, at, put, sync, sync);
   sync();
   if (act) {
     for (int k = t; k < NZH; k += TL) {
-      const C z = buf[reg_slot<NZ>(k)];
-      const C w = buf[reg_slot<NZ>(k == 0 ? 0 : NZ - k)];
+      const C z = buf[reg_slot<NZ, C>(k)];
+      const C w = buf[reg_slot<NZ, C>(k == 0 ? 0 : NZ - k)];
       ra[k] = mk<C>(T(0.5) * (z.x + w.x), T(0.5) * (z.y - w.y));
       ra[ld + k] = mk<C>(T(0.5) * (z.y + w.y), T(-0.5) * (z.x - w.x));
     }
@@ -252,7 +253,7 @@ __global__ void __launch_bounds__(ls3_ax_threads(NL, 2 * (int)sizeof(T), AXIS ? 
                                   ls3_minb(ls3_ax_threads(NL, 2 * (int)sizeof(T), AXIS ? 3 : 6), 2 * (int)sizeof(T)))
     ls3_axis_reg(const Ls3dRep* __restrict__ reps, const Ls3dState* __restrict__ st, const int* __restrict__ sel) {
   using C = C_t<T>;
-  constexpr int NC = AXIS ? 3 : 6, TL = reg_sched(NL).t, W = ls3_tile(NL, sizeof(C)), SL = reg_slots(NL);
+  constexpr int NC = AXIS ? 3 : 6, TL = reg_sched(NL, sizeof(C)).t, W = ls3_tile(NL, sizeof(C)), SL = reg_slots(NL, sizeof(C));
   constexpr int TH = ls3_ax_threads(NL, sizeof(C), NC);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int c0 = (blockIdx.x % (6 / NC)) * NC;
@@ -283,14 +284,14 @@ __global__ void __launch_bounds__(ls3_ax_threads(NL, 2 * (int)sizeof(T), AXIS ? 
   };
   auto load = [&](int i) -> C { return g[i * js]; };
   if constexpr (AXIS) {
-    reg_line<NL, SIGN, C>(t, act, tw, load, at, [&](int i, C v) { g[i * js] = v; }, sync, [] {});
+    reg_line<NL, SIGN, 0, C>(t, act, tw, load, at, [&](int i, C v) { g[i * js] = v; }, sync, [] {});
   } else {
-    auto put = [&](int i, C v) { buf[reg_slot<NL>(i) * W] = v; };
-    reg_line<NL, -1, C>(t, act, tw, load, at, put, sync, [] {});
+    auto put = [&](int i, C v) { buf[reg_slot<NL, C>(i) * W] = v; };
+
+    reg_line<NL, -1, 0, C>(t, act, tw, load, at, put, sync, [] {});
     __syncthreads();
     // Gamma0 in the precision of the pass: FP64 iterations in double, the
-    // FP32 phase of a mixed plan in float.  With u the wave vector, n = u/|u|
-    // only enters squared, so one division by |u|^2 replaces the square root.
+    // FP32 phase of a mixed plan in float
     const T scale = T(1.0 / (double)R.N);
     const T a0 = (T)S.inv2mu0, b0 = (T)S.Bc;
     const T uy = (T)fftfreq3(o, ny) / (T)ny;
@@ -299,29 +300,47 @@ __global__ void __launch_bounds__(ls3_ax_threads(NL, 2 * (int)sizeof(T), AXIS ? 
     for (int e = threadIdx.x; e < W * NL; e += TH) {
       const int w = e % W, kx = e / W, kz = k0 + w;
       if (w >= tcw) continue;
-      C* p = lines + reg_slot<NL>(kx) * W + w;
+      C* p = lines + reg_slot<NL, C>(kx) * W + w;
       C tv[6];
 #pragma unroll
       for (int k = 0; k < 6; ++k) tv[k] = p[k * (SL * W)];
       const T ux = (T)fftfreq3(kx, nx) / (T)nx, uz = (T)fftfreq3(kz, nz) / (T)nz;
       const T uu = ux * ux + uy * uy + uz * uz;
-      const T i2 = uu > T(0) ? T(1) / uu : T(0);  // the mean stays zero
       const bool nqx = (nx & 1) == 0 && 2 * kx == nx, nqz = (nz & 1) == 0 && 2 * kz == nz;
       const bool nq = nqx || nqy || nqz;
-      const T f = (nq ? T(0.5) : T(1)) * scale * i2;
       C ev[6];
-      gamma3d_apply_t<T>(tv, ux, uy, uz, a0 * f, b0 * f * i2, ev);
-      if (nq) {
-        C fv[6];
-        gamma3d_apply_t<T>(tv, nqx ? -ux : ux, nqy ? -uy : uy, nqz ? -uz : uz, a0 * f, b0 * f * i2, fv);
+      if constexpr (sizeof(T) == 8) {
+        // with u the wave vector, n = u/|u| only enters squared, so one
+        // division by |u|^2 replaces the square root
+        const T i2 = uu > T(0) ? T(1) / uu : T(0);  // the mean stays zero
+        const T f = (nq ? T(0.5) : T(1)) * scale * i2;
+        gamma3d_apply_t<T>(tv, ux, uy, uz, a0 * f, b0 * f * i2, ev);
+        if (nq) {
+          C fv[6];
+          gamma3d_apply_t<T>(tv, nqx ? -ux : ux, nqy ? -uy : uy, nqz ? -uz : uz, a0 * f, b0 * f * i2, fv);
 #pragma unroll
-        for (int k = 0; k < 6; ++k) ev[k] = cadd(ev[k], fv[k]);
+          for (int k = 0; k < 6; ++k) ev[k] = cadd(ev[k], fv[k]);
+        }
+      } else {
+        // the roundings of the FP32 passes (see reg_sched32)
+        const T inv = T(1) / sqrt(uu), n0 = ux * inv, n1 = uy * inv, n2 = uz * inv;
+        gamma3d_apply_t<T>(tv, n0, n1, n2, a0, b0, ev);
+        if (nq) {
+          C fv[6];
+          gamma3d_apply_t<T>(tv, nqx ? -n0 : n0, nqy ? -n1 : n1, nqz ? -n2 : n2, a0, b0, fv);
+#pragma unroll
+          for (int k = 0; k < 6; ++k) ev[k] = mk<C>(T(0.5) * (ev[k].x + fv[k].x), T(0.5) * (ev[k].y + fv[k].y));
+        }
+        const bool mean = kx == 0 && o == 0 && kz == 0;
+#pragma unroll
+        for (int k = 0; k < 6; ++k)
+          ev[k] = mean ? mk<C>(T(0), T(0)) : mk<C>(ev[k].x * scale, ev[k].y * scale);
       }
 #pragma unroll
       for (int k = 0; k < 6; ++k) p[k * (SL * W)] = ev[k];
     }
     __syncthreads();
-    reg_line<NL, +1, C>(t, act, tw, [&](int i) -> C { return buf[reg_slot<NL>(i) * W]; }, at,
+    reg_line<NL, +1, 0, C>(t, act, tw, [&](int i) -> C { return buf[reg_slot<NL, C>(i) * W]; }, at,
                         [&](int i, C v) { g[i * js] = v; }, sync, sync);
   }
 }
@@ -351,7 +370,7 @@ template <typename T, int N, bool FINAL> static const Ls3Line* ls3_make() {
     k.y[1] = (const void*)ls3_axis_reg<T, N, 1, 1>;
     k.x = (const void*)ls3_axis_reg<T, N, 0, 0>;
     k.zp = ls3_zp(N);
-    k.z_threads = ls3_z_threads(N);
+    k.z_threads = ls3_z_threads(N, cs);
     k.tile = ls3_tile(N, cs);
     k.y_threads = ls3_ax_threads(N, cs, 3);
     k.x_threads = ls3_ax_threads(N, cs, 6);

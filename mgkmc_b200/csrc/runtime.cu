@@ -93,23 +93,31 @@ const void* twiddles(int n, int prec) {
   return d;
 }
 
-// Step twiddles of the register FFT of length n: for each step s >= 1 the
-// entries W_{NS R}^{r k} at [r - 1][k], k < NS; one table per (device, n,
-// precision), kept until process exit.
+// Twiddles of the register FFT of length n: for each pass after the first
+// (the steps' radices in FP64; make_sched's passes in FP32, the angle as m / n
+// there, so that the floats are those of twiddles()) the entries W_{NS R}^{r k}
+// at [r - 1][k], k < NS; one table per (device, n, precision), kept until
+// process exit.
 template <typename C> static void fill_reg(int n, std::vector<C>& h) {
-  const RegSched q = reg_sched(n);
-  int ns = q.r[0];
-  for (int s = 1; s < q.ns; ++s) {
-    for (int r = 1; r < q.r[s]; ++r)
+  const RegSched q = reg_sched(n, sizeof(C));
+  std::vector<int> pass;
+  for (int s = 0; s < q.ns; ++s) {
+    const int rb = sizeof(C) == 16 ? 1 : q.rb[s];
+    pass.push_back(q.r[s] / rb);
+    if (rb > 1) pass.push_back(rb);
+  }
+  int ns = pass[0];
+  for (size_t p = 1; p < pass.size(); ++p) {
+    for (int r = 1; r < pass[p]; ++r)
       for (int k = 0; k < ns; ++k) {
-        const long double ang =
-            -2.0L * 3.14159265358979323846264338327950288L * (long double)(r * k) / (long double)(ns * q.r[s]);
+        const int m = r * k * (n / (ns * pass[p]));
+        const long double ang = -2.0L * 3.14159265358979323846264338327950288L * (long double)m / (long double)n;
         C c;
         c.x = (decltype(C::x))cosl(ang);
         c.y = (decltype(C::x))sinl(ang);
         h.push_back(c);
       }
-    ns *= q.r[s];
+    ns *= pass[p];
   }
 }
 
