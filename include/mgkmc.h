@@ -317,10 +317,9 @@ MGK_API int mgk_fs3d_destroy(mgk_fs3d_t plan);
  * reference's C4); Fp: device (3,3,nx,ny,nz) plastic deformation gradient or
  * NULL (no F_p: the reference's tangent branch without F_p). */
 /* Precision form of the Krylov matvecs: MGK_FP64 (default), or MGK_MIXED:
- * the tangent product K:dF, the FFTs and the projection of the CG matvecs in
- * FP32, while the Newton right-hand side (-G:P, -G:K:DbarF), the CG vectors x
- * and r, every inner product and norm, the line search and the macro loop
- * stay FP64.  No counterpart in the reference (FP64 only). */
+ * the tangent product K:dF, the FFTs, the projection and the vectors of CG in
+ * FP32, while the Newton right-hand side (-G:P, -G:K:DbarF), every inner product
+ * and norm, the line search and the macro loop stay FP64.  No counterpart in the reference (FP64 only). */
 MGK_API int mgk_fs3d_set_precision(mgk_fs3d_t plan, int precision);
 MGK_API int mgk_fs3d_set_material(mgk_fs3d_t plan, const double* lam, const double* mu, const double* Fp,
                                   mgk_stream_t stream);
@@ -363,16 +362,18 @@ MGK_API int mgk_fs3d_set_plane_strain(mgk_fs3d_t plan, int on);
  * J = det(F) F33. */
 MGK_API int mgk_fs3d_set_plane_stress(mgk_fs3d_t plan, int on);
 /* Autotuner: times one Krylov iteration of each kernel family that can serve
- * the plan (warp-line passes, sides 64/96/128; CTA-wide passes) on the current
- * state and keeps the faster; *chosen 1 warp-line, 0 CTA-wide.  Call after a
+ * the plan (register FFTs on the axes that have one, in the mixed form warp-line
+ * passes for sides 64/96/128; CTA-wide passes) on the current state and keeps
+ * the faster; *chosen 1 register or warp-line, 0 CTA-wide.  Call after a
  * step (the state must be valid); leaves the Krylov vectors unspecified.  No
  * counterpart in the reference. */
 MGK_API int mgk_fs3d_autotune(mgk_fs3d_t plan, int reps, int* chosen, float* best_ms, mgk_stream_t stream);
-/* Timing hook: mean duration (ms, CUDA events on `stream`) of the six kernels
- * of one Krylov iteration (z forward with K:p, y pass, x pass with G, inverse
- * y pass, z inverse with p.q, CG update), ms_out[6]; fp32 = 1 times the mixed
- * form's FP32 kernels.  Leaves the Krylov vectors in an unspecified state.
- * No counterpart in the reference. */
+/* Timing hook: mean duration (ms, CUDA events on `stream`) of the six stages
+ * of one Krylov iteration, ms_out[6]: z stage with K:p, forward y, forward x with
+ * G and p.q, inverse y, inverse x with the direction, CG update; fp32 = 1 the
+ * mixed form's FP32 kernels: z forward with K:p, y, x with G, inverse y, z
+ * inverse with p.q, CG update.  Leaves the Krylov vectors in an unspecified
+ * state.  No counterpart in the reference. */
 MGK_API int mgk_fs3d_profile(mgk_fs3d_t plan, int fp32, int reps, float* ms_out, mgk_stream_t stream);
 
 /* ------------------------------------------------------ 2D STZ / KMC --- */

@@ -56,8 +56,8 @@ def build_finite_strain_bc_3d(driving_component, eps_target_step, mixed_targets,
 
 class Fs3dSolver:
     """Plan-owning 3D finite-strain solver on one device.  ``precision``:
-    "fp64" (the reference's arithmetic) or "mixed" (FP32 Krylov matvecs; the
-    Newton residual, CG vectors, inner products and norms stay FP64)."""
+    "fp64" (the reference's arithmetic) or "mixed" (FP32 Krylov matvecs and
+    vectors; the Newton residual, inner products and norms stay FP64)."""
 
     def __init__(self, nx, ny, nz, model="svk", device=None, precision="fp64"):
         torch = _torch()
@@ -107,16 +107,17 @@ class Fs3dSolver:
         return np.array(out[:]).reshape(3, 3), self.info
 
     def profile_kernels(self, fp32=False, reps=20, stream=None):
-        """Mean ms of the six kernels of one Krylov iteration (z fwd, y, x+G,
-        y inv, z inv, update); leaves the Krylov vectors unspecified."""
+        """Mean ms of the six stages of one Krylov iteration (FP64: z with K:p,
+        y, x+G, y inv, x inv, update; FP32: z fwd with K:p, y, x+G, y inv,
+        z inv, update); leaves the Krylov vectors unspecified."""
         ms = (ctypes.c_float * 6)()
         L.check(L.lib().mgk_fs3d_profile(self._h, 1 if fp32 else 0, int(reps), ms, L.stream_ptr(stream)),
                 "mgk_fs3d_profile")
         return list(ms)
 
     def autotune(self, reps=5, stream=None):
-        """Keeps the faster kernel family (1 warp-line, 0 CTA-wide) for this
-        plan, timed on its current state (call after a step)."""
+        """Keeps the faster kernel family (1 register or warp-line FFTs, 0
+        CTA-wide) for this plan, timed on its current state (call after a step)."""
         ch, ms = ctypes.c_int(), ctypes.c_float()
         L.check(L.lib().mgk_fs3d_autotune(self._h, int(reps), ctypes.byref(ch), ctypes.byref(ms),
                                           L.stream_ptr(stream)), "mgk_fs3d_autotune")

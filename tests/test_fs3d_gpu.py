@@ -175,3 +175,32 @@ def test_autotune_keeps_results():
         s.get(F)
         Fs.append(F.cpu().numpy())
     assert rel(Fs[1], Fs[0]) < 1e-10
+
+
+@pytest.mark.parametrize("shape,model,with_fp", [((24, 27, 32), "neo_hookean", True), ((36, 48, 54), "svk", True),
+                                                 ((72, 2, 81), "neo_hookean", False), ((96, 3, 108), "svk", False),
+                                                 ((128, 4, 144), "neo_hookean", True), ((162, 1, 192), "svk", True),
+                                                 ((3, 216, 24), "neo_hookean", True), ((2, 243, 27), "neo_hookean", False),
+                                                 ((256, 1, 256), "neo_hookean", True), ((4, 192, 243), "svk", True)])
+def test_register_lines_match_general_passes(shape, model, with_fp, monkeypatch):
+    # every line length with a register FFT, on each axis beside axes without
+    # one, against the general passes (which the oracle tests pin): the same
+    # FP64 operations, so the fields of one converged load step agree to
+    # rounding (bounds of the test above)
+    import torch
+    from mgkmc_b200.finite_strain_simulator import Fs3dSolver, build_finite_strain_bc_3d
+    lam, mu, Fp = W.fs3d_material_dev(*shape, 3, "cuda")
+    out = []
+    for flag in ("1", "0"):
+        monkeypatch.setenv("MGK_FS_FAST", flag)
+        s = Fs3dSolver(*shape, model=model)
+        s.set_material(lam, mu, Fp if with_fp else None)
+        F = torch.eye(3, dtype=torch.float64, device="cuda").reshape(3, 3, 1, 1, 1).expand(3, 3, *shape).contiguous()
+        s.set_F(F)
+        Fb, _, Pt, Pm = build_finite_strain_bc_3d((0, 0), 0.005, {(1, 1): 0.0, (2, 2): 0.0})
+        s.step(Fb, (0, 0), Pt, Pm, 90e9, 0.35, 1e-10, 1e-9, 40, 1e3, 40)
+        P = torch.empty_like(F)
+        s.get(F, P)
+        out.append((F.cpu().numpy(), P.cpu().numpy()))
+    assert rel(out[0][0], out[1][0]) < 1e-10
+    assert rel(out[0][1], out[1][1]) < 1e-9
