@@ -362,10 +362,9 @@ MGK_API int mgk_fs3d_set_plane_strain(mgk_fs3d_t plan, int on);
  * J = det(F) F33. */
 MGK_API int mgk_fs3d_set_plane_stress(mgk_fs3d_t plan, int on);
 /* Autotuner: times one Krylov iteration of each kernel family that can serve
- * the plan (register FFTs on the axes that have one, in the mixed form warp-line
- * passes for sides 64/96/128; CTA-wide passes) on the current state and keeps
- * the faster; *chosen 1 register or warp-line, 0 CTA-wide.  Call after a
- * step (the state must be valid); leaves the Krylov vectors unspecified.  No
+ * the plan (register FFTs on the axes that have one; CTA-wide passes) on the
+ * current state and keeps the faster; *chosen 1 register, 0 CTA-wide.  Call
+ * after a step (the state must be valid); leaves the Krylov vectors unspecified.  No
  * counterpart in the reference. */
 MGK_API int mgk_fs3d_autotune(mgk_fs3d_t plan, int reps, int* chosen, float* best_ms, mgk_stream_t stream);
 /* Timing hook: mean duration (ms, CUDA events on `stream`) of the six stages

@@ -50,6 +50,7 @@
 #include "fs3d_dev.cuh"
 #include "fs3d_line.cuh"
 #include "fs3d_mixed.cuh"
+#include "fs3d_mixed_line.cuh"
 
 namespace mgk {
 
@@ -64,6 +65,17 @@ const FsLine* fs_line(int n) {
     if (const FsLine* k = f(n)) return k;
   return nullptr;
 }
+
+namespace fs32 {
+const MixedLine* mixed_line_0(int n);
+const MixedLine* mixed_line_1b(int n);
+const MixedLine* mixed_line_1c(int n);
+const MixedLine* mixed_line(int n, int alt) {
+  if (!alt) return mixed_line_0(n);
+  const MixedLine* k = mixed_line_1b(n);
+  return k ? k : mixed_line_1c(n);
+}
+}  // namespace fs32
 
 template <typename T> __device__ __forceinline__ T det3(const T* A) {
   return A[0] * (A[4] * A[8] - A[5] * A[7]) - A[1] * (A[3] * A[8] - A[5] * A[6]) + A[2] * (A[3] * A[7] - A[4] * A[6]);
@@ -619,11 +631,13 @@ struct mgk_fs3d_plan {
   int prec = MGK_FP64;
   float* f32 = nullptr;  // p, q, r, x, F_p^-1, and the FP64 tangent state of its right-hand sides
   FftLen fft32[3];
+  const void* rtw32[3];
+  const fs32::MixedLine* line32[3];
   // device-side Krylov loop graphs, one per precision (0 FP64, 1 FP32)
   cudaGraph_t cg_graph[2] = {nullptr, nullptr};
   cudaGraphExec_t cg_exec[2] = {nullptr, nullptr};
   int graph_mode = -1;  // -1 untried, 1 graphs, 0 host-driven loop
-  int fast = 1;         // register-FFT (FP32: warp-line) kernels where the sides have them
+  int fast = 1;         // register-FFT kernels on the axes that have them
   // plane strain embedded as (nx, 1, ny): the out-of-plane F_yy = 1 adds N
   // to ||F||^2, which the 2D solver's Newton norm does not contain
   double ff_offset = 0.0;
@@ -656,6 +670,7 @@ static fs32::Fs32Args fs32_args(mgk_fs3d_t p) {
   a.N = p->N; a.has_fp = p->has_fp; a.model = p->model;
   a.fx = p->fft[0]; a.fy = p->fft[1]; a.fz = p->fft[2];
   a.fx32 = p->fft32[0]; a.fy32 = p->fft32[1]; a.fz32 = p->fft32[2];
+  for (int q = 0; q < 3; ++q) a.rtw32[q] = p->rtw32[q];
   a.Fpi = p->Fpi; a.P = p->P; a.r = p->X;
   float* f = p->f32;
   a.p32 = f; a.q32 = f + 9 * p->N; a.r32 = f + 18 * p->N; a.x32 = f + 27 * p->N; a.Fpi32 = f + 36 * p->N;
@@ -665,6 +680,8 @@ static fs32::Fs32Args fs32_args(mgk_fs3d_t p) {
   a.part = p->part; a.sc = p->sc;
   return a;
 }
+// whether the right-hand side takes the warp-line passes (and the FP32 passes
+// their roundings)
 static bool fs32_fast(mgk_fs3d_t p) {
   return p->fast && fs32::fs_fast_len(p->nx) && fs32::fs_fast_len(p->ny) && fs32::fs_fast_len(p->nz);
 }
@@ -722,41 +739,47 @@ static FsLaunch fs_x_launch(mgk_fs3d_t p, int inverse, int kind) {
   return {fn, p->ny * ((p->nzh + p->tcx - 1) / p->tcx), 256, p->xsmem};
 }
 
-// The launches of one mixed-form matvec (mode 0) or right-hand side (FP64; mode 1
-// uniform, 2 P): z forward with the tangent product, y, x with G, y inverse, z
-// inverse; returns their number.
-template <typename T> static int fs32_matvec(mgk_fs3d_t p, int mode, FsLaunch L[6]) {
+// The CTA-wide passes' launches (T float: the matvec's; double: a right-hand
+// side's, mode 1 uniform, 2 P): z forward, y, x with G, y inverse, z inverse.
+template <typename T> static void fs32_general(mgk_fs3d_t p, int mode, FsLaunch L[5]) {
   using namespace fs32;
   constexpr int zm = sizeof(T) == 8 ? 1 : 0;  // z inverse: q and p.q, or r and r.r
+  const int zl = (int)(p->N / p->nz / 2), ntile = (p->nzh + p->tc - 1) / p->tc;
+  const size_t zs = p->zsmem * sizeof(T) / 8, ys = 2 * 9 * (size_t)p->tc * p->ny * 2 * sizeof(T),
+               xs = 2 * 9 * (size_t)p->tc * p->nx * 2 * sizeof(T);
+  if constexpr (zm == 0) L[0] = {(const void*)fs_zfwd_kernel<0, T>, zl, 256, zs};
+  else L[0] = {mode == 1 ? (const void*)fs_zfwd_kernel<1, T> : (const void*)fs_zfwd_kernel<2, T>, zl, 256, zs};
+  L[1] = {(const void*)fs_ypass_kernel<-1, T>, p->nx * ntile, 256, ys};
+  L[2] = {(const void*)fs_xg_kernel<T>, p->ny * ntile, 256, xs};
+  L[3] = {(const void*)fs_ypass_kernel<1, T>, p->nx * ntile, 256, ys};
+  L[4] = {(const void*)fs_zinv_kernel<zm, T>, zl, 256, zs};
+}
+static void fs32_rhs(mgk_fs3d_t p, int mode, FsLaunch L[5]) {
+  using namespace fs32;
+  if (!fs32_fast(p)) return fs32_general<double>(p, mode, L);
+  const int zl = (int)(p->N / p->nz / 2), ntile = 3 * ((p->nzh + kFsTile - 1) / kFsTile);
+  const size_t zs = 9 * (size_t)fs_pl(p->nz) * 16, ys = 3 * (size_t)kFsTile * fs_pl(p->ny) * 16,
+               xs = 3 * (size_t)kFsTile * fs_pl(p->nx) * 16;
+  L[0] = {mode == 1 ? (const void*)fs_zfwd_fast_kernel<1> : (const void*)fs_zfwd_fast_kernel<2>, zl, 96, zs};
+  L[1] = {(const void*)fs_axis_fast_kernel<-1, false>, p->nx * ntile, 96, ys};
+  L[2] = {(const void*)fs_axis_fast_kernel<-1, true>, p->ny * ntile, 96, xs};
+  L[3] = {(const void*)fs_axis_fast_kernel<1, false>, p->nx * ntile, 96, ys};
+  L[4] = {(const void*)fs_zinv_fast64_kernel, zl, 96, zs};
+}
+// the matvec's launches: register FFTs on the axes that have one
+static void fs32_matvec(mgk_fs3d_t p, FsLaunch L[5]) {
+  fs32_general<float>(p, 0, L);
+  if (!p->fast) return;
   const int zl = (int)(p->N / p->nz / 2);
-  int k = 0;
-  if (fs32_fast(p)) {
-    constexpr int csz = 2 * (int)sizeof(T), ncy = fs_axis_nc(false, sizeof(T)), ncx = fs_axis_nc(true, sizeof(T));
-    const int ntile = (p->nzh + kFsTile - 1) / kFsTile;
-    const size_t zs = 9 * (size_t)fs_pl(p->nz, csz) * csz;
-    const size_t ys = ncy * (size_t)kFsTile * fs_pl(p->ny, csz) * csz, xs = ncx * (size_t)kFsTile * fs_pl(p->nx, csz) * csz;
-    if constexpr (zm == 0) {
-      L[k++] = {(const void*)fs_kp_kernel, 4 * p->nblk, 256, 0};
-      L[k++] = {(const void*)fs_zfwd_fast_kernel<3, T>, zl, 96, zs};
-    } else {
-      L[k++] = {mode == 1 ? (const void*)fs_zfwd_fast_kernel<1, T> : (const void*)fs_zfwd_fast_kernel<2, T>, zl, 96, zs};
-    }
-    L[k++] = {(const void*)fs_axis_fast_kernel<-1, T, false>, p->nx * ntile * (9 / ncy), 32 * ncy, ys};
-    L[k++] = {(const void*)fs_axis_fast_kernel<-1, T, true>, p->ny * ntile * (9 / ncx), 32 * ncx, xs};
-    L[k++] = {(const void*)fs_axis_fast_kernel<1, T, false>, p->nx * ntile * (9 / ncy), 32 * ncy, ys};
-    L[k++] = {fs_zinv_fast_fn<zm, T>(), zl, 96, zs};
-  } else {
-    const int ntile = (p->nzh + p->tc - 1) / p->tc;
-    const size_t zs = p->zsmem * sizeof(T) / 8, ys = 2 * 9 * (size_t)p->tc * p->ny * 2 * sizeof(T),
-                 xs = 2 * 9 * (size_t)p->tc * p->nx * 2 * sizeof(T);
-    if constexpr (zm == 0) L[k++] = {(const void*)fs_zfwd_kernel<0, T>, zl, 256, zs};
-    else L[k++] = {mode == 1 ? (const void*)fs_zfwd_kernel<1, T> : (const void*)fs_zfwd_kernel<2, T>, zl, 256, zs};
-    L[k++] = {(const void*)fs_ypass_kernel<-1, T>, p->nx * ntile, 256, ys};
-    L[k++] = {(const void*)fs_xg_kernel<T>, p->ny * ntile, 256, xs};
-    L[k++] = {(const void*)fs_ypass_kernel<1, T>, p->nx * ntile, 256, ys};
-    L[k++] = {(const void*)fs_zinv_kernel<zm, T>, zl, 256, zs};
+  if (const fs32::MixedLine* k = p->line32[2]) {
+    L[0] = {k->zfwd, (zl + k->zp - 1) / k->zp, k->zf_threads, (size_t)k->zf_bytes};
+    L[4] = {k->zinv, zl, k->zi_threads, (size_t)k->zi_bytes};
   }
-  return k;
+  if (const fs32::MixedLine* k = p->line32[1])
+    for (int inv = 0; inv < 2; ++inv)
+      L[inv ? 3 : 1] = {k->y[inv], 3 * p->nx * ((p->nzh + k->yw - 1) / k->yw), k->y_threads, (size_t)k->y_bytes};
+  if (const fs32::MixedLine* k = p->line32[0])
+    L[2] = {k->x, p->ny * ((p->nzh + k->xw - 1) / k->xw), k->x_threads, (size_t)k->x_bytes};
 }
 
 // Raise the shared-memory limits of the kernels that the plan launches in its
@@ -766,10 +789,13 @@ static int fs_raise(mgk_fs3d_t p) {
   cudaError_t e = cudaSuccess;
   auto up = [&](const FsLaunch& l) { if (e == cudaSuccess && l.smem > 46 * 1024) e = raise_smem(l.fn, l.smem); };
   if (p->prec == MGK_MIXED) {
-    FsLaunch L[6];
-    for (int k = fs32_matvec<float>(p, 0, L); k-- > 0;) up(L[k]);
-    for (int m = 1; m < 3; ++m)
-      for (int k = fs32_matvec<double>(p, m, L); k-- > 0;) up(L[k]);
+    FsLaunch L[5];
+    fs32_matvec(p, L);
+    for (const FsLaunch& l : L) up(l);
+    for (int m = 1; m < 3; ++m) {
+      fs32_rhs(p, m, L);
+      for (const FsLaunch& l : L) up(l);
+    }
   }
   // a mixed plan's FP64 kernels run under the profiler
   for (int m = 0; m < 4; ++m) up(fs_z_launch(p, m));
@@ -867,8 +893,12 @@ extern "C" int mgk_fs3d_set_precision(mgk_fs3d_t p, int precision) {
   MGK_REQUIRE(precision == MGK_FP64 || precision == MGK_MIXED, "mgk_fs3d_set_precision: bad precision");
   if (precision == MGK_MIXED && !p->f32) {
     const int n[3] = {p->nx, p->ny, p->nz};
-    for (int q = 0; q < 3; ++q)
-      if (!(p->fft32[q].tw = twiddles(n[q], 1))) return MGK_OOM;
+    const bool alt = !fs32_fast(p);
+    for (int q = 0; q < 3; ++q) {
+      p->line32[q] = fs32::mixed_line(n[q], alt);
+      p->rtw32[q] = p->line32[q] ? twiddles_reg(n[q], MGK_MIXED) : nullptr;
+      if (!(p->fft32[q].tw = twiddles(n[q], 1)) || (p->line32[q] && !p->rtw32[q])) return MGK_OOM;
+    }
     // one allocation: the FP32 planes (an even number of floats), the FP64 state
     if (cudaMalloc(&p->f32, sizeof(float) * p->N * 46 + sizeof(double) * p->N * fs32::kState) != cudaSuccess) {
       cudaGetLastError();
@@ -930,10 +960,10 @@ template <typename A> static int fs_run(const FsLaunch& l, A& a, cudaStream_t s)
 static int fs_rhs(mgk_fs3d_t p, bool uniform, cudaStream_t s) {
   if (p->prec == MGK_MIXED) {
     fs32::Fs32Args b = fs32_args(p);
-    FsLaunch l[6];
-    const int n = fs32_matvec<double>(p, uniform ? 1 : 2, l);
-    for (int k = 0; k < n; ++k)
-      if (int rc = fs_run(l[k], b, s)) return rc;
+    FsLaunch l[5];
+    fs32_rhs(p, uniform ? 1 : 2, l);
+    for (const FsLaunch& k : l)
+      if (int rc = fs_run(k, b, s)) return rc;
     fs32::fs_to_f32_kernel<<<p->nblk, 256, 0, s>>>(9 * p->N, b.r, b.r32);
     MGK_CUDA(cudaGetLastError());
     MGK_CUDA(cudaMemsetAsync(b.x32, 0, sizeof(float) * 9 * p->N, s));
@@ -956,13 +986,12 @@ static int fs_field(mgk_fs3d_t p, cudaStream_t s) {
 }
 
 // the FP64 matvec's five launches, up to the CG update
-static int fs_matvec(mgk_fs3d_t p, FsLaunch l[6]) {
+static void fs_matvec(mgk_fs3d_t p, FsLaunch l[5]) {
   l[0] = fs_x_launch(p, 1, 0);
   l[1] = fs_y_launch(p, 1);
   l[2] = fs_z_launch(p, 0);
   l[3] = fs_y_launch(p, 0);
   l[4] = fs_x_launch(p, 0, 0);
-  return 5;
 }
 
 static int fs_read_scalars(mgk_fs3d_t p, cudaStream_t s) {
@@ -998,7 +1027,7 @@ struct FsLoop {
   struct Node {
     FsLaunch l;
     void** args;
-  } head, body[9];
+  } head, body[8];
 };
 static void fs_loop(mgk_fs3d_t p, int f, FsLoop& L) {
   L.a = fs_args(p);
@@ -1010,9 +1039,10 @@ static void fs_loop(mgk_fs3d_t p, int f, FsLoop& L) {
   L.ah[0] = &L.a; L.ah[1] = &L.h; L.ah[2] = &L.use_cond;
   L.bz[0] = &L.b; L.bz[1] = &L.zl; L.bz[2] = &L.h; L.bz[3] = &L.use_cond;
   L.bn[0] = &L.b; L.bn[1] = &L.nb; L.bn[2] = &L.h; L.bn[3] = &L.use_cond;
-  FsLaunch l[6];
-  const int n = f ? fs32_matvec<float>(p, 0, l) : fs_matvec(p, l);
-  for (int k = 0; k < n; ++k) L.body[L.n++] = {l[k], f ? L.b1 : L.a1};
+  FsLaunch l[5];
+  if (f) fs32_matvec(p, l);
+  else fs_matvec(p, l);
+  for (const FsLaunch& k : l) L.body[L.n++] = {k, f ? L.b1 : L.a1};
   if (f) {
     L.head = {{(const void*)fs32::fs_scalar_kernel<2>, 1, 256, 0}, L.bz};
     L.body[L.n++] = {{(const void*)fs32::fs_scalar_kernel<0>, 1, 256, 0}, L.bz};
@@ -1061,7 +1091,7 @@ static int fs_build_graph(mgk_fs3d_t p, int f) {
     if (cudaGraphAddNode(&wn, g, &n0, 1, &cp) != cudaSuccess) rc = MGK_CUDA_ERROR;
     else body = cp.conditional.phGraph_out[0];
   }
-  cudaGraphNode_t kn[9];
+  cudaGraphNode_t kn[8];
   for (int k = 0; k < L.n; ++k) add(body, &kn[k], k ? &kn[k - 1] : nullptr, L.body[k]);
   cudaGraphExec_t x = nullptr;
   if (rc == MGK_OK && cudaGraphInstantiate(&x, g, 0) != cudaSuccess) rc = MGK_CUDA_ERROR;
@@ -1171,13 +1201,13 @@ extern "C" int mgk_fs3d_profile(mgk_fs3d_t p, int fp32, int reps, float* ms_out,
   const int f = fp32 ? 1 : 0;
   FsLoop L;
   fs_loop(p, f, L);
-  // output of each launch: FP64 {x inv, y inv, z, y, x, update}; FP32 {(K:p,) z,
-  // y, x, y inv, z inv, scalars + update + scalars}
-  int slot[9];
+  // output of each launch: FP64 {x inv, y inv, z, y, x, update}; FP32 {z, y, x, y
+  // inv, z inv, scalars, update, scalars}
+  int slot[8];
   static const int slot64[6] = {4, 3, 0, 1, 2, 5};
-  for (int k = 0; k < L.n; ++k) slot[k] = f ? std::max(0, std::min(k - (L.n - 8), 5)) : slot64[k];
-  cudaEvent_t ev[10];
-  for (int i = 0; i < 10; ++i) MGK_CUDA(cudaEventCreate(&ev[i]));
+  for (int k = 0; k < L.n; ++k) slot[k] = f ? std::min(k, 5) : slot64[k];
+  cudaEvent_t ev[9];
+  for (int i = 0; i < 9; ++i) MGK_CUDA(cudaEventCreate(&ev[i]));
   double acc[6] = {0, 0, 0, 0, 0, 0};
   int rc = MGK_OK;
   for (int r = 0; r < reps && rc == MGK_OK; ++r) {
@@ -1193,21 +1223,19 @@ extern "C" int mgk_fs3d_profile(mgk_fs3d_t p, int fp32, int reps, float* ms_out,
       acc[slot[k]] += ms;
     }
   }
-  for (int i = 0; i < 10; ++i) cudaEventDestroy(ev[i]);
+  for (int i = 0; i < 9; ++i) cudaEventDestroy(ev[i]);
   if (rc != MGK_OK) { cudaGetLastError(); set_error("mgk_fs3d_profile: kernel failure"); return rc; }
   for (int k = 0; k < 6; ++k) ms_out[k] = (float)(acc[k] / reps);
   return MGK_OK;
 }
 
 // Autotuner: times one Krylov iteration of each kernel family that can serve
-// the plan (register FFTs on the axes that have one, or in the mixed form the
-// warp-line passes when every side is 64/96/128; the general passes always) on
-// the current state and keeps the faster one.
+// the plan (register FFTs on the axes that have one; the general passes always)
+// on the current state and keeps the faster one.
 extern "C" int mgk_fs3d_autotune(mgk_fs3d_t p, int reps, int* chosen, float* best_ms, mgk_stream_t stream) {
   MGK_REQUIRE(p && reps >= 1 && p->has_material, "mgk_fs3d_autotune: bad argument");
   const int f = p->prec == MGK_MIXED ? 1 : 0;
-  p->fast = 1;
-  const bool can_fast = f ? fs32_fast(p) : p->line[0] || p->line[1] || p->line[2];
+  const bool can_fast = f ? p->line32[0] || p->line32[1] || p->line32[2] : p->line[0] || p->line[1] || p->line[2];
   int best = 0;
   float best_t = 0.0f;
   for (int k = 0; k < (can_fast ? 2 : 1); ++k) {

@@ -1,115 +1,11 @@
-// Krylov kernels of the finite-strain solver's mixed form: FP32 matvecs on
-// FP32 CG vectors held as 9 real fields.
-//
-// The FP64 form's vectors are potentials in Fourier space (fs3d.cu), which
-// takes half of the time; this form keeps the real fields and every rounding of
-// the passes below, its FP64 right-hand sides included.  With F_p the tangent as
-// the reference applies it is not symmetric and Newton converges linearly: a
-// solve ends some 1e-6 (of the stress) from its limit wherever the increments
-// reach the tolerance, and CG in FP32 carries a changed last bit into that.  The
-// 128^3 load step on FP32 potentials (54 instead of 106 ms) ended 8e-8 from the
-// FP64 result, this one 1e-6; right-hand sides that differ in the last bits of
-// FP64 alone moved it by 3e-8.
+// Kernels of the mixed form (fs3d_mixed_dev.cuh): the CTA-wide FP32 passes for
+// lengths without a register FFT (fs3d_mixed_line.cuh), the FP64 right-hand
+// side's passes, the CG update and scalars.
 #pragma once
-#include "fs3d_dev.cuh"
+#include "fs3d_mixed_dev.cuh"
 
 namespace mgk {
 namespace fs32 {
-
-struct Fs32Args {
-  int nx, ny, nz, nzh, ld, tc;
-  long long N;
-  int has_fp, model;
-  FftLen fx, fy, fz;
-  const double* Fpi;
-  const double* P;
-  double *r, *st64;
-  double2* spec;
-  double* part;
-  FsScalars* sc;
-  FftLen fx32, fy32, fz32;
-  const float* Fpi32;
-  float *p32, *q32, *r32, *x32, *st32;
-};
-
-// Tangent state planes: Fe (9), S_ref (6: 00 11 22 12 02 01), C^-1 (6, same
-// order; Neo-Hookean only), lambda, c (mu - lambda ln Je for Neo-Hookean, mu
-// for SVK), F_p flag (1 where F_p^-1 is not the identity).
-constexpr int kState = 24;
-
-// the planes and FFT tables that precision T reads
-template <typename T> struct FsP;
-template <> struct FsP<double> {
-  static __device__ __forceinline__ const double* Fpi(const Fs32Args& a) { return a.Fpi; }
-  static __device__ __forceinline__ double* st(const Fs32Args& a) { return a.st64; }
-  static __device__ __forceinline__ double2* spec(const Fs32Args& a) { return a.spec; }
-  static __device__ __forceinline__ const FftLen& fx(const Fs32Args& a) { return a.fx; }
-  static __device__ __forceinline__ const FftLen& fy(const Fs32Args& a) { return a.fy; }
-  static __device__ __forceinline__ const FftLen& fz(const Fs32Args& a) { return a.fz; }
-};
-template <> struct FsP<float> {
-  static __device__ __forceinline__ const float* Fpi(const Fs32Args& a) { return a.Fpi32; }
-  static __device__ __forceinline__ float* st(const Fs32Args& a) { return a.st32; }
-  static __device__ __forceinline__ float2* spec(const Fs32Args& a) { return reinterpret_cast<float2*>(a.spec); }
-  static __device__ __forceinline__ const FftLen& fx(const Fs32Args& a) { return a.fx32; }
-  static __device__ __forceinline__ const FftLen& fy(const Fs32Args& a) { return a.fy32; }
-  static __device__ __forceinline__ const FftLen& fz(const Fs32Args& a) { return a.fz32; }
-};
-
-// symmetric 3x3 from its 6 stored components (00 11 22 12 02 01)
-template <typename T> __device__ __forceinline__ void sym_load(const T* st, long long N, int off, long long i, T* M) {
-  const T a00 = st[(off + 0) * N + i], a11 = st[(off + 1) * N + i], a22 = st[(off + 2) * N + i];
-  const T a12 = st[(off + 3) * N + i], a02 = st[(off + 4) * N + i], a01 = st[(off + 5) * N + i];
-  M[0] = a00; M[1] = a01; M[2] = a02;
-  M[3] = a01; M[4] = a11; M[5] = a12;
-  M[6] = a02; M[7] = a12; M[8] = a22;
-}
-
-// trans2(K4 : trans2(d)) from the tangent state (the kdf of VoxelLaw with
-// Fe, S_ref, C^-1 precomputed; F_p^-1 read only where the flag is set).
-template <typename T>
-__device__ __forceinline__ void kdf_state(const Fs32Args& a, long long i, const T* d, T* out) {
-  const long long N = a.N;
-  const T* st = FsP<T>::st(a);
-  T Fe[9], Sref[9], X[9], Tm[9], Y[9];
-  for (int q = 0; q < 9; ++q) Fe[q] = st[q * N + i];
-  sym_load(st, N, 9, i, Sref);
-  const T lam = st[21 * N + i], c = st[22 * N + i];
-  const bool fp = a.has_fp && st[23 * N + i] != T(0);
-  T Fpi[9];
-  if (fp) {
-    const T* fpp = FsP<T>::Fpi(a);
-    for (int q = 0; q < 9; ++q) Fpi[q] = fpp[q * N + i];
-  }
-  mtm(Fe, d, Tm);
-  if (fp) mm(Tm, Fpi, X);
-  else for (int q = 0; q < 9; ++q) X[q] = Tm[q];
-  if (a.model == 0) {
-    const T tr = X[0] + X[4] + X[8];
-    for (int r = 0; r < 3; ++r)
-      for (int s2 = 0; s2 < 3; ++s2) Y[3 * r + s2] = c * (X[3 * r + s2] + X[3 * s2 + r]) + (r == s2 ? lam * tr : T(0));
-  } else {
-    T Ci[9], CX[9], Xs[9], U[9];
-    sym_load(st, N, 15, i, Ci);
-    mm(Ci, X, CX);
-    const T tr = CX[0] + CX[4] + CX[8];
-    for (int r = 0; r < 3; ++r)
-      for (int s2 = 0; s2 < 3; ++s2) Xs[3 * r + s2] = X[3 * r + s2] + X[3 * s2 + r];
-    mm(Ci, Xs, U);
-    mm(U, Ci, Xs);
-    for (int q = 0; q < 9; ++q) Y[q] = lam * tr * Ci[q] + c * Xs[q];
-  }
-  T A[9], B[9];
-  mmt(Sref, d, A);  // S_ref d^T
-  if (fp) { mm(Fpi, Y, Tm); mmt(Tm, Fe, B); }
-  else mmt(Y, Fe, B);
-  if (a.has_fp) {
-    for (int q = 0; q < 9; ++q) out[q] = A[q] + B[q];
-  } else {
-    for (int r = 0; r < 3; ++r)
-      for (int s2 = 0; s2 < 3; ++s2) out[3 * r + s2] = A[3 * s2 + r] + B[3 * s2 + r];
-  }
-}
 
 // z-line forward: MODE 0 CG (p = r + beta p, or p = r when beta = 0; A = K:p),
 // 1 uniform (A = K:dbar), 2 residual (A = P).  R2C along z of pairs of
@@ -359,7 +255,17 @@ template <int MODE>
 __global__ void fs_scalar_kernel(Fs32Args a, int nb, cudaGraphConditionalHandle cond, int use_cond) {
   __shared__ double red[32];
   double s = 0;
-  for (int i = threadIdx.x; i < nb; i += blockDim.x) s += a.part[i];
+  // sixteen loads in flight, added in order (one CTA sums a partial of every pair
+  // of z-lines: 17 us at 128^3 one load after the other)
+  int i = threadIdx.x;
+  for (; i + 15 * (int)blockDim.x < nb; i += 16 * blockDim.x) {
+    double v[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = a.part[i + k * blockDim.x];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) s += v[k];
+  }
+  for (; i < nb; i += blockDim.x) s += a.part[i];
   s = block_sum(s, red);
   if (threadIdx.x != 0) return;
   FsScalars& S = *a.sc;
@@ -382,62 +288,33 @@ __global__ void fs_scalar_kernel(Fs32Args a, int nb, cudaGraphConditionalHandle 
   }
 }
 
-// Krylov direction and tangent product, per voxel: p = r + beta p (p = r
-// when beta = 0), A = K:p from the tangent state, A written to the q planes
-// (free until the inverse z pass writes q).  Elementwise at full occupancy;
-// the z forward pass (MODE 3) then only transforms A.
-__global__ void __launch_bounds__(256) fs_kp_kernel(Fs32Args a) {
-  const long long N = a.N;
-  const double beta = a.sc->beta;
-  float* pp = a.p32;
-  const float* rr = a.r32;
-  float* qq = a.q32;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
-    float d[9], out[9];
-    for (int q = 0; q < 9; ++q) {
-      const double rv = (double)rr[q * N + i];
-      const float pn = beta == 0.0 ? (float)rv : (float)(rv + beta * (double)pp[q * N + i]);
-      pp[q * N + i] = pn;
-      d[q] = pn;
-    }
-    kdf_state<float>(a, i, d, out);
-    for (int q = 0; q < 9; ++q) qq[q * N + i] = out[q];
-  }
-}
-
 // ------------------------------------------------- warp-line 3D passes ---
-// The same five matvec stages for grids whose sides are 64, 96 or 128 (the
-// served and benchmark sizes): lines sit in padded shared memory and
-// each warp transforms its own lines with warp-local passes.
-//   axis kernels: CTA of NC warps per tile of kFsTile kz columns at one x (y
-//     pass) or one y (x pass); warp c transforms component c0 + c's lines.  The
-//     x pass applies G between the forward and inverse transforms (CTA
-//     barrier); G couples the three components of a row of the tensor only.
-//     FP64 CTAs hold 3 components (one row; three CTAs per tile: 5 resident
-//     CTAs of 3 warps per SM instead of one of 9 at the registers an FP64 line
-//     pair needs), FP32 CTAs all 9.
-//   z kernels: CTA of 3 warps per pair of z-lines; the per-voxel stage (K:p or
-//     P, or q and the p.q sums) uses all threads, warp w transforms the lines
-//     of components 3w..3w+2.
+// The FP64 right-hand side's stages for grids whose sides are 64, 96 or 128:
+// lines sit in padded shared memory and each warp transforms its own lines with
+// warp-local passes.
+//   axis kernels: CTA of 3 warps (one tensor row: G couples its three components
+//     only) per tile of kFsTile kz columns at one x (y pass) or one y (x pass,
+//     with G between the transforms); a warp transforms a component's lines.
+//   z kernels: CTA of 3 warps per pair of z-lines; the per-voxel stage uses all
+//     threads, warp w transforms the lines of components 3w..3w+2.
 constexpr int kFsTile = 4;
 
 __host__ __device__ constexpr bool fs_fast_len(int n) { return n == 64 || n == 96 || n == 128; }
-__host__ __device__ constexpr int fs_pl(int n, int csz) {
-  return csz == 16 ? n + n / 8 + 1 : ((n + n / 16 + 2) & ~1);
-}
+__host__ __device__ constexpr int fs_pl(int n) { return n + n / 8 + 1; }
 
-template <int SIGN, typename T, int NL, bool XG, int NC>
+template <int SIGN, int NL, bool XG>
 __device__ __forceinline__ void fs_axis_body(const Fs32Args& a, int o, int k0, int c0, long long obase,
                                              long long jstride, unsigned char* smem) {
-  using C = C_t<T>;
+  using T = double;
+  using C = double2;
   constexpr int PL = padded_len<C>(NL);
-  constexpr int TC = kFsTile;
+  constexpr int TC = kFsTile, NC = 3;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nzh = a.nzh;
   const int tcw = min(TC, nzh - k0);
   const long long plane = (long long)a.nx * a.ny * a.ld;
   C* lines = reinterpret_cast<C*>(smem);  // line (c * TC + t), c relative to c0
-  C* spec = FsP<T>::spec(a) + c0 * plane;
+  C* spec = a.spec + c0 * plane;
   constexpr int TOT = NC * NL * TC;
   for (int e = threadIdx.x; e < TOT; e += NC * 32) {
     const int c = e / (NL * TC);
@@ -448,7 +325,7 @@ __device__ __forceinline__ void fs_axis_body(const Fs32Args& a, int o, int k0, i
   }
   cp_async_wait_all();
   __syncthreads();
-  const C* tw = reinterpret_cast<const C*>((XG ? FsP<T>::fx(a) : FsP<T>::fy(a)).tw);
+  const C* tw = reinterpret_cast<const C*>((XG ? a.fx : a.fy).tw);
   C* l0 = lines + warp * TC * PL;  // warp = component
   warp_fft<NL, XG ? -1 : SIGN, 2>(l0, PL, tw, lane);
   warp_fft<NL, XG ? -1 : SIGN, 2>(l0 + 2 * PL, PL, tw, lane);
@@ -495,18 +372,13 @@ __device__ __forceinline__ void fs_axis_body(const Fs32Args& a, int o, int k0, i
   }
 }
 
-// components per CTA of the axis kernels (FP32 keeps 9: measured faster at
-// 128^3), and resident-CTA targets for the register allocator
-__host__ __device__ constexpr int fs_axis_nc(bool, int tsz) { return tsz == 4 ? 9 : 3; }
-__host__ __device__ constexpr int fs_axis_minb(bool xg, int tsz) { return fs_axis_nc(xg, tsz) == 3 ? 5 : (tsz == 8 ? 1 : 3); }
-
 // y pass (XG = false) or x pass with G (XG = true); grid = (nx or ny) * ntile
-// * (9 / NC), the component group fastest
-template <int SIGN, typename T, bool XG>
-__global__ void __launch_bounds__(fs_axis_nc(XG, sizeof(T)) * 32, fs_axis_minb(XG, sizeof(T)))
+// * 3, the component group fastest
+template <int SIGN, bool XG>
+__global__ void __launch_bounds__(3 * 32, 5)
     fs_axis_fast_kernel(Fs32Args a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  constexpr int NC = fs_axis_nc(XG, sizeof(T));
+  constexpr int NC = 3;
   const int ntile = (a.nzh + kFsTile - 1) / kFsTile;
   const int cg = blockIdx.x % (9 / NC);
   const int item = blockIdx.x / (9 / NC);
@@ -515,7 +387,7 @@ __global__ void __launch_bounds__(fs_axis_nc(XG, sizeof(T)) * 32, fs_axis_minb(X
   const long long obase = XG ? (long long)a.ld : (long long)a.ny * a.ld;
   const long long jstride = XG ? (long long)a.ny * a.ld : (long long)a.ld;
   const int nl = XG ? a.nx : a.ny;
-#define MGK_AX_CASE(n) case n: fs_axis_body<SIGN, T, n, XG, NC>(a, o, k0, cg * NC, obase, jstride, smem_raw); break;
+#define MGK_AX_CASE(n) case n: fs_axis_body<SIGN, n, XG>(a, o, k0, cg * NC, obase, jstride, smem_raw); break;
   switch (nl) {
     MGK_AX_CASE(64) MGK_AX_CASE(96) MGK_AX_CASE(128)
     default: break;
@@ -523,12 +395,12 @@ __global__ void __launch_bounds__(fs_axis_nc(XG, sizeof(T)) * 32, fs_axis_minb(X
 #undef MGK_AX_CASE
 }
 
-// z forward: per-voxel stage (MODE 0: p = r + beta p and K:p; 1: K:dbar;
-// 2: P; 3: A from the q planes, written by fs_kp_kernel), R2C along z of the
-// pair of z-lines, 9 components.
-template <int MODE, typename T, int NZ>
+// z forward: per-voxel stage (MODE 1: K:dbar; 2: P), R2C along z of the pair of
+// z-lines, 9 components.
+template <int MODE, int NZ>
 __device__ __forceinline__ void fs_zfwd_body(const Fs32Args& a, unsigned char* smem) {
-  using C = C_t<T>;
+  using T = double;
+  using C = double2;
   constexpr int PL = padded_len<C>(NZ);
   constexpr int NZH = NZ / 2 + 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -543,9 +415,6 @@ __device__ __forceinline__ void fs_zfwd_body(const Fs32Args& a, unsigned char* s
       const long long i = (l0 + h) * NZ + z;
       if (MODE == 2) {
         for (int q = 0; q < 9; ++q) out[h][q] = (T)a.P[q * N + i];
-      } else if (MODE == 3) {
-        const float* qq = a.q32;
-        for (int q = 0; q < 9; ++q) out[h][q] = qq[q * N + i];
       } else {
         T d[9];
         for (int q = 0; q < 9; ++q) d[q] = (T)a.sc->dbar[q];
@@ -556,10 +425,10 @@ __device__ __forceinline__ void fs_zfwd_body(const Fs32Args& a, unsigned char* s
     for (int q = 0; q < 9; ++q) lines[q * PL + pz] = mk<C>(out[0][q], out[1][q]);
   }
   __syncthreads();
-  const C* tw = reinterpret_cast<const C*>(FsP<T>::fz(a).tw);
+  const C* tw = reinterpret_cast<const C*>(a.fz.tw);
   C* lw = lines + 3 * warp * PL;
   warp_fft<NZ, -1, 3>(lw, PL, tw, lane);
-  C* spec = FsP<T>::spec(a);
+  C* spec = a.spec;
   for (int cc = 0; cc < 3; ++cc) {
     const int c = 3 * warp + cc;
     const C* ln = lines + c * PL;
@@ -573,10 +442,10 @@ __device__ __forceinline__ void fs_zfwd_body(const Fs32Args& a, unsigned char* s
   }
 }
 
-template <int MODE, typename T>
+template <int MODE>
 __global__ void __launch_bounds__(3 * 32) fs_zfwd_fast_kernel(Fs32Args a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-#define MGK_ZF_CASE(n) case n: fs_zfwd_body<MODE, T, n>(a, smem_raw); break;
+#define MGK_ZF_CASE(n) case n: fs_zfwd_body<MODE, n>(a, smem_raw); break;
   switch (a.nz) {
     MGK_ZF_CASE(64) MGK_ZF_CASE(96) MGK_ZF_CASE(128)
     default: break;
@@ -584,11 +453,11 @@ __global__ void __launch_bounds__(3 * 32) fs_zfwd_fast_kernel(Fs32Args a) {
 #undef MGK_ZF_CASE
 }
 
-// z inverse: C2R along z of the pair of z-lines; MODE 0: q and the p.q
-// partial; MODE 1 (FP64): r = -result, x = 0, the r.r partial.
-template <int MODE, typename T, int NZ>
+// z inverse: C2R along z of the pair of z-lines; r = -result, the r.r partial
+template <int NZ>
 __device__ __forceinline__ void fs_zinv_body(const Fs32Args& a, unsigned char* smem, double* red) {
-  using C = C_t<T>;
+  using T = double;
+  using C = double2;
   constexpr int PL = padded_len<C>(NZ);
   constexpr int NZH = NZ / 2 + 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -597,7 +466,7 @@ __device__ __forceinline__ void fs_zinv_body(const Fs32Args& a, unsigned char* s
   const long long plane = (long long)a.nx * a.ny * a.ld;
   const int ld = a.ld;
   C* lines = reinterpret_cast<C*>(smem);
-  const C* spec = FsP<T>::spec(a);
+  const C* spec = a.spec;
   constexpr int U = (NZH + 31) / 32;
   for (int cc = 0; cc < 3; ++cc) {
     const int c = 3 * warp + cc;
@@ -623,11 +492,9 @@ __device__ __forceinline__ void fs_zinv_body(const Fs32Args& a, unsigned char* s
     }
   }
   __syncwarp();
-  const C* tw = reinterpret_cast<const C*>(FsP<T>::fz(a).tw);
+  const C* tw = reinterpret_cast<const C*>(a.fz.tw);
   warp_fft<NZ, +1, 3>(lines + 3 * warp * PL, PL, tw, lane);
   __syncthreads();
-  float* qq = a.q32;
-  const float* pp = a.p32;
   double acc = 0;
   for (int z = threadIdx.x; z < NZ; z += 3 * 32) {
     const int pz = pidx<C>(z);
@@ -636,13 +503,8 @@ __device__ __forceinline__ void fs_zinv_body(const Fs32Args& a, unsigned char* s
       for (int h = 0; h < 2; ++h) {
         const long long i = (l0 + h) * NZ + z;
         const T val = h == 0 ? v.x : v.y;
-        if (MODE == 0) {
-          qq[c * N + i] = val;
-          acc += (double)pp[c * N + i] * (double)val;
-        } else {
-          a.r[c * N + i] = -(double)val;
-          acc += (double)val * (double)val;
-        }
+        a.r[c * N + i] = -(double)val;
+        acc += (double)val * (double)val;
       }
     }
   }
@@ -650,28 +512,15 @@ __device__ __forceinline__ void fs_zinv_body(const Fs32Args& a, unsigned char* s
   if (threadIdx.x == 0) a.part[blockIdx.x] = acc;
 }
 
-template <int MODE, typename T>
-__device__ __forceinline__ void fs_zinv_fast_entry(const Fs32Args& a) {
+__global__ void __launch_bounds__(3 * 32, 5) fs_zinv_fast64_kernel(Fs32Args a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double red[32];
-#define MGK_ZI_CASE(n) case n: fs_zinv_body<MODE, T, n>(a, smem_raw, red); break;
+#define MGK_ZI_CASE(n) case n: fs_zinv_body<n>(a, smem_raw, red); break;
   switch (a.nz) {
     MGK_ZI_CASE(64) MGK_ZI_CASE(96) MGK_ZI_CASE(128)
     default: break;
   }
 #undef MGK_ZI_CASE
-}
-
-// FP32 kernel (the compiler's own register target), and the FP64 kernel with
-// a register target of 5 resident CTAs per SM (measured faster than 4 at
-// 128^3 despite a few spilled registers; the forward z pass is not)
-template <int MODE, typename T>
-__global__ void __launch_bounds__(3 * 32) fs_zinv_fast_kernel(Fs32Args a) { fs_zinv_fast_entry<MODE, T>(a); }
-template <int MODE>
-__global__ void __launch_bounds__(3 * 32, 5) fs_zinv_fast64_kernel(Fs32Args a) { fs_zinv_fast_entry<MODE, double>(a); }
-template <int MODE, typename T> static void* fs_zinv_fast_fn() {
-  if constexpr (sizeof(T) == 8) return (void*)fs_zinv_fast64_kernel<MODE>;
-  else return (void*)fs_zinv_fast_kernel<MODE, T>;
 }
 
 // FP32 copies of n doubles

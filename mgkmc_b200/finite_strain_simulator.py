@@ -116,8 +116,7 @@ class Fs3dSolver:
         return list(ms)
 
     def autotune(self, reps=5, stream=None):
-        """Keeps the faster kernel family (1 register or warp-line FFTs, 0
-        CTA-wide) for this plan, timed on its current state (call after a step)."""
+        """Keeps the faster kernel family (1 register FFTs, 0 CTA-wide) for this plan, timed on its current state (call after a step)."""
         ch, ms = ctypes.c_int(), ctypes.c_float()
         L.check(L.lib().mgk_fs3d_autotune(self._h, int(reps), ctypes.byref(ch), ctypes.byref(ms),
                                           L.stream_ptr(stream)), "mgk_fs3d_autotune")

@@ -204,3 +204,29 @@ def test_register_lines_match_general_passes(shape, model, with_fp, monkeypatch)
         out.append((F.cpu().numpy(), P.cpu().numpy()))
     assert rel(out[0][0], out[1][0]) < 1e-10
     assert rel(out[0][1], out[1][1]) < 1e-9
+
+
+@pytest.mark.parametrize("shape,model,with_fp", [((24, 27, 32), "neo_hookean", True), ((36, 48, 54), "svk", True),
+                                                 ((64, 2, 72), "neo_hookean", False), ((81, 4, 96), "svk", False),
+                                                 ((108, 4, 128), "neo_hookean", True), ((144, 1, 162), "svk", True),
+                                                 ((3, 192, 216), "neo_hookean", True), ((2, 243, 24), "neo_hookean", False)])
+def test_mixed_register_lines_keep_the_general_roundings(shape, model, with_fp, monkeypatch):
+    # the mixed form's register FFTs repeat the CTA-wide passes' FP32
+    # operations and sums: the same bits, on axes of every length
+    import torch
+    from mgkmc_b200.finite_strain_simulator import Fs3dSolver, build_finite_strain_bc_3d
+    lam, mu, Fp = W.fs3d_material_dev(*shape, 3, "cuda")
+    out = []
+    for flag in ("1", "0"):
+        monkeypatch.setenv("MGK_FS_FAST", flag)
+        s = Fs3dSolver(*shape, model=model, precision="mixed")
+        s.set_material(lam, mu, Fp if with_fp else None)
+        F = torch.eye(3, dtype=torch.float64, device="cuda").reshape(3, 3, 1, 1, 1).expand(3, 3, *shape).contiguous()
+        s.set_F(F)
+        Fb, _, Pt, Pm = build_finite_strain_bc_3d((0, 0), 0.005, {(1, 1): 0.0, (2, 2): 0.0})
+        _, info = s.step(Fb, (0, 0), Pt, Pm, 90e9, 0.35, 1e-8, 1e-6, 40, 1e6, 40)
+        P = torch.empty_like(F)
+        s.get(F, P)
+        out.append((F.cpu().numpy(), P.cpu().numpy(), info.krylov_iterations))
+    assert out[0][2] == out[1][2]
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
