@@ -177,16 +177,16 @@ MGK_API int mgk_ls2d_solve_batch(mgk_ls2d_t plan, int nsel, const int* sel, cons
                                  mgk_stream_t stream);
 
 /* Autotuner: times one iteration of every kernel family that can serve the
- * plan (warp-line kernels for sides up to 256 / 512 / 1024 with their column
- * tiles, and the CTA-wide passes with theirs) on the selection, `reps` times
- * each, and keeps the fastest (FP64 plus FP32 kernels for mixed plans).
- * *chosen: 0 CTA-wide, or 256/512/1024; *best_ms: its iteration time.  Leaves
+ * plan (the register-FFT kernels, which 256, 512 and 1024 all name, and the
+ * CTA-wide passes) on the selection, `reps` times each, and keeps the fastest
+ * (FP64 plus FP32 kernels for mixed plans).  *chosen: 0 CTA-wide, or
+ * 256/512/1024; *best_ms: its iteration time.  Leaves
  * the replicas' iterates unspecified (call before solving).  No counterpart in
  * the reference. */
 MGK_API int mgk_ls2d_autotune(mgk_ls2d_t plan, int nsel, const int* sel, const double* eps_bar, int reps,
                               int* chosen, float* best_ms, mgk_stream_t stream);
 
-/* Sets the kernel family directly (0 CTA-wide, 256/512/1024 warp-line; at
+/* Sets the kernel family directly (0 CTA-wide, 256/512/1024 register FFTs; at
  * least the plan's largest side), e.g. one the autotuner chose for an equal
  * plan.  Synchronises the device.  No counterpart in the reference. */
 MGK_API int mgk_ls2d_set_family(mgk_ls2d_t plan, int family);

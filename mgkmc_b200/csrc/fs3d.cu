@@ -33,9 +33,9 @@
 // What bounds it: memory.  In numbers of one real value per voxel an iteration
 // moves 15 + 15 + 30 + 15 + 12 + 18 = 105 (12 of them the tangent state); with
 // real CG vectors, 9 spectra in the x passes and a state of 24 planes it moved
-// 213.  A Neo-Hookean FP64 load step of 152 .. 156 iterations: 64^3 30.1 -> 13.1
-// ms, 96^3 87 -> 40 ms, 128^3 180 -> 84 ms (0.55 of the measured copy rate over an
-// iteration's 1.76 GB); 72^3, which had no warp-line kernels, 68 -> 19 ms.  Host
+// 213.  A Neo-Hookean FP64 load step of 152 .. 156 iterations: 64^3 30.1 -> 11.9
+// ms, 96^3 87 -> 40 ms, 128^3 180 -> 77 ms (0.57 of the measured copy rate over an
+// iteration's 1.76 GB); 72^3, which had no warp-line kernels, 68 -> 18 ms.  Host
 // reads are one per Newton iteration: the trial state is evaluated behind the
 // Krylov loop, writes the next tangent state and is accepted by a swap.
 //
@@ -417,13 +417,32 @@ __global__ void __launch_bounds__(256) fs_update_kernel(FsArgs a, cudaGraphCondi
   });
 }
 
+// Sums of K values over the CTA (the tree of block_sum(), for all of them at
+// once: 2 barriers, not 3 K, which took 0.5 ms of a 64^3 load step): out[k] for
+// every thread.
+template <int K> __device__ __forceinline__ void block_sums(const double* v, double (*red)[32], double* out) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const double s = warp_sum(v[k]);
+    if (lane == 0) red[k][wid] = s;
+  }
+  __syncthreads();
+  for (int k = wid; k < K; k += nw) {
+    const double s = warp_sum(lane < nw ? red[k][lane] : 0.0);
+    if (lane == 0) out[k] = s;
+  }
+  __syncthreads();
+}
+
 // Constitutive evaluation at F + alpha (x + dbar) (at F without use_x): writes
 // Fout, Pout and the tangent state there; min Je, NaN count, sum F^2, sum x^2 and the Cauchy stress means (cauchy_from_P_3d) are
 // reduced by the CTA that arrives last.  16 values per CTA.
-// x32, st32: the mixed form's increment and tangent state (null: FP64).
-__global__ void fs_constitutive_kernel(FsArgs a, double alpha, int use_dbar, int use_x, const float* __restrict__ x32,
+// x32, st32: the mixed form's increment and tangent state (null: FP64).  Two CTAs
+// per SM (128 registers, 158 without being asked): 485 -> 290 us at 128^3, mixed.
+__global__ void __launch_bounds__(256, 2) fs_constitutive_kernel(FsArgs a, double alpha, int use_dbar, int use_x, const float* __restrict__ x32,
                                        float* __restrict__ st32) {
-  __shared__ double red[32];
+  __shared__ double red[12][32], sum[12];
   const long long N = a.N;
   double mnJ = INFINITY, nan = 0, FF = 0, xx = 0;
   double sg[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
@@ -461,9 +480,10 @@ __global__ void fs_constitutive_kernel(FsArgs a, double alpha, int use_dbar, int
   double v[13] = {0};
   v[0] = nan; v[1] = FF; v[2] = xx;
   for (int q = 0; q < 9; ++q) v[3 + q] = sg[q];
-  for (int q = 0; q < 12; ++q) {
-    const double t = block_sum(v[q], red);
-    if (threadIdx.x == 0) a.part[(size_t)blockIdx.x * 16 + q] = t;
+  block_sums<12>(v, red, sum);
+  if (threadIdx.x < 12) {
+    a.part[(size_t)blockIdx.x * 16 + threadIdx.x] = sum[threadIdx.x];
+    __threadfence();
   }
   // min Je
   __shared__ double mn[32];
@@ -483,11 +503,10 @@ __global__ void fs_constitutive_kernel(FsArgs a, double alpha, int use_dbar, int
   if (!s_last) return;
   __threadfence();
   const int nb = gridDim.x;
-  for (int q = 0; q < 12; ++q) {
-    double s = 0;
-    for (int i = threadIdx.x; i < nb; i += blockDim.x) s += __ldcg(&a.part[(size_t)i * 16 + q]);
-    v[q] = block_sum(s, red);
-  }
+  for (int q = 0; q < 12; ++q) v[q] = 0;
+  for (int i = threadIdx.x; i < nb; i += blockDim.x)
+    for (int q = 0; q < 12; ++q) v[q] += __ldcg(&a.part[(size_t)i * 16 + q]);
+  block_sums<12>(v, red, sum);
   m = INFINITY;
   for (int i = threadIdx.x; i < nb; i += blockDim.x) m = fmin(m, __ldcg(&a.part[(size_t)i * 16 + 12]));
   for (int o = 16; o > 0; o >>= 1) m = fmin(m, __shfl_down_sync(0xffffffffu, m, o));
@@ -497,10 +516,10 @@ __global__ void fs_constitutive_kernel(FsArgs a, double alpha, int use_dbar, int
     FsScalars& S = *a.sc;
     double r = INFINITY;
     for (int w = 0; w < (int)(blockDim.x + 31) / 32; ++w) r = fmin(r, mn[w]);
-    S.nan = v[0];
-    S.FF = v[1];
-    S.xx = v[2];
-    for (int q = 0; q < 9; ++q) S.sig[q] = v[3 + q] / (double)a.N;
+    S.nan = sum[0];
+    S.FF = sum[1];
+    S.xx = sum[2];
+    for (int q = 0; q < 9; ++q) S.sig[q] = sum[3 + q] / (double)a.N;
     S.minJe = r;
   }
 }
@@ -511,29 +530,29 @@ struct FsBegin {
   double F_bar[9], tol2, kmax;
 };
 __global__ void fs_begin_kernel(FsArgs a, FsBegin b) {
-  __shared__ double red[32];
+  __shared__ double red[9][32], sum[9];
   __shared__ int s_last;
   double s[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < a.N; i += (long long)gridDim.x * blockDim.x)
     for (int q = 0; q < 9; ++q) s[q] += a.F[q * a.N + i];
-  for (int q = 0; q < 9; ++q) {
-    const double t = block_sum(s[q], red);
-    if (threadIdx.x == 0) a.part[(size_t)blockIdx.x * 16 + q] = t;
-  }
-  if (threadIdx.x == 0) {
+  block_sums<9>(s, red, sum);
+  if (threadIdx.x < 9) {
+    a.part[(size_t)blockIdx.x * 16 + threadIdx.x] = sum[threadIdx.x];
     __threadfence();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
     s_last = atomicInc(a.counter, gridDim.x - 1) == gridDim.x - 1;
   }
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  for (int q = 0; q < 9; ++q) {
-    double t = 0;
-    for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) t += __ldcg(&a.part[(size_t)i * 16 + q]);
-    t = block_sum(t, red);
-    if (threadIdx.x == 0) a.sc->dbar[q] = b.F_bar[q] - t / (double)a.N;
-  }
+  for (int q = 0; q < 9; ++q) s[q] = 0;
+  for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x)
+    for (int q = 0; q < 9; ++q) s[q] += __ldcg(&a.part[(size_t)i * 16 + q]);
+  block_sums<9>(s, red, sum);
   if (threadIdx.x == 0) {
+    for (int q = 0; q < 9; ++q) a.sc->dbar[q] = b.F_bar[q] - sum[q] / (double)a.N;
     a.sc->tol2 = b.tol2;
     a.sc->kmax = b.kmax;
     a.sc->err = 0.0;
@@ -717,7 +736,7 @@ static const FsLine* fs_kernels(mgk_fs3d_t p, int axis) { return p->fast ? p->li
 static FsLaunch fs_z_launch(mgk_fs3d_t p, int mode) {
   const int pairs = (int)(p->N / p->nz / 2);
   if (const FsLine* k = fs_kernels(p, 2))
-    return {k->z[p->model][mode], (pairs + k->zp - 1) / k->zp, k->z_threads, (size_t)k->z_bytes};
+    return {k->z[p->model][mode], pairs, k->z_threads, (size_t)k->z_bytes};
   const void* fn = mode == 0   ? (p->model ? (const void*)fs_z_kernel<0, 1> : (const void*)fs_z_kernel<0, 0>)
                    : mode == 1 ? (p->model ? (const void*)fs_z_kernel<1, 1> : (const void*)fs_z_kernel<1, 0>)
                    : mode == 2 ? (const void*)fs_z_kernel<2, 0>
@@ -772,7 +791,7 @@ static void fs32_matvec(mgk_fs3d_t p, FsLaunch L[5]) {
   if (!p->fast) return;
   const int zl = (int)(p->N / p->nz / 2);
   if (const fs32::MixedLine* k = p->line32[2]) {
-    L[0] = {k->zfwd, (zl + k->zp - 1) / k->zp, k->zf_threads, (size_t)k->zf_bytes};
+    L[0] = {k->zfwd, zl, k->zf_threads, (size_t)k->zf_bytes};
     L[4] = {k->zinv, zl, k->zi_threads, (size_t)k->zi_bytes};
   }
   if (const fs32::MixedLine* k = p->line32[1])
@@ -1106,7 +1125,7 @@ static int fs_build_graph(mgk_fs3d_t p, int f) {
 }
 
 static int fs_krylov_status(mgk_fs3d_t p) {
-  if (p->h_sc->err != 0.0) { set_error("mgk_fs3d_step: a bulk copy did not complete"); return MGK_CUDA_ERROR; }
+  if (p->h_sc->err != 0.0) { set_error("mgk_fs3d_step: a bulk copy wait gave up (device timeout)"); return MGK_TIMEOUT; }
   if (!isfinite(p->h_sc->rr)) { set_error("mgk_fs3d_step: non-finite Krylov residual"); return MGK_NONFINITE; }
   return MGK_OK;
 }

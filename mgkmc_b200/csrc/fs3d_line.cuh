@@ -2,7 +2,7 @@
 // instantiation per line length; axes of other lengths take the general
 // kernels of fs3d.cu.
 //
-//   z-line   CTA of fs_zp pairs of z-lines x 9 components x T threads: C2R of
+//   z-line   CTA of a pair of z-lines x 9 components x T threads: C2R of
 //            the increment's spectrum, K:p per voxel, R2C of the product; the
 //            real fields exist in shared memory only;
 //   y pass   CTA of one tensor row (3 components) x tile of kz columns;
@@ -20,21 +20,23 @@ namespace mgk {
 constexpr int fs_round32(int n) { return (n + 31) / 32 * 32; }
 // row pitch of the half spectra: rows start on 64-byte boundaries
 __host__ __device__ constexpr int fs_ld(int n) { return (n / 2 + 1 + 3) / 4 * 4; }
-constexpr int fs_zp(int n) { return reg_sched64(n).t <= 9 ? 2 : 1; }
-constexpr int fs_z_threads(int n) { return fs_round32(9 * reg_sched64(n).t * fs_zp(n)); }
+constexpr int fs_z_threads(int n) { return fs_round32(9 * reg_sched64(n).t); }
 // kz columns per tile: whole 32-byte sectors per row, within 432 threads for
 // the six lines of the x pass
 constexpr int fs_tile(int n) { return reg_sched64(n).t <= 18 ? 4 : 2; }
 constexpr int fs_ax_threads(int n, int nc) { return fs_round32(nc * fs_tile(n) * reg_sched64(n).t); }
 // exchange buffers; they first hold the pairs' spectrum rows as copied
 constexpr int fs_z_bytes(int n) {
-  const int a = fs_zp(n) * 9 * reg_slots(n, 16), b = fs_zp(n) * 18 * fs_ld(n);
+  const int a = 9 * reg_slots(n, 16), b = 18 * fs_ld(n);
   return (a > b ? a : b) * 16;
 }
 constexpr int fs_ax_bytes(int n, int nc) { return nc * fs_tile(n) * reg_slots(n, 16) * 16; }
-// resident CTAs asked of the register allocator: 128 registers per thread
-constexpr int fs_minb(int threads) {
-  const int b = 65536 / (threads * 128);
+// resident CTAs asked of the register allocator: 128 registers per thread, in the
+// x passes 112 (a third CTA of 192 threads at 128 points, 118 registers without
+// being asked: 80 and 98 us -> 73 and 80 us; in the y passes the spills cost more:
+// 57 and 63 us -> 96 and 82 us)
+constexpr int fs_minb(int threads, int regs = 128) {
+  const int b = 65536 / (threads * regs);
   return b < 1 ? 1 : b;
 }
 
@@ -46,42 +48,40 @@ __global__ void __launch_bounds__(fs_z_threads(NZ),
                                   fs_minb(fs_z_threads(NZ)))
     fs_zline_reg(FsArgs a) {
   using C = double2;
-  constexpr int TL = reg_sched(NZ, sizeof(C)).t, P = fs_zp(NZ), TH = fs_z_threads(NZ), SL = reg_slots(NZ, sizeof(C));
+  constexpr int TL = reg_sched64(NZ).t, TH = fs_z_threads(NZ), SL = reg_slots(NZ, sizeof(C));
   constexpr int NZH = NZ / 2 + 1, ld = fs_ld(NZ);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bar;
   const long long N = a.N, plane = a.plane;
-  const long long p0 = (long long)blockIdx.x * P;  // first pair
-  const int np = (int)min((long long)P, (long long)a.nx * a.ny / 2 - p0);
+  const long long l0 = 2LL * blockIdx.x;  // first line
   C* lines = reinterpret_cast<C*>(smem_raw);
   C* spec = reinterpret_cast<C*>(a.spec);
   if constexpr (MODE == 0 || MODE == 3) {
     if (threadIdx.x == 0) {
-      // the pairs' half-spectrum rows, contiguous per component
-      const uint32_t bytes = 2u * np * ld * sizeof(C);
+      // the pair's half-spectrum rows, contiguous per component
+      const uint32_t bytes = 2u * ld * sizeof(C);
       mbar_init(&bar, 1);
       fence_mbar_init();
       mbar_arrive_expect_tx(&bar, 9u * bytes);
 #pragma unroll
-      for (int q = 0; q < 9; ++q) bulk_g2s(lines + q * 2 * P * ld, spec + q * plane + 2 * p0 * ld, bytes, &bar);
+      for (int q = 0; q < 9; ++q) bulk_g2s(lines + q * 2 * ld, spec + q * plane + l0 * ld, bytes, &bar);
     }
   }
   if constexpr (MODE == 0) {
     // the voxels' tangent state into L2 meanwhile (rows that start on 16 bytes)
     if (threadIdx.x >= 32 && threadIdx.x < 32 + (MODEL == 1 ? 12 : 11)) {
-      const double* f = reinterpret_cast<const double*>(a.st) + (threadIdx.x - 32) * N + 2 * p0 * NZ;
-      const uint32_t bytes = 2u * np * NZ * sizeof(double);
+      const double* f = reinterpret_cast<const double*>(a.st) + (threadIdx.x - 32) * N + l0 * NZ;
+      const uint32_t bytes = 2u * NZ * sizeof(double);
       if (((reinterpret_cast<uintptr_t>(f) | bytes) & 15) == 0)
         asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(f), "r"(bytes) : "memory");
     }
   }
   const C* tw = reinterpret_cast<const C*>(a.rtw[2]);
-  const int line = threadIdx.x / TL, t = threadIdx.x % TL;  // line = 9 pair + component
-  const int pr = line / 9, c = line - 9 * pr;
-  const bool act = line < 9 * P && pr < np;
+  const int c = min(threadIdx.x / TL, 8), t = threadIdx.x % TL;
+  const bool act = threadIdx.x < 9 * TL;
   const bool third = c % 3 == 2;  // its spectrum is uz times the potential's
-  C* buf = lines + (line < 9 * P ? line : 0) * SL;
-  C* ra = spec + c * plane + 2 * (p0 + pr) * ld;  // the pair's two rows: ra, ra + ld
+  C* buf = lines + c * SL;
+  C* ra = spec + c * plane + l0 * ld;  // the pair's two rows: ra, ra + ld
   auto at = [&](int s) -> C& { return buf[s]; };
   auto put = [&](int i, C v) { buf[reg_slot<NZ, C>(i)] = v; };
   auto sync = [] {
@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(fs_z_threads(NZ),
       if (threadIdx.x == 0) a.sc->err = 1.0;
       return;
     }
-    const C* sa = lines + (c * P + pr) * 2 * ld;
+    const C* sa = lines + c * 2 * ld;
     auto load = [&](int k) -> C {
       const int ks = 2 * k <= NZ ? k : NZ - k;
       C x = sa[ks], y = sa[ld + ks];
@@ -111,11 +111,10 @@ __global__ void __launch_bounds__(fs_z_threads(NZ),
     __syncthreads();
   }
   if constexpr (MODE == 3) {
-    for (int e = threadIdx.x; e < 9 * P * NZ; e += TH) {
-      const int l = e / NZ, z = e - l * NZ, q = l / 9, k = l - 9 * q;
-      if (q >= np) break;
-      const C v = lines[l * SL + reg_slot<NZ, C>(z)];
-      double* X = a.X + k * N + 2 * (p0 + q) * NZ + z;
+    for (int e = threadIdx.x; e < 9 * NZ; e += TH) {
+      const int k = e / NZ, z = e - k * NZ;
+      const C v = lines[k * SL + reg_slot<NZ, C>(z)];
+      double* X = a.X + k * N + l0 * NZ + z;
       X[0] = v.x;
       X[NZ] = v.y;
     }
@@ -124,10 +123,10 @@ __global__ void __launch_bounds__(fs_z_threads(NZ),
   // one voxel per thread and round, the two lines of a pair interleaved
   // (8-byte words of consecutive lanes in consecutive banks)
 #pragma unroll 1
-  for (int e = threadIdx.x; e < 2 * np * NZ; e += TH) {
-    const int h = e & 1, v = e >> 1, q = v / NZ, z = v - q * NZ;
-    const long long i = (2 * (p0 + q) + h) * NZ + z;
-    double* vx = reinterpret_cast<double*>(lines + q * 9 * SL + reg_slot<NZ, C>(z)) + h;
+  for (int e = threadIdx.x; e < 2 * NZ; e += TH) {
+    const int h = e & 1, z = e >> 1;
+    const long long i = (l0 + h) * NZ + z;
+    double* vx = reinterpret_cast<double*>(lines + reg_slot<NZ, C>(z)) + h;
     double d[9], out[9];
     if constexpr (MODE == 2) {
 #pragma unroll
@@ -225,7 +224,7 @@ __global__ void __launch_bounds__(fs_ax_threads(NL, 3),
 // fs_contract().
 template <int NL, bool RHS>
 __global__ void __launch_bounds__(fs_ax_threads(NL, 6),
-                                  fs_minb(fs_ax_threads(NL, 6)))
+                                  fs_minb(fs_ax_threads(NL, 6), 112))
     fs_xfwd_reg(FsArgs a) {
   using C = double2;
   constexpr int TL = reg_sched(NL, sizeof(C)).t, W = fs_tile(NL), SL = reg_slots(NL, sizeof(C));
@@ -268,7 +267,7 @@ __global__ void __launch_bounds__(fs_ax_threads(NL, 6),
 // Inverse x pass: the direction's potential v and its lines X = ux v and v.
 template <int NL, bool FINAL>
 __global__ void __launch_bounds__(fs_ax_threads(NL, 6),
-                                  fs_minb(fs_ax_threads(NL, 6)))
+                                  fs_minb(fs_ax_threads(NL, 6), 112))
     fs_xinv_reg(FsArgs a) {
   using C = double2;
   constexpr int TL = reg_sched(NL, sizeof(C)).t, W = fs_tile(NL), SL = reg_slots(NL, sizeof(C));
@@ -315,7 +314,7 @@ struct FsLine {
   const void* y[2];     // forward, inverse
   const void* xf[2];    // matvec, right-hand side
   const void* xi[2];    // direction, final
-  int zp, z_threads, tile, y_threads, x_threads;
+  int z_threads, tile, y_threads, x_threads;
   int z_bytes, y_bytes, x_bytes;
 };
 const FsLine* fs_line(int n);  // null: no instantiation
@@ -335,7 +334,6 @@ template <int N> static const FsLine* fs_make() {
     k.xf[1] = (const void*)fs_xfwd_reg<N, true>;
     k.xi[0] = (const void*)fs_xinv_reg<N, false>;
     k.xi[1] = (const void*)fs_xinv_reg<N, true>;
-    k.zp = fs_zp(N);
     k.z_threads = fs_z_threads(N);
     k.tile = fs_tile(N);
     k.y_threads = fs_ax_threads(N, 3);

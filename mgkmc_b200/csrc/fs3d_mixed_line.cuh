@@ -5,7 +5,7 @@
 // CTA-wide passes of other grids, which remain for lengths without a register
 // FFT).  Sums keep their order.
 //
-//   z forward  CTA of pairs of z-lines x 9 components x T threads: p = r + beta
+//   z forward  CTA of a pair of z-lines x 9 components x T threads: p = r + beta
 //              p, A = K:p per voxel into shared memory, R2C;
 //   y          CTA of one tensor row (3 components) x tile of kz columns;
 //   x          all 9 components x tile: forward, G, inverse;
@@ -14,9 +14,9 @@
 // What bounds them: HBM, 45 + 2 x 18 + 18 + 27 floats per voxel.  The former
 // passes crossed shared memory about twice per radix pass and wrote A to memory
 // between K:p and the z transform.  At 128^3, before and now (CUDA events around
-// each launch): K:p with z forward 202 and 134 us, y 56 and 37, x 88 and 65, y
+// each launch): K:p with z forward 202 and 133 us, y 56 and 37, x 88 and 65, y
 // inverse 53 and 33, z inverse 66 and 54.  72^3, from CTA-wide passes: 301 and
-// 133 us an iteration.
+// 129 us an iteration.
 #pragma once
 #include "fft_reg.cuh"
 #include "fs3d_mixed_dev.cuh"
@@ -28,9 +28,9 @@ namespace fs32 {
 constexpr int up32(int n) { return (n + 31) / 32 * 32; }
 constexpr int ml_t(int n) { return reg_sched32(n).t; }
 constexpr int ml_ld(int n) { return (n / 2 + 1 + 3) / 4 * 4; }  // row pitch of the half spectra
-// z forward: pairs per CTA
-constexpr int ml_zp(int n) { return ml_t(n) <= 9 ? 2 : 1; }
-constexpr int ml_zf_threads(int n) { return up32(9 * ml_t(n) * ml_zp(n)); }
+// one pair of lines per z CTA: with two, 64^3 took 13.9 instead of 12.7 ms a load
+// step, 96^3 45 instead of 39
+constexpr int ml_zf_threads(int n) { return up32(9 * ml_t(n)); }
 // z inverse: the threads (and with them the order of the sums) of the passes
 // that it replaces
 constexpr int ml_zi_threads(int alt) { return alt ? 256 : 96; }
@@ -40,7 +40,7 @@ constexpr int ml_yw(int n) { return ml_t(n) <= 9 ? 8 : ml_t(n) <= 18 ? 4 : 2; }
 constexpr int ml_xw(int n) { return ml_t(n) <= 14 ? 4 : 2; }
 constexpr int ml_y_threads(int n) { return up32(3 * ml_yw(n) * ml_t(n)); }
 constexpr int ml_x_threads(int n) { return up32(9 * ml_xw(n) * ml_t(n)); }
-constexpr int ml_zf_bytes(int n) { return ml_zp(n) * 9 * reg_slots(n, 8) * 8; }
+constexpr int ml_zf_bytes(int n) { return 9 * reg_slots(n, 8) * 8; }
 constexpr int ml_zi_bytes(int n) {
   const int a = 9 * reg_slots(n, 8), b = 18 * ml_ld(n);
   return (a > b ? a : b) * 8;
@@ -52,19 +52,18 @@ constexpr int ml_minb(int threads) { return 65536 / (threads * 80) < 1 ? 1 : 655
 template <int NZ, int ALT>
 __global__ void __launch_bounds__(ml_zf_threads(NZ), ml_minb(ml_zf_threads(NZ))) ml_zfwd(Fs32Args a) {
   using C = float2;
-  constexpr int TL = ml_t(NZ), P = ml_zp(NZ), TH = ml_zf_threads(NZ), SL = reg_slots(NZ, 8), NZH = NZ / 2 + 1;
+  constexpr int TL = ml_t(NZ), TH = ml_zf_threads(NZ), SL = reg_slots(NZ, 8), NZH = NZ / 2 + 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const long long N = a.N, plane = (long long)a.nx * a.ny * a.ld;
-  const long long p0 = (long long)blockIdx.x * P;  // first pair
-  const int np = (int)min((long long)P, (long long)a.nx * a.ny / 2 - p0);
+  const long long l0 = 2LL * blockIdx.x;  // first line
   C* lines = reinterpret_cast<C*>(smem_raw);
   const double beta = a.sc->beta;
   // one voxel per thread and round, the two lines of a pair interleaved
 #pragma unroll 1
-  for (int e = threadIdx.x; e < 2 * np * NZ; e += TH) {
-    const int h = e & 1, v = e >> 1, q = v / NZ, z = v - q * NZ;
-    const long long i = (2 * (p0 + q) + h) * NZ + z;
-    float* vx = reinterpret_cast<float*>(lines + q * 9 * SL + reg_slot<NZ, C>(z)) + h;
+  for (int e = threadIdx.x; e < 2 * NZ; e += TH) {
+    const int h = e & 1, z = e >> 1;
+    const long long i = (l0 + h) * NZ + z;
+    float* vx = reinterpret_cast<float*>(lines + reg_slot<NZ, C>(z)) + h;
     float d[9], out[9];
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
@@ -78,10 +77,9 @@ __global__ void __launch_bounds__(ml_zf_threads(NZ), ml_minb(ml_zf_threads(NZ)))
     for (int k = 0; k < 9; ++k) vx[k * 2 * SL] = out[k];
   }
   __syncthreads();
-  const int line = threadIdx.x / TL, t = threadIdx.x % TL;  // line = 9 pair + component
-  const int pr = line / 9, c = line - 9 * pr;
-  const bool act = line < 9 * P && pr < np;
-  C* buf = lines + (line < 9 * P ? line : 0) * SL;
+  const int c = min(threadIdx.x / TL, 8), t = threadIdx.x % TL;
+  const bool act = threadIdx.x < 9 * TL;
+  C* buf = lines + c * SL;
   auto at = [&](int s) -> C& { return buf[s]; };
   auto sync = [] {
     if constexpr (32 % TL == 0) __syncwarp();
@@ -92,7 +90,7 @@ __global__ void __launch_bounds__(ml_zf_threads(NZ), ml_minb(ml_zf_threads(NZ)))
                            [&](int i, C v) { buf[reg_slot<NZ, C>(i)] = v; }, sync, sync);
   sync();
   if (act) {
-    C* ra = reinterpret_cast<C*>(a.spec) + c * plane + 2 * (p0 + pr) * a.ld;
+    C* ra = reinterpret_cast<C*>(a.spec) + c * plane + l0 * a.ld;
     for (int k = t; k < NZH; k += TL) {
       const C z = buf[reg_slot<NZ, C>(k)];
       const C w = buf[reg_slot<NZ, C>(k == 0 ? 0 : NZ - k)];
@@ -259,7 +257,7 @@ __global__ void __launch_bounds__(ml_x_threads(NL), ml_minb(ml_x_threads(NL))) m
 // The kernels of one line length, with their launch shapes.
 struct MixedLine {
   const void *zfwd, *zinv, *y[2], *x;
-  int zp, zf_threads, zi_threads, yw, xw, y_threads, x_threads;
+  int zf_threads, zi_threads, yw, xw, y_threads, x_threads;
   int zf_bytes, zi_bytes, y_bytes, x_bytes;
 };
 const MixedLine* mixed_line(int n, int alt);  // null: no instantiation
@@ -272,7 +270,6 @@ template <int N, int ALT> static const MixedLine* mixed_make() {
     k.y[0] = (const void*)ml_ypass<N, -1, ALT>;
     k.y[1] = (const void*)ml_ypass<N, 1, ALT>;
     k.x = (const void*)ml_xpass<N, ALT>;
-    k.zp = ml_zp(N);
     k.zf_threads = ml_zf_threads(N);
     k.zi_threads = ml_zi_threads(ALT);
     k.yw = ml_yw(N);
