@@ -1624,8 +1624,52 @@ static int ls2d_set_variant(mgk_ls2d_t p, int v) {
   return MGK_OK;
 }
 
-extern "C" int mgk_ls2d_profile_batch(mgk_ls2d_t p, int nsel, const int* sel, const double* eps_bar, int fp32,
-                                      int reps, float* row_ms, float* col_ms, mgk_stream_t stream);
+static int profile_setup(mgk_ls2d_t p, int nsel, const int* sel, const double* eps_bar, cudaStream_t s);
+
+// Mean time of an iteration as the loop's body runs it, the groups side by side:
+// a graph of `reps` bodies, each waiting for the whole one before it.
+static int time_iterations(mgk_ls2d_t p, bool f32, int reps, float* ms, cudaStream_t s) {
+  Loop2& a = p->last;
+  int rc = launch2(a, kFirst, f32, 1, s);
+  if (rc) return rc;
+  cudaGraph_t g = nullptr;
+  cudaGraphExec_t x = nullptr;
+  cudaEvent_t ev[2] = {nullptr, nullptr};
+  auto run = [&]() -> int {
+    MGK_CUDA(cudaGraphCreate(&g, 0));
+    std::vector<cudaGraphNode_t> prev, rows;
+    for (int r = 0; r < reps; ++r) {
+      rows.clear();
+      for (Grp2& gr : a.grp) {
+        cudaGraphNode_t col, row;
+        MGK_CUDA(with_stage2(a, gr, kCol, f32, 1, 0, 0, 0, [&](const Launch2& L, void** args) {
+          return add_node2(g, &col, prev.data(), prev.size(), L, args);
+        }));
+        MGK_CUDA(with_stage2(a, gr, kRow, f32, 1, 0, 0, 0, [&](const Launch2& L, void** args) {
+          return add_node2(g, &row, &col, 1, L, args);
+        }));
+        rows.push_back(row);
+      }
+      prev = rows;
+    }
+    MGK_CUDA(cudaGraphInstantiate(&x, g, 0));
+    for (int i = 0; i < 2; ++i) MGK_CUDA(cudaEventCreate(&ev[i]));
+    MGK_CUDA(cudaGraphLaunch(x, s));  // warm-up
+    MGK_CUDA(cudaEventRecord(ev[0], s));
+    MGK_CUDA(cudaGraphLaunch(x, s));
+    MGK_CUDA(cudaEventRecord(ev[1], s));
+    MGK_CUDA(cudaEventSynchronize(ev[1]));
+    MGK_CUDA(cudaEventElapsedTime(ms, ev[0], ev[1]));
+    *ms /= reps;
+    return MGK_OK;
+  };
+  rc = run();
+  for (int i = 0; i < 2; ++i)
+    if (ev[i]) cudaEventDestroy(ev[i]);
+  if (x) cudaGraphExecDestroy(x);
+  if (g) cudaGraphDestroy(g);
+  return rc;
+}
 
 extern "C" int mgk_ls2d_set_family(mgk_ls2d_t p, int family) {
   MGK_REQUIRE(p, "mgk_ls2d_set_family: null plan");
@@ -1646,11 +1690,15 @@ extern "C" int mgk_ls2d_autotune(mgk_ls2d_t p, int nsel, const int* sel, const d
   for (int k = 0; k < nc; ++k) {
     int st = ls2d_set_variant(p, cands[k]);
     if (st) return st;
-    float r64 = 0, c64 = 0, r32 = 0, c32 = 0;
-    st = mgk_ls2d_profile_batch(p, nsel, sel, eps_bar, 0, reps, &r64, &c64, stream);
-    if (st == MGK_OK && p->prec == MGK_MIXED) st = mgk_ls2d_profile_batch(p, nsel, sel, eps_bar, 1, reps, &r32, &c32, stream);
+    float t64 = 0, t32 = 0;
+    st = profile_setup(p, nsel, sel, eps_bar, (cudaStream_t)stream);
+    if (st == MGK_OK) st = time_iterations(p, false, reps, &t64, (cudaStream_t)stream);
+    if (st == MGK_OK && p->prec == MGK_MIXED) {
+      st = profile_setup(p, nsel, sel, eps_bar, (cudaStream_t)stream);
+      if (st == MGK_OK) st = time_iterations(p, true, reps, &t32, (cudaStream_t)stream);
+    }
     if (st) return st;
-    const float t = r64 + c64 + r32 + c32;
+    const float t = t64 + t32;
     if (k == 0 || t < best_t) { best_t = t; best = cands[k]; }
   }
   int st = ls2d_set_variant(p, best);
@@ -1935,17 +1983,13 @@ static int profile_stages(mgk_ls2d_t p, bool f32, float* row_ms, float* col_ms, 
   return MGK_OK;
 }
 
-extern "C" int mgk_ls2d_profile_batch(mgk_ls2d_t p, int nsel, const int* sel, const double* eps_bar, int fp32,
-                                      int reps, float* row_ms, float* col_ms, mgk_stream_t stream) {
-  MGK_REQUIRE(p && eps_bar && row_ms && col_ms && reps > 0, "mgk_ls2d_profile: bad argument");
-  MGK_REQUIRE(!fp32 || p->prec == MGK_MIXED, "mgk_ls2d_profile: FP32 kernels need a mixed-precision plan");
-  cudaStream_t s = (cudaStream_t)stream;
+static int profile_setup(mgk_ls2d_t p, int nsel, const int* sel, const double* eps_bar, cudaStream_t s) {
   // set up the selection with a zero-iteration solve, then time iterations
   // with tolerance 0 and an unreachable cap so every replica stays active
   std::vector<const double*> init(nsel, nullptr);
   std::vector<double*> outs(nsel, nullptr);
   int rc = mgk_ls2d_solve_batch(p, nsel, sel, eps_bar, init.data(), outs.data(), outs.data(), 0, 0.0, nullptr,
-                                stream);
+                                (mgk_stream_t)s);
   if (rc) return rc;
   rc = staging_wait(p);
   if (rc) return rc;
@@ -1965,6 +2009,16 @@ extern "C" int mgk_ls2d_profile_batch(mgk_ls2d_t p, int nsel, const int* sel, co
   p->h_ctl->bodies = 0;
   MGK_CUDA(cudaMemcpyAsync(p->d_ctl, p->h_ctl, sizeof(Ls2dCtl), cudaMemcpyHostToDevice, s));
   MGK_CUDA(cudaStreamSynchronize(s));
+  return MGK_OK;
+}
+
+extern "C" int mgk_ls2d_profile_batch(mgk_ls2d_t p, int nsel, const int* sel, const double* eps_bar, int fp32,
+                                      int reps, float* row_ms, float* col_ms, mgk_stream_t stream) {
+  MGK_REQUIRE(p && eps_bar && row_ms && col_ms && reps > 0, "mgk_ls2d_profile: bad argument");
+  MGK_REQUIRE(!fp32 || p->prec == MGK_MIXED, "mgk_ls2d_profile: FP32 kernels need a mixed-precision plan");
+  cudaStream_t s = (cudaStream_t)stream;
+  int rc = profile_setup(p, nsel, sel, eps_bar, s);
+  if (rc) return rc;
   return profile_stages(p, fp32 != 0, row_ms, col_ms, reps, s);
 }
 

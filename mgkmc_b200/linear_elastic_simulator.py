@@ -135,7 +135,7 @@ class Ls2dBatch:
     def autotune(self, reps, eps_bars, n=5, stream=None):
         """Times every kernel family that can serve this plan on the selection
         and keeps the fastest; returns (family, ms per iteration): 0 for the
-        CTA-wide passes, 256/512/1024 for the warp-line kernels.  Replicas must
+        CTA-wide passes, 256/512/1024 for the register-FFT kernels.  Replicas must
         have their material; their iterates are left unspecified."""
         k = len(reps)
         sel = (ctypes.c_int * k)(*[int(r) for r in reps])
@@ -148,7 +148,7 @@ class Ls2dBatch:
         return ch.value, ms.value
 
     def set_family(self, family):
-        """Kernel family (0 CTA-wide, 256/512/1024 warp-line), e.g. one chosen
+        """Kernel family (0 CTA-wide, 256/512/1024 register FFTs), e.g. one chosen
         by ``autotune`` for an equal plan."""
         L.check(L.lib().mgk_ls2d_set_family(self._h, int(family)), "mgk_ls2d_set_family")
         self.family = int(family)
