@@ -220,8 +220,7 @@ __device__ __forceinline__ C* fft_any(C* a, C* b, int nlines, int ld, const FftL
 // stores of the early Stockham passes hit distinct banks).  Each pass reads
 // all of a lane's butterfly inputs into registers, synchronises the warp,
 // then writes the outputs in place: only the line's lanes synchronise between
-// passes (__syncwarp, or a named barrier for two-warp lines), so
-// warps of a CTA progress independently.
+// passes (__syncwarp), so warps of a CTA progress independently.
 namespace mgk {
 
 template <typename C> __device__ __forceinline__ int pidx(int i) {
@@ -234,28 +233,21 @@ template <typename C> constexpr int padded_len(int n) {
   return sizeof(C) == 16 ? n + n / 8 + 1 : ((n + n / 16 + 1 + 1) & ~1);
 }
 
-// Synchronises the G lanes that share a line: the warp (G = 32) or two
-// warps through named barrier `bid` (G = 64; ids 1.., 0 is __syncthreads).
-template <int G> __device__ __forceinline__ void grp_sync(int bid) {
-  if constexpr (G == 32) __syncwarp();
-  else asm volatile("bar.sync %0, %1;" ::"r"(bid), "n"(G) : "memory");
-}
-
-template <int N, int SIGN, int L, int P, int NS, int G, typename C>
-__device__ __forceinline__ void warp_pass(C* a, int stride, const C* __restrict__ tw, int lane, int bid) {
+template <int N, int SIGN, int L, int P, int NS, typename C>
+__device__ __forceinline__ void warp_pass(C* a, int stride, const C* __restrict__ tw, int lane) {
   constexpr RadixList S = make_sched(N);
   if constexpr (P < S.np) {
     constexpr int R = S.r[P];
     constexpr int nb = N / R;
-    constexpr int U = (nb + G - 1) / G;
+    constexpr int U = (nb + 31) / 32;
     constexpr int tws = N / (NS * R);
     C v[L][U][R];
 #pragma unroll
     for (int l = 0; l < L; ++l)
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        const int j = lane + G * u;
-        if (nb % G == 0 || j < nb) {
+        const int j = lane + 32 * u;
+        if (nb % 32 == 0 || j < nb) {
           if constexpr (nb % kPadPeriod<C> == 0) {
             // j + r*nb: the padding of r*nb is a constant, so one padded base
             const int pj = l * stride + pidx<C>(j);
@@ -267,11 +259,11 @@ __device__ __forceinline__ void warp_pass(C* a, int stride, const C* __restrict_
           }
         }
       }
-    grp_sync<G>(bid);
+    __syncwarp();
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int j = lane + G * u;
-      if (nb % G == 0 || j < nb) {
+      const int j = lane + 32 * u;
+      if (nb % 32 == 0 || j < nb) {
         const int k = j % NS;
         C w[R];
         if constexpr (NS > 1) {
@@ -309,16 +301,16 @@ __device__ __forceinline__ void warp_pass(C* a, int stride, const C* __restrict_
         }
       }
     }
-    grp_sync<G>(bid);
-    warp_pass<N, SIGN, L, P + 1, NS * R, G>(a, stride, tw, lane, bid);
+    __syncwarp();
+    warp_pass<N, SIGN, L, P + 1, NS * R>(a, stride, tw, lane);
   }
 }
 
 // L lines at a, a + stride, ... (padded layout), transformed in place by the
-// G lanes of the calling group (lane in [0, G)).  tw: the W_N^m table.
-template <int N, int SIGN, int L, int G = 32, typename C>
-__device__ __forceinline__ void warp_fft(C* a, int stride, const C* __restrict__ tw, int lane, int bid = 0) {
-  warp_pass<N, SIGN, L, 0, 1, G>(a, stride, tw, lane, bid);
+// calling warp.  tw: the W_N^m table.
+template <int N, int SIGN, int L, typename C>
+__device__ __forceinline__ void warp_fft(C* a, int stride, const C* __restrict__ tw, int lane) {
+  warp_pass<N, SIGN, L, 0, 1>(a, stride, tw, lane);
 }
 
 // line lengths with a compiled warp-line FFT
@@ -327,24 +319,15 @@ __host__ __device__ constexpr bool warp_fft_len(int n) {
          n == 1024;
 }
 
-// 16- or 8-byte asynchronous global -> shared copies (cp.async, completion
-// tracked per thread with commit/wait groups)
+// 16-byte asynchronous global -> shared copies (cp.async, completion tracked per
+// thread with commit/wait groups)
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
                "l"(src)
                : "memory");
 }
-__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
-               "l"(src)
-               : "memory");
-}
 __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-}
-template <typename C> __device__ __forceinline__ void cp_async_elem(C* dst, const C* src) {
-  if constexpr (sizeof(C) == 16) cp_async16(dst, src);
-  else cp_async8(dst, src);
 }
 
 }  // namespace mgk

@@ -321,7 +321,7 @@ __device__ __forceinline__ void fs_axis_body(const Fs32Args& a, int o, int k0, i
     const int rem = e - c * NL * TC;
     const int j = rem / TC, t = rem - j * TC;
     if (t < tcw)
-      cp_async_elem(&lines[(c * TC + t) * PL + pidx<C>(j)], &spec[c * plane + o * obase + j * jstride + k0 + t]);
+      cp_async16(&lines[(c * TC + t) * PL + pidx<C>(j)], &spec[c * plane + o * obase + j * jstride + k0 + t]);
   }
   cp_async_wait_all();
   __syncthreads();
