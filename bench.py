@@ -605,7 +605,7 @@ def run_finite_strain(n, peak):
         ms = s.profile_kernels(fp32=(prec == "mixed"), reps=10)
         w = 8.0 if prec == "fp64" else 4.0
         # bytes of one Krylov iteration: potentials in FP64, real fields in the mixed form
-        it_bytes = (105.0 if prec == "fp64" else 213.0) * w * N
+        it_bytes = (105.0 if prec == "fp64" else 195.0) * w * N
         stages = (["z_Kp", "y", "x_G_pq", "y_inv", "x_inv_p", "cg_update"] if prec == "fp64" else
                   ["z_fwd_Kp", "y", "x_G", "y_inv", "z_inv_pq", "cg_update"])
         out[prec] = {"seconds": sec, "load_steps_per_s": 11 / sec,
@@ -791,7 +791,7 @@ def run_ours(a):
     traffic = 242.4e6 * (N * B) / (32 * 256 * 256)
     roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
             "traffic": traffic, "traffic_source": "ncu capture, profiles/ls2d_warp_kernels_256x32_fp64.md",
-            "kernel": "ls2d_row_fast_kernel<double,256,true,true> (C2R + update + tau + R2C along y) over the batch",
+            "kernel": "ls2_row_reg<double,256> (C2R + update + tau + R2C along y) over the batch",
             "peak_kind": peak_kind, "bytes_per_launch": row_bytes,
             "kernels_us": {"row_fp64": row64 * 1e3, "col_fp64": col64 * 1e3, "row_fp32": row32 * 1e3,
                            "col_fp32": col32 * 1e3},
