@@ -14,7 +14,7 @@
 // What bounds them: HBM, 45 + 2 x 18 + 18 + 27 floats per voxel.  The former
 // passes crossed shared memory about twice per radix pass and wrote A to memory
 // between K:p and the z transform.  At 128^3, before and now (CUDA events around
-// each launch): K:p with z forward 202 and 133 us, y 56 and 37, x 88 and 65, y
+// each launch): K:p with z forward 202 and 133 us, y 56 and 37, x 88 and 61, y
 // inverse 53 and 33, z inverse 66 and 54.  72^3, from CTA-wide passes: 301 and
 // 129 us an iteration.
 #pragma once
@@ -47,7 +47,10 @@ constexpr int ml_zi_bytes(int n) {
 }
 constexpr int ml_y_bytes(int n) { return 3 * ml_yw(n) * reg_slots(n, 8) * 8; }
 constexpr int ml_x_bytes(int n) { return 9 * ml_xw(n) * reg_slots(n, 8) * 8; }
-constexpr int ml_minb(int threads) { return 65536 / (threads * 80) < 1 ? 1 : 65536 / (threads * 80); }
+constexpr int ml_minb(int threads, int regs = 80) { return 65536 / (threads * regs) < 1 ? 1 : 65536 / (threads * regs); }
+// x pass: a third CTA of 288 threads where no step has more than 16 points per
+// thread (128 points: 65 -> 60 us; 96 points, radix 24: 39.0 and 39.5 us)
+constexpr int ml_x_regs(int n) { return reg_sched32(n).r[0] > 16 || reg_sched32(n).r[1] > 16 ? 80 : 72; }
 
 template <int NZ, int ALT>
 __global__ void __launch_bounds__(ml_zf_threads(NZ), ml_minb(ml_zf_threads(NZ))) ml_zfwd(Fs32Args a) {
@@ -197,7 +200,7 @@ __global__ void __launch_bounds__(ml_y_threads(NL), ml_minb(ml_y_threads(NL))) m
 
 // x pass with G; grid = ny * ntile
 template <int NL, int ALT>
-__global__ void __launch_bounds__(ml_x_threads(NL), ml_minb(ml_x_threads(NL))) ml_xpass(Fs32Args a) {
+__global__ void __launch_bounds__(ml_x_threads(NL), ml_minb(ml_x_threads(NL), ml_x_regs(NL))) ml_xpass(Fs32Args a) {
   using C = float2;
   constexpr int TL = ml_t(NL), W = ml_xw(NL), SL = reg_slots(NL, 8), TH = ml_x_threads(NL);
   extern __shared__ __align__(16) unsigned char smem_raw[];
