@@ -879,9 +879,12 @@ extern "C" int mgk_fs3d_create(int nx, int ny, int nz, int model, mgk_fs3d_t* ou
   p->F = f; p->Ftr = f + 9 * N; p->P = f + 18 * N; p->Ptr = f + 27 * N; p->X = f + 36 * N; p->Fpi = f + 45 * N;
   p->lam = f + 54 * N; p->mu = f + 55 * N;
   if (cudaMallocHost(&p->h_sc, sizeof(FsScalars)) != cudaSuccess) return fail(MGK_OOM);
+  // The memsets run on the legacy stream and do not hold the host up; the caller's
+  // stream need not wait for that one, so the plan leaves here with them done.
+  // (The spectra and Krylov vectors start unset: every entry is written before it is read.)
   if (cudaMemset(p->fields, 0, sizeof(double) * N * (9 * 6 + 2)) != cudaSuccess ||
-      cudaMemset(p->spec, 0, sizeof(double2) * 21 * (size_t)p->plane) != cudaSuccess ||
-      cudaMemset(p->counter, 0, sizeof(unsigned int)) != cudaSuccess || cudaMemset(p->sc, 0, sizeof(FsScalars)) != cudaSuccess)
+      cudaMemset(p->counter, 0, sizeof(unsigned int)) != cudaSuccess || cudaMemset(p->sc, 0, sizeof(FsScalars)) != cudaSuccess ||
+      cudaStreamSynchronize(0) != cudaSuccess)
     return fail(MGK_CUDA_ERROR);
   const char* env = getenv("MGK_FS_FAST");
   p->fast = !(env && env[0] == '0');

@@ -58,6 +58,30 @@ bool fft_schedule(int n, FftLen* f) {
   return true;
 }
 
+// A device copy of the table h, complete on return: a copy from pageable memory
+// may still be on its way when cudaMemcpy returns, and the streams that will read
+// the table need not wait for the legacy one.
+template <typename C> static void* upload(const std::vector<C>& h) {
+  void* d = nullptr;
+  if (cudaMalloc(&d, h.size() * sizeof(C)) != cudaSuccess) return nullptr;
+  if (cudaMemcpy(d, h.data(), h.size() * sizeof(C), cudaMemcpyHostToDevice) != cudaSuccess ||
+      cudaStreamSynchronize(0) != cudaSuccess) {
+    cudaFree(d);
+    return nullptr;
+  }
+  return d;
+}
+
+template <typename C> static void* upload_twiddles(int n) {
+  std::vector<C> h(n);
+  for (int m = 0; m < n; ++m) {
+    const long double ang = -2.0L * 3.14159265358979323846264338327950288L * (long double)m / (long double)n;
+    h[m].x = (decltype(C::x))cosl(ang);
+    h[m].y = (decltype(C::x))sinl(ang);
+  }
+  return upload(h);
+}
+
 // Twiddle tables W_n^m = exp(-2 pi i m / n), one per (device, n, precision);
 // they live until process exit (a few tens of KB in total).
 const void* twiddles(int n, int prec) {
@@ -69,26 +93,8 @@ const void* twiddles(int n, int prec) {
   auto key = std::make_tuple(dev, n, prec);
   auto it = cache.find(key);
   if (it != cache.end()) return it->second;
-  void* d = nullptr;
-  const size_t bytes = (size_t)n * (prec == MGK_FP64 ? sizeof(double2) : sizeof(float2));
-  if (cudaMalloc(&d, bytes) != cudaSuccess) return nullptr;
-  if (prec == MGK_FP64) {
-    std::vector<double2> h(n);
-    for (int m = 0; m < n; ++m) {
-      long double ang = -2.0L * 3.14159265358979323846264338327950288L * (long double)m / (long double)n;
-      h[m].x = (double)cosl(ang);
-      h[m].y = (double)sinl(ang);
-    }
-    if (cudaMemcpy(d, h.data(), bytes, cudaMemcpyHostToDevice) != cudaSuccess) return nullptr;
-  } else {
-    std::vector<float2> h(n);
-    for (int m = 0; m < n; ++m) {
-      long double ang = -2.0L * 3.14159265358979323846264338327950288L * (long double)m / (long double)n;
-      h[m].x = (float)cosl(ang);
-      h[m].y = (float)sinl(ang);
-    }
-    if (cudaMemcpy(d, h.data(), bytes, cudaMemcpyHostToDevice) != cudaSuccess) return nullptr;
-  }
+  void* d = prec == MGK_FP64 ? upload_twiddles<double2>(n) : upload_twiddles<float2>(n);
+  if (!d) return nullptr;
   cache[key] = d;
   return d;
 }
@@ -119,16 +125,6 @@ template <typename C> static void fill_reg(int n, std::vector<C>& h) {
       }
     ns *= pass[p];
   }
-}
-
-template <typename C> static void* upload(const std::vector<C>& h) {
-  void* d = nullptr;
-  if (cudaMalloc(&d, h.size() * sizeof(C)) != cudaSuccess) return nullptr;
-  if (cudaMemcpy(d, h.data(), h.size() * sizeof(C), cudaMemcpyHostToDevice) != cudaSuccess) {
-    cudaFree(d);
-    return nullptr;
-  }
-  return d;
 }
 
 const void* twiddles_reg(int n, int prec) {
