@@ -198,6 +198,11 @@ MGK_API int mgk_ls2d_set_family(mgk_ls2d_t plan, int family);
  * counterpart in the reference (its solves are synchronous). */
 MGK_API int mgk_ls2d_collect(mgk_ls2d_t plan, int nsel, const int* sel, mgk_ls_info* infos, mgk_stream_t stream);
 
+/* Test hook: leaves replica `rep`'s arrival counter at `count` (below its row
+ * items, and 256), as a solve does in which a device wait gave up
+ * (MGK_TIMEOUT).  No counterpart in the reference. */
+MGK_API int mgk_ls2d_leave_arrivals(mgk_ls2d_t plan, int rep, int count, mgk_stream_t stream);
+
 /* Timing hook: runs `reps` LS iterations (tolerance 0) and returns the mean
  * duration of the row kernel (C2R+update+tau+R2C along y) and of the column
  * kernel (FFT+Gamma+IFFT along x), timed with CUDA events on `stream`.
@@ -287,6 +292,8 @@ MGK_API int mgk_ls3d_solve_batch(mgk_ls3d_t plan, int nsel, const int* sel, cons
                                  const double* const* eps_init, double* const* eps_out,
                                  double* const* sig_out, int max_iter, double tol, mgk_ls_info3* infos,
                                  mgk_stream_t stream);
+/* Test hook, as mgk_ls2d_leave_arrivals (count below the replica's z-line items). */
+MGK_API int mgk_ls3d_leave_arrivals(mgk_ls3d_t plan, int rep, int count, mgk_stream_t stream);
 
 /* After a KMC flip changed voxel (x, y) = d_xy[0..1] (device int64, e.g.
  * from mgk_kmc2d_event) of the caller's eigenstrain field, copy that voxel

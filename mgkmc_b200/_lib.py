@@ -69,6 +69,8 @@ _SIGS = {
                                   POINTER(ctypes.c_float), _P]),
     "mgk_ls2d_set_family": (c_int, [_P, c_int]),
     "mgk_ls2d_collect": (c_int, [_P, c_int, POINTER(c_int), POINTER(LsInfo), _P]),
+    "mgk_ls2d_leave_arrivals": (c_int, [_P, c_int, c_int, _P]),
+    "mgk_ls3d_leave_arrivals": (c_int, [_P, c_int, c_int, _P]),
     "mgk_ls2d_solve_batch": (c_int, [_P, c_int, POINTER(c_int), POINTER(c_double), POINTER(c_void_p),
                                      POINTER(c_void_p), POINTER(c_void_p), c_int, c_double, POINTER(LsInfo), _P]),
     "mgk_ls2d_profile_batch": (c_int, [_P, c_int, POINTER(c_int), POINTER(c_double), c_int, c_int,

@@ -199,9 +199,12 @@ __global__ void __launch_bounds__(kThreads) ls2d_means_kernel(const Ls2dRep* rep
 // Solve start for each selected replica: eps_bar, caps and the initial field
 // (linear_elastic_simulator.py:32-41), and the antisymmetric part's
 // contribution to the first diff and norm.  fp32: the loop starts with a mixed
-// plan's FP32 phase, which needs the FP32 field only.  grid = (G, nsel).
+// plan's FP32 phase, which needs the FP32 field only.  The replica's arrival
+// counter of the row kernel starts at zero whatever the call before it left: a row
+// CTA whose copy wait gave up does not arrive.  grid = (G, nsel).
 __global__ void __launch_bounds__(kThreads) ls2d_begin_kernel(const Ls2dRep* reps, Ls2dState* st, const int* sel,
-                                                              double* partials, unsigned int* ctr, int fp32) {
+                                                              double* partials, unsigned int* ctr,
+                                                              unsigned int* arrivals, int fp32) {
   __shared__ double res[2];
   const int r = sel[blockIdx.y];
   const Ls2dRep& R = reps[r];
@@ -250,6 +253,7 @@ __global__ void __launch_bounds__(kThreads) ls2d_begin_kernel(const Ls2dRep* rep
     S.done = R.max_iter <= 0 ? 2 : 0;
     S.status = MGK_OK;
     S.diff = 0;
+    arrivals[r] = 0;
     if (!init) { S.extra_d0 = 0; S.extra_n0 = 2.0 * (double)N * abar * abar; }
   }
 }
@@ -1879,7 +1883,7 @@ extern "C" int mgk_ls2d_solve_batch(mgk_ls2d_t p, int nsel, const int* sel, cons
   if (any_init)
     ls2d_means_kernel<<<dim3(G, nsel), kThreads, 0, s>>>(p->d_reps, p->d_st, d_sel, p->d_part, p->d_voxctr);
   ls2d_begin_kernel<<<dim3(G, nsel), kThreads, 0, s>>>(p->d_reps, p->d_st, d_sel, p->d_part, p->d_voxctr,
-                                                       mixed && n_active > 0);
+                                                       p->d_repctr, mixed && n_active > 0);
   MGK_CUDA(cudaGetLastError());
   if (n_active > 0) {
     if (p->aa_m > 0) {
@@ -1950,6 +1954,13 @@ extern "C" int mgk_ls2d_solve(mgk_ls2d_t p, const double* eps_bar, const double*
   MGK_REQUIRE(p && eps_bar, "mgk_ls2d_solve: null argument");
   int r0 = 0;
   return mgk_ls2d_solve_batch(p, 1, &r0, eps_bar, &eps_init, &eps_out, &sig_out, max_iter, tol, info, stream);
+}
+
+extern "C" int mgk_ls2d_leave_arrivals(mgk_ls2d_t p, int rep, int count, mgk_stream_t stream) {
+  MGK_REQUIRE(p && rep >= 0 && rep < p->nrep && count >= 0 && count < p->reps[rep].row_items && count < 256,
+              "mgk_ls2d_leave_arrivals: bad argument");
+  MGK_CUDA(cudaMemsetAsync(p->d_repctr + rep, count, 1, (cudaStream_t)stream));  // the low byte; the others are zero
+  return MGK_OK;
 }
 
 // ----------------------------------------------------------- profiling ---
@@ -2224,7 +2235,7 @@ extern "C" int mgk_ls2d_solve_noalloc(int nx, int ny, int plane_mode, const doub
   ls2d_material_kernel<<<G, kThreads, 0, s>>>(d_rep, d_st, 0, E, nu, eps_plastic, plane_mode, 1, 0, 0.0, part, d_vox);
   MGK_CUDA(cudaGetLastError());
   if (eps_init) ls2d_means_kernel<<<dim3(G, 1), kThreads, 0, s>>>(d_rep, d_st, d_sel, part, d_vox);
-  ls2d_begin_kernel<<<dim3(G, 1), kThreads, 0, s>>>(d_rep, d_st, d_sel, part, d_vox, 0);
+  ls2d_begin_kernel<<<dim3(G, 1), kThreads, 0, s>>>(d_rep, d_st, d_sel, part, d_vox, d_ctr, 0);
   MGK_CUDA(cudaGetLastError());
   if (max_iter > 0) {
     ls2d_row_kernel<double, double, false, true><<<rows, kThreads, row_smem, s>>>(

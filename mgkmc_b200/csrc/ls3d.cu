@@ -197,9 +197,11 @@ __global__ void ls3d_finalize_kernel(const Ls3dRep* reps, Ls3dState* st, const i
   if (lane == 0) out[q] = a * (mode == 2 ? 1.0 : 1.0 / (double)reps[r].N);
 }
 
-// initial field (linear_elastic_simulator.py:302-313); grid (G, nsel)
+// initial field (linear_elastic_simulator.py:302-313); grid (G, nsel).  arrivals:
+// the z-line kernels' counters, which start at zero whatever the call before left (a
+// CTA whose copy wait gave up does not arrive)
 __global__ void __launch_bounds__(kT3, 3) ls3d_begin_kernel(const Ls3dRep* reps, Ls3dState* st, const int* sel,
-                                                            double* partials) {
+                                                            double* partials, unsigned int* arrivals) {
   __shared__ double buf[9 * kT3];
   const int r = sel[blockIdx.y];
   const Ls3dRep& R = reps[r];
@@ -253,6 +255,7 @@ __global__ void __launch_bounds__(kT3, 3) ls3d_begin_kernel(const Ls3dRep* reps,
     S.done = R.max_iter <= 0 ? 2 : 0;
     S.status = MGK_OK;
     S.diff = 0;
+    arrivals[r] = 0;
     if (!R.init) {
       S.extra_d0 = 0;
       S.extra_n0 = 2.0 * (double)N * (ab[0] * ab[0] + ab[1] * ab[1] + ab[2] * ab[2]);
@@ -1151,7 +1154,7 @@ extern "C" int mgk_ls3d_solve_batch(mgk_ls3d_t p, int nsel, const int* sel, cons
                                               (int)offsetof(Ls3dState, means), 1);
     MGK_CUDA(cudaGetLastError());
   }
-  ls3d_begin_kernel<<<dim3(G, nsel), kT3, 0, s>>>(p->d_reps, p->d_st, d_sel, p->d_part);
+  ls3d_begin_kernel<<<dim3(G, nsel), kT3, 0, s>>>(p->d_reps, p->d_st, d_sel, p->d_part, p->d_repctr);
   MGK_CUDA(cudaGetLastError());
   if (any_init) {
     ls3d_finalize_kernel<<<nsel, 32 * 2, 0, s>>>(p->d_reps, p->d_st, d_sel, p->d_part, G,
@@ -1234,5 +1237,12 @@ extern "C" int mgk_ls3d_solve_batch(mgk_ls3d_t p, int nsel, const int* sel, cons
     }
     if (worst) { set_error("mgk_ls3d_solve: non-finite residual"); return worst; }
   }
+  return MGK_OK;
+}
+
+extern "C" int mgk_ls3d_leave_arrivals(mgk_ls3d_t p, int rep, int count, mgk_stream_t stream) {
+  MGK_REQUIRE(p && rep >= 0 && rep < p->nrep && count >= 0 && count < p->reps[rep].zl_items && count < 256,
+              "mgk_ls3d_leave_arrivals: bad argument");
+  MGK_CUDA(cudaMemsetAsync(p->d_repctr + rep, count, 1, (cudaStream_t)stream));  // the low byte; the others are zero
   return MGK_OK;
 }

@@ -240,7 +240,7 @@ __device__ void ls3d_decide(const Ls3dRep& R, Ls3dState& S, int r, int item, dou
     const unsigned int still = atomicExch(&ctl->still, 0u);
     ctl->decided = 0;
     ctl->n_active = still;
-    const bool go = still > 0 && atomicAdd(&ctl->bodies, 0u) <= (unsigned int)guard_cap;
+    const bool go = still > 0 && atomicAdd(&ctl->bodies, 0u) <= (unsigned int)guard_cap && *(volatile int*)&ctl->error == 0;
     ctl->any = go ? 1 : 0;
     if (use_cond) cudaGraphSetConditional(cond, go ? 1u : 0u);
   }
