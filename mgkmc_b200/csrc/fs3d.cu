@@ -373,10 +373,6 @@ __global__ void __launch_bounds__(256) fs_xinv_kernel(FsArgs a) {
 }
 
 // ------------------------------------------------------------ CG scalars ---
-// whether the device-side Krylov loop runs another iteration
-__device__ __forceinline__ bool fs_go(const FsScalars& S) {
-  return isfinite(S.rr) && S.rr > S.tol2 * S.bb && S.kcount < S.kmax && S.err == 0.0;
-}
 __global__ void fs_loop_head(FsArgs a, cudaGraphConditionalHandle cond) {
   cudaGraphSetConditional(cond, fs_go(*a.sc) ? 1u : 0u);
 }

@@ -15,6 +15,13 @@ struct FsScalars {
   double pad;
 };
 
+// Whether the device-side Krylov loop of either precision form runs another
+// iteration: the residual is finite and above the tolerance, the iteration cap is
+// not reached, and no bounded wait gave up (the vectors are stale then).
+__device__ __forceinline__ bool fs_go(const FsScalars& S) {
+  return isfinite(S.rr) && S.rr > S.tol2 * S.bb && S.kcount < S.kmax && S.err == 0.0;
+}
+
 struct FsArgs {
   int nx, ny, nz, nzh, ld;
   int tcx, tcy;  // kz columns per CTA of the general axis passes

@@ -249,8 +249,7 @@ __global__ void __launch_bounds__(256) fs_update_kernel(Fs32Args a) {
 // fixed-order sum of nb partials; MODE 0: pq -> alpha; 1: r.r -> beta, rr,
 // one more Krylov iteration counted; 2: right-hand side -> rr = bb, beta = 0,
 // iteration count reset.  MODEs 1 and 2 decide, when use_cond, whether the
-// device-side Krylov loop runs another iteration: rr > tol^2 bb, finite, and
-// below the iteration cap.
+// device-side Krylov loop runs another iteration (fs_go()).
 template <int MODE>
 __global__ void fs_scalar_kernel(Fs32Args a, int nb, cudaGraphConditionalHandle cond, int use_cond) {
   __shared__ double red[32];
@@ -282,10 +281,7 @@ __global__ void fs_scalar_kernel(Fs32Args a, int nb, cudaGraphConditionalHandle 
     S.beta = 0.0;
     S.kcount = 0.0;
   }
-  if (MODE != 0 && use_cond) {
-    const bool go = isfinite(S.rr) && S.rr > S.tol2 * S.bb && S.kcount < S.kmax;
-    cudaGraphSetConditional(cond, go ? 1u : 0u);
-  }
+  if (MODE != 0 && use_cond) cudaGraphSetConditional(cond, fs_go(S) ? 1u : 0u);
 }
 
 // ------------------------------------------------- warp-line 3D passes ---
