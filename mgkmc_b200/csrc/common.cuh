@@ -78,7 +78,8 @@ template <typename T> __device__ T block_sum(T v, T* red /* >= 32 entries */) {
 inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
 
 // Raises a kernel's dynamic shared-memory limit on the current device to at
-// least `bytes` (never lowers it: plans of different sizes share kernels).
+// least `bytes` (never lowers it: plans of different sizes share kernels), where
+// that is more than any kernel may use as it is.
 cudaError_t raise_smem(const void* fn, size_t bytes);
 
 }  // namespace mgk

@@ -798,11 +798,10 @@ static void fs32_matvec(mgk_fs3d_t p, FsLaunch L[5]) {
 }
 
 // Raise the shared-memory limits of the kernels that the plan launches in its
-// family and precision, where they need it (a kernel that is named here is loaded,
-// some 0.1 ms the first time).
+// family and precision, where they need it.
 static int fs_raise(mgk_fs3d_t p) {
   cudaError_t e = cudaSuccess;
-  auto up = [&](const FsLaunch& l) { if (e == cudaSuccess && l.smem > 46 * 1024) e = raise_smem(l.fn, l.smem); };
+  auto up = [&](const FsLaunch& l) { if (e == cudaSuccess) e = raise_smem(l.fn, l.smem); };
   if (p->prec == MGK_MIXED) {
     FsLaunch L[5];
     fs32_matvec(p, L);

@@ -1095,17 +1095,6 @@ static int plan_alloc(mgk_ls2d_t p, void** ptr, size_t bytes) {
   return MGK_OK;
 }
 
-// raises the shared-memory limits of a replica's register-FFT kernels
-static int ls2d_line_attrs(int nx, int ny, int kind) {
-  const Ls2Line *kx = ls2_line(nx, kind), *ky = ls2_line(ny, kind);
-  for (int w = 0; w < 2; ++w) {
-    for (int law = 0; law < 4; ++law)
-      if (ky->row[law][w]) MGK_CUDA(raise_smem(ky->row[law][w], ky->r_bytes[w]));
-    MGK_CUDA(raise_smem(kx->col[w], kx->c_bytes[w]));
-  }
-  return MGK_OK;
-}
-
 static void ls2d_drop_graphs(mgk_ls2d_t p) {
   for (auto& e : p->gcache) {
     cudaGraphExecDestroy(e.x);
@@ -1215,9 +1204,6 @@ extern "C" int mgk_ls2d_create_batch(int nrep, const int* nxs, const int* nys, i
         if (mixed) R.rtw32[q] = reinterpret_cast<const float2*>(twiddles_reg(n[q], MGK_MIXED));
         if (!R.rtw[q] || (mixed && !R.rtw32[q])) return fail(MGK_OOM);
       }
-      int rc = ls2d_line_attrs(nx, ny, kLs2Fp64);
-      if (rc == MGK_OK && mixed) rc = ls2d_line_attrs(nx, ny, p->fast ? kLs2Fp32 : kLs2Fp32Wide);
-      if (rc) return fail(rc);
     }
     row_smem = std::max(row_smem, 2 * 3 * (size_t)ny * c64);
     col_smem = std::max(col_smem, 2 * 3 * (size_t)R.tc * nx * c64);
@@ -1253,9 +1239,7 @@ extern "C" int mgk_ls2d_create_batch(int nrep, const int* nxs, const int* nys, i
   p->col_smem = col_smem;
   p->row_smem32 = row_smem32;
   p->col_smem32 = col_smem32;
-  int st = ls2d_set_attrs<double, double>(row_smem, col_smem);
-  if (st == MGK_OK && mixed) st = ls2d_set_attrs<float, float>(row_smem32, col_smem32);
-  if (st) return fail(st);
+  int st = MGK_OK;
   const int G = grid_blocks(p->maxN);
   p->part_doubles = std::max((size_t)2 * p->total_row_items, (size_t)nrep * G * 8);
   void* v = nullptr;
@@ -1748,8 +1732,11 @@ extern "C" int mgk_ls2d_collect(mgk_ls2d_t p, int nsel, const int* sel, mgk_ls_i
 
 // The selection by launch groups (the CTA-wide replicas first, then each
 // shape), its order and the loop's signature.  A group takes the wide forms
-// when these give at least two CTAs per SM.
-static void ls2d_group(mgk_ls2d_t p, const std::vector<int>& selv, Loop2& a, std::vector<int>& sig) {
+// when these give at least two CTAs per SM.  The shared-memory limits are raised
+// here and not in the constructor: of five sides' 50 kernels (4 laws, 2 widths) a
+// solve launches 10, and the first one named of a translation unit loads it (created
+// after a plan of other sides, one 64^2 grid 18 -> 3 ms, five sides 40 -> 5 ms).
+static int ls2d_group(mgk_ls2d_t p, const std::vector<int>& selv, Loop2& a, std::vector<int>& sig) {
   const int nsel = (int)selv.size();
   constexpr int kFill = 296;
   a = Loop2();
@@ -1769,6 +1756,11 @@ static void ls2d_group(mgk_ls2d_t p, const std::vector<int>& selv, Loop2& a, std
   c.row_local = c.row_map + c.rows;
   c.col_map = c.row_local + c.rows;
   c.col_local = c.col_map + c.cols;
+  if (c.n) {
+    int rc = ls2d_set_attrs<double, double>(a.rs, a.cs);
+    if (rc == MGK_OK && p->prec == MGK_MIXED) rc = ls2d_set_attrs<float, float>(a.rs32, a.cs32);
+    if (rc) return rc;
+  }
   sig = {p->law, p->aa_m, nsel, c.n, c.rows, c.cols};
   if (c.n) a.grp.push_back(c);
   std::vector<char> placed(p->nrep, 0);
@@ -1797,10 +1789,17 @@ static void ls2d_group(mgk_ls2d_t p, const std::vector<int>& selv, Loop2& a, std
     g.wr = (long long)g.n * ceil_div(g.nx / 2, g.ky->pairs[1]) >= kFill;
     g.wc = (long long)g.n * ceil_div(g.nyh, g.kx->cols[1]) >= kFill;
     if (g.kx32) g.wc32 = (long long)g.n * ceil_div(g.nyh, g.kx32->cols[1]) >= kFill;
+    MGK_CUDA(raise_smem(g.ky->row[p->law][g.wr], g.ky->r_bytes[g.wr]));
+    MGK_CUDA(raise_smem(g.kx->col[g.wc], g.kx->c_bytes[g.wc]));
+    if (g.kx32) {
+      MGK_CUDA(raise_smem(g.ky32->row[0][g.wr], g.ky32->r_bytes[g.wr]));
+      MGK_CUDA(raise_smem(g.kx32->col[g.wc32], g.kx32->c_bytes[g.wc32]));
+    }
     sig.insert(sig.end(), {R.nx, R.ny, g.n});
     a.grp.push_back(g);
   }
   a.grp[0].lead = 1;
+  return MGK_OK;
 }
 
 extern "C" int mgk_ls2d_solve_batch(mgk_ls2d_t p, int nsel, const int* sel, const double* eps_bar,
@@ -1829,7 +1828,7 @@ extern "C" int mgk_ls2d_solve_batch(mgk_ls2d_t p, int nsel, const int* sel, cons
   if (rc) return rc;
   Loop2& a = p->last;
   std::vector<int> sig;
-  ls2d_group(p, selv, a, sig);
+  if ((rc = ls2d_group(p, selv, a, sig))) return rc;
   // per-call records, the selection and the CTA-wide group's maps
   const Grp2& cg = a.grp[0];
   int* row_map = p->h_maps + nsel;

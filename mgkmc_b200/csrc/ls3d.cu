@@ -626,17 +626,6 @@ static int a3(mgk_ls3d_t p, void** ptr, size_t bytes) {
   return MGK_OK;
 }
 
-// raises the shared-memory limits of a replica's register-FFT kernels
-static int ls3_attrs(const Ls3dRep& R, int prec) {
-  const Ls3Line *kx = ls3_line(R.nx, prec), *ky = ls3_line(R.ny, prec), *kz = ls3_line(R.nz, prec);
-  for (int law : {0, 1, 3})
-    if (kz->zline[law]) MGK_CUDA(raise_smem(kz->zline[law], kz->z_bytes));
-  MGK_CUDA(raise_smem(ky->y[0], ky->y_bytes));
-  MGK_CUDA(raise_smem(ky->y[1], ky->y_bytes));
-  MGK_CUDA(raise_smem(kx->x, kx->x_bytes));
-  return MGK_OK;
-}
-
 static void drop_graphs3(mgk_ls3d_t p) {
   for (auto& e : p->gcache) {
     cudaGraphExecDestroy(e.x);
@@ -666,7 +655,6 @@ extern "C" int mgk_ls3d_set_precision(mgk_ls3d_t p, int precision) {
         R.rtw32[q] = reinterpret_cast<const float2*>(twiddles_reg(n[q], 1));
         if (!R.rtw32[q]) return MGK_OOM;
       }
-      if (ls3_attrs(R, MGK_MIXED)) return MGK_CUDA_ERROR;
       p->has_material[r] = 0;  // the FP32 copies come with the next set_material
     }
     MGK_CUDA(cudaMemcpy(p->d_reps, p->reps.data(), sizeof(Ls3dRep) * p->nrep, cudaMemcpyHostToDevice));
@@ -739,7 +727,6 @@ extern "C" int mgk_ls3d_create_batch(int nrep, const int* nxs, const int* nys, c
         R.rtw[q] = reinterpret_cast<const double2*>(twiddles_reg(side[q], MGK_FP64));
         if (!R.rtw[q]) return fail(MGK_OOM);
       }
-      if (int rc = ls3_attrs(R, MGK_FP64)) return fail(rc);
     } else {
       p->zl_smem = std::max(p->zl_smem, 2 * 6 * (size_t)R.nz * sizeof(double2));
       p->ax_smem = std::max(p->ax_smem, 2 * 6 * (size_t)R.tc * std::max(R.nx, R.ny) * sizeof(double2));
@@ -757,14 +744,6 @@ extern "C" int mgk_ls3d_create_batch(int nrep, const int* nxs, const int* nys, c
     R.spec = reinterpret_cast<double2*>(sp);
   }
   int st;
-  if (p->zl_smem && (raise_smem((const void*)ls3d_zline_kernel<true>, (int)p->zl_smem) ||
-      raise_smem((const void*)ls3d_zline_kernel<false>, (int)p->zl_smem) ||
-      raise_smem((const void*)ls3d_axis_kernel<1, -1>, (int)p->ax_smem) ||
-      raise_smem((const void*)ls3d_axis_kernel<1, 1>, (int)p->ax_smem) ||
-      raise_smem((const void*)ls3d_axis_kernel<0, 0>, (int)p->ax_smem))) {
-    set_error("mgk_ls3d_create: cudaFuncSetAttribute failed");
-    return fail(MGK_CUDA_ERROR);
-  }
   const int G = g3(p->maxN);
   const size_t part = std::max((size_t)2 * p->tot_zl, (size_t)nrep * G * 18);
   void* v = nullptr;
@@ -1070,6 +1049,9 @@ extern "C" int mgk_ls3d_solve_batch(mgk_ls3d_t p, int nsel, const int* sel, cons
   }
   int rc = wait3(p);
   if (rc) return rc;
+  // shared-memory limits are raised below as the kernels are taken up, not in the
+  // constructor: the first one named of a translation unit loads it (a 72x54x48 plan,
+  // created first: 8 .. 15 -> 4 ms)
   Loop3 a{p->d_reps, p->d_st, p->d_part, p->d_repctr, p->d_ctl, p->zl_smem, p->ax_smem, p->d_maps, nsel,
           g3(p->maxN), p->law, {}};
   // the selection by groups: the CTA-wide replicas first, then each shape
@@ -1086,7 +1068,14 @@ extern "C" int mgk_ls3d_solve_batch(mgk_ls3d_t p, int nsel, const int* sel, cons
     const int* m = p->d_maps + nsel;
     g.zm = m; g.zl = g.zm + g.czl; g.ym = g.zl + g.czl; g.yl = g.ym + g.cy; g.xm = g.yl + g.cy; g.xl = g.xm + g.cx;
     sig.insert(sig.end(), {nsel, g.n, g.czl, g.cy, g.cx});
-    if (g.n) a.grp.push_back(g);
+    if (g.n) {
+      MGK_CUDA(raise_smem((const void*)ls3d_zline_kernel<true>, p->zl_smem));
+      MGK_CUDA(raise_smem((const void*)ls3d_zline_kernel<false>, p->zl_smem));
+      MGK_CUDA(raise_smem((const void*)ls3d_axis_kernel<1, -1>, p->ax_smem));
+      MGK_CUDA(raise_smem((const void*)ls3d_axis_kernel<1, 1>, p->ax_smem));
+      MGK_CUDA(raise_smem((const void*)ls3d_axis_kernel<0, 0>, p->ax_smem));
+      a.grp.push_back(g);
+    }
   }
   std::vector<char> placed(p->nrep, 0);
   for (int q = 0; q < nsel; ++q) {
@@ -1108,6 +1097,11 @@ extern "C" int mgk_ls3d_solve_batch(mgk_ls3d_t p, int nsel, const int* sel, cons
       ++g.n;
     }
     sig.insert(sig.end(), {R.nx, R.ny, R.nz, g.n});
+    for (int stage = 0; stage < 4; ++stage)
+      for (int f32 = 0; f32 <= (g.kx32 ? 1 : 0); ++f32) {
+        const Launch3 l = stage3(a, g, stage, f32 != 0);
+        MGK_CUDA(raise_smem(l.fn, l.smem));
+      }
     a.grp.push_back(g);
   }
   a.grp[0].lead = 1;
