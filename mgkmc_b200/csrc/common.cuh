@@ -6,6 +6,8 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <vector>
+
 #include "../../include/mgkmc.h"
 
 namespace mgk {
@@ -81,5 +83,28 @@ inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
 // least `bytes` (never lowers it: plans of different sizes share kernels), where
 // that is more than any kernel may use as it is.
 cudaError_t raise_smem(const void* fn, size_t bytes);
+
+// Up to `want` non-blocking streams of a priority on the current device, each with
+// an event, lent to one call at a time: making them costs 60 us a piece, so they
+// are kept, at most kSideStreams per device and priority (a call gets fewer when
+// the others are out).  The borrower returns them with no work in flight.
+constexpr size_t kSideStreams = 16;
+struct SideStream {
+  cudaStream_t s;
+  cudaEvent_t done;
+};
+class SideStreams {
+ public:
+  SideStreams(size_t want, int priority);
+  ~SideStreams();
+  SideStreams(const SideStreams&) = delete;
+  SideStreams& operator=(const SideStreams&) = delete;
+  size_t size() const { return v.size(); }
+  const SideStream& operator[](size_t i) const { return v[i]; }
+
+ private:
+  std::vector<SideStream> v;
+  int device = -1, priority;
+};
 
 }  // namespace mgk

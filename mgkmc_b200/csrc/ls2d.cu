@@ -52,6 +52,8 @@
 
 #include <algorithm>
 #include <mutex>
+#include <set>
+#include <utility>
 #include <vector>
 
 #include "common.cuh"
@@ -1007,6 +1009,7 @@ struct Grp2 {
   const int *row_map = nullptr, *row_local = nullptr, *col_map = nullptr, *col_local = nullptr;
   int rows = 0, cols = 0;    // CTA-wide: items over its replicas
   int lead = 0;              // counts the loop bodies
+  Ls2dCtl* ctl = nullptr;    // its loop's control block
 };
 
 struct Loop2 {
@@ -1014,7 +1017,7 @@ struct Loop2 {
   Ls2dState* st = nullptr;
   double* part = nullptr;
   unsigned int* ctr = nullptr;
-  Ls2dCtl* ctl = nullptr;
+  Ls2dCtl* ctl = nullptr;                     // one for the graph's loop, or one per group (host_loop)
   size_t rs = 0, cs = 0, rs32 = 0, cs32 = 0;  // shared memory of the CTA-wide passes
   const int* sel = nullptr;
   int nsel = 0, G = 0, law = 0;
@@ -1046,7 +1049,8 @@ struct mgk_ls2d_plan {
   std::vector<char> has_material;
   Ls2dRep* h_reps = nullptr;      // pinned staging of the table
   int* h_maps = nullptr;          // pinned staging: row_map, row_local, col_map, col_local, sel
-  Ls2dCtl* h_ctl = nullptr;
+  Ls2dCtl* h_ctl = nullptr;       // 2 nctl: staging, and the host-driven loop's copies
+  int nctl = 0;                   // control blocks: the plan's distinct shapes, and one
   Ls2dState* h_state = nullptr;
   cudaEvent_t staged = nullptr;   // last upload from the staging buffers
   bool staged_pending = false;
@@ -1074,6 +1078,7 @@ struct mgk_ls2d_plan {
   };
   std::vector<GraphEntry> gcache;
   int graph_mode = 1;  // 0: host-driven loop
+  std::vector<std::pair<std::vector<int>, int>> sights;  // uses of selections of several shapes without a graph
   Loop2 last;          // the last call's launches (the timing hook repeats its stages)
   // Anderson mixing inside the loop (one replica per solve): depth, ring
   // buffer of (3 + 2 m) strain fields, state and per-block partial sums
@@ -1251,7 +1256,12 @@ extern "C" int mgk_ls2d_create_batch(int nrep, const int* nxs, const int* nys, i
   p->d_reps = reinterpret_cast<Ls2dRep*>(v);
   if ((st = plan_alloc(p, &v, sizeof(Ls2dState) * nrep))) return fail(st);
   p->d_st = reinterpret_cast<Ls2dState*>(v);
-  if ((st = plan_alloc(p, &v, sizeof(Ls2dCtl)))) return fail(st);
+  {
+    std::set<std::pair<int, int>> shapes;
+    for (int r = 0; r < nrep; ++r) shapes.insert({nxs[r], nys[r]});
+    p->nctl = (int)shapes.size() + 1;
+  }
+  if ((st = plan_alloc(p, &v, sizeof(Ls2dCtl) * p->nctl))) return fail(st);
   p->d_ctl = reinterpret_cast<Ls2dCtl*>(v);
   const size_t nmaps = 2 * (size_t)p->total_row_items + 2 * (size_t)p->total_col_items + nrep;
   if ((st = plan_alloc(p, &v, sizeof(int) * nmaps))) return fail(st);
@@ -1261,11 +1271,11 @@ extern "C" int mgk_ls2d_create_batch(int nrep, const int* nxs, const int* nys, i
   p->d_voxctr = p->d_repctr + nrep;
   if (cudaMemset(p->d_repctr, 0, sizeof(unsigned int) * 2 * nrep) != cudaSuccess ||
       cudaMemset(p->d_st, 0, sizeof(Ls2dState) * nrep) != cudaSuccess ||
-      cudaMemset(p->d_ctl, 0, sizeof(Ls2dCtl)) != cudaSuccess)
+      cudaMemset(p->d_ctl, 0, sizeof(Ls2dCtl) * p->nctl) != cudaSuccess)
     return fail(MGK_CUDA_ERROR);
   if (cudaMallocHost(&p->h_reps, sizeof(Ls2dRep) * nrep) != cudaSuccess ||
       cudaMallocHost(&p->h_maps, sizeof(int) * nmaps) != cudaSuccess ||
-      cudaMallocHost(&p->h_ctl, sizeof(Ls2dCtl)) != cudaSuccess ||
+      cudaMallocHost(&p->h_ctl, sizeof(Ls2dCtl) * 2 * p->nctl) != cudaSuccess ||
       cudaMallocHost(&p->h_state, sizeof(Ls2dState) * nrep) != cudaSuccess)
     return fail(MGK_OOM);
   if (cudaEventCreateWithFlags(&p->staged, cudaEventDisableTiming) != cudaSuccess) return fail(MGK_CUDA_ERROR);
@@ -1463,7 +1473,7 @@ static cudaError_t with_stage2(Loop2& a, Grp2& g, int stage, bool f32, int final
                        (size_t)kx->c_bytes[w]}, x);
     }
     const int w = g.wr;
-    void* x[] = {&a.reps, &a.st, &g.sel, &a.part, &a.ctr, &a.ctl, &h, &use, &cap, &g.lead, &stage, &final};
+    void* x[] = {&a.reps, &a.st, &g.sel, &a.part, &a.ctr, &g.ctl, &h, &use, &cap, &g.lead, &stage, &final};
     return f(Launch2{ky->row[f32 ? 0 : a.law][w], dim3(g.n * ceil_div(g.nx / 2, ky->pairs[w])),
                      dim3(ky->r_threads[w]), (size_t)ky->r_bytes[w]}, x);
   }
@@ -1477,15 +1487,19 @@ static cudaError_t with_stage2(Loop2& a, Grp2& g, int stage, bool f32, int final
                                         : (const void*)ls2d_row_kernel<float, float, false, false>)
                        : (stage == kRow ? (const void*)ls2d_row_kernel<double, double, true, true>
                                         : (const void*)ls2d_row_kernel<double, double, false, true>);
-  void* x[] = {&a.reps, &a.st, &g.row_map, &g.row_local, &a.part, &a.ctr, &a.ctl, &h, &use, &cap};
+  void* x[] = {&a.reps, &a.st, &g.row_map, &g.row_local, &a.part, &a.ctr, &g.ctl, &h, &use, &cap};
   return f(Launch2{fn, dim3(g.rows), dim3(kThreads), f32 ? a.rs32 : a.rs}, x);
 }
 
+static int launch2(Loop2& a, Grp2& g, int stage, bool f32, int final, cudaStream_t s) {
+  MGK_CUDA(with_stage2(a, g, stage, f32, final, 0, 0, 0, [&](const Launch2& L, void** args) {
+    return cudaLaunchKernel(L.fn, L.grid, L.block, args, L.smem, s);
+  }));
+  return MGK_OK;
+}
 static int launch2(Loop2& a, int stage, bool f32, int final, cudaStream_t s) {
   for (Grp2& g : a.grp)
-    MGK_CUDA(with_stage2(a, g, stage, f32, final, 0, 0, 0, [&](const Launch2& L, void** args) {
-      return cudaLaunchKernel(L.fn, L.grid, L.block, args, L.smem, s);
-    }));
+    if (int rc = launch2(a, g, stage, f32, final, s)) return rc;
   return MGK_OK;
 }
 
@@ -1503,13 +1517,13 @@ static void* aa_update_fn(int m) {
   }
 }
 
-static int launch_body(Loop2& a, bool f32, cudaStream_t s) {
-  int rc = launch2(a, kCol, f32, !f32, s);
-  if (rc == MGK_OK) rc = launch2(a, kRow, f32, !f32, s);
+static int launch_body(Loop2& a, Grp2& g, bool f32, cudaStream_t s) {
+  int rc = launch2(a, g, kCol, f32, !f32, s);
+  if (rc == MGK_OK) rc = launch2(a, g, kRow, f32, !f32, s);
   if (rc == MGK_OK && !f32 && a.aa_m > 0) {
     void* args[] = {&a.reps, &a.st, &a.sel, &a.aa_buf, &a.aa, &a.aa_m, &a.aa_part};
     MGK_CUDA(cudaLaunchKernel(aa_update_fn(a.aa_m), dim3(a.aa_nb), dim3(kAaThreads), args, 0, s));
-    rc = launch2(a, kFirst, false, 1, s);  // the mix and tau of the mixed iterate
+    rc = launch2(a, g, kFirst, false, 1, s);  // the mix and tau of the mixed iterate
   }
   return rc;
 }
@@ -1601,6 +1615,73 @@ static int build_graph(mgk_ls2d_t p, Loop2& a, int cap, cudaGraph_t* gout, cudaG
   *gout = g;
   *xout = x;
   return MGK_OK;
+}
+
+// The loop driven from the host, from the first tau on; the caller's stream has
+// drained when it returns.  Each group runs on a stream of its own (as far as there
+// are side streams) with its own control block and phase.  The host launches kBodies iterations per group (body by
+// body, the groups in turn) before it looks at the control blocks: a body too many is
+// two launches that return at once.
+static int host_loop(mgk_ls2d_t p, Loop2& a, int max_iter, cudaStream_t s) {
+  constexpr int kBodies = 4;
+  const bool mixed = p->prec == MGK_MIXED;
+  const size_t G = a.grp.size();
+  struct Run {
+    cudaStream_t s;
+    bool f32;
+    int left;  // bodies of this phase yet to launch
+  };
+  std::vector<Run> run(G);
+  int priority = 0;
+  MGK_CUDA(cudaStreamGetPriority(s, &priority));
+  const SideStreams side(G - 1, priority);
+  auto loop = [&]() -> int {
+    // the fork's event joins later: a wait means the record before it
+    if (side.size()) MGK_CUDA(cudaEventRecord(side[0].done, s));
+    for (size_t i = 0; i < side.size(); ++i) MGK_CUDA(cudaStreamWaitEvent(side[i].s, side[0].done, 0));
+    for (size_t i = 0; i < G; ++i) {
+      run[i] = {i > 0 && i <= side.size() ? side[i - 1].s : s, mixed, max_iter};
+      if (int e = launch2(a, a.grp[i], kFirst, mixed, !mixed, run[i].s)) return e;
+    }
+    for (size_t open = G; open > 0;) {
+      for (int b = 0; b < kBodies; ++b)
+        for (size_t i = 0; i < G; ++i)
+          if (run[i].left > 0) {
+            if (int e = launch_body(a, a.grp[i], run[i].f32, run[i].s)) return e;
+            --run[i].left;
+          }
+      for (size_t i = 0; i < side.size(); ++i) {
+        MGK_CUDA(cudaEventRecord(side[i].done, side[i].s));
+        MGK_CUDA(cudaStreamWaitEvent(s, side[i].done, 0));
+      }
+      Ls2dCtl* c = p->h_ctl + p->nctl;
+      MGK_CUDA(cudaMemcpyAsync(c, a.ctl, sizeof(Ls2dCtl) * G, cudaMemcpyDeviceToHost, s));
+      MGK_CUDA(cudaStreamSynchronize(s));
+      open = 0;
+      for (size_t i = 0; i < G; ++i) {
+        if (c[i].error) {
+          set_error("mgk_ls2d_solve: a bulk copy wait gave up (device timeout)");
+          return MGK_TIMEOUT;
+        }
+        if (!c[i].any) run[i].left = 0;
+        if (run[i].left == 0 && run[i].f32) {  // the FP32 phase is over: on to the FP64 iterations
+          Grp2& g = a.grp[i];
+          run[i].f32 = false;
+          run[i].left = max_iter;
+          if (!g.ky) ls2d_promote_kernel<<<dim3(a.G, g.n), kThreads, 0, run[i].s>>>(a.reps, g.sel);
+          ls2d_phase2_kernel<<<1, 32, 0, run[i].s>>>(a.st, g.sel, g.n, g.ctl);
+          MGK_CUDA(cudaGetLastError());
+          if (int e = launch2(a, g, kPromote, false, 1, run[i].s)) return e;
+        }
+        open += run[i].left > 0;
+      }
+    }
+    return MGK_OK;
+  };
+  const int rc = loop();
+  if (rc)
+    for (size_t i = 0; i < side.size(); ++i) cudaStreamSynchronize(side[i].s);
+  return rc;
 }
 
 // Switches the plan's kernel family (see mgk_ls2d_plan::fast).
@@ -1762,6 +1843,7 @@ static int ls2d_group(mgk_ls2d_t p, const std::vector<int>& selv, Loop2& a, std:
     if (rc) return rc;
   }
   sig = {p->law, p->aa_m, nsel, c.n, c.rows, c.cols};
+  c.sel = p->d_maps;
   if (c.n) a.grp.push_back(c);
   std::vector<char> placed(p->nrep, 0);
   for (int q = 0; q < nsel; ++q) {
@@ -1799,7 +1881,25 @@ static int ls2d_group(mgk_ls2d_t p, const std::vector<int>& selv, Loop2& a, std:
     a.grp.push_back(g);
   }
   a.grp[0].lead = 1;
+  for (Grp2& g : a.grp) g.ctl = a.ctl;
   return MGK_OK;
+}
+
+// Whether a selection of several shapes whose caller waits for it is driven from the
+// host: at its first kHostUses uses.  Its graph takes 360 us to instantiate with five
+// shapes (135 with one, 55 for every further branch of a body; mixed plans have two
+// bodies), most of a warm-started solve, and an ensemble's selections change from
+// round to round; a host-driven solve of 3 .. 5 shapes takes 20 us less to 80 us more.
+// First solve of a fresh plan of the five sides 128 .. 512, warm: 815 -> 466 us (660
+// with the one pair of kernels for all shapes that the register passes replaced).
+static bool ls2d_host_first(mgk_ls2d_t p, const std::vector<int>& sig) {
+  constexpr int kHostUses = 4;
+  constexpr size_t kSights = 64;
+  for (auto& e : p->sights)
+    if (e.first == sig) return e.second < kHostUses && ++e.second <= kHostUses;
+  if (p->sights.size() >= kSights) p->sights.erase(p->sights.begin());
+  p->sights.push_back({sig, 1});
+  return true;
 }
 
 extern "C" int mgk_ls2d_solve_batch(mgk_ls2d_t p, int nsel, const int* sel, const double* eps_bar,
@@ -1861,16 +1961,19 @@ extern "C" int mgk_ls2d_solve_batch(mgk_ls2d_t p, int nsel, const int* sel, cons
       for (int i = 0; i < H.col_items; ++i) { col_map[ci] = r; col_local[ci] = i; ++ci; }
     }
   const int n_active = max_iter > 0 ? nsel : 0;
-  p->h_ctl->n_active = (unsigned int)n_active;
-  p->h_ctl->decided = 0;
-  p->h_ctl->still = 0;
-  p->h_ctl->bodies = 0;
-  p->h_ctl->any = n_active > 0;
-  p->h_ctl->error = 0;
+  const char* env = getenv("MGK_NO_GRAPH_WHILE");
+  if (env && env[0] == '1') p->graph_mode = 0;
+  const bool hosted = p->graph_mode == 0 || (infos && a.grp.size() > 1 && ls2d_host_first(p, sig));
+  const size_t nc = hosted ? a.grp.size() : 1;
+  for (size_t i = 0; i < nc; ++i) {
+    const int n = n_active == 0 ? 0 : hosted ? a.grp[i].n : nsel;
+    p->h_ctl[i] = Ls2dCtl{(unsigned int)n, 0u, 0u, 0u, n > 0, 0};
+    if (hosted) a.grp[i].ctl = a.ctl + i;
+  }
   const size_t nm = nsel + 2 * (size_t)(ri + ci);
   MGK_CUDA(cudaMemcpyAsync(p->d_maps, p->h_maps, sizeof(int) * nm, cudaMemcpyHostToDevice, s));
   MGK_CUDA(cudaMemcpyAsync(p->d_reps, p->h_reps, sizeof(Ls2dRep) * p->nrep, cudaMemcpyHostToDevice, s));
-  MGK_CUDA(cudaMemcpyAsync(p->d_ctl, p->h_ctl, sizeof(Ls2dCtl), cudaMemcpyHostToDevice, s));
+  MGK_CUDA(cudaMemcpyAsync(p->d_ctl, p->h_ctl, sizeof(Ls2dCtl) * nc, cudaMemcpyHostToDevice, s));
   MGK_CUDA(cudaEventRecord(p->staged, s));
   p->staged_pending = true;
 
@@ -1894,12 +1997,9 @@ extern "C" int mgk_ls2d_solve_batch(mgk_ls2d_t p, int nsel, const int* sel, cons
       ls2d_aa_init_kernel<<<p->aa_nb, kThreads, 0, s>>>(p->d_reps, d_sel, p->aa_buf, p->d_aa);
       MGK_CUDA(cudaGetLastError());
     }
-    if ((rc = launch2(a, kFirst, mixed, !mixed, s))) return rc;
-    const int cap = (max_iter + 2 > 1000 ? max_iter + 2 : 1000);
-    const char* env = getenv("MGK_NO_GRAPH_WHILE");
-    if (env && env[0] == '1') p->graph_mode = 0;
     cudaGraphExec_t exec = nullptr;
-    if (p->graph_mode == 1) {
+    if (!hosted) {
+      const int cap = (max_iter + 2 > 1000 ? max_iter + 2 : 1000);
       for (auto& e : p->gcache)
         if (e.cap >= cap && e.sig == sig) exec = e.x;
       if (!exec) {
@@ -1913,29 +2013,23 @@ extern "C" int mgk_ls2d_solve_batch(mgk_ls2d_t p, int nsel, const int* sel, cons
           }
           p->gcache.push_back({sig, cap, g, exec});
         } else {
+          exec = nullptr;
           p->graph_mode = 0;
         }
       }
     }
-    if (p->graph_mode == 1) {
+    if (exec) {
+      if ((rc = launch2(a, kFirst, mixed, !mixed, s))) return rc;
       MGK_CUDA(cudaGraphLaunch(exec, s));
     } else {
-      // host-driven loop: poll the device flag after each iteration
-      for (int phase = mixed ? 1 : 2; phase <= 2; ++phase) {
-        if (phase == 2 && mixed) {
-          if (!a.grp[0].ky) ls2d_promote_kernel<<<dim3(G, a.grp[0].n), kThreads, 0, s>>>(p->d_reps, d_sel);
-          ls2d_phase2_kernel<<<1, 32, 0, s>>>(p->d_st, d_sel, nsel, p->d_ctl);
-          MGK_CUDA(cudaGetLastError());
-          if ((rc = launch2(a, kPromote, false, 1, s))) return rc;
+      if (!hosted && a.grp.size() > 1) {  // no graph after all: the groups' own control blocks
+        for (size_t i = 0; i < a.grp.size(); ++i) {
+          p->h_ctl[p->nctl + i] = Ls2dCtl{(unsigned int)a.grp[i].n, 0u, 0u, 0u, 1, 0};
+          a.grp[i].ctl = a.ctl + i;
         }
-        for (int it = 0; it < max_iter; ++it) {
-          if ((rc = launch_body(a, phase == 1, s))) return rc;
-          Ls2dCtl hc;
-          MGK_CUDA(cudaMemcpyAsync(&hc, p->d_ctl, sizeof(Ls2dCtl), cudaMemcpyDeviceToHost, s));
-          MGK_CUDA(cudaStreamSynchronize(s));
-          if (!hc.any) break;
-        }
+        MGK_CUDA(cudaMemcpyAsync(p->d_ctl, p->h_ctl + p->nctl, sizeof(Ls2dCtl) * a.grp.size(), cudaMemcpyHostToDevice, s));
       }
+      if ((rc = host_loop(p, a, max_iter, s))) return rc;
     }
   }
   auto out = p->law == 1   ? ls2d_output_kernel<1>

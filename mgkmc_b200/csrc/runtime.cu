@@ -40,6 +40,51 @@ cudaError_t raise_smem(const void* fn, size_t bytes) {
   return e;
 }
 
+namespace {
+struct SidePool {
+  std::mutex m;
+  struct Kind {
+    size_t made = 0;
+    std::vector<SideStream> free;
+  };
+  std::map<std::pair<int, int>, Kind> kinds;  // by device and priority
+};
+// never destroyed: it may be needed while the process ends
+SidePool& side_pool() {
+  static SidePool* p = new SidePool();
+  return *p;
+}
+}  // namespace
+
+SideStreams::SideStreams(size_t want, int prio) : priority(prio) {
+  if (want == 0 || cudaGetDevice(&device) != cudaSuccess) return;
+  SidePool& P = side_pool();
+  std::lock_guard<std::mutex> g(P.m);
+  SidePool::Kind& k = P.kinds[{device, priority}];
+  while (v.size() < want) {
+    if (k.free.empty()) {
+      SideStream n{};
+      if (k.made == kSideStreams || cudaStreamCreateWithPriority(&n.s, cudaStreamNonBlocking, priority) != cudaSuccess) break;
+      if (cudaEventCreateWithFlags(&n.done, cudaEventDisableTiming) != cudaSuccess) {
+        cudaStreamDestroy(n.s);
+        break;
+      }
+      ++k.made;
+      k.free.push_back(n);
+    }
+    v.push_back(k.free.back());
+    k.free.pop_back();
+  }
+}
+
+SideStreams::~SideStreams() {
+  if (v.empty()) return;
+  SidePool& P = side_pool();
+  std::lock_guard<std::mutex> g(P.m);
+  SidePool::Kind& k = P.kinds[{device, priority}];
+  k.free.insert(k.free.end(), v.begin(), v.end());
+}
+
 bool fft_schedule(int n, FftLen* f) {
   if (n < 1 || n > 4096) return false;
   int m = n, a = 0, b = 0;
