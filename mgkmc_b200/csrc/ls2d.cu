@@ -415,7 +415,7 @@ __global__ void __launch_bounds__(256) ls2d_row_kernel(const Ls2dRep* __restrict
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  ls2d_decide(R, S, partials, ctl, cond, use_cond, guard_cap, red, FINAL);
+  ls2d_decide(R, S, partials, ctl, cond, use_cond, guard_cap, FINAL);
 }
 
 // Column kernel: FFT along x, Gamma0_sym, inverse FFT along x, for a tile of
@@ -1952,7 +1952,6 @@ extern "C" int mgk_ls2d_solve_batch(mgk_ls2d_t p, int nsel, const int* sel, cons
       H.aa = p->aa_m > 0 ? p->d_aa : nullptr;
       H.aa_x = p->aa_m > 0 ? p->aa_buf : nullptr;
       H.aa_dG = p->aa_m > 0 ? p->aa_buf + (size_t)(3 + p->aa_m) * 3 * (size_t)H.N : nullptr;
-      if (g.ky) H.row_items = ceil_div(H.nx / 2, g.ky->pairs[g.wr]);
       H.row_first = first;
       first += H.row_items;
       p->h_maps[k] = r;

@@ -10,6 +10,7 @@
 namespace mgk {
 
 constexpr int kAaMax = 8;  // deepest Anderson history
+constexpr int kMaxPairs = 2048;  // row pairs of a replica (sides up to 4096)
 struct Ls2dAA;
 
 struct Ls2dRep {
@@ -326,20 +327,30 @@ __device__ __forceinline__ void law_sigma(double m, double l, double dxx, double
   }
 }
 
-// Convergence decision of replica r once the last of its row items has
-// written its partial sums (all threads of the CTA call; thread 0 decides).
-// The last replica to decide sets the graph while-node's condition.
+// Convergence decision of replica r once the last of its row pairs' partial sums
+// is written (all threads of the CTA call, in whole warps; thread 0 decides): a
+// warp tree over every 32 pairs, then one over their results, so that the order of
+// the sums does not depend on the CTA's size.  The last replica to decide sets the graph while-node's condition.
 // final: this phase's decision is the last one (FP64 iterations).
 static __device__ void ls2d_decide(const Ls2dRep& R, Ls2dState& S, const double* partials, Ls2dCtl* ctl,
-                                   cudaGraphConditionalHandle cond, int use_cond, int guard_cap, double* red,
-                                   bool final) {
-  double a = 0, b = 0;
-  for (int i = threadIdx.x; i < R.row_items; i += blockDim.x) {
-    a += __ldcg(&partials[2 * (R.row_first + i)]);
-    b += __ldcg(&partials[2 * (R.row_first + i) + 1]);
+                                   cudaGraphConditionalHandle cond, int use_cond, int guard_cap, bool final) {
+  __shared__ double2 part32[kMaxPairs / 32];
+  const double2* p = reinterpret_cast<const double2*>(partials) + R.row_first;
+  const int lane = threadIdx.x & 31, n32 = (R.row_items + 31) / 32;
+#pragma unroll 2
+  for (int g = threadIdx.x >> 5; g < n32; g += blockDim.x >> 5) {
+    const int i = 32 * g + lane;
+    double2 v = i < R.row_items ? __ldcg(p + i) : make_double2(0.0, 0.0);
+    v.x = warp_sum(v.x);
+    v.y = warp_sum(v.y);
+    if (lane == 0) part32[g] = v;
   }
-  a = block_sum(a, red);
-  b = block_sum(b, red);
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  double a = 0, b = 0;
+  for (int g = lane; g < n32; g += 32) { a += part32[g].x; b += part32[g].y; }
+  a = warp_sum(a);
+  b = warp_sum(b);
   if (threadIdx.x != 0) return;
   if (S.iter == 0) { a += S.extra_d0; b += S.extra_n0; }
   else { b += 2.0 * (double)R.N * S.abar * S.abar; }

@@ -34,15 +34,17 @@ constexpr int ls2_pairs(int n) { return reg_sched64(n).t <= 9 ? 4 : reg_sched64(
 // threads: those of the transforms, and enough for equal rounds of the voxel
 // stage of at most 128 (256 for the longer lines) voxel pairs
 constexpr int ls2_r_threads(int n, int p, int csz) {
-  const int fft = 3 * reg_sched(n, csz).t * p, vox = p * n, cap = n <= 256 ? 128 : 256;
+  const int fft = 3 * reg_sched(n, csz).t * p, vox = p * ls2_round32(n), cap = n <= 256 ? 128 : 256;
   const int rounds = (vox + cap - 1) / cap, per = (vox + rounds - 1) / rounds;
   return ls2_round32(fft > per ? fft : per);
 }
 // columns per CTA: rows of 64 bytes in the wide kernel where the CTA stays
-// below 432 threads, of 32 or 16 otherwise; 16 in the narrow one
+// below 432 threads, of 32 or 16 otherwise; 16 in the narrow one.  Lines of at most
+// 32 points have the wide form only: their narrow CTA is a single warp, whose
+// one-round loops the compiler contracts differently.
 constexpr int ls2_cols(int n, int csz, bool wide) {
   const int t = reg_sched(n, csz).t, one = 16 / csz;
-  return wide ? (t * one <= 36 ? 4 * one : t * one <= 72 ? 2 * one : csz == 16 ? 2 : one) : one;
+  return wide || n <= 32 ? (t * one <= 36 ? 4 * one : t * one <= 72 ? 2 * one : csz == 16 ? 2 : one) : one;
 }
 constexpr int ls2_c_threads(int n, int w, int csz) { return ls2_round32(3 * w * reg_sched(n, csz).t); }
 // row pitch of the half spectra
@@ -100,8 +102,15 @@ __global__ void __launch_bounds__(ls2_r_threads(NY, P, 2 * (int)sizeof(T)),
   using C = C_t<T>;
   constexpr int TL = reg_sched(NY, sizeof(C)).t, TH = ls2_r_threads(NY, P, sizeof(C)), SL = reg_slots(NY, sizeof(C));
   constexpr int NYH = NY / 2 + 1;
+  // A pair's sums behind the update norm do not depend on P: its voxel pairs, padded
+  // to whole warps, are folded warp by warp (K = 1), or after the K rounds in which the
+  // CTA of either form takes them up alike; where there is one form, after the loop.
+  constexpr bool ONE = ls2_pairs(NY) == 1;
+  constexpr int NYP = ls2_round32(NY), T1 = ls2_r_threads(NY, 1, sizeof(C));
+  constexpr int K = T1 == ls2_r_threads(NY, ls2_pairs(NY), sizeof(C)) && NYP % T1 == 0 ? NYP / T1 : 1;
+  constexpr int NCH = ONE || K > 1 ? TH / 32 : NYP / 32;  // parts of a pair's sum
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ double red[32];
+  __shared__ double chunk[2][P * NCH];
   __shared__ int s_last;
   __shared__ __align__(8) uint64_t bar;
   const int per = (reps[sel[0]].nx / 2 + P - 1) / P;
@@ -187,60 +196,75 @@ __global__ void __launch_bounds__(ls2_r_threads(NY, P, 2 * (int)sizeof(T)),
     if (first != 0 && R.aa) nmix = aa_load(R, gam);
   const bool img_only = LAW != 0 && first == 0 && R.aa != nullptr;
   double d2 = 0, n2 = 0;
+  // the warp's 32 sums of each kind: the low lanes fold d2, the high ones n2
+  auto fold = [&](int part) {
+    const bool low = (threadIdx.x & 16) == 0;
+    double v = (low ? d2 : n2) + __shfl_xor_sync(0xffffffffu, low ? n2 : d2, 16);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o, 16);
+    if ((threadIdx.x & 15) == 0) chunk[low ? 0 : 1][part] = v;
+    d2 = n2 = 0;
+  };
 #pragma unroll 1
-  for (int e = threadIdx.x; e < np * NY; e += TH) {
-    const int q = e / NY, y = e - q * NY;
-    C* vx = lines + q * 3 * SL + reg_slot<NY, C>(y);
-    // every input of the two voxels before the first store
-    double o[2][3], m[2], l[2], pl[2][3];
+  for (int e = threadIdx.x; e < np * NYP; e += TH) {
+    const int q = e / NYP, y = e - q * NYP;
+    if (NY == NYP || y < NY) {
+      C* vx = lines + q * 3 * SL + reg_slot<NY, C>(y);
+      // every input of the two voxels before the first store
+      double o[2][3], m[2], l[2], pl[2][3];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const long long i = (2LL * (p0 + q) + h) * NY + y;
+      for (int h = 0; h < 2; ++h) {
+        const long long i = (2LL * (p0 + q) + h) * NY + y;
 #pragma unroll
-      for (int k = 0; k < 3; ++k)
-        o[h][k] = sizeof(T) == 8 && first == 2 ? (double)R.eps32[k * N + i] : (double)eps[k * N + i];
-      m[h] = (double)mu[i];
-      l[h] = (double)lam[i];
+        for (int k = 0; k < 3; ++k)
+          o[h][k] = sizeof(T) == 8 && first == 2 ? (double)R.eps32[k * N + i] : (double)eps[k * N + i];
+        m[h] = (double)mu[i];
+        l[h] = (double)lam[i];
 #pragma unroll
-      for (int k = 0; k < 3; ++k) pl[h][k] = (double)ep[k * N + i];
-    }
-    T tr[2][3];
+        for (int k = 0; k < 3; ++k) pl[h][k] = (double)ep[k * N + i];
+      }
+      T tr[2][3];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const long long i = (2LL * (p0 + q) + h) * NY + y;
-      double ev[3];
-      if (first == 0) {
-        const C z0 = vx[0], z1 = vx[SL], z2 = vx[2 * SL];
-        ev[0] = eb0 + (double)(h == 0 ? z0.x : z0.y);
-        ev[1] = eb1 + (double)(h == 0 ? z1.x : z1.y);
-        ev[2] = eb2 + (double)(h == 0 ? z2.x : z2.y);
-        const double q0 = ev[0] - o[h][0], q1 = ev[1] - o[h][1], q2 = ev[2] - o[h][2];
-        d2 += q0 * q0 + q1 * q1 + 2.0 * q2 * q2;
-        n2 += o[h][0] * o[h][0] + o[h][1] * o[h][1] + 2.0 * o[h][2] * o[h][2];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) eps[k * N + i] = (T)ev[k];
-      } else {
-#pragma unroll
-        for (int k = 0; k < 3; ++k) ev[k] = o[h][k];
-        if constexpr (LAW != 0)
-          if (R.aa) aa_mix_voxel(R, i, nmix, gam, ev);  // the mixed iterate
-        if (sizeof(T) == 8 && first == 2)
+      for (int h = 0; h < 2; ++h) {
+        const long long i = (2LL * (p0 + q) + h) * NY + y;
+        double ev[3];
+        if (first == 0) {
+          const C z0 = vx[0], z1 = vx[SL], z2 = vx[2 * SL];
+          ev[0] = eb0 + (double)(h == 0 ? z0.x : z0.y);
+          ev[1] = eb1 + (double)(h == 0 ? z1.x : z1.y);
+          ev[2] = eb2 + (double)(h == 0 ? z2.x : z2.y);
+          const double q0 = ev[0] - o[h][0], q1 = ev[1] - o[h][1], q2 = ev[2] - o[h][2];
+          d2 += q0 * q0 + q1 * q1 + 2.0 * q2 * q2;
+          n2 += o[h][0] * o[h][0] + o[h][1] * o[h][1] + 2.0 * o[h][2] * o[h][2];
 #pragma unroll
           for (int k = 0; k < 3; ++k) eps[k * N + i] = (T)ev[k];
-      }
-      if (img_only) continue;
-      const double tre = ev[0] + ev[1];
-      double s0, s1, s2;  // LAW 0 linear; 1 secant, 2 Rose, 3 Landau (FP64 plans)
-      law_sigma<LAW>(m[h], l[h], ev[0] - pl[h][0], ev[1] - pl[h][1], ev[2] - pl[h][2], law_a, law_b, law_ps, s0, s1,
-                     s2, R.lp);
-      tr[h][0] = (T)(s0 - (2 * mu0 * ev[0] + lam0 * tre));
-      tr[h][1] = (T)(s1 - (2 * mu0 * ev[1] + lam0 * tre));
-      tr[h][2] = (T)(s2 - 2 * mu0 * ev[2]);
-    }
-    if (img_only) continue;
+        } else {
 #pragma unroll
-    for (int k = 0; k < 3; ++k) vx[k * SL] = mk<C>(tr[0][k], tr[1][k]);
+          for (int k = 0; k < 3; ++k) ev[k] = o[h][k];
+          if constexpr (LAW != 0)
+            if (R.aa) aa_mix_voxel(R, i, nmix, gam, ev);  // the mixed iterate
+          if (sizeof(T) == 8 && first == 2)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) eps[k * N + i] = (T)ev[k];
+        }
+        if (img_only) continue;
+        const double tre = ev[0] + ev[1];
+        double s0, s1, s2;  // LAW 0 linear; 1 secant, 2 Rose, 3 Landau (FP64 plans)
+        law_sigma<LAW>(m[h], l[h], ev[0] - pl[h][0], ev[1] - pl[h][1], ev[2] - pl[h][2], law_a, law_b, law_ps, s0, s1,
+                       s2, R.lp);
+        tr[h][0] = (T)(s0 - (2 * mu0 * ev[0] + lam0 * tre));
+        tr[h][1] = (T)(s1 - (2 * mu0 * ev[1] + lam0 * tre));
+        tr[h][2] = (T)(s2 - 2 * mu0 * ev[2]);
+      }
+      if (!img_only)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) vx[k * SL] = mk<C>(tr[0][k], tr[1][k]);
+    }
+    if constexpr (!ONE)
+      if (first == 0 && (K == 1 || y >= NYP - TH)) fold(K == 1 ? e >> 5 : q * NCH + (threadIdx.x >> 5));
   }
+  if constexpr (ONE)
+    if (first == 0) fold(threadIdx.x >> 5);
   if (!img_only) {
     __syncthreads();
     reg_line<NY, -1, ALT, C>(t, act, tw, [&](int i) -> C { return buf[reg_slot<NY, C>(i)]; }, at, put, sync, sync);
@@ -256,20 +280,22 @@ __global__ void __launch_bounds__(ls2_r_threads(NY, P, 2 * (int)sizeof(T)),
     }
   }
   if (first != 0) return;
-  d2 = block_sum(d2, red);
-  n2 = block_sum(n2, red);
-  if (threadIdx.x == 0) {
-    const int item = R.row_first + loc;
-    partials[2 * item] = d2;
-    partials[2 * item + 1] = n2;
-    __threadfence();
-    const unsigned int k = atomicInc(&rep_counter[r], (unsigned int)R.row_items - 1);  // self-resetting
-    s_last = (k == (unsigned int)R.row_items - 1);
+  __syncthreads();
+  for (int q = threadIdx.x >> 5; q < np; q += TH / 32) {
+    const int lane = threadIdx.x & 31;
+    const double a = warp_sum(lane < NCH ? chunk[0][q * NCH + lane] : 0.0);
+    const double b = warp_sum(lane < NCH ? chunk[1][q * NCH + lane] : 0.0);
+    if (lane == 0) {
+      reinterpret_cast<double2*>(partials)[R.row_first + p0 + q] = make_double2(a, b);
+      __threadfence();
+    }
   }
+  if constexpr (P > 1) __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicInc(&rep_counter[r], (unsigned int)per - 1) == (unsigned int)per - 1;  // self-resetting
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  ls2d_decide(R, S, partials, ctl, cond, use_cond, guard_cap, red, final != 0);
+  ls2d_decide(R, S, partials, ctl, cond, use_cond, guard_cap, final != 0);
 }
 
 // Thread = (component, t, column), the column fastest: a warp's loads cover
