@@ -354,7 +354,8 @@ __device__ __forceinline__ void reg_bfly(C* v, int j, const C* __restrict__ tw) 
   }
 }
 
-// The transform of one line by its T threads (t in [0, T)).
+// The transform of one line by its T threads (t in [0, T); TT: other than the
+// schedule's, which changes no rounding).
 //   load(i)      the input point i (any source)
 //   at(slot)     reference to the line's exchange slot
 //   store(i, v)  the result point i; it may write at(reg_slot(i)) in place
@@ -363,11 +364,12 @@ __device__ __forceinline__ void reg_bfly(C* v, int j, const C* __restrict__ tw) 
 //   pre()        called once by every thread between its loads and the first
 //                exchange: inputs that lie in exchange buffers have been read
 //                by the threads it synchronises
-template <int N, int SIGN, int ALT, typename C, typename Load, typename At, typename Store, typename Sync, typename Pre>
+template <int N, int SIGN, int ALT, typename C, int TT = 0, typename Load, typename At, typename Store, typename Sync,
+          typename Pre>
 __device__ __forceinline__ void reg_line(int t, bool act, const C* __restrict__ tw, Load load, At at, Store store,
                                          Sync sync, Pre pre) {
   constexpr RegSched Q = reg_sched(N, sizeof(C));
-  constexpr int R0 = Q.r[0], T = Q.t, P0 = reg_p0(N, sizeof(C));
+  constexpr int R0 = Q.r[0], T = TT ? TT : Q.t, P0 = reg_p0(N, sizeof(C));
   {
     constexpr int NB = N / R0, U = (NB + T - 1) / T;
     C v[U][R0];

@@ -28,13 +28,23 @@ namespace mgk {
 
 // ------------------------------------------------------------ geometry ---
 constexpr int ls2_round32(int n) { return (n + 31) / 32 * 32; }
+// Threads per line: the schedule's, or half of them in the wide form of FP32 lines of
+// three steps of at most 8 points, whose butterflies then fill a thread's registers
+// (256^2 x 32: row 55.0 -> 51.5 us, column 34.6 -> 31.1; 512^2 x 8: 61.1 -> 59.5, 39.4 ->
+// 31.7; the kernels before the register passes: 49.8 and 38.0, 78 and 61).  One small
+// grid wants the warps (256^2 x 1: row 15.7, at half 16.6), radix 9 the registers (162^2
+// x 64: row 48.8, at half 57.3).
+constexpr int ls2_t(int n, int csz, bool wide) {
+  const RegSched q = reg_sched(n, csz);
+  return wide && csz == 8 && q.ns == 3 && q.r[0] <= 8 && q.r[1] <= 8 && q.r[2] <= 8 ? q.t / 2 : q.t;
+}
 // row pairs per CTA of the wide kernel: about 100 transform threads in FP64
 // (the same in FP32: a replica's items do not depend on the phase)
 constexpr int ls2_pairs(int n) { return reg_sched64(n).t <= 9 ? 4 : reg_sched64(n).t <= 18 ? 2 : 1; }
 // threads: those of the transforms, and enough for equal rounds of the voxel
 // stage of at most 128 (256 for the longer lines) voxel pairs
-constexpr int ls2_r_threads(int n, int p, int csz) {
-  const int fft = 3 * reg_sched(n, csz).t * p, vox = p * ls2_round32(n), cap = n <= 256 ? 128 : 256;
+constexpr int ls2_r_threads(int n, int p, int tl) {
+  const int fft = 3 * tl * p, vox = p * ls2_round32(n), cap = n <= 256 ? 128 : 256;
   const int rounds = (vox + cap - 1) / cap, per = (vox + rounds - 1) / rounds;
   return ls2_round32(fft > per ? fft : per);
 }
@@ -43,10 +53,10 @@ constexpr int ls2_r_threads(int n, int p, int csz) {
 // 32 points have the wide form only: their narrow CTA is a single warp, whose
 // one-round loops the compiler contracts differently.
 constexpr int ls2_cols(int n, int csz, bool wide) {
-  const int t = reg_sched(n, csz).t, one = 16 / csz;
+  const int t = ls2_t(n, csz, wide), one = 16 / csz;
   return wide || n <= 32 ? (t * one <= 36 ? 4 * one : t * one <= 72 ? 2 * one : csz == 16 ? 2 : one) : one;
 }
-constexpr int ls2_c_threads(int n, int w, int csz) { return ls2_round32(3 * w * reg_sched(n, csz).t); }
+constexpr int ls2_c_threads(int w, int tl) { return ls2_round32(3 * w * tl); }
 // row pitch of the half spectra
 constexpr int ls2_ld(int n) { return (n / 2 + 1 + 3) / 4 * 4; }
 // exchange buffers; they first hold the pairs' spectrum rows as copied
@@ -93,21 +103,21 @@ __device__ __forceinline__ void l2_prefetch2(const void* p, uint32_t bytes) {
 // the field as is (first tau of a phase, or of a mixed iterate); 2 does so
 // from the FP32 field of a mixed plan, which becomes the FP64 one.  final: see
 // ls2d_decide.  lead: this launch counts the loop bodies.
-template <typename T, int NY, int P, int LAW, int ALT>
-__global__ void __launch_bounds__(ls2_r_threads(NY, P, 2 * (int)sizeof(T)),
-                                  ls2_minb(ls2_r_threads(NY, P, 2 * (int)sizeof(T)), 2 * (int)sizeof(T)))
+template <typename T, int NY, int P, int TL, int LAW, int ALT>
+__global__ void __launch_bounds__(ls2_r_threads(NY, P, TL), ls2_minb(ls2_r_threads(NY, P, TL), 2 * (int)sizeof(T)))
     ls2_row_reg(const Ls2dRep* __restrict__ reps, Ls2dState* st, const int* __restrict__ sel, double* partials,
                 unsigned int* rep_counter, Ls2dCtl* ctl, cudaGraphConditionalHandle cond, int use_cond, int guard_cap,
                 int lead, int first, int final) {
   using C = C_t<T>;
-  constexpr int TL = reg_sched(NY, sizeof(C)).t, TH = ls2_r_threads(NY, P, sizeof(C)), SL = reg_slots(NY, sizeof(C));
+  constexpr int TH = ls2_r_threads(NY, P, TL), SL = reg_slots(NY, sizeof(C));
   constexpr int NYH = NY / 2 + 1;
   // A pair's sums behind the update norm do not depend on P: its voxel pairs, padded
   // to whole warps, are folded warp by warp (K = 1), or after the K rounds in which the
   // CTA of either form takes them up alike; where there is one form, after the loop.
-  constexpr bool ONE = ls2_pairs(NY) == 1;
-  constexpr int NYP = ls2_round32(NY), T1 = ls2_r_threads(NY, 1, sizeof(C));
-  constexpr int K = T1 == ls2_r_threads(NY, ls2_pairs(NY), sizeof(C)) && NYP % T1 == 0 ? NYP / T1 : 1;
+  constexpr bool ONE = ls2_pairs(NY) == 1 && ls2_t(NY, sizeof(C), false) == ls2_t(NY, sizeof(C), true);
+  constexpr int NYP = ls2_round32(NY), T1 = ls2_r_threads(NY, 1, ls2_t(NY, sizeof(C), false));
+  constexpr int T2 = ls2_r_threads(NY, ls2_pairs(NY), ls2_t(NY, sizeof(C), true));
+  constexpr int K = T1 == T2 && NYP % T1 == 0 ? NYP / T1 : 1;
   constexpr int NCH = ONE || K > 1 ? TH / 32 : NYP / 32;  // parts of a pair's sum
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double chunk[2][P * NCH];
@@ -180,7 +190,7 @@ __global__ void __launch_bounds__(ls2_r_threads(NY, P, 2 * (int)sizeof(T)),
       if (k == 0 || 2 * k == NY) { a.y = 0; b.y = 0; }
       return 2 * k <= NY ? mk<C>(a.x - b.y, a.y + b.x) : mk<C>(a.x + b.y, b.x - a.y);
     };
-    reg_line<NY, +1, ALT, C>(t, act, tw, load, at, put, sync, [] { __syncthreads(); });
+    reg_line<NY, +1, ALT, C, TL>(t, act, tw, load, at, put, sync, [] { __syncthreads(); });
   }
   __syncthreads();
   const double mu0 = S.mu0, lam0 = S.lam0;
@@ -267,7 +277,7 @@ __global__ void __launch_bounds__(ls2_r_threads(NY, P, 2 * (int)sizeof(T)),
     if (first == 0) fold(threadIdx.x >> 5);
   if (!img_only) {
     __syncthreads();
-    reg_line<NY, -1, ALT, C>(t, act, tw, [&](int i) -> C { return buf[reg_slot<NY, C>(i)]; }, at, put, sync, sync);
+    reg_line<NY, -1, ALT, C, TL>(t, act, tw, [&](int i) -> C { return buf[reg_slot<NY, C>(i)]; }, at, put, sync, sync);
     sync();
     if (act) {
       C* ra = spec + ((long long)c * nx + 2 * (p0 + pr)) * ld;
@@ -300,12 +310,11 @@ __global__ void __launch_bounds__(ls2_r_threads(NY, P, 2 * (int)sizeof(T)),
 
 // Thread = (component, t, column), the column fastest: a warp's loads cover
 // whole rows of the tile, and the exchange is stored column-fastest too.
-template <typename T, int NX, int W, int ALT>
-__global__ void __launch_bounds__(ls2_c_threads(NX, W, 2 * (int)sizeof(T)),
-                                  ls2_minb(ls2_c_threads(NX, W, 2 * (int)sizeof(T)), 2 * (int)sizeof(T)))
+template <typename T, int NX, int W, int TL, int ALT>
+__global__ void __launch_bounds__(ls2_c_threads(W, TL), ls2_minb(ls2_c_threads(W, TL), 2 * (int)sizeof(T)))
     ls2_col_reg(const Ls2dRep* __restrict__ reps, const Ls2dState* __restrict__ st, const int* __restrict__ sel) {
   using C = C_t<T>;
-  constexpr int TL = reg_sched(NX, sizeof(C)).t, SL = reg_slots(NX, sizeof(C)), TH = ls2_c_threads(NX, W, sizeof(C));
+  constexpr int SL = reg_slots(NX, sizeof(C)), TH = ls2_c_threads(W, TL);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int nyh = reps[sel[0]].nyh, per = (nyh + W - 1) / W;
   const int r = sel[blockIdx.x / per], k0 = blockIdx.x % per * W;
@@ -325,7 +334,7 @@ __global__ void __launch_bounds__(ls2_c_threads(NX, W, 2 * (int)sizeof(T)),
     if constexpr (32 % (TL * W) == 0) __syncwarp();
     else __syncthreads();
   };
-  reg_line<NX, -1, ALT, C>(t, act, tw, [&](int i) -> C { return g[i * ld]; }, at, put, sync, [] {});
+  reg_line<NX, -1, ALT, C, TL>(t, act, tw, [&](int i) -> C { return g[i * ld]; }, at, put, sync, [] {});
   __syncthreads();
   // Gamma0 in the precision of the pass.
   const T scale = (T)(1.0 / ((double)NX * (double)ny));
@@ -390,7 +399,7 @@ __global__ void __launch_bounds__(ls2_c_threads(NX, W, 2 * (int)sizeof(T)),
     p[2 * SL * W] = exy;
   }
   __syncthreads();
-  reg_line<NX, +1, ALT, C>(t, act, tw, [&](int i) -> C { return buf[reg_slot<NX, C>(i) * W]; }, at,
+  reg_line<NX, +1, ALT, C, TL>(t, act, tw, [&](int i) -> C { return buf[reg_slot<NX, C>(i) * W]; }, at,
                       [&](int i, C v) { g[i * ld] = v; }, sync, sync);
 }
 
@@ -412,26 +421,27 @@ template <typename T, int N, int ALT> static const Ls2Line* ls2_make() {
   constexpr int cs = 2 * (int)sizeof(T);
   static const Ls2Line L = [] {
     constexpr int P = ls2_pairs(N), W0 = ls2_cols(N, cs, false), W1 = ls2_cols(N, cs, true);
+    constexpr int T0 = ls2_t(N, cs, false), T1 = ls2_t(N, cs, true);
     Ls2Line k{};
-    k.row[0][0] = (const void*)ls2_row_reg<T, N, 1, 0, ALT>;
-    k.row[0][1] = (const void*)ls2_row_reg<T, N, P, 0, ALT>;
+    k.row[0][0] = (const void*)ls2_row_reg<T, N, 1, T0, 0, ALT>;
+    k.row[0][1] = (const void*)ls2_row_reg<T, N, P, T1, 0, ALT>;
     if constexpr (sizeof(T) == 8) {
-      k.row[1][0] = (const void*)ls2_row_reg<T, N, 1, 1, 0>;
-      k.row[1][1] = (const void*)ls2_row_reg<T, N, P, 1, 0>;
-      k.row[2][0] = (const void*)ls2_row_reg<T, N, 1, 2, 0>;
-      k.row[2][1] = (const void*)ls2_row_reg<T, N, P, 2, 0>;
-      k.row[3][0] = (const void*)ls2_row_reg<T, N, 1, 3, 0>;
-      k.row[3][1] = (const void*)ls2_row_reg<T, N, P, 3, 0>;
+      k.row[1][0] = (const void*)ls2_row_reg<T, N, 1, T0, 1, 0>;
+      k.row[1][1] = (const void*)ls2_row_reg<T, N, P, T1, 1, 0>;
+      k.row[2][0] = (const void*)ls2_row_reg<T, N, 1, T0, 2, 0>;
+      k.row[2][1] = (const void*)ls2_row_reg<T, N, P, T1, 2, 0>;
+      k.row[3][0] = (const void*)ls2_row_reg<T, N, 1, T0, 3, 0>;
+      k.row[3][1] = (const void*)ls2_row_reg<T, N, P, T1, 3, 0>;
     }
-    k.col[0] = (const void*)ls2_col_reg<T, N, W0, ALT>;
-    k.col[1] = (const void*)ls2_col_reg<T, N, W1, ALT>;
-    const int p[2] = {1, P}, w[2] = {W0, W1};
+    k.col[0] = (const void*)ls2_col_reg<T, N, W0, T0, ALT>;
+    k.col[1] = (const void*)ls2_col_reg<T, N, W1, T1, ALT>;
+    const int p[2] = {1, P}, w[2] = {W0, W1}, t[2] = {T0, T1};
     for (int i = 0; i < 2; ++i) {
       k.pairs[i] = p[i];
-      k.r_threads[i] = ls2_r_threads(N, p[i], cs);
+      k.r_threads[i] = ls2_r_threads(N, p[i], t[i]);
       k.r_bytes[i] = ls2_r_bytes(N, p[i], cs);
       k.cols[i] = w[i];
-      k.c_threads[i] = ls2_c_threads(N, w[i], cs);
+      k.c_threads[i] = ls2_c_threads(w[i], t[i]);
       k.c_bytes[i] = ls2_c_bytes(N, w[i], cs);
     }
     return k;
