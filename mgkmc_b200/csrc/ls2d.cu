@@ -85,7 +85,7 @@ constexpr int kThreads = 256;
 
 // Sums over a replica's CTAs of K <= 8 values per thread, in a fixed order:
 // warp trees, the warps, then (in the CTA that arrives last) one warp per
-// value over the CTAs' partials.  part: the replica's gridDim.x slots of 8;
+// value over the CTAs' partials.  part: the replica's gridDim.x slots of K;
 // ctr: its arrival counter (left at zero).  True in the last CTA only, with
 // the sums in res.  A launch for the last step alone took 4 .. 7 us.
 template <int K>
@@ -103,7 +103,7 @@ __device__ __forceinline__ bool grid_sums(const double* v, double* part, unsigne
     double t = 0;
 #pragma unroll
     for (int k = 0; k < kThreads / 32; ++k) t += w[k][threadIdx.x];
-    part[blockIdx.x * 8 + threadIdx.x] = t;
+    part[blockIdx.x * K + threadIdx.x] = t;
     __threadfence();
   }
   __syncthreads();
@@ -113,7 +113,7 @@ __device__ __forceinline__ bool grid_sums(const double* v, double* part, unsigne
   __threadfence();
   if (wid < K) {
     double a = 0;
-    for (int i = lane; i < (int)gridDim.x; i += 32) a += __ldcg(&part[i * 8 + wid]);
+    for (int i = lane; i < (int)gridDim.x; i += 32) a += __ldcg(&part[i * K + wid]);
     a = warp_sum(a);
     if (lane == 0) res[wid] = a;
   }
@@ -1060,7 +1060,8 @@ struct mgk_ls2d_plan {
   int* d_maps = nullptr;
   unsigned int* d_repctr = nullptr;
   double* d_part = nullptr;
-  double* d_mat_part = nullptr;   // partials of the material kernel
+  double* d_mat_part = nullptr;   // partials of the material kernel, each replica's from mat_off
+  std::vector<size_t> mat_off;
   size_t part_doubles = 0;
   int total_row_items = 0, total_col_items = 0;
   unsigned int* d_voxctr = nullptr;  // arrival counters of the per-voxel kernels, per replica
@@ -1250,7 +1251,13 @@ extern "C" int mgk_ls2d_create_batch(int nrep, const int* nxs, const int* nys, i
   void* v = nullptr;
   if ((st = plan_alloc(p, &v, sizeof(double) * p->part_doubles))) return fail(st);
   p->d_part = reinterpret_cast<double*>(v);
-  if ((st = plan_alloc(p, &v, sizeof(double) * 8 * kPerVoxelBlocks * nrep))) return fail(st);
+  // two sums per CTA: replicas may be set on different streams, so each has its own
+  size_t mat = 0;
+  for (int r = 0; r < nrep; ++r) {
+    p->mat_off.push_back(mat);
+    mat += 2 * (size_t)grid_blocks(p->reps[r].N);
+  }
+  if ((st = plan_alloc(p, &v, sizeof(double) * mat))) return fail(st);
   p->d_mat_part = reinterpret_cast<double*>(v);
   if ((st = plan_alloc(p, &v, sizeof(Ls2dRep) * nrep))) return fail(st);
   p->d_reps = reinterpret_cast<Ls2dRep*>(v);
@@ -1315,7 +1322,7 @@ static int ls2d_set_fields(mgk_ls2d_t p, int rep, const double* E, const double*
   const int grid = grid_blocks(R.N);
   ls2d_material_kernel<<<grid, kThreads, 0, s>>>(p->d_reps, p->d_st, rep, E, nu, epsp, p->plane_mode, set_moduli,
                                                  set_moduli == 2 ? (p->law == 2 ? 2 : 1) : 0, p->law_b,
-                                                 p->d_mat_part + (size_t)rep * 8 * kPerVoxelBlocks, p->d_voxctr + rep);
+                                                 p->d_mat_part + p->mat_off[rep], p->d_voxctr + rep);
   MGK_CUDA(cudaGetLastError());
   return MGK_OK;
 }
