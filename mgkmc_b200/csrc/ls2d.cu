@@ -1431,7 +1431,10 @@ extern "C" int mgk_ls2d_set_anderson(mgk_ls2d_t p, int m) {
       int dev = 0, sms = 148;
       if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
       p->aa_nb = std::max(1, std::min(8 * sms, ceil_div(3 * p->maxN, kAaThreads)));
+      // zeroed (the legacy stream waited for): the timing hooks run first passes before
+      // any solve has set the mix
       if (cudaMalloc((void**)&p->d_aa, sizeof(Ls2dAA)) != cudaSuccess ||
+          cudaMemset(p->d_aa, 0, sizeof(Ls2dAA)) != cudaSuccess || cudaStreamSynchronize(0) != cudaSuccess ||
           cudaMalloc((void**)&p->aa_part, sizeof(double) * 2 * kAaMax * p->aa_nb) != cudaSuccess) {
         cudaGetLastError();
         set_error("mgk_ls2d_set_anderson: cudaMalloc failed");
