@@ -626,6 +626,8 @@ static int a3(mgk_ls3d_t p, void** ptr, size_t bytes) {
   return MGK_OK;
 }
 
+static int wait3(mgk_ls3d_t p);
+
 static void drop_graphs3(mgk_ls3d_t p) {
   for (auto& e : p->gcache) {
     cudaGraphExecDestroy(e.x);
@@ -657,7 +659,12 @@ extern "C" int mgk_ls3d_set_precision(mgk_ls3d_t p, int precision) {
       }
       p->has_material[r] = 0;  // the FP32 copies come with the next set_material
     }
-    MGK_CUDA(cudaMemcpy(p->d_reps, p->reps.data(), sizeof(Ls3dRep) * p->nrep, cudaMemcpyHostToDevice));
+    // the staged records too: a solve uploads all of them, those of replicas that it
+    // leaves out as they were staged last
+    int st = wait3(p);
+    if (st) return st;
+    memcpy(p->h_reps, p->reps.data(), sizeof(Ls3dRep) * p->nrep);
+    MGK_CUDA(cudaMemcpy(p->d_reps, p->h_reps, sizeof(Ls3dRep) * p->nrep, cudaMemcpyHostToDevice));
   }
   p->prec = precision;
   return MGK_OK;
