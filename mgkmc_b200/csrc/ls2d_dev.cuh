@@ -352,6 +352,10 @@ static __device__ void ls2d_decide(const Ls2dRep& R, Ls2dState& S, const double*
   a = warp_sum(a);
   b = warp_sum(b);
   if (threadIdx.x != 0) return;
+  // the control block's words at once, ahead of the chain of atomics below (n_active is
+  // stable until every active replica has decided)
+  const unsigned int n_act = *(volatile unsigned int*)&ctl->n_active, bodies = *(volatile unsigned int*)&ctl->bodies;
+  const int error = *(volatile int*)&ctl->error;
   if (S.iter == 0) { a += S.extra_d0; b += S.extra_n0; }
   else { b += 2.0 * (double)R.N * S.abar * S.abar; }
   const double diff = sqrt(a) / (sqrt(b) + 1e-20);
@@ -370,7 +374,6 @@ static __device__ void ls2d_decide(const Ls2dRep& R, Ls2dState& S, const double*
     else if (diff < tol1 || S.phase_iter >= kMixedPhase1Cap) S.done = 1;
     else keep = 1;
   }
-  const unsigned int n_act = ctl->n_active;  // stable until every active replica has decided
   if (keep) atomicAdd(&ctl->still, 1u);
   __threadfence();
   const unsigned int d = atomicAdd(&ctl->decided, 1u);
@@ -379,7 +382,7 @@ static __device__ void ls2d_decide(const Ls2dRep& R, Ls2dState& S, const double*
     const unsigned int still = atomicExch(&ctl->still, 0u);
     ctl->decided = 0;
     ctl->n_active = still;
-    const bool go = still > 0 && atomicAdd(&ctl->bodies, 0u) <= (unsigned int)guard_cap && *(volatile int*)&ctl->error == 0;
+    const bool go = still > 0 && bodies <= (unsigned int)guard_cap && error == 0;
     ctl->any = go ? 1 : 0;
     if (use_cond) cudaGraphSetConditional(cond, go ? 1u : 0u);
   }

@@ -213,6 +213,9 @@ __device__ void ls3d_decide(const Ls3dRep& R, Ls3dState& S, int r, int item, dou
   a = block_sum(a, red);
   b = block_sum(b, red);
   if (threadIdx.x != 0) return;
+  // the control block's words at once, ahead of the chain of atomics below
+  const unsigned int n_act = *(volatile unsigned int*)&ctl->n_active, bodies = *(volatile unsigned int*)&ctl->bodies;
+  const int error = *(volatile int*)&ctl->error;
   if (S.iter == 0) { a += S.extra_d0; b += S.extra_n0; }
   else b += 2.0 * (double)N * (S.abar[0] * S.abar[0] + S.abar[1] * S.abar[1] + S.abar[2] * S.abar[2]);
   const double diff = sqrt(a) / (sqrt(b) + 1e-20);
@@ -231,7 +234,6 @@ __device__ void ls3d_decide(const Ls3dRep& R, Ls3dState& S, int r, int item, dou
     else if (diff < tol1 || S.phase_iter >= kL3Phase1Cap) S.done = 1;
     else keep = 1;
   }
-  const unsigned int n_act = ctl->n_active;
   if (keep) atomicAdd(&ctl->still, 1u);
   __threadfence();
   const unsigned int dcount = atomicAdd(&ctl->decided, 1u);
@@ -240,7 +242,7 @@ __device__ void ls3d_decide(const Ls3dRep& R, Ls3dState& S, int r, int item, dou
     const unsigned int still = atomicExch(&ctl->still, 0u);
     ctl->decided = 0;
     ctl->n_active = still;
-    const bool go = still > 0 && atomicAdd(&ctl->bodies, 0u) <= (unsigned int)guard_cap && *(volatile int*)&ctl->error == 0;
+    const bool go = still > 0 && bodies <= (unsigned int)guard_cap && error == 0;
     ctl->any = go ? 1 : 0;
     if (use_cond) cudaGraphSetConditional(cond, go ? 1u : 0u);
   }
