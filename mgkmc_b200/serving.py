@@ -507,11 +507,18 @@ class Server:
                 if t.need[0] == "solve":
                     solving.append(t)
         b.tasks = alive
+        # The ragged bucket's selections differ from round to round (in an ensemble of 96,
+        # 2,800 of 12,000 occur once) and it has no other bucket to overlap with: it waits
+        # for its solves, which runs new selections from the host instead of building a
+        # graph for each (that ensemble, 100 events: 173 -> 199 events/s).
+        alone = self.ragged is not None
         for tol, group in _by_tol(solving):  # one launch per tolerance in use
-            b.plan.solve([t.slot for t in group], [t.need[1] for t in group], [t.need[2] for t in group],
-                         [t.need[3] for t in group], eps_init=[t.need[4] for t in group],
-                         max_iter=self.ls_max_iter, tol=tol, sync=False, stream=b.stream)
-        b.solving = solving
+            infos = b.plan.solve([t.slot for t in group], [t.need[1] for t in group], [t.need[2] for t in group],
+                                 [t.need[3] for t in group], eps_init=[t.need[4] for t in group],
+                                 max_iter=self.ls_max_iter, tol=tol, sync=alone, stream=b.stream)
+            for t, info in zip(group, infos or ()):
+                t.send = info
+        b.solving = [] if alone else solving
         b.inflight = list(alive)  # tasks admitted during the round join the next one
         b.event.record(b.stream)
 
