@@ -786,11 +786,11 @@ def run_ours(a):
     achieved = row_bytes / (row64 * 1e-3) / 1e9
     # DRAM read+write bytes of one launch of this kernel on this workload (32 x
     # 256^2, FP64), from the ncu capture summarised in
-    # profiles/ls2d_warp_kernels_256x32_fp64.md; scaled by voxels for other
+    # profiles/ls2d_register_passes_256x32.md; scaled by voxels for other
     # batch sizes or grids (the traffic per voxel does not depend on them)
-    traffic = 242.4e6 * (N * B) / (32 * 256 * 256)
+    traffic = 242.5e6 * (N * B) / (32 * 256 * 256)
     roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-            "traffic": traffic, "traffic_source": "ncu capture, profiles/ls2d_warp_kernels_256x32_fp64.md",
+            "traffic": traffic, "traffic_source": "ncu capture, profiles/ls2d_register_passes_256x32.md",
             "kernel": "ls2_row_reg<double,256> (C2R + update + tau + R2C along y) over the batch",
             "peak_kind": peak_kind, "bytes_per_launch": row_bytes,
             "kernels_us": {"row_fp64": row64 * 1e3, "col_fp64": col64 * 1e3, "row_fp32": row32 * 1e3,

@@ -31,8 +31,8 @@ constexpr int fs_z_bytes(int n) {
   return (a > b ? a : b) * 16;
 }
 constexpr int fs_ax_bytes(int n, int nc) { return nc * fs_tile(n) * reg_slots(n, 16) * 16; }
-// resident CTAs asked of the register allocator: 128 registers per thread, in the
-// x passes 112 (a third CTA of 192 threads at 128 points, 118 registers without
+// resident CTAs asked of the register allocator: as many as 128 registers per thread
+// allow, rounded down (the compiler takes what is left over), in the x passes 112 (a third CTA of 192 threads at 128 points, 118 registers without
 // being asked: 80 and 98 us -> 73 and 80 us; in the y passes the spills cost more:
 // 57 and 63 us -> 96 and 82 us)
 constexpr int fs_minb(int threads, int regs = 128) {

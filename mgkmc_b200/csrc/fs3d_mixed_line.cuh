@@ -32,7 +32,9 @@ constexpr int ml_ld(int n) { return (n / 2 + 1 + 3) / 4 * 4; }  // row pitch of 
 // step, 96^3 45 instead of 39
 constexpr int ml_zf_threads(int n) { return up32(9 * ml_t(n)); }
 // z inverse: the threads (and with them the order of the sums) of the passes
-// that it replaces
+// that it replaces.  The nine lines have to fit: 256 points, 32 threads a line, have
+// no instantiation, and an axis of that length takes the CTA-wide passes (the FP64
+// form has one)
 constexpr int ml_zi_threads(int alt) { return alt ? 256 : 96; }
 // columns per tile: 64-byte rows in y, 32-byte rows in x, less on lines of many
 // threads

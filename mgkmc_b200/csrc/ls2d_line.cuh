@@ -14,9 +14,10 @@
 // kernel comes in two widths: P pairs or W columns per CTA for a selection
 // that fills the GPU twice over, one pair or column (the sector waste is served
 // by L2) below that, which spreads a 64^2 grid over 32 CTAs instead of 8.
-// FP64, 256^2 x 32 per launch, before and now: row 83.7 and 62.6 us (285 MB:
-// 0.70 of the measured copy rate), column 50.2 and 37.7 us; 1024^2 x 1: 71.5 and
-// 45 us, 49.3 and 39.3 us.  FP32, 1024^2 x 1: 58.9 and 36.3 us, 44.8 and 21.3 us.
+// CUDA events around each launch, the warp-line kernels before and these: FP64,
+// 256^2 x 32: row 94.6 and 70.2 us (285 MB: 0.62 of the measured copy rate), column
+// 60.5 and 44 us (0.35); 1024^2 x 1: 67 and 45 us, 43 and 40 us.  FP32, 256^2 x 32: row
+// 49.9 and 51 us, column 38 and 30.6 us; 1024^2 x 1: 50.7 and 36 us, 33 and 24 us.
 // 432x324, 162x243 and 288x216 together, whose sides had no warp-line kernel: an
 // iteration took 101 us in the CTA-wide passes and takes 45 us.
 #pragma once
@@ -65,8 +66,10 @@ constexpr int ls2_r_bytes(int n, int p, int csz) {
   return (a > b ? a : b) * csz;
 }
 constexpr int ls2_c_bytes(int n, int w, int csz) { return 3 * w * reg_slots(n, csz) * csz; }
-// resident CTAs asked of the register allocator: 128 registers per thread in
-// FP64, 80 in FP32
+// Resident CTAs asked of the register allocator: as many as 128 registers per thread
+// allow in FP64, 80 in FP32, rounded down.  Where that leaves registers over, the
+// compiler takes them: blocks of 192 threads get two CTAs and up to 168 registers
+// (the FP64 column pass: 158 at 256 points, 160 at 1024, 12 warps per SM).
 constexpr int ls2_minb(int threads, int csz) {
   const int b = 65536 / (threads * (csz == 16 ? 128 : 80));
   return b < 1 ? 1 : b > 16 ? 16 : b;

@@ -54,8 +54,9 @@ constexpr int ls3_z_bytes(int n, int csz) {
   return (a > b ? a : b) * csz;
 }
 constexpr int ls3_ax_bytes(int n, int csz, int nc) { return nc * ls3_tile(n, csz) * reg_slots(n, csz) * csz; }
-// resident CTAs asked of the register allocator: 128 registers per thread in
-// FP64, 80 in FP32
+// resident CTAs asked of the register allocator: as many as 128 registers per thread
+// allow in FP64, 80 in FP32, rounded down (blocks of 192 threads, as the x pass at 128
+// points, get two and up to 168 registers: 162)
 constexpr int ls3_minb(int threads, int csz) {
   const int b = 65536 / (threads * (csz == 16 ? 128 : 80));
   return b < 1 ? 1 : b;
