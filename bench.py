@@ -814,7 +814,7 @@ def run_ours(a):
                                 f"one batched solve launch per size per round, the sizes on their own streams")
         if a.ensemble_ragged:
             _, rag = run_ensemble(reqs, ragged=True)
-            rag["workload"] = "the same replicas in one ragged plan: one launch per solver stage for all replicas"
+            rag["workload"] = "the same replicas in one ragged plan: one launch per side and solver stage"
             ensemble["ragged"] = rag
     serving = None
     if world == 1 and a.serve_window > 0:

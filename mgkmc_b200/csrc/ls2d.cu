@@ -8,7 +8,7 @@
 //
 // A plan holds `nrep` independent replicas (grids of any supported size, so a
 // batch may be ragged).  A solve call selects a subset of them; every stage
-// is one launch over all selected replicas.
+// is one launch per shape among the selected replicas.
 //
 // HBM layout per replica (SoA planes of N = nx*ny, C order):
 //   mu, lam                 Lame fields (plane strain or plane stress lambda)
@@ -31,7 +31,8 @@
 // CTA of each replica to finish a row kernel reduces that replica's partial
 // sums in a fixed order (deterministic), decides its convergence on the
 // device, and the last replica to decide sets the condition of the CUDA
-// graph while-node that holds the loop, so a solve needs no host round trip.
+// graph while-node that holds the loop, so a solve needs no host round trip (new
+// selections of several shapes are driven from the host first, see ls2d_host_first).
 //
 // Precision forms: FP64 (the reference's arithmetic), and mixed: FP32
 // storage, FFTs and Gamma0 until the update norm falls below max(tol, 2e-6)

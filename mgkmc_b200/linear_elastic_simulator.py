@@ -112,7 +112,7 @@ class Ls2dBatch:
 
     def solve(self, reps, eps_bars, eps_out, sig_out, eps_init=None, max_iter=200, tol=1e-6, sync=True,
               stream=None):
-        """Solve replicas ``reps`` (one launch per stage for all of them).
+        """Solve replicas ``reps`` (one launch per stage and shape).
         eps_bars: sequence of (2,2); eps_out/sig_out/eps_init: sequences of
         tensors (or None entries).  Returns the list of LsInfo when sync."""
         n = len(reps)

@@ -139,7 +139,7 @@ class _Task:
 class _Bucket:
     """A batched 2D LS plan with a stream: ``slots`` replicas of side n, or
     one replica per entry of ``sizes`` (a ragged bucket: replicas of several
-    sides advance in one launch per solver stage)."""
+    sides advance together, one launch per side and solver stage)."""
 
     def __init__(self, torch, n, slots, precision, sizes=None, priority=0):
         from .linear_elastic_simulator import Ls2dBatch
@@ -756,7 +756,7 @@ def run_ensemble(requests, slots=None, ragged=False, **server_kw):
     once when slots allow) and returns (results, summary with events/s).
     ragged=False: one bucket per side, one batched solve launch per side per
     round, the sides' buckets on their own streams; True: one ragged bucket
-    with a slot per replica, one launch per solver stage for all replicas of
+    with a slot per replica, one launch per side and solver stage for the replicas of
     a round."""
     from collections import Counter
     cnt = Counter(r.n for r in requests)
